@@ -87,9 +87,8 @@ constexpr int kAdjThreads = 128;
 
 // G(d) of grad_a W = G(d) (x_a - x_b) and dG/dd.
 // Gaussian: G = -2 k exp(-q^2)/h^2; Wendland C2: G = -5 k (1 - q/2)^3 / h^2.
-// (1/h is loop-invariant: the compiler hoists it out of the pair loops.)
 __device__ __forceinline__ void kernel_g(const Params& P, double d, double& G, double& dG) {
-    const double ih = 1.0 / P.h, q = d * ih, kf = P.kfactor, ih2 = ih * ih;
+    const double ih = P.inv_h, q = d * ih, kf = P.kfactor, ih2 = ih * ih;
     if (P.kernel_model == SPH_KERNEL_GAUSSIAN) {
         const double ex = exp(-(q * q));
         G = -2.0 * kf * ex * ih2;
@@ -104,7 +103,7 @@ __device__ __forceinline__ void kernel_g(const Params& P, double d, double& G, d
 // kernel_g and the kernel value W(d) of compute_kernel (whose d-derivative is
 // G(d) d) from one exponential.
 __device__ __forceinline__ void kernel_gw(const Params& P, double d, double& G, double& dG, double& W) {
-    const double ih = 1.0 / P.h, q = d * ih, kf = P.kfactor, ih2 = ih * ih;
+    const double ih = P.inv_h, q = d * ih, kf = P.kfactor, ih2 = ih * ih;
     if (P.kernel_model == SPH_KERNEL_GAUSSIAN) {
         const double ex = exp(-(q * q));
         G = -2.0 * kf * ex * ih2;
@@ -144,26 +143,26 @@ template <typename R, bool MS = false, bool MUSCL = false>
 __device__ __forceinline__ PSide load_side(const Sorted<R>& D, int s) {
     PSide o;
     o.x = D.pos[s];
-    const double4 k = D.kin[s];
+    const double4 k = load4(&D.kin[s]);
     o.u = k.x; o.v = k.y; o.rho = k.z; o.p = k.w;
-    const typename VT<R>::V4 ax = D.aux[s];
+    const typename VT<R>::V4 ax = load4(&D.aux[s]);
     o.m = D.mass[s];
-    o.ir = 1.0 / o.rho;
+    o.ir = rcp64(o.rho);
     o.V = o.m * o.ir;
     o.c = (double)ax.z;
     o.sm = (double)ax.w;
-    const typename VT<R>::V4 n1 = D.nb1[s];
+    const typename VT<R>::V4 n1 = load4(&D.nb1[s]);
     const double gs = grad_scale<R>();
     o.t0 = (double)n1.x; o.t1 = (double)n1.y; o.t2 = (double)n1.z; o.g0 = gs * n1.w;
     o.g1 = gs * D.nb2[s].x;
-    o.bi = D.binv64[s];
+    o.bi = load4(&D.binv64[s]);
     o.water = D.type[s] == SPH_TYPE_WATER;
     o.near = (D.flags[s] & 2) != 0;
     o.ax = o.ay = 0.0;
     o.gp0 = o.gp1 = o.gu0 = o.gu1 = o.gv0 = o.gv1 = 0.0;
     if (MUSCL) {
         // nb2 = (grad rho y, grad p x, grad p y, grad u x), nb3 = (grad u y, grad v x, grad v y, .)
-        const typename VT<R>::V4 n2 = D.nb2[s], n3 = D.nb3[s];
+        const typename VT<R>::V4 n2 = load4(&D.nb2[s]), n3 = load4(&D.nb3[s]);
         o.gp0 = gs * n2.y; o.gp1 = gs * n2.z; o.gu0 = gs * n2.w; o.gu1 = gs * n3.x;
         o.gv0 = gs * n3.y; o.gv1 = gs * n3.z;
     }
@@ -189,7 +188,20 @@ struct PBar {
     double gpa0, gpa1, gua0, gua1, gva0, gva1, gpb0, gpb1, gub0, gub1, gvb0, gvb1;
 };
 
-// Reverse of muscl_limiter on the branch the forward took: lim is one of 0,
+// The MUSCL limiter (function_module.f90:34-80) with the reference's arguments and
+// both increments, its two sign branches folded into one (with s = sign(dj) the
+// dj <= 0 branch is the dj > 0 branch on (-di, -dj), negated).
+__device__ __forceinline__ void muscl_limiter_ij(double di, double dj, double dij, double& li, double& lj) {
+    const double s = dj > 0.0 ? 1.0 : -1.0;
+    const double sdi = s * di, sdj = s * dj;
+    const double m = max(0.0, max(min(1.3 * sdi, sdj), min(sdi, 1.3 * sdj)));
+    const double half = 0.5 * dij, lim = s * m;
+    const bool big = m > s * half && m > 0.0, first = sdi > sdj;
+    li = big ? (first ? half : 0.0) : lim;
+    lj = big ? (first ? 0.0 : half) : lim;
+}
+
+// Reverse of muscl_limiter_ij on the branch the forward took: lim is one of 0,
 // 1.3 di, dj, di, 1.3 dj (the min / max chain), or the large-jump branch gives
 // dij/2 to one side.  From the adjoints (lib, ljb) of (li, lj), the adjoints of
 // (di, dj, dij).
@@ -244,7 +256,7 @@ template <bool MS = false, bool MUSCL = false, bool HLLC = false>
 __device__ __forceinline__ void rev_pair(const Params& P, const PSide& A, const PSide& B, double lr, double l0,
                                          double l1, PBar& o, bool a_lower = true) {
     const double r0 = A.x.x - B.x.x, r1 = A.x.y - B.x.y;
-    const double d2 = r0 * r0 + r1 * r1, d = sqrt(d2), id = 1.0 / d, id2 = id * id;
+    const double d2 = r0 * r0 + r1 * r1, id = rsqrt64(d2), d = d2 * id, id2 = id * id;
     double G, dG;
     kernel_g(P, d, G, dG);
     const double n0 = A.bi.x * r0 + A.bi.y * r1, n1 = A.bi.z * r0 + A.bi.w * r1;
@@ -268,16 +280,16 @@ __device__ __forceinline__ void rev_pair(const Params& P, const PSide& A, const 
         dpi = 0.5 * (gIp0 * xj0 + gIp1 * xj1); dpj = -0.5 * (gJp0 * xj0 + gJp1 * xj1);
         dui = 0.5 * (gIu0 * xj0 + gIu1 * xj1); duj = -0.5 * (gJu0 * xj0 + gJu1 * xj1);
         dvi = 0.5 * (gIv0 * xj0 + gIv1 * xj1); dvj = -0.5 * (gJv0 * xj0 + gJv1 * xj1);
-        muscl_limiter<double>(dpi, dpj, -sI * dp, lpi, lpj);
-        muscl_limiter<double>(dui, duj, -sI * du0, lui, luj);
-        muscl_limiter<double>(dvi, dvj, -sI * du1, lvi, lvj);
+        muscl_limiter_ij(dpi, dpj, -sI * dp, lpi, lpj);
+        muscl_limiter_ij(dui, duj, -sI * du0, lui, luj);
+        muscl_limiter_ij(dvi, dvj, -sI * du1, lvi, lvj);
     }
     const double Su = lui + luj, Sv = lvi + lvj, Sp = lpi + lpj;
     // U_L - U_R = -(v_a - v_b + sI (l_i + l_j)).r / d
     const double vxm = MUSCL ? (du0 + sI * Su) * r0 + (du1 + sI * Sv) * r1 : vx;
     const double dU = -vxm * id;
     const double rbar = 0.5 * (A.rho + B.rho), cbar = 0.5 * (A.c + B.c);
-    const double irbar = 1.0 / rbar, ic0 = 1.0 / P.sqrt_c0;
+    const double irbar = rcp64(rbar), ic0 = P.inv_sqrt_c0;
     const double Pbar = 0.5 * (A.p + B.p);
     // Riemann state
     double PA, w0, w1, bR = 0.0, kk = 0.0;
@@ -305,7 +317,7 @@ __device__ __forceinline__ void rev_pair(const Params& P, const PSide& A, const 
         const double dpp = sIh * dp;
         hrL = a_lower ? A.rho : B.rho; hrR = a_lower ? B.rho : A.rho;
         hcL = a_lower ? A.c : B.c; hcR = a_lower ? B.c : A.c;
-        hCL = hrL * hcL; hCR = hrR * hcR; hiC = 1.0 / (hCL + hCR);
+        hCL = hrL * hcL; hCR = hrR * hcR; hiC = rcp64(hCL + hCR);
         hsL = (hCL * hdVh + dpp) * hiC;
         hsR = (dpp - hCR * hdVh) * hiC;
         const double hh = 0.5 * hdVh;
@@ -340,7 +352,7 @@ __device__ __forceinline__ void rev_pair(const Params& P, const PSide& A, const 
     const double den_phi = d2 + fh2;
     double phi = 0.0, Pi = 0.0, iden = 0.0;
     if (av) {
-        iden = 1.0 / den_phi;
+        iden = rcp64(den_phi);
         phi = P.h * vx * iden;
         Pi = (-P.alpha * cbar * phi + P.beta * (phi * phi)) * irbar;
     }
@@ -883,12 +895,12 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_a(Params P, Sorted<R> D, Ad
         const double2 xb = D.pos[b];
         const double4 kb = D.kin[b];
         const double r0 = xc.x - xb.x, r1 = xc.y - xb.y;
-        const double d = sqrt(r0 * r0 + r1 * r1), id = 1.0 / d;
+        const double d2 = r0 * r0 + r1 * r1, id = rsqrt64(d2), d = d2 * id;
         double G, dG, W;
         kernel_gw(P, d, G, dG, W);
         if (MS) {
             const double mb = D.mass[b];
-            const double rs = kc.z + kb.z, irs = 1.0 / rs;
+            const double rs = kc.z + kb.z, irs = rcp64(rs);
             const double2 g = A.gavg[b], l = lg[b];
             const double lb0 = g.x + l.x, lb1 = g.y + l.y;
             // own sum: f = eps m_b W / rs times (v_b - v_c)
@@ -978,7 +990,7 @@ __global__ void k_shift_sum(Params P, Sorted<R> D, Adj A) {
         const int b = (int)(D.pairs[(size_t)e * P.nbr_stride + a] & 0x7fffffffu);
         const double2 xb = D.pos[b];
         const double r0 = xa.x - xb.x, r1 = xa.y - xb.y;
-        const double d = sqrt(r0 * r0 + r1 * r1);
+        const double d2 = r0 * r0 + r1 * r1, d = d2 * rsqrt64(d2);
         double G, dG, W;
         kernel_gw(P, d, G, dG, W);
         const double q = W * iwdx, q2 = q * q;
@@ -1007,7 +1019,7 @@ __global__ void k_adj_shift(Params P, Sorted<R> D, Adj A) {
         if (mc.x == 0.0 && mc.y == 0.0 && mb.x == 0.0 && mb.y == 0.0) continue;
         const double2 xb = D.pos[b];
         const double r0 = xc.x - xb.x, r1 = xc.y - xb.y;
-        const double d = sqrt(r0 * r0 + r1 * r1), id = 1.0 / d;
+        const double d2 = r0 * r0 + r1 * r1, id = rsqrt64(d2), d = d2 * id;
         double G, dG, W;
         kernel_gw(P, d, G, dG, W);
         const double q = W * iwdx, q2 = q * q, q4 = q2 * q2;
@@ -1740,7 +1752,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_drag(Params P, Sorted<R> D,
             const double4 ka = c_is_a ? kc : kb, kbb = c_is_a ? kb : kc;
             const double Va = c_is_a ? Vc : Vb, Vbb = c_is_a ? Vb : Vc;
             const double r0 = c_is_a ? xc.x - xb.x : xb.x - xc.x, r1 = c_is_a ? xc.y - xb.y : xb.y - xc.y;
-            const double d2 = r0 * r0 + r1 * r1, d = sqrt(d2), id = 1.0 / d, id2 = id * id;
+            const double d2 = r0 * r0 + r1 * r1, id = rsqrt64(d2), d = d2 * id, id2 = id * id;
             double G, dG;
             kernel_g(P, d, G, dG);
             const double L0 = bi.x * r0 + bi.y * r1, L1 = bi.z * r0 + bi.w * r1;

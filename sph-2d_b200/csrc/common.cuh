@@ -31,11 +31,14 @@ struct Params {
     double ghost_h, ghost_r, ghost_kf, shock_t, grav[2];
     // kernel / pair search
     double h, r_cut, cut_min, kfactor, gauss_e9, q_zero;
+    double s_cut, s_min;     // the support test on the squared distance: the largest s with
+                             // sqrt(s) <= r_cut, the smallest with sqrt(s) >= cut_min
+    double inv_h, half_inv_h, inv_h2, gk;   // 1/h, 1/(2h), 1/h^2; grad_a W = gk e^{-q^2} r or gk t^3 r
     double r2_list;          // squared neighbour-list radius (support * (1 + skin))
     float r2_list32;         // the same for the mixed path's FP32 test on the hi positions,
                              // widened to cover their rounding (a superset of the FP64 list)
     // equation of state
-    double rho0, c0sq, sqrt_c0, eos_b, pb;
+    double rho0, c0sq, sqrt_c0, inv_sqrt_c0, eos_b, pb;
     int eos;
     // solver coefficients
     double nu, alpha, beta, fai, delta, delta_alpha, eps;
@@ -98,9 +101,50 @@ __device__ __forceinline__ bool in_support(const Params& P, double dx, double dy
     return d <= P.r_cut && d >= P.cut_min;
 }
 
+// The same test without the square root: sqrt is monotonic and correctly rounded
+// on both sides, so with s rounded as above d <= r_cut is s <= s_cut and
+// d >= cut_min is s >= s_min for the bounds derive_params finds; the pair set is
+// the same, bit for bit.  s2: the squared distance.
+__device__ __forceinline__ bool in_support_s2(const Params& P, double dx, double dy, double& s2) {
+    s2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+    return s2 <= P.s_cut && s2 >= P.s_min;
+}
+
 // A product rounded on its own (never fused into a following add).
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// FP64 reciprocal and reciprocal square root for the pair loops: the hardware's
+// coarse approximation (about 20 bits) corrected by one third-order Newton
+// (Householder) step.  With r0 = (1 - e0)/x the first gives r0 (1 + e + e^2),
+// e = 1 - x r0, relative error e^3; with y0 = (1 - e0)/sqrt(x) the second gives
+// y0 (1 + e/2 + 3 e^2/8), e = 1 - x y0^2, relative error of order e^3: both far
+// below the rounding of the last multiply-add, so they are within about one ulp.
+// No branch and 3 / 5 FP64 operations, where the quotient and the square root
+// followed by a quotient take a multiple of that and a special-case branch
+// (tests/test_gpu_fp64_math.py measures them against the correctly rounded
+// values).  For the arguments of the pair loops: positive, normal, not huge.
+__device__ __forceinline__ double rcp64(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ double rsqrt64(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);      // y has 21 significant bits: y y is exact
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// One 32-byte record: a single 256-bit load for FP64 (cudaMalloc'd arrays of
+// 32-byte elements, so every element is 32-byte aligned), 128-bit for FP32.
+__device__ __forceinline__ double4 load4(const double4* p) {
+    double4 v;
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 load4(const float4* p) { return *p; }
 
 // Plain accumulator for the FP64 path.
 struct DSum {

@@ -32,6 +32,12 @@ namespace sph {
 // moving-square solvers (P.ms), whose XSPH sum is formed here and which keep
 // the hi + lo differences; compile-time so that the Taylor-Green launches carry
 // none of its registers.
+//
+// FP64 at 2048^2: 3.16 -> 2.54 ms per step (three launches) with the support test
+// on the squared distance, the kernel gradient without a division (and without
+// the distance at all for the Gaussian), 256-bit record loads and 5 blocks per SM
+// (92 registers; 4 blocks 2.56, 6 blocks with 36 B spilled 2.84).  Bound by the
+// L1 data stage (67 % busy) and load latency.
 #ifndef SPH_PASS_A_F32_BLOCKS
 #define SPH_PASS_A_F32_BLOCKS 8
 #endif
@@ -39,7 +45,7 @@ namespace sph {
 #define SPH_PASS_A_F32_MS_BLOCKS 7
 #endif
 template <typename R, bool HLREC, bool MS>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_BLOCKS : SPH_PASS_A_F32_BLOCKS) : 4)
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_BLOCKS : SPH_PASS_A_F32_BLOCKS) : (MS ? 4 : 5))
     k_pass_a(Params P, Sorted<R> D) {
     using V4 = typename VT<R>::V4;
     constexpr bool F32 = sizeof(R) == 4;
@@ -78,7 +84,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
     R vb_n = R(0);
     auto fetch = [&](int bb) {
         if (HL) { xbhl_n = __ldg(&D.xhl[bb]); kbh_n = __ldg(&D.kh[bb]); if (LO) kbl_n = __ldg(&D.kl[bb]); }
-        else { xb_n = __ldg(&D.pos[bb]); kb_n = D.kin[bb]; }
+        else { xb_n = __ldg(&D.pos[bb]); kb_n = load4(&D.kin[bb]); }
         vb_n = D.aux[bb].y;
     };
     if (nn > 0) fetch((int)(ent_n & 0x7fffffffu));
@@ -97,24 +103,35 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
         const double dxd = HL ? 0.0 : xa.x - xb.x, dyd = HL ? 0.0 : xa.y - xb.y;
         const float dxf = HL ? (xa_hl.x - xbhl.x) + (xa_hl.z - xbhl.z) : 0.f;
         const float dyf = HL ? (xa_hl.y - xbhl.y) + (xa_hl.w - xbhl.w) : 0.f;
-        R d, inv_d;
+        R d = R(0), inv_d = R(0);
+        double s2 = 0.0;                 // FP64: the squared distance
         if (F32) {
             const R s = HL ? (R)(dxf * dxf + dyf * dyf) : (R)(dxd * dxd + dyd * dyd);
             if (!(s <= r2cut) || s < r2min) continue;
             inv_d = rsqrtf(s);
             d = s * inv_d;
         } else {
-            double dd;
-            if (!in_support(P, dxd, dyd, dd)) continue;
-            d = (R)dd;
-            inv_d = R(1) / d;
+            if (!in_support_s2(P, dxd, dyd, s2)) continue;
         }
         D.pairs[(size_t)np * P.nbr_stride + a] = ent;
         ++np;
         const R dx = HL ? (R)dxf : (R)dxd, dy = HL ? (R)dyf : (R)dyd;
         // grad_a W = g(d) (x_a - x_b)  (compute_kernel)
         R gs, wk;
-        {
+        if constexpr (!F32) {
+            // FP64: q/(d h) = 1/h^2 folded into gk, so the Gaussian needs no distance
+            // and Wendland C2 only q = s rsqrt(s) / h
+            if (P.kernel_model == SPH_KERNEL_GAUSSIAN) {
+                const double ex = exp(-(s2 * P.inv_h2));
+                wk = (R)((ex - P.gauss_e9) * P.kfactor);
+                gs = (R)(ex * P.gk);
+            } else {
+                const double hq = s2 * rsqrt64(s2) * P.half_inv_h;      // q / 2
+                const double t = 1.0 - hq, t2 = t * t;
+                wk = (R)(P.kfactor * (1.0 + 4.0 * hq) * (t2 * t2));
+                gs = (R)(P.gk * (t2 * t));
+            }
+        } else {
             const R q = d * inv_h;
             const R kf = (R)P.kfactor;
             if (P.kernel_model == SPH_KERNEL_GAUSSIAN) {
@@ -200,13 +217,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
         tyy = (R)((2 * nut * syy - kk - blin) * rho);
     }
     // FP32 records: the gradients halved (exact), since pass C uses only
-    // 1/2 grad phi, and w = 1/rho (rounded FP32 reciprocal of the FP32 density),
-    // which pass C reads instead of forming it for every pair
+    // 1/2 grad phi.  nb3.w = 1/rho (FP32: the rounded reciprocal of the FP32
+    // density), which pass C reads instead of forming it for every pair
     if (F32)
         for (int c = 0; c < 8; ++c) gr[c] *= R(0.5);
     D.nb1[a] = mk4<R>(txx, txy, tyy, gr[0]);
     D.nb2[a] = mk4<R>(gr[1], gr[2], gr[3], gr[4]);
-    D.nb3[a] = mk4<R>(gr[5], gr[6], gr[7], F32 ? (R)__frcp_rn((float)rho_a) : R(0));
+    D.nb3[a] = mk4<R>(gr[5], gr[6], gr[7], F32 ? (R)__frcp_rn((float)rho_a) : (R)(1.0 / rho_a));
     const R fv = fra;
     D.fra_v[a] = fv;
     uint8_t fl = 0;

@@ -33,73 +33,75 @@
 
 namespace sph {
 
-template <typename R>
-__device__ __forceinline__ void muscl_limiter(R di, R dj, R dij, R& li, R& lj) {
-    // The reference's two sign branches folded into one: with s = sign(dj)
-    // (+1 when dj > 0, else -1) the dj <= 0 branch is the dj > 0 branch applied
-    // to (-di, -dj) and negated, since min and max swap under negation:
-    //   lim = s max(0, max(min(1.3 s di, s dj), min(s di, 1.3 s dj))),
-    //   lim < dij/2 (dj <= 0) <=> s lim > s dij/2,  di < dj <=> s di > s dj.
-    // The same values as the branches (zero increments may carry the other
-    // sign), one min/max chain, no divergence between the lanes of a warp.
-    const R b = R(1.3);
-    const R s = dj > R(0) ? R(1) : R(-1);
-    const R sdi = s * di, sdj = s * dj;
-    const R m = max(R(0), max(min(b * sdi, sdj), min(sdi, b * sdj)));     // s * lim >= 0
-    const R half = R(0.5) * dij;
-    const bool big = m > s * half && m > R(0);
-    const bool first = sdi > sdj;
-    const R lim = s * m;
-    const R off = dij * R(0);
-    li = big ? (first ? half : off) : lim;
-    lj = big ? (first ? off : half) : lim;
-}
-
-// The FP32 form: multiplying by s = +-1 is a flip of the sign bit (taken from
-// dj), and s dj = |dj|.  dj = +0 takes s = +1 instead of -1; both give m = 0,
-// big = false and li = lj = 0, so the values are those of the form above
-// (a zero increment may carry the other sign).
-template <>
-__device__ __forceinline__ void muscl_limiter<float>(float di, float dj, float dij, float& li, float& lj) {
-    const float b = 1.3f;
+// The MUSCL limiter (function_module.f90:34-80) of one field, for particle a of
+// the pair (a, b), written without the pair's orientation.  With A = -1/2 grad
+// phi_a.(x_a - x_b) and B = 1/2 grad phi_b.(x_a - x_b) the reference's arguments are
+// (di, dj) = (A, B) when a is pair_i and (B, A) when it is pair_j, and
+// dij = phi_j - phi_i = -sgn dphi with dphi = phi_a - phi_b, sgn = +-1.  Folding
+// its two sign branches (the dj <= 0 branch is the dj > 0 one on (-di, -dj),
+// negated) its value is
+//   lim = s max(0, max(min(1.3 s di, s dj), min(s di, 1.3 s dj))),  s = sign(dj),
+// replaced by dij/2 for one side and 0 for the other when s lim > s dij/2.  lim is
+// symmetric in di and dj (it is 0 when their signs differ), so s and both
+// products can be taken from (A, B) directly; the side that keeps dij/2 is the
+// one with the larger s d, which is a when s A > s B (or >= when a is pair_j).
+// Returned: L = sgn (li + lj), the sum in a's frame, and own, a's increment times
+// sgn; flip = the sign bit of sgn.
+//
+// FP32: with the arguments selected by a_is_i (the form without the selects has
+// fewer instructions between the neighbour-record loads and measured 1 % slower:
+// mixed pass C 2.77 -> 2.80 ms per step at 2048^2).
+__device__ __forceinline__ void muscl_limiter(float A, float B, float dphi, bool a_is_i, unsigned, float& L,
+                                              float& own) {
+    const float sgn = a_is_i ? 1.f : -1.f;
+    const float di = a_is_i ? A : B, dj = a_is_i ? B : A, dij = -(sgn * dphi);
     const unsigned sb = __float_as_uint(dj) & 0x80000000u;
     const float sdi = __uint_as_float(__float_as_uint(di) ^ sb), sdj = fabsf(dj);
-    const float m = fmaxf(0.f, fmaxf(fminf(b * sdi, sdj), fminf(sdi, b * sdj)));
+    const float m = fmaxf(0.f, fmaxf(fminf(1.3f * sdi, sdj), fminf(sdi, 1.3f * sdj)));
     const float half = 0.5f * dij;
     const bool big = m > __uint_as_float(__float_as_uint(half) ^ sb) && m > 0.f;
     const bool first = sdi > sdj;
     const float lim = __uint_as_float(__float_as_uint(m) ^ sb);
-    li = big ? (first ? half : 0.f) : lim;
-    lj = big ? (first ? 0.f : half) : lim;
+    L = sgn * (big ? half : 2.f * lim);
+    own = sgn * (big ? (first == a_is_i ? half : 0.f) : lim);
+}
+// FP64: without the selects (a 64-bit select is two instructions); multiplying by
+// s or sgn is a flip of the sign bit in the high word, so the only use of a_is_i
+// is the tie, and both members of a pair form the same bits.
+__device__ __forceinline__ double flip_sign(double v, int hi_bit) {
+    return __hiloint2double(__double2hiint(v) ^ hi_bit, __double2loint(v));
+}
+__device__ __forceinline__ void muscl_limiter(double A, double B, double dphi, bool a_is_i, unsigned flip, double& L,
+                                              double& own) {
+    const int sb = __double2hiint(B) & (int)0x80000000u;
+    const double x = flip_sign(A, sb), y = fabs(B);
+    // max(min(1.3 x, y), min(x, 1.3 y)) = min(1.3 min(x, y), max(x, y)) for x, y >= 0
+    // (for x <= 0 both are <= 0 and m = 0)
+    const bool gt = x > y;
+    const double lo = gt ? y : x, hi = gt ? x : y;
+    const double l3 = 1.3 * lo;
+    const double m = l3 < hi ? l3 : hi;
+    const double hb = -0.5 * dphi;
+    const int t = sb ^ (int)flip;
+    const bool pos = x > 0.0;                        // with y > 0 too: m > 0
+    const bool big = pos && m > flip_sign(hb, t) && m > 0.0;
+    const bool mine = gt || (x == y && !a_is_i);
+    const double lim = pos ? flip_sign(m, t) : 0.0;
+    L = big ? hb : 2.0 * lim;
+    own = big ? (mine ? hb : 0.0) : lim;
 }
 
-// The same FP32 limiter with its results as a pair term uses them: the sum
-// L = li + lj (half when one increment is clamped to dij/2, else 2 lim) and the
-// increment of this particle's side (li when it is pair_i, else lj).
-__device__ __forceinline__ void muscl_limiter_sum(float di, float dj, float dij, bool a_is_i, float& L, float& own) {
-    const float b = 1.3f;
-    const unsigned sb = __float_as_uint(dj) & 0x80000000u;
-    const float sdi = __uint_as_float(__float_as_uint(di) ^ sb), sdj = fabsf(dj);
-    const float m = fmaxf(0.f, fmaxf(fminf(b * sdi, sdj), fminf(sdi, b * sdj)));
-    const float half = 0.5f * dij;
-    const bool big = m > __uint_as_float(__float_as_uint(half) ^ sb) && m > 0.f;
-    const bool first = sdi > sdj;
-    const float lim = __uint_as_float(__float_as_uint(m) ^ sb);
-    L = big ? half : 2.f * lim;
-    own = big ? (first == a_is_i ? half : 0.f) : lim;
-}
-
-// Reciprocal and quotient in the pair loop: correctly rounded, except the
-// FP32 1/rho-bar and artificial-viscosity quotient (fast_quot: __fdividef,
-// about 2 ulp).  Fast forms everywhere made mixed pass C slower (3.46 -> 3.85 ms
+// Reciprocal and quotient in the pair loop.  FP32: correctly rounded, except the
+// 1/rho-bar and artificial-viscosity quotient (fast_quot: __fdividef, about 2
+// ulp).  Fast forms everywhere made mixed pass C slower (3.46 -> 3.85 ms
 // per step at 2048^2: fewer instructions between the neighbour-record loads);
 // these two alone took it from 2.80 to 2.75 ms with the velocity L2 against
-// FP64 unchanged (2.78e-6 after 100 steps).
-__device__ __forceinline__ double rcp(double x) { return 1.0 / x; }
+// FP64 unchanged (2.78e-6 after 100 steps).  FP64: the Newton reciprocal.
+__device__ __forceinline__ double rcp(double x) { return rcp64(x); }
 __device__ __forceinline__ float rcp(float x) { return __frcp_rn(x); }
 template <typename R>
 __device__ __forceinline__ R quot(R a, R b) { return a / b; }
-__device__ __forceinline__ double fast_quot(double a, double b) { return a / b; }
+__device__ __forceinline__ double fast_quot(double a, double b) { return a * rcp64(b); }
 __device__ __forceinline__ float fast_quot(float a, float b) { return __fdividef(a, b); }
 
 // Per-particle state a thread needs for one side of a pair.
@@ -126,6 +128,15 @@ struct Side {
 #ifndef SPH_PASS_C_F32_BLOCKS
 #define SPH_PASS_C_F32_BLOCKS 4
 #endif
+//
+// FP64 at 2048^2 (MUSCL, ms per step of three launches): 7.30 with correctly
+// rounded square roots, reciprocals and quotients and the limiter's and frame's
+// 64-bit selects; 6.02 with rsqrt64 / rcp64, m_b/rho_b read as V_b, the
+// orientation-free limiter and 256-bit record loads; 5.46 with the neighbour's
+// records loaded one iteration ahead (kept: 168 registers, 3 blocks per SM; 4
+// blocks without the prefetch 5.89).  ncu at 1024^2, 398 -> 270 M warp
+// instructions, 654 -> 431 us: FP64 pipe 50 % busy, L1 data stage 67 % (176 B of
+// records per neighbour), 58 % issue-active.
 template <typename R, bool MUSCL, bool MS, bool SHIFT>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIFT_BLOCKS : SPH_PASS_C_F32_BLOCKS) : 3)
     k_pass_c(Params P, Sorted<R> D) {
@@ -165,17 +176,17 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
     if (MS) avg_a = D.avg[a];
 
     const R hbar = (R)P.h;
-    const R inv_h = (R)(1.0 / P.h);
-    const R gk = (R)((P.kernel_model == SPH_KERNEL_GAUSSIAN ? -2.0 : -5.0) * P.kfactor / (P.h * P.h));
-    const R inv_sqc0 = (R)(1.0 / P.sqrt_c0);
+    const R inv_h = (R)P.inv_h;
+    const R gk = (R)P.gk;
+    const R inv_sqc0 = (R)P.inv_sqrt_c0;
     const R nu2 = (R)(2.0 * P.nu), alpha = (R)P.alpha, beta = (R)P.beta;
     const R fh2 = (R)((P.fai * P.h) * (P.fai * P.h));
     const R dlt2h = (R)(2.0 * P.delta * P.h);
     const R dla_dh = (R)(P.delta * P.h);
     const R dla_h = (R)(P.delta_alpha * P.h);
     const R eps2 = (R)(2.0 * P.eps);
-    // 1/rho: the FP32 MUSCL records carry it (nb3.w, the same rounded reciprocal)
-    constexpr bool RREC = F32 && MUSCL;
+    // 1/rho: the MUSCL records carry it (nb3.w)
+    constexpr bool RREC = MUSCL;
     const R inv_rho_a = RREC ? (R)S.nb3.w : rcp(rho_a);
     const R rho0_over_rho_a = (R)P.rho0 * inv_rho_a;
     const R dla_rho = dla_h * rho0_over_rho_a;
@@ -184,13 +195,12 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
     cont.init(); accx.init(); accy.init();
     R xsx = R(0), xsy = R(0);
     double shx = 0.0, shy = 0.0;   // shifting sum, FP64 in both paths
-    const double inv_h64 = 1.0 / P.h, inv_h2_64 = inv_h64 * inv_h64, inv_wdx = 1.0 / P.w_dx;
+    const double inv_h64 = P.inv_h, inv_h2_64 = P.inv_h2, inv_wdx = 1.0 / P.w_dx;
 
     // the pairs pass A found inside the support at this RHS
     unsigned ent_n = nn > 0 ? __ldg(&D.pairs[a]) : 0u;
     // software pipeline: the pair entry two iterations ahead; the neighbour's
-    // position and (mixed path) its records one iteration ahead
-    constexpr bool PRE = HL;
+    // position and its records one iteration ahead
     unsigned ent_nn = nn > 1 ? __ldg(&D.pairs[(size_t)P.nbr_stride + a]) : 0u;
     double2 xb_n = make_double2(0.0, 0.0);
     float4 xbhl_n = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -199,16 +209,16 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
     Side<R> T_n;
     auto load_records = [&](int bb, Side<R>& t) {
         if (HL) { t.kh = D.kh[bb]; t.kl = D.kl[bb]; }
-        else t.kin = D.kin[bb];
-        t.aux = D.aux[bb]; t.nb1 = D.nb1[bb]; t.nb2 = D.nb2[bb];
-        if (MUSCL) t.nb3 = D.nb3[bb];
+        else t.kin = load4(&D.kin[bb]);
+        t.aux = load4(&D.aux[bb]); t.nb1 = load4(&D.nb1[bb]); t.nb2 = load4(&D.nb2[bb]);
+        if (MUSCL) t.nb3 = load4(&D.nb3[bb]);
     };
     if (nn > 0) {
         const int b0 = (int)(ent_n & 0x7fffffffu);
         if (X64) xb_n = __ldg(&D.pos[b0]);
         else xbhl_n = __ldg(&D.xhl[b0]);
         if (VPRE) vd_n = __ldg(&D.vol64[b0]);
-        if (PRE) load_records(b0, T_n);
+        load_records(b0, T_n);
     }
     for (int e = 0; e < nn; ++e) {
         const unsigned ent = ent_n;
@@ -217,15 +227,14 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         const double2 xb = xb_n;
         const float4 xbhl = xbhl_n;
         const double vd_b = vd_n;
-        Side<R> T;
-        if (PRE) T = T_n;
+        const Side<R> T = T_n;
         if (e + 1 < nn) {
             ent_n = ent_nn;
             const int b1 = (int)(ent_n & 0x7fffffffu);
             if (X64) xb_n = __ldg(&D.pos[b1]);
             else xbhl_n = __ldg(&D.xhl[b1]);
             if (VPRE) vd_n = __ldg(&D.vol64[b1]);
-            if (PRE) load_records(b1, T_n);
+            load_records(b1, T_n);
             if (e + 2 < nn) ent_nn = __ldg(&D.pairs[(size_t)(e + 2) * P.nbr_stride + a]);
         }
         // x_a - x_b: FP64, or hi/lo in FP32 (the mixed SHIFT launch: the FP32
@@ -240,21 +249,21 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
             inv_d = rsqrtf(s);
             d = s * inv_d;
         } else {
-            d = (R)sqrt(dxd * dxd + dyd * dyd);
-            inv_d = R(1) / d;
+            const double s = dxd * dxd + dyd * dyd;
+            inv_d = (R)rsqrt64(s);
+            d = (R)(s * (double)inv_d);
         }
-        if (!PRE) load_records(b, T);
         // the pair's i and j members (only the moving-square HLLC state reads
         // them; everything else is formed from a's and b's records directly)
         const Side<R>& I = a_is_i ? S : T;
         const Side<R>& J = a_is_i ? T : S;
         const R sgn = a_is_i ? R(1) : R(-1);
-        // AB (the mixed MUSCL Taylor-Green launch): the pair terms are formed in a's
+        // AB (the FP64 and the mixed MUSCL Taylor-Green launches): the pair terms are formed in a's
         // frame, x_a - x_b and phi_a - phi_b, instead of the pair's i/j frame.
         // Negation is exact, so a term odd in the orientation takes the i/j-frame
-        // bits times sgn and the sgn of the final sums cancels it: sgn stays only
-        // where the MUSCL limiter needs the i/j frame.
-        constexpr bool AB = F32 && MUSCL && !MS;
+        // bits times sgn and the sgn of the final sums cancels it; only the MUSCL
+        // limiter looks at the orientation.
+        constexpr bool AB = !MS && (MUSCL || !F32);
         // position_difference_ij = x_i - x_j (find_particle_pair.f90:79-107) = sgn (x_a - x_b);
         // xij: that, or x_a - x_b in AB
         R xab0, xab1;
@@ -273,13 +282,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
             drho_ji = -(fsg * (R)((S.kh.z - T.kh.z) + (S.kl.z - T.kl.z)));
             rho_a_ = (R)S.kh.z; rho_b = (R)T.kh.z;
         } else {
-            du = sgn * (R)(S.kin.x - T.kin.x); dv = sgn * (R)(S.kin.y - T.kin.y);
-            dp = sgn * (R)(S.kin.w - T.kin.w);
-            drho_ji = -(sgn * (R)(S.kin.z - T.kin.z));
+            du = fsg * (R)(S.kin.x - T.kin.x); dv = fsg * (R)(S.kin.y - T.kin.y);
+            dp = fsg * (R)(S.kin.w - T.kin.w);
+            drho_ji = -(fsg * (R)(S.kin.z - T.kin.z));
             rho_a_ = (R)S.kin.z; rho_b = (R)T.kin.z;
         }
-        // compute_kernel: W and dwdx(k) = g (x_i - x_j).  FP32: g with
-        // q/(d h) = 1/h^2 folded into a constant (gk)
+        // compute_kernel: W and dwdx(k) = g (x_i - x_j), g with q/(d h) = 1/h^2
+        // folded into a constant (gk)
         R w, g;
         {
             const R q = d * inv_h;
@@ -287,12 +296,12 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
             if (P.kernel_model == SPH_KERNEL_GAUSSIAN) {
                 const R ex = exp(-(q * q));
                 w = (ex - (R)P.gauss_e9) * kf;
-                g = F32 ? ex * gk : ex * (R(-2) * q) * inv_d * inv_h * kf;
+                g = ex * gk;
             } else {
                 const R t = R(1) - R(0.5) * q;
                 const R t3 = t * t * t;
                 w = kf * (R(1) + R(2) * q) * (t3 * t);
-                g = F32 ? t3 * gk : kf * (R(-5) * q * t3) * inv_d * inv_h;
+                g = t3 * gk;
             }
         }
         const R dw0 = g * xij0, dw1 = g * xij1;
@@ -303,50 +312,37 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         const R rbar = R(0.5) * (rho_a_ + rho_b);
         const R inv_rbar = fast_quot(R(1), rbar);
         const R e0 = -xij0 * inv_d, e1 = -xij1 * inv_d;     // x_j - x_i direction (both solvers)
-        // Riemann states.  li/lj are the MUSCL reconstruction increments
-        // (function_module.f90:34-80); the modified solver has none.
-        R lpi = R(0), lpj = R(0), lui = R(0), luj = R(0), lvi = R(0), lvj = R(0);
+        // Riemann states.  lp, lu, lv are the sums of the MUSCL reconstruction
+        // increments of both sides and ou, ov this side's (muscl_limiter, in a's
+        // frame); the other solvers have none.
+        R lp = R(0), lu = R(0), lv = R(0), ou = R(0), ov = R(0);
         if (MUSCL) {
-            // DelPhi_i = 0.5 grad phi_i.(x_j - x_i), DelPhi_j = -0.5 grad phi_j.(x_j - x_i):
-            // with ga = 0.5 grad phi_a.(x_a - x_b), gb = 0.5 grad phi_b.(x_a - x_b),
-            // (DelPhi_i, DelPhi_j) = (-ga, gb) when a is pair_i and (gb, -ga) when it is
-            // pair_j.  The products are rounded separately and fused in a fixed order,
-            // so both members of the pair form the same bits.
-            // nb2 = (grad rho y, grad p x, grad p y, grad u x), nb3 = (grad u y, grad v x, grad v y, 1/rho),
-            // the gradients halved in the FP32 records
-            // (the FP32 records hold 1/2 grad phi, so the halving is already done, exactly)
+            // 1/2 grad phi.(x_a - x_b) of both particles; the products are rounded
+            // separately and fused in a fixed order, so both members of the pair form
+            // the same bits.  nb2 = (grad rho y, grad p x, grad p y, grad u x),
+            // nb3 = (grad u y, grad v x, grad v y, 1/rho); the FP32 records hold
+            // 1/2 grad phi, so the halving is already done, exactly.
             auto half_dot = [&](R g0, R g1) { return (F32 ? R(1) : R(0.5)) * fma(g1, xab1, mul_rn(g0, xab0)); };
             const R gpa = half_dot(S.nb2.y, S.nb2.z), gpb = half_dot(T.nb2.y, T.nb2.z);
             const R gua = half_dot(S.nb2.w, S.nb3.x), gub = half_dot(T.nb2.w, T.nb3.x);
             const R gva = half_dot(S.nb3.y, S.nb3.z), gvb = half_dot(T.nb3.y, T.nb3.z);
-            if constexpr (AB) {
-                // the limiter in the i/j frame (dij = phi_j - phi_i = -sgn (phi_a - phi_b)),
-                // its sum and own-side increment taken back to a's frame by sgn;
-                // lpi etc. then hold sgn L and the own increment (lpj, luj, lvj unused)
-                float L, own;
-                muscl_limiter_sum(a_is_i ? -gpa : gpb, a_is_i ? gpb : -gpa, -(sgn * dp), a_is_i, L, own);
-                lpi = sgn * L;
-                muscl_limiter_sum(a_is_i ? -gua : gub, a_is_i ? gub : -gua, -(sgn * du), a_is_i, L, own);
-                lui = sgn * L; luj = sgn * own;
-                muscl_limiter_sum(a_is_i ? -gva : gvb, a_is_i ? gvb : -gva, -(sgn * dv), a_is_i, L, own);
-                lvi = sgn * L; lvj = sgn * own;
-            } else {
-                muscl_limiter<R>(a_is_i ? -gpa : gpb, a_is_i ? gpb : -gpa, -dp, lpi, lpj);
-                muscl_limiter<R>(a_is_i ? -gua : gub, a_is_i ? gub : -gua, -du, lui, luj);
-                muscl_limiter<R>(a_is_i ? -gva : gvb, a_is_i ? gvb : -gva, -dv, lvi, lvj);
-            }
+            const unsigned flip = ~ent & 0x80000000u;
+            R own;
+            muscl_limiter(-gpa, gpb, dp, a_is_i, flip, lp, own);
+            muscl_limiter(-gua, gub, du, a_is_i, flip, lu, ou);
+            muscl_limiter(-gva, gvb, dv, a_is_i, flip, lv, ov);
         }
-        // U_L - U_R and P_L - P_R from the differences (AB: the frame's e0, e1 and
+        // U_L - U_R and P_L - P_R from the differences (the frame's e0, e1 and
         // differences; the product is the i/j frame's)
-        const R dU = AB ? (du + lui) * e0 + (dv + lvi) * e1 : (du + lui + luj) * e0 + (dv + lvi + lvj) * e1;
+        const R dU = (du + lu) * e0 + (dv + lv) * e1;
         const R Pbar = HL ? R(0.5) * ((R)S.kh.w + (R)T.kh.w) : R(0.5) * ((R)S.kin.w + (R)T.kin.w);
         R PA, wa0, wa1;          // this side's star pressure and velocity minus star velocity
-        if (AB) { wa0 = R(0.5) * du + luj; wa1 = R(0.5) * dv + lvj; }
-        else if (a_is_i) { wa0 = R(0.5) * du + lui; wa1 = R(0.5) * dv + lvi; }
-        else { wa0 = R(-0.5) * du - luj; wa1 = R(-0.5) * dv - lvj; }
+        if (AB) { wa0 = R(0.5) * du + ou; wa1 = R(0.5) * dv + ov; }
+        else if (a_is_i) { wa0 = R(0.5) * du; wa1 = R(0.5) * dv; }
+        else { wa0 = R(-0.5) * du; wa1 = R(-0.5) * dv; }
         if (!MS || !P.hllc) {
-            // AB: dP and U* - Ubar in a's frame; sU e is the i/j frame's product
-            const R dP = AB ? dp + lpi : dp + lpi + lpj;
+            // dP and U* - Ubar in the frame; sU e is the same product in either
+            const R dP = dp + lp;
             const R sU = R(0.5) * dP * (inv_rbar * inv_sqc0);               // U* - Ubar
             const R bR = min(R(3) * (max(dU, R(0))), cbar);
             const R Ps = Pbar + R(0.5) * bR * rbar * dU;
@@ -412,8 +408,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         } else {
             // HLLC in the pair frame (Moving_Square.../Solver_Normalized_HLLC_Riemann_Delta.f90:207-322),
             // FP64 path: the reference's own operations
-            const double ed0 = -(a_is_i ? dxd : -dxd) / sqrt(dxd * dxd + dyd * dyd);
-            const double ed1 = -(a_is_i ? dyd : -dyd) / sqrt(dxd * dxd + dyd * dyd);
+            const double ed0 = (double)e0, ed1 = (double)e1;
             const double uI = I.kin.x, vI = I.kin.y, uJ = J.kin.x, vJ = J.kin.y;
             const double VL0 = ed0 * uI + ed1 * vI, VL1 = -ed1 * uI + ed0 * vI;
             const double VR0 = ed0 * uJ + ed1 * vJ, VR1 = -ed1 * uJ + ed0 * vJ;
@@ -454,7 +449,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         R dr = R(2) * rho_a * Vb * (fsg * (wa0 * nd0 + wa1 * nd1));
         // pressure force (:374-388)
         const R rho_ij = inv_rho_a * (RREC ? (R)T.nb3.w : rcp(rho_b));
-        const R fp = R(-2) * PA * rho_ij * mb;
+        // (FP64: m_b / rho_b is V_b)
+        const R fp = F32 ? R(-2) * PA * rho_ij * mb : R(-2) * PA * (inv_rho_a * Vb);
         R tx = fp * nd0, ty = fp * nd1;
         // artificial viscosity (:392-417)
         const R inv_r2 = inv_d * inv_d;
@@ -465,11 +461,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
             tx += mb * (-Pi * nd0);
             ty += mb * (-Pi * nd1);
         }
-        // (x_i - x_j).B^-1 dwdx / r^2, shared by the laplacian and delta-SPH (FP32)
+        // (x_i - x_j).B^-1 dwdx / r^2, shared by the laplacian and delta-SPH
         const R xnd = (xij0 * nd0 + xij1 * nd1) * inv_r2;
         if (!MS || P.laplacian == 1) {
             // Morris laplacian (:432-436)
-            const R lf = F32 ? Vb * nu2 * xnd : Vb * nu2 * (xij0 * nd0 + xij1 * nd1) * inv_r2;
+            const R lf = Vb * nu2 * xnd;
             tx += lf * du;
             ty += lf * dv;
         } else {
@@ -479,7 +475,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
             ty += lf * nd1;
         }
         // delta-alpha artificial internal acceleration (:442-446)
-        const R tt = F32 ? dla_rho * cbar * (vx * inv_r2) * Vb : dla_h * cbar * vx * inv_r2 * rho0_over_rho_a * Vb;
+        const R tt = dla_rho * cbar * (vx * inv_r2) * Vb;
         tx += tt * nd0;
         ty += tt * nd1;
         // SPS force, unnormalised dwdx and the neighbour's SPS mass (:450-492);
@@ -498,8 +494,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         // XSPH average velocity (:495-500; modified solver only)
         if (!MUSCL && !MS && P.xsph) {
             const R f = eps2 * mb * rcp(rho_a_ + rho_b) * w;
-            xsx -= sgn * (f * du);
-            xsy -= sgn * (f * dv);
+            xsx -= fsg * (f * du);
+            xsy -= fsg * (f * dv);
         }
         // delta-SPH density diffusion (:552-583): psi = (rho_j - rho_i) - 0.5 (grad rho_i + grad rho_j).(x_j - x_i)
         if (water) {
@@ -510,11 +506,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
                 const R f = R(2) * drho_ji * inv_r2;
                 const R gsc = F32 ? R(2) : R(1);      // FP32 records: 1/2 grad rho
                 const R p0 = -(f * xij0) - gsc * sg0, p1 = -(f * xij1) - gsc * sg1;
-                dr += sgn * (dla_dh * cbar * (p0 * nd0 + p1 * nd1) * Vb);
+                dr += fsg * (dla_dh * cbar * (p0 * nd0 + p1 * nd1) * Vb);
             } else {
                 const R psi = drho_ji + (F32 ? R(1) : R(0.5)) * (sg0 * xij0 + sg1 * xij1);
-                const R tma = F32 ? -xnd : -(xij0 * nd0 + xij1 * nd1) * inv_r2;
-                dr += fsg * (dlt2h * cbar * psi * tma * Vb);
+                dr += fsg * (dlt2h * cbar * psi * (-xnd) * Vb);
             }
         }
         cont.add(dr);
@@ -583,7 +578,7 @@ __global__ void __launch_bounds__(128, 12) k_shift_gather(Params P, Sorted<R> D)
     }
     const int nn = D.npairs[a];
     const double2 xa = D.pos[a];
-    const double inv_h64 = 1.0 / P.h, inv_h2_64 = inv_h64 * inv_h64, inv_wdx = 1.0 / P.w_dx;
+    const double inv_h64 = P.inv_h, inv_h2_64 = P.inv_h2, inv_wdx = 1.0 / P.w_dx;
     double shx = 0.0, shy = 0.0;
     // the pair entry two iterations ahead, the neighbour's position and volume one ahead
     unsigned ent_n = nn > 0 ? __ldg(&D.pairs[a]) : 0u;

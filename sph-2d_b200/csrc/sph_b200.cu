@@ -197,7 +197,18 @@ int derive_params(const sph_config& c, Params& P) {
         P.sps_blin = 2.0 / 3.0 * 0.0066;
         P.q_zero = 1.0e-8;
     }
-    P.rho0 = c.rho0; P.c0sq = c.c0sq; P.sqrt_c0 = sqrt(c.c0sq); P.eos_b = c.c0sq * c.rho0 / 7.0; P.pb = c.background_p;
+    P.inv_h = 1.0 / c.h;
+    P.half_inv_h = 0.5 / c.h;
+    P.inv_h2 = P.inv_h * P.inv_h;
+    P.gk = (c.kernel_model == SPH_KERNEL_GAUSSIAN ? -2.0 : -5.0) * P.kfactor / (c.h * c.h);
+    // in_support's bounds on the squared distance (see in_support_s2)
+    P.s_cut = P.r_cut * P.r_cut;
+    while (sqrt(P.s_cut) > P.r_cut) P.s_cut = nextafter(P.s_cut, 0.0);
+    while (sqrt(nextafter(P.s_cut, HUGE_VAL)) <= P.r_cut) P.s_cut = nextafter(P.s_cut, HUGE_VAL);
+    P.s_min = P.cut_min * P.cut_min;
+    while (sqrt(P.s_min) < P.cut_min) P.s_min = nextafter(P.s_min, HUGE_VAL);
+    while (sqrt(nextafter(P.s_min, 0.0)) >= P.cut_min) P.s_min = nextafter(P.s_min, 0.0);
+    P.rho0 = c.rho0; P.c0sq = c.c0sq; P.sqrt_c0 = sqrt(c.c0sq); P.inv_sqrt_c0 = 1.0 / P.sqrt_c0; P.eos_b = c.c0sq * c.rho0 / 7.0; P.pb = c.background_p;
     P.nu = c.nu; P.alpha = c.alpha; P.beta = c.beta; P.fai = c.fai;
     P.delta = c.delta; P.delta_alpha = c.delta_alpha; P.eps = c.xsph_eps;
     const double sr = c.kernel_scale * c.h;

@@ -21,8 +21,6 @@ struct Staging {
     double* r_drho;
     double2* r_acc;
     double2* r_avg;
-    int* cnt;         // scratch pair that sizes the image scan's temporary storage
-    int* off;
     // image counts and offsets of this step, kept for routing image adjoints:
     // left/right images of host i sit at n_host + lr_off[i] + k (k < lr_cnt[i]),
     // bottom/top images of source s at n_host + n_lr + tb_off[s] + k (k < tb_cnt[s])
@@ -44,72 +42,279 @@ __device__ __forceinline__ double2 wrap_position(const Params& P, double2 x) {
     return x;
 }
 
-// --- 2. images: count per source, then emit at scanned offsets -------------
-// axis 0: left/right images of the host particles (:98-148),
-// axis 1: bottom/top images of host particles and left/right images (:156-206).
-// cnt: the routing counts of this axis (lr_cnt / tb_cnt), scanned in place into
-// the routing offsets (lr_off / tb_off) that k_img_emit reads
-// axis 0 (sources = the host particles) wraps the positions first.
-__global__ void k_img_count(Params P, Staging S, int n_src, int axis, int* cnt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_src) return;
-    int c = 0;
-    if (S.type[i] != SPH_TYPE_ILL) {
-        double2 xy = S.pos[i];
-        if (axis == 0) {
-            const double2 w = wrap_position(P, xy);
-            if (w.x != xy.x || w.y != xy.y) S.pos[i] = w;
-            xy = w;
+// --- 2. images and the counting sort into cells -----------------------------
+// The step set-up is six launches with no host wait on its critical path:
+//   k_img_count   wraps the host positions and counts each block's images; the
+//                 last block to finish scans the block sums and posts the totals
+//                 to the host (which reads them while the next kernels run, to
+//                 size the launches that follow)
+//   k_img_emit    writes the images at their offsets, the cell key of every
+//                 particle and its arrival number in its cell
+//   k_cell_scan   exclusive scan of the cell counts (last block: of the block sums)
+//   k_place       cell ranges; particle -> slot, unordered inside a cell
+//   k_gather_sorted  orders each cell by id while it copies the arrays: the same
+//                 order as a stable sort of the keys
+//   k_build_lists
+// Bound by launch latency below about 10^5 particles and by HBM above.  Against
+// image counts and offsets by two library scans with a host wait each, a library
+// radix sort and separate key and range passes (18 launches), same slot order:
+// images + sort + lists 166 -> 59 us per step at 100^2 (FP64), 195 -> 85 us at
+// 401^2 and 1.11 -> 0.98 ms at 2048^2 (mixed).
+constexpr int kImgThreads = 1024;         // host particles per block
+constexpr int kScanThreads = 1024;        // cell scan: kScanCells cells per block
+constexpr int kScanShift = 12, kScanCells = 1 << kScanShift;
+
+// What the set-up kernels share (device memory of the handle).
+struct SetupBuf {
+    int4* blk;            // [image blocks] image sums (x: left/right, y: bottom/top of host
+                          // particles, z: bottom/top of left/right images), then exclusive
+    int* tot;             // [3] their totals
+    unsigned* done;       // [2] blocks finished (image count, cell scan); left at 0
+    unsigned* key;        // [cap] cell of particle i (id order), ncells = not binned
+    int* rank;            // [cap] its arrival number in the cell
+    int* cnt;             // [ncells + 1] particles per cell
+    int* pre;             // [ncells + 1] exclusive scan within the scan block
+    int* blkoff;          // [scan blocks] offset of the scan block
+    unsigned* perm;       // [cap] slot -> id, unordered inside a cell
+    int ncells;
+};
+
+// Totals the host waits for (page-locked, mapped): written by the device, seq last.
+struct HostBox {
+    int tot[3];
+    volatile unsigned seq;
+    unsigned status;
+    int nsurf;
+    double diag[8];
+};
+
+__device__ __forceinline__ int band_count(double v, double lo, double hi, double band) {
+    return (v <= (lo + band) && v >= lo ? 1 : 0) + (v >= (hi - band) && v <= hi ? 1 : 0);
+}
+
+// Exclusive scan over one block of up to 1024 threads; total returned to all.
+template <typename T>
+__device__ __forceinline__ T block_scan(T v, T* sh, T& total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    T inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    if (lane == 31) sh[w] = inc;
+    __syncthreads();
+    if (w == 0) {
+        T x = lane < (int)(blockDim.x >> 5) ? sh[lane] : T(0);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const T u = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += u;
         }
-        double x = axis == 0 ? xy.x : xy.y;
-        double lo = P.box_lo[axis], hi = P.box_hi[axis];
-        if (x <= (lo + P.band) && x >= lo) c++;
-        if (x >= (hi - P.band) && x <= hi) c++;
+        sh[lane] = x;
     }
-    cnt[i] = c;
+    __syncthreads();
+    total = sh[(blockDim.x >> 5) - 1];
+    const T base = w > 0 ? sh[w - 1] : T(0);
+    __syncthreads();
+    return base + inc - v;
 }
 
-__global__ void k_img_emit(Params P, Staging S, int n_src, int axis, int base, const int* off) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_src || S.type[i] == SPH_TYPE_ILL) return;
-    double2 x = S.pos[i];
-    double v = axis == 0 ? x.x : x.y;
-    double lo = P.box_lo[axis], hi = P.box_hi[axis], L = hi - lo;
-    int o = base + off[i];
-    for (int side = 0; side < 2; ++side) {
-        bool in = side == 0 ? (v <= (lo + P.band) && v >= lo) : (v >= (hi - P.band) && v <= hi);
-        if (!in) continue;
+// True in every thread of the last block of the grid to get here (its earlier
+// writes to global memory, and every other block's, are then visible).
+__device__ __forceinline__ bool last_block(unsigned* done, int* sh_flag) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned t = atomicAdd(done, 1u);
+        *sh_flag = t == gridDim.x - 1;
+    }
+    __syncthreads();
+    const bool last = *sh_flag != 0;
+    if (last) {
+        __threadfence();
+        if (threadIdx.x == 0) *done = 0u;
+    }
+    return last;
+}
+
+// axis 0: left/right images of the host particles (Distribute_Period_Boundary_Particle.f90:98-148),
+// axis 1: bottom/top images of host particles and of left/right images (:156-206).
+// A left/right image has its source's y, so every count is a function of the
+// host particle.  Packed sums: 20 bits each (at most 4 per particle).
+__device__ __forceinline__ void image_counts(const Params& P, double2 x, bool ill, int& lr, int& tb) {
+    lr = tb = 0;
+    if (ill) return;
+    lr = band_count(x.x, P.box_lo[0], P.box_hi[0], P.band);
+    tb = band_count(x.y, P.box_lo[1], P.box_hi[1], P.band);
+}
+
+__global__ void __launch_bounds__(kImgThreads) k_img_count(Params P, Staging S, SetupBuf B, HostBox* box, unsigned seq) {
+    __shared__ unsigned long long sh[32];
+    __shared__ int flag;
+    const int i = blockIdx.x * kImgThreads + threadIdx.x;
+    for (int c = i; c <= B.ncells; c += gridDim.x * kImgThreads) B.cnt[c] = 0;
+    int lr = 0, tb = 0;
+    if (i < P.n_host) {
+        const double2 xy = S.pos[i];
+        const bool ill = S.type[i] == SPH_TYPE_ILL;
+        const double2 w = wrap_position(P, xy);
+        if (!ill && (w.x != xy.x || w.y != xy.y)) S.pos[i] = w;
+        image_counts(P, w, ill, lr, tb);
+    }
+    unsigned long long total;
+    block_scan<unsigned long long>((unsigned long long)lr | ((unsigned long long)tb << 20) |
+                                       ((unsigned long long)(lr * tb) << 40), sh, total);
+    if (threadIdx.x == 0)
+        B.blk[blockIdx.x] = make_int4((int)(total & 0xfffff), (int)((total >> 20) & 0xfffff), (int)(total >> 40), 0);
+    if (!last_block(&B.done[0], &flag)) return;
+    // the last block: exclusive scan of the block sums, then the totals
+    __shared__ int shi[32];
+    int run[3] = {0, 0, 0};
+    const int nb = gridDim.x;
+    for (int b0 = 0; b0 < nb; b0 += kImgThreads) {
+        const int b = b0 + threadIdx.x;
+        const int4 v = b < nb ? __ldcg(&B.blk[b]) : make_int4(0, 0, 0, 0);
+        int t0, t1, t2;
+        const int e0 = block_scan<int>(v.x, shi, t0), e1 = block_scan<int>(v.y, shi, t1),
+                  e2 = block_scan<int>(v.z, shi, t2);
+        if (b < nb) B.blk[b] = make_int4(run[0] + e0, run[1] + e1, run[2] + e2, 0);
+        run[0] += t0; run[1] += t1; run[2] += t2;
+    }
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 3; ++k) { B.tot[k] = run[k]; box->tot[k] = run[k]; }
+        __threadfence_system();
+        box->seq = seq;
+    }
+}
+
+// Cell key (row-major cells of edge >= list radius) and arrival number of id o.
+// Particles that are not binned (Assign_boundary_particles.f90:82) or off the
+// grid go past the last cell.
+__device__ __forceinline__ void cell_key(const Params& P, const SetupBuf& B, int o, double2 x, int t, unsigned* status) {
+    unsigned key = (unsigned)B.ncells;
+    if (t != SPH_TYPE_ILL && t != 0) {
+        const double fx = floor((x.x - P.gx0) / P.cs), fy = floor((x.y - P.gy0) / P.cs);
+        const int cx = (int)fx, cy = (int)fy;
+        if (fx >= 0.0 && fy >= 0.0 && cx < P.gnx && cy < P.gny) key = (unsigned)(cy * P.gnx + cx);
+        else atomicOr(status, ST_DOMAIN);
+    }
+    B.key[o] = key;
+    B.rank[o] = atomicAdd(&B.cnt[key], 1);
+}
+
+// One image of host particle i with id o.
+__device__ __forceinline__ void put_image(const Params& P, const Staging& S, const SetupBuf& B, int i, int o, double2 x,
+                                          int cap, unsigned* status) {
+    if (o >= cap) return;                       // the host sees the total and stops
+    S.pos[o] = x;
+    S.vel[o] = S.vel[i];
+    S.rho[o] = S.rho[i];
+    S.mass[o] = S.mass[i];
+    S.smass[o] = S.smass[i];
+    S.type[o] = SPH_TYPE_PERIODIC;
+    S.itype[o] = SPH_TYPE_PERIODIC;
+    cell_key(P, B, o, x, SPH_TYPE_PERIODIC, status);
+}
+
+// periodic: emit the images, numbered as the reference appends them (left/right
+// images in host order, bottom/top images of the host particles, then of the
+// left/right images; the low side first).  route: also keep the counts and
+// offsets for the reverse sweep.
+__global__ void __launch_bounds__(kImgThreads) k_img_emit(Params P, Staging S, SetupBuf B, int cap, int periodic,
+                                                          int route, unsigned* status) {
+    __shared__ unsigned long long sh[32];
+    const int i = blockIdx.x * kImgThreads + threadIdx.x;
+    const bool live = i < P.n_host;
+    double2 x = make_double2(0.0, 0.0);
+    int t = SPH_TYPE_ILL;
+    if (live) { x = S.pos[i]; t = S.type[i]; }
+    if (live) cell_key(P, B, i, x, t, status);
+    if (!periodic) return;
+    int lr, tb;
+    image_counts(P, x, t == SPH_TYPE_ILL, lr, tb);
+    unsigned long long total;
+    const unsigned long long e = block_scan<unsigned long long>(
+        (unsigned long long)lr | ((unsigned long long)tb << 20) | ((unsigned long long)(lr * tb) << 40), sh, total);
+    if (!live || (lr == 0 && tb == 0 && !route)) return;
+    const int4 base = B.blk[blockIdx.x];
+    const int n_lr = B.tot[0], tb_host = B.tot[1];
+    const int o_lr = base.x + (int)(e & 0xfffff), o_tb = base.y + (int)((e >> 20) & 0xfffff),
+              o_lt = tb_host + base.z + (int)(e >> 40);
+    const int first_tb = P.n_host + n_lr;
+    if (route) {
+        S.lr_cnt[i] = lr; S.lr_off[i] = o_lr;
+        S.tb_cnt[i] = tb; S.tb_off[i] = o_tb;
+        for (int k = 0; k < lr; ++k) {
+            const int s = P.n_host + o_lr + k;
+            if (s < cap) { S.tb_cnt[s] = tb; S.tb_off[s] = o_lt + k * tb; }
+        }
+    }
+    if (lr == 0 && tb == 0) return;
+    const double Lx = P.box_hi[0] - P.box_lo[0], Ly = P.box_hi[1] - P.box_lo[1];
+    // sides of each axis in order: low side (shift +L), high side (-L)
+    const bool xlo = x.x <= (P.box_lo[0] + P.band) && x.x >= P.box_lo[0];
+    const bool xhi = x.x >= (P.box_hi[0] - P.band) && x.x <= P.box_hi[0];
+    const bool ylo = x.y <= (P.box_lo[1] + P.band) && x.y >= P.box_lo[1];
+    const bool yhi = x.y >= (P.box_hi[1] - P.band) && x.y <= P.box_hi[1];
+    // k = 0: the particle itself, then its left/right images
+    int o = P.n_host + o_lr, k = 0;
+#pragma unroll 1
+    for (int sx = -1; sx < 2; ++sx) {
+        if ((sx == 0 && !xlo) || (sx == 1 && !xhi)) continue;
         double2 y = x;
-        double sh = side == 0 ? L : -L;
-        if (axis == 0) y.x = x.x + sh; else y.y = x.y + sh;
-        S.pos[o] = y;
-        S.vel[o] = S.vel[i];
-        S.rho[o] = S.rho[i];
-        S.mass[o] = S.mass[i];
-        S.smass[o] = S.smass[i];
-        S.type[o] = SPH_TYPE_PERIODIC;
-        S.itype[o] = SPH_TYPE_PERIODIC;
-        ++o;
+        if (sx >= 0) {
+            y.x = x.x + (sx == 0 ? Lx : -Lx);
+            put_image(P, S, B, i, o, y, cap, status);
+            ++o;
+        }
+        int q = first_tb + (sx < 0 ? o_tb : o_lt + k * tb);
+        if (sx >= 0) ++k;
+        if (ylo) { put_image(P, S, B, i, q, make_double2(y.x, y.y + Ly), cap, status); ++q; }
+        if (yhi) put_image(P, S, B, i, q, make_double2(y.x, y.y + (-Ly)), cap, status);
     }
 }
 
-// --- 3. cell keys (row-major cells of edge >= list radius) -----------------
-__global__ void k_cell_keys(Params P, const double2* pos, const int* type, unsigned* keys, unsigned* vals,
-                            unsigned* status, unsigned dead_key) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n_tot) return;
-    vals[i] = (unsigned)i;
-    int t = type[i];
-    if (t == SPH_TYPE_ILL || t == 0) { keys[i] = dead_key; return; }   // not binned (Assign_boundary_particles.f90:82)
-    double2 x = pos[i];
-    double fx = floor((x.x - P.gx0) / P.cs), fy = floor((x.y - P.gy0) / P.cs);
-    int cx = (int)fx, cy = (int)fy;
-    if (!(fx >= 0.0 && fy >= 0.0 && cx < P.gnx && cy < P.gny)) {
-        atomicOr(status, ST_DOMAIN);
-        keys[i] = dead_key;
-        return;
+// Exclusive scan of the cell counts within blocks of kScanCells cells; the last
+// block scans the block sums.
+__global__ void __launch_bounds__(kScanThreads) k_cell_scan(SetupBuf B) {
+    __shared__ int sh[32];
+    __shared__ int flag;
+    constexpr int per = kScanCells / kScanThreads;
+    const int c0 = blockIdx.x * kScanCells + threadIdx.x * per;
+    int v[per], s = 0;
+#pragma unroll
+    for (int k = 0; k < per; ++k) { v[k] = c0 + k <= B.ncells ? B.cnt[c0 + k] : 0; s += v[k]; }
+    int total;
+    int run = block_scan<int>(s, sh, total);
+#pragma unroll
+    for (int k = 0; k < per; ++k)
+        if (c0 + k <= B.ncells) { B.pre[c0 + k] = run; run += v[k]; }
+    if (threadIdx.x == 0) B.blkoff[blockIdx.x] = total;
+    if (!last_block(&B.done[1], &flag)) return;
+    int sum = 0;
+    for (int b0 = 0; b0 < (int)gridDim.x; b0 += kScanThreads) {
+        const int b = b0 + threadIdx.x;
+        const int u = b < (int)gridDim.x ? __ldcg(&B.blkoff[b]) : 0;
+        int t;
+        const int e = block_scan<int>(u, sh, t);
+        if (b < (int)gridDim.x) B.blkoff[b] = sum + e;
+        sum += t;
     }
-    keys[i] = (unsigned)(cy * P.gnx + cx);
+}
+
+// Cell ranges (-1 for an empty cell), and each particle at its arrival place.
+__global__ void k_place(int n_tot, SetupBuf B, int* cell_start, int* cell_end) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < B.ncells) {
+        const int n = B.cnt[t], st = B.blkoff[t >> kScanShift] + B.pre[t];
+        cell_start[t] = n ? st : -1;
+        cell_end[t] = n ? st + n : -1;
+    }
+    if (t < n_tot) {
+        const unsigned k = B.key[t];
+        B.perm[B.blkoff[k >> kScanShift] + B.pre[k] + B.rank[t]] = (unsigned)t;
+    }
 }
 
 // Device-side arrays in cell-sorted order (templated on the pair precision).
@@ -193,11 +398,20 @@ __device__ __forceinline__ void store_split(Sorted<R>& D, int s, double2 x, doub
 }
 
 // --- 4. gather the id-ordered arrays into cell order -----------------------
+// Thread t holds the particle at place t; its slot is the cell's start plus the
+// number of lower ids in the cell (about 8 reads that the warp shares).
 template <typename R>
-__global__ void k_gather_sorted(Params P, Staging S, Sorted<R> D, const unsigned* perm) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= P.n_tot) return;
-    int i = (int)perm[s];
+__global__ void k_gather_sorted(Params P, Staging S, Sorted<R> D, SetupBuf B) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= P.n_tot) return;
+    const int i = (int)B.perm[t];
+    const unsigned key = B.key[i];
+    int s = t;                         // not binned: any order
+    if (key < (unsigned)B.ncells) {
+        const int st = D.cell_start[key], en = D.cell_end[key];
+        s = st;
+        for (int q = st; q < en; ++q) s += B.perm[q] < (unsigned)i ? 1 : 0;
+    }
     D.id[s] = i;
     D.slot_of[i] = s;
     D.type[s] = S.type[i];
@@ -249,16 +463,6 @@ __global__ void k_unsort(Params P, Staging S, Sorted<R> D) {
     S.r_avg[i] = make_double2((double)D.c_avg[s].x, (double)D.c_avg[s].y);
 }
 
-// --- 5. cell ranges from the sorted keys ----------------------------------
-__global__ void k_cell_ranges(int n, const unsigned* keys, int* start, int* end, unsigned dead_key) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    unsigned k = keys[s];
-    if (k == dead_key) return;
-    if (s == 0 || keys[s - 1] != k) start[k] = s;
-    if (s == n - 1 || keys[s + 1] != k) end[k] = s + 1;
-}
-
 // Pair-rule of find_particle_pair (TGV :76, MS :73-75).
 __device__ __forceinline__ bool pair_allowed(int rule, int ti, int tj) {
     if (rule == SPH_PAIRS_ONE_FLUID) return ti == SPH_TYPE_WATER || tj == SPH_TYPE_WATER;
@@ -268,7 +472,7 @@ __device__ __forceinline__ bool pair_allowed(int rule, int ti, int tj) {
     return true;
 }
 
-// --- 6. neighbour lists ----------------------------------------------------
+// --- 5. neighbour lists ----------------------------------------------------
 // Every particle b != a in the 3x3 cells with |x_a - x_b|^2 <= (support*(1+skin))^2
 // and an allowed type pair.  The exact support test is repeated at every RHS on
 // the current positions, so the list only has to be a superset of the pairs of

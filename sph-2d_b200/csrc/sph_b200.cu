@@ -73,12 +73,13 @@ struct sph_handle {
     Sorted<double> D64{};
     Sorted<float> D32{};
     bool mixed = false;
-    // sort
-    unsigned *keys_in = nullptr, *keys_out = nullptr, *vals_in = nullptr, *vals_out = nullptr;
-    void* cub_tmp = nullptr;
+    // set-up (images, counting sort)
+    SetupBuf B{};
+    HostBox* box = nullptr;         // page-locked, mapped
+    HostBox* d_box = nullptr;       // its device address
+    unsigned box_seq = 0;
+    void* cub_tmp = nullptr;        // pair-offset scan
     size_t cub_bytes = 0;
-    int key_bits = 0;
-    unsigned dead_key = 0;
     int ncells = 0;
     // misc device buffers
     unsigned* d_status = nullptr;
@@ -356,18 +357,17 @@ int unsort(sph_handle* h) {
     return SPH_OK;
 }
 
-// One exclusive scan of cnt[0..n) into off, returning the total on the host.
-int scan_total(sph_handle* h, const int* cnt, int* off, int n, int* total) {
-    if (n <= 0) { *total = 0; return SPH_OK; }
-    size_t bytes = 0;
-    CK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, cnt, off, n, h->stream));
-    if (bytes > h->cub_bytes) return SPH_E_CAPACITY;
-    CK(cub::DeviceScan::ExclusiveSum(h->cub_tmp, bytes, cnt, off, n, h->stream));
-    int last[2];
-    CK(cudaMemcpyAsync(&last[0], off + n - 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(&last[1], cnt + n - 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    *total = last[0] + last[1];
+// Wait for the image totals of set-up number seq (k_img_count writes them to
+// mapped memory while the kernels behind it run).  The stream is queried now and
+// then, so a failed launch ends the wait.
+int wait_totals(sph_handle* h, unsigned seq) {
+    for (unsigned spin = 1; h->box->seq != seq; ++spin) {
+        if ((spin & 0xfff) != 0) continue;
+        const cudaError_t e = cudaStreamQuery(h->stream);
+        if (e == cudaErrorNotReady) continue;
+        CK(e);
+        if (h->box->seq != seq) return SPH_E_CUDA;      // everything queued has run without it
+    }
     return SPH_OK;
 }
 
@@ -378,47 +378,33 @@ int prepare(sph_handle* h) {
     if (rc) return rc;
     Params& P = h->P;
     P.n_host = h->n_host;
+    Sorted<R>& D = sorted<R>(h);
+    const SetupBuf& B = h->B;
     tic(h, PH_IMAGES);
+    const int nhb = blocks(h->n_host, kImgThreads), ncb = blocks(h->ncells + 1, kScanCells);
+    const int periodic = h->cfg.periodic ? 1 : 0;
+    if (periodic) k_img_count<<<nhb, kImgThreads, 0, h->stream>>>(P, h->S, B, h->d_box, ++h->box_seq);
+    else CK(cudaMemsetAsync(B.cnt, 0, sizeof(int) * (size_t)(h->ncells + 1), h->stream));
+    // (the routing of image adjoints is kept once an adjoint run exists)
+    k_img_emit<<<nhb, kImgThreads, 0, h->stream>>>(P, h->S, B, h->cap_tot, periodic, h->adj != nullptr, h->d_status);
+    tic(h, PH_SORT);
+    k_cell_scan<<<ncb, kScanThreads, 0, h->stream>>>(B);
+    CK(cudaGetLastError());
     int n_img = 0;
-    if (h->cfg.periodic) {
-        // left/right images of the host particles; the counts and offsets are
-        // kept for routing image adjoints back to their sources
-        k_img_count<<<blocks(h->n_host, 256), 256, 0, h->stream>>>(P, h->S, h->n_host, 0, h->S.lr_cnt);
-        int n_lr = 0;
-        rc = scan_total(h, h->S.lr_cnt, h->S.lr_off, h->n_host, &n_lr);
-        if (rc) return rc;
-        if (h->n_host + n_lr > h->cap_tot) return SPH_E_CAPACITY;
-        k_img_emit<<<blocks(h->n_host, 256), 256, 0, h->stream>>>(P, h->S, h->n_host, 0, h->n_host, h->S.lr_off);
-        // bottom/top images of host particles and left/right images
-        const int n_src = h->n_host + n_lr;
-        k_img_count<<<blocks(n_src, 256), 256, 0, h->stream>>>(P, h->S, n_src, 1, h->S.tb_cnt);
-        int n_tb = 0;
-        rc = scan_total(h, h->S.tb_cnt, h->S.tb_off, n_src, &n_tb);
-        if (rc) return rc;
-        if (n_src + n_tb > h->cap_tot) return SPH_E_CAPACITY;
-        k_img_emit<<<blocks(n_src, 256), 256, 0, h->stream>>>(P, h->S, n_src, 1, n_src, h->S.tb_off);
+    if (periodic) {
+        if ((rc = wait_totals(h, h->box_seq))) return rc;
+        const int n_lr = h->box->tot[0];
+        n_img = n_lr + h->box->tot[1] + h->box->tot[2];
+        if ((long long)h->n_host + n_img > h->cap_tot) return SPH_E_CAPACITY;
         h->n_lr = n_lr;
-        n_img = n_lr + n_tb;
-        CK(cudaGetLastError());
     }
     h->n_img = n_img;
-    h->launches += h->cfg.periodic ? 4 : 0;
     P.n_tot = h->n_host + n_img;
-    tic(h, PH_SORT);
-    Sorted<R>& D = sorted<R>(h);
-    k_cell_keys<<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, h->S.pos, h->S.type, h->keys_in, h->vals_in,
-                                                              h->d_status, h->dead_key);
-    size_t bytes = h->cub_bytes;
-    CK(cub::DeviceRadixSort::SortPairs(h->cub_tmp, bytes, h->keys_in, h->keys_out, h->vals_in, h->vals_out,
-                                       P.n_tot, 0, h->key_bits, h->stream));
-    k_gather_sorted<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, h->S, D, h->vals_out);
-    CK(cudaMemsetAsync(D.cell_start, 0xff, sizeof(int) * (size_t)h->ncells, h->stream));
-    CK(cudaMemsetAsync(D.cell_end, 0xff, sizeof(int) * (size_t)h->ncells, h->stream));
-    k_cell_ranges<<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P.n_tot, h->keys_out, D.cell_start, D.cell_end,
-                                                                h->dead_key);
+    k_place<<<blocks(std::max(P.n_tot, h->ncells), 256), 256, 0, h->stream>>>(P.n_tot, B, D.cell_start, D.cell_end);
+    k_gather_sorted<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, h->S, D, B);
     k_build_lists<R><<<blocks(P.n_tot, 128), 128, 0, h->stream>>>(P, D, h->d_status);
     CK(cudaGetLastError());
-    h->launches += 4;
+    h->launches += periodic ? 6 : 5;
     h->sorted_valid = true;
     h->staging_valid = false;   // the master state now lives in the sorted arrays
     return SPH_OK;
@@ -1697,7 +1683,8 @@ void destroy(sph_handle* h) {
     if (h->adj) { adj_free_all(h->adj); delete h->adj; }
     void* ptrs[] = {h->S.pos, h->S.vel, h->S.rho, h->S.mass, h->S.smass, h->S.type, h->S.itype, h->S.blabel, h->d_bf,
                     h->S.r_drho, h->S.r_acc,
-                    h->S.r_avg, h->S.cnt, h->S.off, h->S.lr_cnt, h->S.lr_off, h->S.tb_cnt, h->S.tb_off, h->keys_in, h->keys_out, h->vals_in, h->vals_out, h->cub_tmp,
+                    h->S.r_avg, h->S.lr_cnt, h->S.lr_off, h->S.tb_cnt, h->S.tb_off, h->B.blk, h->B.tot, h->B.done, h->B.key, h->B.rank,
+                    h->B.cnt, h->B.pre, h->B.blkoff, h->B.perm, h->cub_tmp,
                     h->d_status, h->d_int, h->d_part, h->d_diag, h->d_xfer, h->d_export, h->d_off64, h->d_cnt_id,
                     h->d_mls, h->d_ghost_ids};
     for (void* p : ptrs) if (p) cudaFree(p);
@@ -1706,6 +1693,7 @@ void destroy(sph_handle* h) {
     if (h->snap_ready) cudaEventDestroy(h->snap_ready);
     if (h->snap_done) cudaEventDestroy(h->snap_done);
     if (h->d_snap) cudaFree(h->d_snap);
+    if (h->box) cudaFreeHost(h->box);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }
@@ -1731,9 +1719,6 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     h->cap_tot = h->cap_host + h->cap_img;
     const int cap = h->cap_tot;
     h->ncells = h->P.gnx * h->P.gny;
-    h->key_bits = 1;
-    while ((1LL << h->key_bits) <= (long long)h->ncells) h->key_bits++;
-    h->dead_key = (unsigned)((1ULL << h->key_bits) - 1);
     h->P.nbr_stride = cap;
     CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
@@ -1746,20 +1731,24 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     CK(dalloc(&h->S.blabel, cap)); CK(cudaMemset(h->S.blabel, 0, sizeof(int) * (size_t)cap));
     CK(dalloc(&h->d_bf, (size_t)6 * blocks(cap, kRedThreads) + 6));
     CK(dalloc(&h->S.r_drho, h->cap_host)); CK(dalloc(&h->S.r_acc, h->cap_host)); CK(dalloc(&h->S.r_avg, h->cap_host));
-    CK(dalloc(&h->S.cnt, cap)); CK(dalloc(&h->S.off, cap));
     CK(dalloc(&h->S.lr_cnt, cap)); CK(dalloc(&h->S.lr_off, cap));
     CK(dalloc(&h->S.tb_cnt, cap)); CK(dalloc(&h->S.tb_off, cap));
-    // sort
-    CK(dalloc(&h->keys_in, cap)); CK(dalloc(&h->keys_out, cap));
-    CK(dalloc(&h->vals_in, cap)); CK(dalloc(&h->vals_out, cap));
+    // set-up
+    SetupBuf& B = h->B;
+    B.ncells = h->ncells;
+    CK(dalloc(&B.blk, blocks(h->cap_host, kImgThreads))); CK(dalloc(&B.tot, 3)); CK(dalloc(&B.done, 2));
+    CK(cudaMemsetAsync(B.done, 0, 2 * sizeof(unsigned), h->stream));
+    CK(dalloc(&B.key, cap)); CK(dalloc(&B.rank, cap)); CK(dalloc(&B.perm, cap));
+    CK(dalloc(&B.cnt, (size_t)h->ncells + 1)); CK(dalloc(&B.pre, (size_t)h->ncells + 1));
+    CK(dalloc(&B.blkoff, blocks((long long)h->ncells + 1, kScanCells)));
+    CK(cudaHostAlloc((void**)&h->box, sizeof(HostBox), cudaHostAllocMapped));
+    memset((void*)h->box, 0, sizeof(HostBox));
+    CK(cudaHostGetDevicePointer((void**)&h->d_box, h->box, 0));
     {
-        size_t b1 = 0, b2 = 0, b3 = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, b1, h->keys_in, h->keys_out, h->vals_in, h->vals_out, cap, 0,
-                                        h->key_bits, h->stream);
-        cub::DeviceScan::ExclusiveSum(nullptr, b2, h->S.cnt, h->S.off, cap, h->stream);
+        size_t b3 = 0;
         long long* dummy = nullptr;
         cub::DeviceScan::ExclusiveSum(nullptr, b3, dummy, dummy, cap, h->stream);
-        h->cub_bytes = std::max(b1, std::max(b2, b3)) + 1024;
+        h->cub_bytes = b3 + 1024;
         CK(cudaMalloc(&h->cub_tmp, h->cub_bytes));
     }
     CK(dalloc(&h->d_status, 1)); CK(cudaMemset(h->d_status, 0, sizeof(unsigned)));

@@ -55,6 +55,7 @@ struct Params {
     int gnx, gny;
     // sizes
     int n_host, n_tot, max_nbr, nbr_stride;
+    int rhs_gen;             // number of the RHS being evaluated (see Sorted::surf_gen)
     double skin_half2;       // (skin/2)^2: allowed squared displacement since the list build
 };
 

@@ -18,6 +18,49 @@
 
 namespace sph {
 
+// Geometric free-surface test of a candidate (Define_freesurface...f90:295-376):
+// normal n = -B^-1 sum(grad W V)/|.|; the candidate is interior as soon as one
+// water neighbour j satisfies  |x_j-x_i| >= 1.414h and |x_j - (x_i + h n)| < h,
+// or |x_j-x_i| < 1.414h and acos(n.(x_j-x_i)/|x_j-x_i|) <= pi/4.
+// Both criteria only accept j within 2h <= support, so the pair list covers them.
+// Pass A calls it for its own particle, whose pair list it has just written.
+template <typename R>
+__device__ __noinline__ bool surface_test(const Params& P, const Sorted<R>& D, int a, int nn, typename VT<R>::V4 bi) {
+    const double2 xa = D.pos[a];
+    // sum_dwdx (:155-156) recomputed here (candidates are rare)
+    double s0 = 0.0, s1 = 0.0;
+    for (int e = 0; e < nn; ++e) {
+        const int b = (int)(D.pairs[(size_t)e * P.nbr_stride + a] & 0x7fffffffu);
+        const double2 xb = D.pos[b];
+        double dx = xa.x - xb.x, dy = xa.y - xb.y, d;
+        if (!in_support(P, dx, dy, d)) continue;
+        double w, gx, gy;
+        kernel_w_dw<double>(P, d, dx, dy, w, gx, gy);
+        const double Vb = (double)D.aux[b].y;
+        s0 += gx * Vb; s1 += gy * Vb;
+    }
+    double n0 = (double)bi.x * s0 + (double)bi.y * s1;
+    double n1 = (double)bi.z * s0 + (double)bi.w * s1;
+    const double len = sqrt(n0 * n0 + n1 * n1);
+    if (isnan(len) || len == 0.0) return false;
+    n0 = -n0 / len; n1 = -n1 / len;
+    const double h = P.h;
+    const double vx = xa.x + h * n0, vy = xa.y + h * n1;
+    for (int e = 0; e < nn; ++e) {
+        const int b = (int)(D.pairs[(size_t)e * P.nbr_stride + a] & 0x7fffffffu);
+        if (D.type[b] != SPH_TYPE_WATER) continue;
+        const double2 xb = D.pos[b];
+        double p0 = xb.x - xa.x, p1 = xb.y - xa.y;
+        double ji = sqrt(p0 * p0 + p1 * p1);
+        double nd = n0 * p0 + n1 * p1;
+        double q0 = xb.x - vx, q1 = xb.y - vy;
+        double jt = sqrt(q0 * q0 + q1 * q1);
+        if (ji >= P.c1414 * h && jt < h) return false;
+        if (ji < P.c1414 * h && acos(nd / ji) <= (P.pi / 4.0)) return false;
+    }
+    return true;
+}
+
 // HLREC: in the mixed path, read the hi/lo float records (position, u, v, rho, p)
 // instead of the FP64 ones and form the pair differences in FP32 from them
 // (see store_split); the adjoint, which runs this pass on stored stage states
@@ -46,7 +89,7 @@ namespace sph {
 #endif
 template <typename R, bool HLREC, bool MS>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_BLOCKS : SPH_PASS_A_F32_BLOCKS) : (MS ? 4 : 5))
-    k_pass_a(Params P, Sorted<R> D) {
+    k_pass_a(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D) {
     using V4 = typename VT<R>::V4;
     constexpr bool F32 = sizeof(R) == 4;
     constexpr bool HL = HLREC && F32;
@@ -227,7 +270,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
     const R fv = fra;
     D.fra_v[a] = fv;
     uint8_t fl = 0;
-    if (P.free_surface && ta == SPH_TYPE_WATER && (double)fv <= P.fs_thr) fl = 4;   // surface candidate (:123)
+    if (P.free_surface && ta == SPH_TYPE_WATER && (double)fv <= P.fs_thr) {   // surface candidate (:123)
+        fl = 4;
+        if (surface_test<R>(P, D, a, np, mk4<R>(m00, m01, m10, m11))) {
+            fl |= 1;
+            *D.surf_gen = P.rhs_gen;            // every writer stores the same value
+        }
+    }
     D.flags[a] = fl;
     if (MS) D.avg[a] = mk2<R>(xs0, xs1);
 }
@@ -238,65 +287,14 @@ void launch_pass_a(const Params& P, const Sorted<R>& D, int nb, cudaStream_t st)
     else k_pass_a<R, HLREC, false><<<nb, 128, 0, st>>>(P, D);
 }
 
-// Geometric free-surface test of the candidates (Define_freesurface...f90:295-376):
-// normal n = -B^-1 sum(grad W V)/|.|; the candidate is interior as soon as one
-// water neighbour j satisfies  |x_j-x_i| >= 1.414h and |x_j - (x_i + h n)| < h,
-// or |x_j-x_i| < 1.414h and acos(n.(x_j-x_i)/|x_j-x_i|) <= pi/4.
-// Both criteria only accept j within 2h <= support, so the list covers them.
-template <typename R>
-// Grid-stride over the particles: candidates are rare, so most threads only
-// read a flag byte, and a grid of 148 x 8 blocks does that with little block
-// scheduling.
-__global__ void k_surface(Params P, Sorted<R> D) {
-    using V4 = typename VT<R>::V4;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < P.n_tot; a += gridDim.x * blockDim.x) {
-    uint8_t fl = D.flags[a];
-    if (!(fl & 4)) continue;
-    const int nn = D.npairs[a];
-    const double2 xa = D.pos[a];
-    // sum_dwdx (:155-156) recomputed here (candidates are rare)
-    double s0 = 0.0, s1 = 0.0;
-    for (int e = 0; e < nn; ++e) {
-        const int b = (int)(D.pairs[(size_t)e * P.nbr_stride + a] & 0x7fffffffu);
-        const double2 xb = D.pos[b];
-        double dx = xa.x - xb.x, dy = xa.y - xb.y, d;
-        if (!in_support(P, dx, dy, d)) continue;
-        double w, gx, gy;
-        kernel_w_dw<double>(P, d, dx, dy, w, gx, gy);
-        const double Vb = (double)D.aux[b].y;
-        s0 += gx * Vb; s1 += gy * Vb;
-    }
-    const V4 bi = D.binv[a];
-    double n0 = (double)bi.x * s0 + (double)bi.y * s1;
-    double n1 = (double)bi.z * s0 + (double)bi.w * s1;
-    double len = sqrt(n0 * n0 + n1 * n1);
-    bool surface = true;
-    if (isnan(len) || len == 0.0) surface = false;
-    else {
-        n0 = -n0 / len; n1 = -n1 / len;
-        const double h = P.h;
-        const double vx = xa.x + h * n0, vy = xa.y + h * n1;
-        for (int e = 0; e < nn && surface; ++e) {
-            const int b = (int)(D.pairs[(size_t)e * P.nbr_stride + a] & 0x7fffffffu);
-            if (D.type[b] != SPH_TYPE_WATER) continue;
-            const double2 xb = D.pos[b];
-            double p0 = xb.x - xa.x, p1 = xb.y - xa.y;
-            double ji = sqrt(p0 * p0 + p1 * p1);
-            double nd = n0 * p0 + n1 * p1;
-            double q0 = xb.x - vx, q1 = xb.y - vy;
-            double jt = sqrt(q0 * q0 + q1 * q1);
-            if (ji >= P.c1414 * h && jt < h) surface = false;
-            else if (ji < P.c1414 * h && acos(nd / ji) <= (P.pi / 4.0)) surface = false;
-        }
-    }
-    D.flags[a] = surface ? (uint8_t)(fl | 1) : (uint8_t)(fl & ~1);
-    }
-}
-
 // Near-free-surface flags (Define_freesurface...f90:418-440): every pair
 // neighbour of a surface particle.  Idempotent byte stores, no atomics needed.
+// The forward's pass C marks its own particle instead (near_surface); this pass
+// serves the adjoint, which re-runs pass A without pass C.  Grid-stride: most
+// RHS have no surface particle and every thread returns at once.
 template <typename R>
 __global__ void k_near(Params P, Sorted<R> D) {
+    if (*D.surf_gen != P.rhs_gen) return;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < P.n_tot; a += gridDim.x * blockDim.x) {
         if (!(D.flags[a] & 1)) continue;
         const int nn = D.npairs[a];
@@ -307,16 +305,12 @@ __global__ void k_near(Params P, Sorted<R> D) {
     }
 }
 
-// The free-surface test and the near-surface flags of one RHS.
 template <typename R>
-void launch_surface(const Params& P, const Sorted<R>& D, cudaStream_t st) {
-    // without free-surface detection pass A marks no candidate, so both kernels
-    // would only read flags
-    if (!P.free_surface) return;
+void launch_near(const Params& P, const Sorted<R>& D, cudaStream_t st) {
+    if (!P.free_surface) return;          // pass A marks no surface particle then
     int nb = (P.n_tot + 127) / 128;
     if (nb > 148 * 8) nb = 148 * 8;
     if (nb == 0) return;
-    k_surface<R><<<nb, 128, 0, st>>>(P, D);
     k_near<R><<<nb, 128, 0, st>>>(P, D);
 }
 

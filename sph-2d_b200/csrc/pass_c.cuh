@@ -104,6 +104,21 @@ __device__ __forceinline__ R quot(R a, R b) { return a / b; }
 __device__ __forceinline__ double fast_quot(double a, double b) { return a * rcp64(b); }
 __device__ __forceinline__ float fast_quot(float a, float b) { return __fdividef(a, b); }
 
+// Is a near the free surface (Define_freesurface...f90:418-440: a pair neighbour
+// is a surface particle)?  The pair lists are symmetric, so a's own list decides;
+// they are only searched at an RHS where pass A found a surface particle.  The
+// mark (bit 1) is kept for the shift and for the host; the other threads read
+// only bit 0, which this store does not change.
+template <typename R>
+__device__ __forceinline__ bool near_surface(const Params& P, const Sorted<R>& D, int a, int nn) {
+    if (!P.free_surface || *D.surf_gen != P.rhs_gen) return false;
+    bool near = false;
+    for (int e = 0; e < nn && !near; ++e)
+        near = (D.flags[D.pairs[(size_t)e * P.nbr_stride + a] & 0x7fffffffu] & 1) != 0;
+    if (near) D.flags[a] = D.flags[a] | 2;
+    return near;
+}
+
 // Per-particle state a thread needs for one side of a pair.
 template <typename R>
 struct Side {
@@ -129,6 +144,12 @@ struct Side {
 #define SPH_PASS_C_F32_BLOCKS 4
 #endif
 //
+// The stage that follows the RHS is applied here (StageArgs), on the particle's
+// own sums: a stage pass of its own read back the rates and the whole state and
+// ran at HBM speed while this kernel leaves HBM at a tenth of its rate.  2048^2,
+// ms per step, pass C + update: mixed 2.77 + 1.18 -> 3.06 + 0.45, FP64
+// 5.48 + 0.85 -> 6.24; 401^2 mixed 140 + 81 -> 158 + 27 us.
+//
 // FP64 at 2048^2 (MUSCL, ms per step of three launches): 7.30 with correctly
 // rounded square roots, reciprocals and quotients and the limiter's and frame's
 // 64-bit selects; 6.02 with rsqrt64 / rcp64, m_b/rho_b read as V_b, the
@@ -139,7 +160,7 @@ struct Side {
 // records per neighbour), 58 % issue-active.
 template <typename R, bool MUSCL, bool MS, bool SHIFT>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIFT_BLOCKS : SPH_PASS_C_F32_BLOCKS) : 3)
-    k_pass_c(Params P, Sorted<R> D) {
+    k_pass_c(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D, const __grid_constant__ StageArgs G) {
     using V4 = typename VT<R>::V4;
     using A = typename Acc<R>::T;
     constexpr bool F32 = sizeof(R) == 4;
@@ -168,7 +189,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
     // pressure terms (:333-374) are the pair-mean (v-bar, P-bar) form the Riemann
     // solvers use near the free surface, so it takes that branch for every pair
     const bool dsph = !MUSCL && !MS && P.dsph;
-    const bool near_a = dsph || (D.flags[a] & 2) != 0;
+    const bool near_a = near_surface(P, D, a, nn) || dsph;
     // delta-SPH and the assembly only apply to integrated particles (Solver :627-635,
     // Moving_Square.../Single_step_compute.f90:273-281)
     const bool water = integrated(P, ta);
@@ -548,14 +569,46 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         }
     }
     // assembly (single_step_compute.f90:152-171, Solver :627-635)
-    D.drho[a] = cont.val();
-    D.acc[a] = water ? mk2<R>(accx.val(), accy.val()) : mk2<R>(R(0), R(0));
-    if (!MS) D.avg[a] = mk2<R>(xsx, xsy);
+    const R drho_a = (R)cont.val();
+    const typename VT<R>::V2 acc_a = water ? mk2<R>((R)accx.val(), (R)accy.val()) : mk2<R>(R(0), R(0));
+    double2 sh = make_double2(0.0, 0.0);
     if (SHIFT) {
         const double4 b64 = D.binv64[a];
         const double c = -P.shift_beta * (P.h * P.h);
-        D.shift[a] = make_double2(c * (b64.x * shx + b64.y * shy), c * (b64.z * shx + b64.w * shy));
+        sh = make_double2(c * (b64.x * shx + b64.y * shy), c * (b64.z * shx + b64.w * shy));
     }
+    const typename VT<R>::V2 avg_o = MS ? avg_a : mk2<R>(xsx, xsy);
+    if (G.mode == STAGE_NONE) {
+        D.drho[a] = drho_a;
+        D.acc[a] = acc_a;
+        if (!MS) D.avg[a] = avg_o;
+        if (SHIFT) D.shift[a] = sh;
+        return;
+    }
+    // the stage that follows this RHS, on a alone: a middle stage writes the other
+    // copy of the records (the neighbours still read this one; particles that are
+    // not integrated are copied), the last one the master state
+    const double dr = (double)drho_a, ax = (double)acc_a.x, ay = (double)acc_a.y, gx = (double)avg_o.x,
+                 gy = (double)avg_o.y;
+    if (!water) {
+        if (G.mode == STAGE_MID) {
+            D.pos_n[a] = D.pos[a]; D.kin_n[a] = D.kin[a]; D.aux_n[a] = D.aux[a];
+            if (F32) { D.vol64_n[a] = D.vol64[a]; D.kh_n[a] = D.kh[a]; D.kl_n[a] = D.kl[a]; D.xhl_n[a] = D.xhl[a]; }
+        }
+        return;
+    }
+    const double2 x0 = D.pos0[a], v0 = D.vel0[a];
+    const double r0 = D.rho0[a];
+    double x, y, u, v, rho;
+    stage_update<R>(D, a, G.stage, G.dt, x0, v0, r0, dr, ax, ay, gx, gy, x, y, u, v, rho);
+    check_skin(P, x0, x, y, G.status);
+    if (G.mode == STAGE_MID) {
+        store_records<R>(P, D, a, make_double2(x, y), u, v, rho, D.mass[a], D.smass[a], true);
+        return;
+    }
+    if (SHIFT && ta == SPH_TYPE_WATER && !(D.flags[a] & 2))
+        shift_by(P, sh, grad_scale<R>() * S.nb1.w, grad_scale<R>() * S.nb2.x, x, y, rho);
+    store_end<R>(P, D, G.S, a, x, y, u, v, rho, dr, ax, ay, gx, gy, G.to_staging, G.status);
 }
 
 // The particle shifting sum of the mixed Taylor-Green path as a gather of its
@@ -565,18 +618,21 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
 // sum inside mixed pass C holds its FP64 values at pass C's register bound and
 // stalls on their loads; here it runs at full occupancy.  Particles the shift
 // does not move (not water, or near the free surface) get 0.  12 blocks of 128
-// per SM (40 registers, 24 B spilled): 0.32 -> 0.29 ms per step at 2048^2
-// against 44 registers at 11 blocks; at 16 blocks (32 registers, 48 B
-// spilled) it was slower.
+// per SM (40 registers): 0.32 -> 0.29 ms per step at 2048^2 against 44 registers
+// at 11 blocks; at 16 blocks (32 registers, 48 B spilled) it was slower.  With
+// the step's last stage behind the sum (StageArgs) 0.45 ms, against 0.29 and 0.30
+// for two passes; 10 blocks 0.49, 8 blocks without spills 0.57.
 template <typename R>
-__global__ void __launch_bounds__(128, 12) k_shift_gather(Params P, Sorted<R> D) {
+__global__ void __launch_bounds__(128, 12) k_shift_gather(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D,
+                                                        const __grid_constant__ StageArgs G) {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
-    if (D.type[a] != SPH_TYPE_WATER || (D.flags[a] & 2)) {
+    const bool moves = D.type[a] == SPH_TYPE_WATER && !(D.flags[a] & 2);
+    if (!moves && G.mode == STAGE_NONE) {
         D.shift[a] = make_double2(0.0, 0.0);
         return;
     }
-    const int nn = D.npairs[a];
+    const int nn = moves ? D.npairs[a] : 0;
     const double2 xa = D.pos[a];
     const double inv_h64 = P.inv_h, inv_h2_64 = P.inv_h2, inv_wdx = 1.0 / P.w_dx;
     double shx = 0.0, shy = 0.0;
@@ -629,7 +685,19 @@ __global__ void __launch_bounds__(128, 12) k_shift_gather(Params P, Sorted<R> D)
     }
     const double4 b64 = D.binv64[a];
     const double c = -P.shift_beta * (P.h * P.h);
-    D.shift[a] = make_double2(c * (b64.x * shx + b64.y * shy), c * (b64.z * shx + b64.w * shy));
+    const double2 sh = make_double2(c * (b64.x * shx + b64.y * shy), c * (b64.z * shx + b64.w * shy));
+    if (G.mode == STAGE_NONE) { D.shift[a] = sh; return; }
+    // the step's last stage (STAGE_END): it writes only a's own master state, so the
+    // positions the other threads are reading stay as they are
+    if (!integrated(P, D.type[a])) return;
+    const typename VT<R>::V2 ac = D.acc[a], av = D.avg[a];
+    const double dr = (double)D.drho[a], ax = (double)ac.x, ay = (double)ac.y, gx = (double)av.x, gy = (double)av.y;
+    const double2 x0 = D.pos0[a];
+    double x, y, u, v, rho;
+    stage_update<R>(D, a, G.stage, G.dt, x0, D.vel0[a], D.rho0[a], dr, ax, ay, gx, gy, x, y, u, v, rho);
+    check_skin(P, x0, x, y, G.status);
+    if (moves) shift_by(P, sh, grad_scale<R>() * D.nb1[a].w, grad_scale<R>() * D.nb2[a].x, x, y, rho);
+    store_end<R>(P, D, G.S, a, x, y, u, v, rho, dr, ax, ay, gx, gy, G.to_staging, G.status);
 }
 
 }  // namespace sph

@@ -377,7 +377,26 @@ struct Sorted {
     float4* kh;       // u, v, rho, p  (hi)
     float4* kl;       //               (lo)
     float4* xhl;      // x hi, y hi, x lo, y lo
+    float2* xh0;      // (float) of the list-build position
+    // the other copy of what a stage writes (position and records): pass C forms
+    // the next stage's state there while its neighbours still read this one
+    double2* pos_n;
+    double4* kin_n;
+    V4* aux_n;
+    double* vol64_n;
+    float4* kh_n;
+    float4* kl_n;
+    float4* xhl_n;
+    int* surf_gen;    // [1] Params::rhs_gen of the last RHS with a surface particle
 };
+
+// The sorted arrays with the two copies exchanged.
+template <typename R>
+inline void swap_stage_state(Sorted<R>& D) {
+    auto sw = [](auto& x, auto& y) { auto t = x; x = y; y = t; };
+    sw(D.pos, D.pos_n); sw(D.kin, D.kin_n); sw(D.aux, D.aux_n); sw(D.vol64, D.vol64_n);
+    sw(D.kh, D.kh_n); sw(D.kl, D.kl_n); sw(D.xhl, D.xhl_n);
+}
 
 // Factor from the stored gradient records (nb1.w, nb2, nb3.xyz) to the
 // gradients: the FP32 records hold 1/2 grad phi (pass C uses only that).
@@ -385,23 +404,178 @@ template <typename R>
 __host__ __device__ constexpr double grad_scale() { return sizeof(R) == 4 ? 2.0 : 1.0; }
 
 // Hi/lo split of the records a particle's pass-C neighbours read (mixed path).
+__device__ __forceinline__ void split_to(float4* kh, float4* kl, float4* xhl, int s, double2 x, double4 k) {
+    const float uh = (float)k.x, vh = (float)k.y, rh = (float)k.z, ph = (float)k.w;
+    kh[s] = make_float4(uh, vh, rh, ph);
+    kl[s] = make_float4((float)(k.x - (double)uh), (float)(k.y - (double)vh), (float)(k.z - (double)rh),
+                        (float)(k.w - (double)ph));
+    const float xh = (float)x.x, yh = (float)x.y;
+    xhl[s] = make_float4(xh, yh, (float)(x.x - (double)xh), (float)(x.y - (double)yh));
+}
 template <typename R>
 __device__ __forceinline__ void store_split(Sorted<R>& D, int s, double2 x, double4 k) {
     if (sizeof(R) != 4) return;
     D.vol64[s] = D.mass[s] / k.z;
-    const float uh = (float)k.x, vh = (float)k.y, rh = (float)k.z, ph = (float)k.w;
-    D.kh[s] = make_float4(uh, vh, rh, ph);
-    D.kl[s] = make_float4((float)(k.x - (double)uh), (float)(k.y - (double)vh), (float)(k.z - (double)rh),
-                          (float)(k.w - (double)ph));
-    const float xh = (float)x.x, yh = (float)x.y;
-    D.xhl[s] = make_float4(xh, yh, (float)(x.x - (double)xh), (float)(x.y - (double)yh));
+    split_to(D.kh, D.kl, D.xhl, s, x, k);
+}
+
+// The records of a state (x, v, rho) with mass m and SPS mass sm; next: into the
+// other copy.
+template <typename R>
+__device__ __forceinline__ void store_records(const Params& P, const Sorted<R>& D, int s, double2 x, double u, double v,
+                                              double rho, double m, double sm, bool next) {
+    double p, c;
+    eos64(P, rho, p, c);
+    const double4 k = make_double4(u, v, rho, p);
+    (next ? D.pos_n : D.pos)[s] = x;
+    (next ? D.kin_n : D.kin)[s] = k;
+    (next ? D.aux_n : D.aux)[s] = mk4<R>((R)m, (R)(m / rho), (R)c, (R)sm);
+    if (sizeof(R) == 4) {
+        (next ? D.vol64_n : D.vol64)[s] = m / rho;
+        if (next) split_to(D.kh_n, D.kl_n, D.xhl_n, s, x, k);
+        else split_to(D.kh, D.kl, D.xhl, s, x, k);
+    }
+}
+
+// Runge-Kutta stages of time_iteration.f90 (water particles only; images and
+// boundary particles keep their step-start state, as the reference only
+// updates type 2 at :944, :978, :1008, :1038):
+//   stage 0  rho = rho0 + drhodt*dt/2, v = v0 + 0.5 dt a + avg, x = x0 + 0.5 dt v    K = K1
+//   stage 1  same with the second RHS                                          K += 2 K2
+//   stage 2  full dt with the third RHS                                        K += 2 K3
+//   stage 3  rho = rho0 + (K + drhodt) dt/6, v = v0 + (K_a + a) dt/6 + avg,
+//            x = x0 + (K_v + v) dt/6 + 0.5 dt^2 a; then Shift_particle_position.
+// Stage 0 uses the rates carried from the previous step (K1 reuse, :940-965)
+// unless this is the first step, when a fresh RHS precedes it (:821).
+//
+// With SPH_INTEGRATOR_EULER_PC (Moving_Square.../SPH_Time_Iteration.f90:304-334) the
+// stages are 10 (predictor) and 11 (corrector):
+//   predictor  rho = rho0 + drhodt dt, x = x0 + dt (v0 + avg) + 0.5 a dt^2, v = v0 + dt a
+//   corrector  rho = rho0 + 0.5 (drhodt + drhodt_p) dt,
+//              x = x0 + 0.5 dt (v_p + v0) + avg dt + 0.5 a dt^2, v = v0 + 0.5 dt (a + a_p)
+//
+// The state a stage takes particle s to from the step-start state (x0, v0, r0)
+// with the rates (dr, a, g), and the sums and carried rates it leaves.
+template <typename R>
+__device__ __forceinline__ void stage_update(const Sorted<R>& D, int s, int stage, double dt, double2 x0, double2 v0,
+                                             double r0, double dr, double ax, double ay, double gx, double gy, double& x,
+                                             double& y, double& u, double& v, double& rho) {
+    using V2 = typename VT<R>::V2;
+    if (stage == 10) {
+        rho = r0 + dr * dt;
+        x = x0.x + dt * (v0.x + gx) + 0.5 * ax * (dt * dt);
+        y = x0.y + dt * (v0.y + gy) + 0.5 * ay * (dt * dt);
+        u = v0.x + dt * ax;
+        v = v0.y + dt * ay;
+        D.ks_r[s] = (R)dr;
+        D.ks_a[s] = mk2<R>((R)ax, (R)ay);
+        D.ks_v[s] = v0;
+    } else if (stage == 11) {
+        const double4 kp = D.kin[s];          // predicted velocity
+        const V2 ka = D.ks_a[s];
+        const double2 kv = D.ks_v[s];
+        rho = r0 + 0.5 * (dr + (double)D.ks_r[s]) * dt;
+        x = x0.x + 0.5 * dt * (kp.x + kv.x) + gx * dt + 0.5 * ax * (dt * dt);
+        y = x0.y + 0.5 * dt * (kp.y + kv.y) + gy * dt + 0.5 * ay * (dt * dt);
+        u = v0.x + 0.5 * dt * (ax + (double)ka.x);
+        v = v0.y + 0.5 * dt * (ay + (double)ka.y);
+    } else if (stage < 3) {
+        const double f = stage < 2 ? 0.5 * dt : dt;
+        rho = stage < 2 ? r0 + dr * dt / 2 : r0 + dr * dt;
+        u = v0.x + f * ax + gx;
+        x = x0.x + f * u;
+        v = v0.y + f * ay + gy;
+        y = x0.y + f * v;
+        if (stage == 0) {
+            D.ks_r[s] = (R)dr;
+            D.ks_a[s] = mk2<R>((R)ax, (R)ay);
+            D.ks_v[s] = make_double2(u, v);
+        } else {
+            D.ks_r[s] = D.ks_r[s] + R(2) * (R)dr;
+            V2 ka = D.ks_a[s];
+            double2 kv = D.ks_v[s];
+            D.ks_a[s] = mk2<R>(ka.x + R(2) * (R)ax, ka.y + R(2) * (R)ay);
+            D.ks_v[s] = make_double2(kv.x + 2 * u, kv.y + 2 * v);
+        }
+    } else {
+        const V2 ka = D.ks_a[s];
+        const double2 kv = D.ks_v[s];
+        rho = r0 + ((double)D.ks_r[s] + dr) * dt / 6.0;
+        u = v0.x + ((double)ka.x + ax) * dt / 6.0 + gx;
+        x = x0.x + ((double)kv.x + u) * dt / 6.0 + 0.5 * dt * dt * ax;
+        v = v0.y + ((double)ka.y + ay) * dt / 6.0 + gy;
+        y = x0.y + ((double)kv.y + v) * dt / 6.0 + 0.5 * dt * dt * ay;
+    }
+    if (stage == 3 || stage == 11) {
+        // rates of this last RHS become next step's K1
+        D.c_drho[s] = (R)dr;
+        D.c_acc[s] = mk2<R>((R)ax, (R)ay);
+        D.c_avg[s] = mk2<R>((R)gx, (R)gy);
+    }
+}
+
+// What a kernel needs to apply the stage that follows it to its own particle.
+struct StageArgs {
+    int mode;             // STAGE_NONE, STAGE_MID (into the other copy), STAGE_END
+    int stage;
+    double dt;
+    int shift;            // STAGE_END: apply the step's shift
+    int to_staging;       // STAGE_END: also write the id-order state
+    unsigned* status;
+    Staging S;
+};
+enum { STAGE_NONE = 0, STAGE_MID = 1, STAGE_END = 2 };
+
+// the neighbour lists stay exact while nobody moved more than half the skin
+__device__ __forceinline__ void check_skin(const Params& P, double2 x0, double x, double y, unsigned* status) {
+    const double ddx = x - x0.x, ddy = y - x0.y;
+    if (ddx * ddx + ddy * ddy > P.skin_half2) atomicOr(status, ST_SKIN);
+}
+
+// The end of a step for particle s: the new master state, and (to_staging) the
+// new state and carried rates of a host particle in the id-order arrays, exactly
+// what k_unsort would copy there, so the next step's set-up and a state read
+// need no unsort pass (static fields are unchanged in staging).
+template <typename R>
+__device__ __forceinline__ void store_end(const Params& P, const Sorted<R>& D, const Staging& S, int s, double x, double y,
+                                          double u, double v, double rho, double dr, double ax, double ay, double gx,
+                                          double gy, int to_staging, unsigned* status) {
+    if (!(isfinite(x) && isfinite(y) && isfinite(u) && isfinite(v) && isfinite(rho))) atomicOr(status, ST_NONFINITE);
+    D.pos0[s] = make_double2(x, y);
+    D.vel0[s] = make_double2(u, v);
+    D.rho0[s] = rho;
+    if (to_staging) {
+        const int i = D.id[s];
+        if (i < P.n_host) {
+            S.pos[i] = make_double2(x, y);
+            S.vel[i] = make_double2(u, v);
+            S.rho[i] = rho;
+            // the carried rates as k_unsort reads them back (rounded to R)
+            S.r_drho[i] = (double)(R)dr;
+            S.r_acc[i] = make_double2((double)(R)ax, (double)(R)ay);
+            S.r_avg[i] = make_double2((double)(R)gx, (double)(R)gy);
+        }
+    }
+}
+
+// The capped shift (Shift_particle_position.f90:108-131) of a water particle not
+// near the free surface: displacement sh, density gradient (g0, g1).
+__device__ __forceinline__ void shift_by(const Params& P, double2 sh, double g0, double g1, double& x, double& y,
+                                         double& rho) {
+    double s0 = sh.x, s1 = sh.y;
+    const double amp = sqrt(s0 * s0 + s1 * s1);
+    if (amp > P.shift_max) { s0 = s0 / amp * P.shift_max; s1 = s1 / amp * P.shift_max; }
+    x = x + s0;
+    y = y + s1;
+    rho = rho + g0 * s0;
+    rho = rho + g1 * s1;
 }
 
 // --- 4. gather the id-ordered arrays into cell order -----------------------
 // Thread t holds the particle at place t; its slot is the cell's start plus the
 // number of lower ids in the cell (about 8 reads that the warp shares).
 template <typename R>
-__global__ void k_gather_sorted(Params P, Staging S, Sorted<R> D, SetupBuf B) {
+__global__ void k_gather_sorted(Params P, Staging S, Sorted<R> D, SetupBuf B, StageArgs G) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.n_tot) return;
     const int i = (int)B.perm[t];
@@ -414,33 +588,41 @@ __global__ void k_gather_sorted(Params P, Staging S, Sorted<R> D, SetupBuf B) {
     }
     D.id[s] = i;
     D.slot_of[i] = s;
-    D.type[s] = S.type[i];
+    const int ty = S.type[i];
+    D.type[s] = ty;
     D.itype[s] = S.itype[i];
     D.blabel[s] = i < P.n_host ? S.blabel[i] : 0;
-    double2 x = S.pos[i];
-    D.pos[s] = x;
+    const double2 x = S.pos[i];
     D.pos0[s] = x;
+    if (sizeof(R) == 4) D.xh0[s] = make_float2((float)x.x, (float)x.y);
     const double2 v = S.vel[i];
     const double rho = S.rho[i], m = S.mass[i], sm = S.smass[i];
     D.vel0[s] = v;
     D.rho0[s] = rho;
     D.mass[s] = m;
     D.smass[s] = sm;
-    // neighbour records of the step-start state (formed here from the values
-    // just gathered, instead of a second pass over the sorted arrays)
-    double p, c;
-    eos64(P, rho, p, c);
-    D.kin[s] = make_double4(v.x, v.y, rho, p);
-    D.aux[s] = mk4<R>((R)m, (R)(m / rho), (R)c, (R)sm);
-    store_split(D, s, x, make_double4(v.x, v.y, rho, p));
-    if (i < P.n_host) {
-        D.c_drho[s] = (R)S.r_drho[i];
-        D.c_acc[s] = mk2<R>((R)S.r_acc[i].x, (R)S.r_acc[i].y);
-        D.c_avg[s] = mk2<R>((R)S.r_avg[i].x, (R)S.r_avg[i].y);
+    double dr = 0.0;
+    double2 a = make_double2(0.0, 0.0), g = a;
+    if (i < P.n_host) { dr = (double)(R)S.r_drho[i]; a = S.r_acc[i]; g = S.r_avg[i]; }
+    a = make_double2((double)(R)a.x, (double)(R)a.y);
+    g = make_double2((double)(R)g.x, (double)(R)g.y);
+    if (G.mode == STAGE_MID) {
+        // the step's first stage with the carried rates, on the values just read
+        // (c_* are next written by the step's end)
+        double2 xn = x;
+        double u = v.x, w = v.y, r = rho;
+        if (integrated(P, ty)) {
+            stage_update<R>(D, s, G.stage, G.dt, x, v, rho, dr, a.x, a.y, g.x, g.y, xn.x, xn.y, u, w, r);
+            check_skin(P, x, xn.x, xn.y, G.status);
+        }
+        store_records<R>(P, D, s, xn, u, w, r, m, sm, false);
     } else {
-        D.c_drho[s] = R(0);
-        D.c_acc[s] = mk2<R>(R(0), R(0));
-        D.c_avg[s] = mk2<R>(R(0), R(0));
+        store_records<R>(P, D, s, x, v.x, v.y, rho, m, sm, false);
+    }
+    if (G.mode != STAGE_MID || !integrated(P, ty)) {
+        D.c_drho[s] = (R)dr;
+        D.c_acc[s] = mk2<R>((R)a.x, (R)a.y);
+        D.c_avg[s] = mk2<R>((R)g.x, (R)g.y);
     }
 }
 
@@ -496,13 +678,13 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
         else if (cnt < P.max_nbr) D.nbr[(size_t)cnt * P.nbr_stride + a] = v;
         ++cnt;
     };
-    // the mixed path tests the FP32 hi positions against the widened radius
+    // the mixed path tests the positions rounded to FP32 against the widened radius
     // r2_list32 (a superset of the FP64 list, see derive_params)
     constexpr bool F32 = sizeof(R) == 4;
-    const float2* xh = reinterpret_cast<const float2*>(D.xhl);     // (x hi, y hi) at 2 s
+    const float2* xh = D.xh0;
     if (ta != SPH_TYPE_ILL && ta != 0) {
-        double2 xa = D.pos[a];
-        const float2 xa_h = F32 ? xh[2 * (size_t)a] : make_float2(0.f, 0.f);
+        double2 xa = D.pos0[a];
+        const float2 xa_h = F32 ? xh[a] : make_float2(0.f, 0.f);
         int ida = D.id[a];
         int cx = (int)floor((xa.x - P.gx0) / P.cs), cy = (int)floor((xa.y - P.gy0) / P.cs);
         int x0 = max(cx - 1, 0), x1 = min(cx + 1, P.gnx - 1);
@@ -528,8 +710,8 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
                 int tb[4], ib[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    if (F32) xbh[k] = __ldg(&xh[2 * (size_t)(b + k)]);
-                    else xb[k] = __ldg(&D.pos[b + k]);
+                    if (F32) xbh[k] = __ldg(&xh[b + k]);
+                    else xb[k] = __ldg(&D.pos0[b + k]);
                     ib[k] = __ldg(&D.id[b + k]);
                     tb[k] = check_type ? __ldg(&D.type[b + k]) : 0;
                 }
@@ -551,11 +733,11 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
                 if (b == a) continue;
                 if (check_type && !pair_allowed(P.pair_rule, ta, D.type[b])) continue;
                 if (F32) {
-                    const float2 xbh = xh[2 * (size_t)b];
+                    const float2 xbh = xh[b];
                     const float dx = xa_h.x - xbh.x, dy = xa_h.y - xbh.y;
                     if (dx * dx + dy * dy > P.r2_list32) continue;
                 } else {
-                    const double2 xb = D.pos[b];
+                    const double2 xb = D.pos0[b];
                     const double dx = xa.x - xb.x, dy = xa.y - xb.y;
                     if (dx * dx + dy * dy > P.r2_list) continue;
                 }

@@ -8,9 +8,10 @@
 // Per time step (time_iteration.f90:781-1073):
 //   prepare: periodic wrap + images (id order), cell keys, radix sort,
 //            cell ranges, neighbour lists with a skin, neighbour records
-//   RHS    : pass A (renormalisation, gradients, SPS) -> surface test ->
-//            near-surface flags -> pass C (fused forces)
-//   stages : k_stage 0..3, shifting fused into the last stage
+//   RHS    : pass A (renormalisation, gradients, SPS, surface test) -> pass C
+//            (near-surface flags, fused forces)
+//   stages : the first in the gather, the others in the kernel that ends each
+//            RHS (pass C, or the mixed path's shifting gather at the step's end)
 #include <cuda_runtime.h>
 #include <cub/cub.cuh>
 
@@ -326,8 +327,12 @@ int alloc_sorted(Sorted<R>& D, int cap, int max_nbr, int ncells) {
     CK(dalloc(&D.nbr, (size_t)cap * max_nbr)); CK(dalloc(&D.nnbr, cap));
     CK(dalloc(&D.pairs, (size_t)cap * max_nbr)); CK(dalloc(&D.npairs, cap));
     CK(dalloc(&D.cell_start, ncells)); CK(dalloc(&D.cell_end, ncells));
+    CK(dalloc(&D.pos_n, cap)); CK(dalloc(&D.kin_n, cap)); CK(dalloc(&D.aux_n, cap));
+    CK(dalloc(&D.surf_gen, 1)); CK(cudaMemset(D.surf_gen, 0, sizeof(int)));
     if (sizeof(R) == 4) {
         CK(dalloc(&D.kh, cap)); CK(dalloc(&D.kl, cap)); CK(dalloc(&D.xhl, cap)); CK(dalloc(&D.vol64, cap));
+        CK(dalloc(&D.kh_n, cap)); CK(dalloc(&D.kl_n, cap)); CK(dalloc(&D.xhl_n, cap)); CK(dalloc(&D.vol64_n, cap));
+        CK(dalloc(&D.xh0, cap));
     }
     CK(cudaMemset(D.nb3, 0, sizeof(*D.nb3) * (size_t)cap));
     CK(cudaMemset(D.flags, 0, (size_t)cap));
@@ -339,7 +344,8 @@ void free_sorted(Sorted<R>& D) {
     void* ptrs[] = {D.id, D.type, D.itype, D.blabel, D.pos, D.pos0, D.vel0, D.rho0, D.mass, D.smass, D.kin, D.aux, D.nb1, D.nb2, D.nb3,
                     D.binv, D.binv64, D.fra_v, D.flags, D.drho, D.acc, D.avg, D.shift, D.ks_r, D.ks_a, D.ks_v, D.c_drho,
                     D.c_acc, D.c_avg, D.nbr, D.nnbr, D.pairs, D.npairs, D.cell_start, D.cell_end, D.kh, D.kl,
-                    D.xhl, D.vol64, D.slot_of, D.nflag};
+                    D.xhl, D.vol64, D.slot_of, D.nflag, D.pos_n, D.kin_n, D.aux_n, D.vol64_n, D.kh_n, D.kl_n, D.xhl_n, D.xh0,
+                    D.surf_gen};
     for (void* p : ptrs) if (p) cudaFree(p);
     D = Sorted<R>{};
 }
@@ -372,8 +378,10 @@ int wait_totals(sph_handle* h, unsigned seq) {
 }
 
 // Step-start set-up: wrap + periodic images, sort, cell ranges, lists, records.
+// first: the step's first stage, applied to the carried rates by the gather
+// (mode STAGE_MID), or none.
 template <typename R>
-int prepare(sph_handle* h) {
+int prepare(sph_handle* h, const StageArgs& first = StageArgs{}) {
     int rc = unsort<R>(h);
     if (rc) return rc;
     Params& P = h->P;
@@ -401,7 +409,7 @@ int prepare(sph_handle* h) {
     h->n_img = n_img;
     P.n_tot = h->n_host + n_img;
     k_place<<<blocks(std::max(P.n_tot, h->ncells), 256), 256, 0, h->stream>>>(P.n_tot, B, D.cell_start, D.cell_end);
-    k_gather_sorted<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, h->S, D, B);
+    k_gather_sorted<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, h->S, D, B, first);
     k_build_lists<R><<<blocks(P.n_tot, 128), 128, 0, h->stream>>>(P, D, h->d_status);
     CK(cudaGetLastError());
     h->launches += periodic ? 6 : 5;
@@ -413,11 +421,42 @@ int prepare(sph_handle* h) {
 template <typename R>
 int keep_stage(sph_handle* h, int j, int k);
 
-// One RHS evaluation on the current stage state.  keep_j >= 0 (the adjoint's
-// segment re-run): the ghost interpolation sums go to gint / gsw and the state
-// after the ghost assignment to stage slot keep_j.
+StageArgs stage_args(sph_handle* h, int mode, int stage, double dt, int shift = 0, int to_staging = 0) {
+    StageArgs g{};
+    g.mode = mode; g.stage = stage; g.dt = dt; g.shift = shift; g.to_staging = to_staging;
+    g.status = h->d_status;
+    g.S = h->S;
+    return g;
+}
+
 template <typename R>
-int rhs(sph_handle* h, int last, int keep_j = -1, double4* gint = nullptr, double* gsw = nullptr) {
+void launch_pass_c(const Params& P, const Sorted<R>& D, const StageArgs& G, bool shift, int nb, cudaStream_t st) {
+    if (P.ms) {
+        if (shift) k_pass_c<R, false, true, true><<<nb, 128, 0, st>>>(P, D, G);
+        else k_pass_c<R, false, true, false><<<nb, 128, 0, st>>>(P, D, G);
+        return;
+    }
+    // (the mixed Taylor-Green launches never carry the shifting sum)
+    if constexpr (sizeof(R) == 8) {
+        if (shift) {
+            if (P.muscl) k_pass_c<R, true, false, true><<<nb, 128, 0, st>>>(P, D, G);
+            else k_pass_c<R, false, false, true><<<nb, 128, 0, st>>>(P, D, G);
+            return;
+        }
+    }
+    if (P.muscl) k_pass_c<R, true, false, false><<<nb, 128, 0, st>>>(P, D, G);
+    else k_pass_c<R, false, false, false><<<nb, 128, 0, st>>>(P, D, G);
+}
+
+// One RHS evaluation on the current stage state.  G: the stage that follows it,
+// applied by its last kernel (STAGE_MID leaves the new state in the other copy
+// of the records, which becomes the current one), or none.  keep_j >= 0 (the
+// adjoint's segment re-run): the ghost interpolation sums go to gint / gsw and
+// the state after the ghost assignment to stage slot keep_j.
+template <typename R>
+int rhs(sph_handle* h, int last, const StageArgs& G = StageArgs{}, int keep_j = -1, double4* gint = nullptr,
+        double* gsw = nullptr) {
+    ++h->P.rhs_gen;
     const Params& P = h->P;
     Sorted<R>& D = sorted<R>(h);
     const int nb = blocks(P.n_tot, 128);
@@ -437,40 +476,20 @@ int rhs(sph_handle* h, int last, int keep_j = -1, double4* gint = nullptr, doubl
     }
     tic(h, PH_A);
     launch_pass_a<R, true>(P, D, nb, h->stream);
-    tic(h, PH_SURF);
-    launch_surface<R>(P, D, h->stream);
     tic(h, PH_C);
     // the mixed Taylor-Green path forms the shifting sum in k_shift_gather after
     // pass C; the FP64 and moving-square launches form it inside pass C
     const bool sep = sizeof(R) == 4 && !P.ms;
     const bool sh = last && h->cfg.shifting;
-    const bool shc = sh && !sep;
-    if (P.ms) {
-        if (shc) k_pass_c<R, false, true, true><<<nb, 128, 0, h->stream>>>(P, D);
-        else k_pass_c<R, false, true, false><<<nb, 128, 0, h->stream>>>(P, D);
-    } else if (P.muscl) {
-        if constexpr (sizeof(R) == 8) {       // the mixed launches never carry the sum
-            if (shc) k_pass_c<R, true, false, true><<<nb, 128, 0, h->stream>>>(P, D);
-            else k_pass_c<R, true, false, false><<<nb, 128, 0, h->stream>>>(P, D);
-        } else {
-            k_pass_c<R, true, false, false><<<nb, 128, 0, h->stream>>>(P, D);
-        }
-    } else {
-        if constexpr (sizeof(R) == 8) {
-            if (shc) k_pass_c<R, false, false, true><<<nb, 128, 0, h->stream>>>(P, D);
-            else k_pass_c<R, false, false, false><<<nb, 128, 0, h->stream>>>(P, D);
-        } else {
-            k_pass_c<R, false, false, false><<<nb, 128, 0, h->stream>>>(P, D);
-        }
-    }
+    launch_pass_c<R>(P, D, sh && sep ? StageArgs{} : G, sh && !sep, nb, h->stream);
     if constexpr (sizeof(R) == 4) if (sh && sep) {
         // timed with the update: shifting is part of the step's second pass
         tic(h, PH_UPDATE);
-        k_shift_gather<R><<<nb, 128, 0, h->stream>>>(P, D);
+        k_shift_gather<R><<<nb, 128, 0, h->stream>>>(P, D, G);
         h->launches += 1;
     }
     CK(cudaGetLastError());
-    h->launches += P.free_surface ? 4 : 2;
+    h->launches += 2;
     if (P.has_body && (last || h->bf_every_rhs)) {
         const int nbf = blocks(P.n_tot, kRedThreads);      // <= blocks(cap_tot), the partial buffer size
         double* fin = h->d_bf + (size_t)6 * blocks(h->cap_tot, kRedThreads);
@@ -483,17 +502,18 @@ int rhs(sph_handle* h, int last, int keep_j = -1, double4* gint = nullptr, doubl
             h->launches += 1;
         }
     }
+    if (G.mode == STAGE_MID) swap_stage_state(D);
     h->n_rhs++;
     h->have_rhs = true;
     return SPH_OK;
 }
 
 template <typename R>
-int stage(sph_handle* h, int st, double dt, int use_carried, int do_shift, int to_staging = 0) {
+int stage(sph_handle* h, int st, double dt, int use_carried, int do_shift) {
     const Params& P = h->P;
     tic(h, PH_UPDATE);
     k_stage<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, sorted<R>(h), st, dt, use_carried, do_shift,
-                                                             h->d_status, h->S, to_staging);
+                                                             h->d_status);
     CK(cudaGetLastError());
     h->launches += 1;
     return SPH_OK;
@@ -566,35 +586,31 @@ int run_steps(sph_handle* h, int nsteps, double dt) {
     for (int s = 0; s < nsteps; ++s) {
         int rc = step_begin<R>(h, dt);
         if (rc) return rc;
-        rc = prepare<R>(h);
-        if (rc) return rc;
-        const int first = h->step_count == 0;
+        const bool first = h->step_count == 0;
+        const bool pc = h->cfg.integrator == SPH_INTEGRATOR_EULER_PC;
+        const int st0 = pc ? 10 : 0, stn = pc ? 11 : 3;
         // density re-initialisation after every mls_every-th step (1-based step number)
         const bool mls = h->P.mls_order != 0 && (h->step_count + 1) % h->P.mls_every == 0;
-        const int shift_now = mls ? 0 : h->cfg.shifting;
-        // the Taylor-Green driver's final stage keeps the id-order staging current
-        // (the moving-square ghost assignment and MLS change the sorted state
-        // after or outside it)
-        const int to_staging = (!h->P.ms && !h->P.ghost_assign && !mls) ? 1 : 0;
-        if (first) { rc = rhs<R>(h, 0); if (rc) return rc; }
         const bool mls1 = mls && h->P.mls_order == 1;
-        if (h->cfg.integrator == SPH_INTEGRATOR_EULER_PC) {
-            rc = stage<R>(h, 10, dt, first ? 0 : 1, 0); if (rc) return rc;
-            rc = rhs<R>(h, 1); if (rc) return rc;
-            if (mls1 && (rc = mls1_on_last_rhs<R>(h))) return rc;
-            rc = stage<R>(h, 11, dt, 0, shift_now); if (rc) return rc;
+        // the first stage: by the gather on the carried rates, or after a fresh RHS
+        if ((rc = prepare<R>(h, first ? StageArgs{} : stage_args(h, STAGE_MID, st0, dt)))) return rc;
+        if (first && ((rc = rhs<R>(h, 0)) || (rc = stage<R>(h, st0, dt, 0, 0)))) return rc;
+        if (!pc)
+            for (int k = 1; k < 3; ++k)
+                if ((rc = rhs<R>(h, 0, stage_args(h, STAGE_MID, k, dt)))) return rc;
+        if (mls) {
+            // the re-initialisation works on the state after the last stage (order 1:
+            // on the last RHS), before the shift
+            if ((rc = rhs<R>(h, 1)) || (mls1 && (rc = mls1_on_last_rhs<R>(h))) || (rc = stage<R>(h, stn, dt, 0, 0)) ||
+                (rc = reinit_density<R>(h, h->cfg.shifting)))
+                return rc;
         } else {
-            rc = stage<R>(h, 0, dt, first ? 0 : 1, 0); if (rc) return rc;
-            rc = rhs<R>(h, 0); if (rc) return rc;
-            rc = stage<R>(h, 1, dt, 0, 0); if (rc) return rc;
-            rc = rhs<R>(h, 0); if (rc) return rc;
-            rc = stage<R>(h, 2, dt, 0, 0); if (rc) return rc;
-            rc = rhs<R>(h, 1); if (rc) return rc;
-            if (mls1 && (rc = mls1_on_last_rhs<R>(h))) return rc;
-            rc = stage<R>(h, 3, dt, 0, shift_now, to_staging); if (rc) return rc;
+            // the Taylor-Green driver's final stage keeps the id-order staging current
+            // (the moving-square ghost assignment changes the sorted state outside it)
+            const int to_staging = (!pc && !h->P.ms && !h->P.ghost_assign) ? 1 : 0;
+            if ((rc = rhs<R>(h, 1, stage_args(h, STAGE_END, stn, dt, h->cfg.shifting, to_staging)))) return rc;
             if (to_staging) h->staging_valid = true;
         }
-        if (mls && (rc = reinit_density<R>(h, h->cfg.shifting))) return rc;
         tic(h, -1);
         h->step_count++;
         h->n_steps++;
@@ -1190,7 +1206,7 @@ int step_keep(sph_handle* h, double dt, int j, bool full) {
             const size_t o = (size_t)j * X->cap_tot;
             {
                 PaSwap<R> sw(h, j);
-                if ((rc = rhs<R>(h, 1, j, X->pa_gint + o, X->pa_gsw + o)) ||
+                if ((rc = rhs<R>(h, 1, StageArgs{}, j, X->pa_gint + o, X->pa_gsw + o)) ||
                     (rc = stage<R>(h, 11, dt, 0, h->cfg.shifting)))
                     return rc;
             }
@@ -1249,6 +1265,7 @@ int step_keep(sph_handle* h, double dt, int j, bool full) {
 // from V's FP64 state first (the same records the forward's stage wrote).
 template <typename R>
 void adj_pass_a(sph_handle* h, const Sorted<R>& V) {
+    ++h->P.rhs_gen;
     const Params& P = h->P;
     const int nb = blocks(P.n_tot, 128);
     if constexpr (sizeof(R) == 4) {
@@ -1258,8 +1275,8 @@ void adj_pass_a(sph_handle* h, const Sorted<R>& V) {
     } else {
         launch_pass_a<R, false>(P, V, nb, h->stream);
     }
-    launch_surface<R>(P, V, h->stream);
-    h->launches += P.free_surface ? 3 : 1;
+    launch_near<R>(P, V, h->stream);
+    h->launches += P.free_surface ? 2 : 1;
 }
 
 // Reverse of one RHS evaluation on the stage state V, with the rate adjoints
@@ -1408,6 +1425,7 @@ int adj_step(sph_handle* h, bool first, int j) {
 // arrays refilled from what the segment re-run left.
 template <typename R>
 void adj_rhs_ms_values(sph_handle* h, const Sorted<R>& V, int kept_j) {
+    ++h->P.rhs_gen;
     const Params& P = h->P;
     AdjCtx* X = h->adj;
     const bool ghosts = P.ghost_assign && h->n_ghost > 0;
@@ -1426,7 +1444,7 @@ void adj_rhs_ms_values(sph_handle* h, const Sorted<R>& V, int kept_j) {
         h->launches += 1;
     }
     launch_pass_a<R, false>(P, V, blocks(P.n_tot, kAdjThreads), h->stream);
-    launch_surface<R>(P, V, h->stream);
+    launch_near<R>(P, V, h->stream);
 }
 
 // Reverse of one moving-square RHS evaluation on the state V with the rate

@@ -5,22 +5,6 @@
 
 namespace sph {
 
-// Runge-Kutta stages of time_iteration.f90 (water particles only; images and
-// boundary particles keep their step-start state, as the reference only
-// updates type 2 at :944, :978, :1008, :1038):
-//   stage 0  rho = rho0 + drhodt*dt/2, v = v0 + 0.5 dt a + avg, x = x0 + 0.5 dt v    K = K1
-//   stage 1  same with the second RHS                                          K += 2 K2
-//   stage 2  full dt with the third RHS                                        K += 2 K3
-//   stage 3  rho = rho0 + (K + drhodt) dt/6, v = v0 + (K_a + a) dt/6 + avg,
-//            x = x0 + (K_v + v) dt/6 + 0.5 dt^2 a; then Shift_particle_position.
-// Stage 0 uses the rates carried from the previous step (K1 reuse, :940-965)
-// unless this is the first step, when a fresh RHS precedes it (:821).
-//
-// With SPH_INTEGRATOR_EULER_PC (Moving_Square.../SPH_Time_Iteration.f90:304-334) the
-// stages are 10 (predictor) and 11 (corrector):
-//   predictor  rho = rho0 + drhodt dt, x = x0 + dt (v0 + avg) + 0.5 a dt^2, v = v0 + dt a
-//   corrector  rho = rho0 + 0.5 (drhodt + drhodt_p) dt,
-//              x = x0 + 0.5 dt (v_p + v0) + avg dt + 0.5 a dt^2, v = v0 + 0.5 dt (a + a_p)
 // Shift_particle_position.f90:108-131: the capped displacement of the last RHS's
 // shifting sum and the first-order density correction, for water particles
 // that are not near the free surface.
@@ -28,23 +12,16 @@ template <typename R>
 __device__ __forceinline__ void apply_shift(const Params& P, const Sorted<R>& D, int s, double& x, double& y,
                                             double& rho) {
     if (D.type[s] != SPH_TYPE_WATER || (D.flags[s] & 2)) return;
-    const double2 sh = D.shift[s];
-    double s0 = sh.x, s1 = sh.y;
-    const double amp = sqrt(s0 * s0 + s1 * s1);
-    if (amp > P.shift_max) { s0 = s0 / amp * P.shift_max; s1 = s1 / amp * P.shift_max; }
-    x = x + s0;
-    y = y + s1;
-    rho = rho + grad_scale<R>() * D.nb1[s].w * s0;
-    rho = rho + grad_scale<R>() * D.nb2[s].x * s1;
+    shift_by(P, D.shift[s], grad_scale<R>() * D.nb1[s].w, grad_scale<R>() * D.nb2[s].x, x, y, rho);
 }
 
+// A stage as a pass of its own: where the rates are not carried by the kernel
+// before it (the first step, a density re-initialisation, the adjoint's segment
+// re-run).  Elsewhere the first stage is applied by k_gather_sorted, the middle
+// ones and the last by k_pass_c or k_shift_gather (StageArgs).
 template <typename R>
-// to_staging (final stages of the Taylor-Green driver): also write the new
-// master state and carried rates of each host particle to the id-order staging
-// arrays, exactly what k_unsort would copy there, so the next step's set-up and
-// a state read need no unsort pass (static fields are unchanged in staging).
 __global__ void k_stage(Params P, Sorted<R> D, int stage, double dt, int use_carried, int do_shift,
-                        unsigned* status, Staging S, int to_staging) {
+                        unsigned* status) {
     using V2 = typename VT<R>::V2;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
@@ -61,90 +38,13 @@ __global__ void k_stage(Params P, Sorted<R> D, int stage, double dt, int use_car
         ax = (double)a.x; ay = (double)a.y; gx = (double)g.x; gy = (double)g.y;
     }
     double rho, u, v, x, y;
-    if (stage == 10) {
-        rho = r0 + dr * dt;
-        x = x0.x + dt * (v0.x + gx) + 0.5 * ax * (dt * dt);
-        y = x0.y + dt * (v0.y + gy) + 0.5 * ay * (dt * dt);
-        u = v0.x + dt * ax;
-        v = v0.y + dt * ay;
-        D.ks_r[s] = (R)dr;
-        D.ks_a[s] = mk2<R>((R)ax, (R)ay);
-        D.ks_v[s] = v0;
-    } else if (stage == 11) {
-        const double4 kp = D.kin[s];          // predicted velocity
-        const V2 ka = D.ks_a[s];
-        const double2 kv = D.ks_v[s];
-        rho = r0 + 0.5 * (dr + (double)D.ks_r[s]) * dt;
-        x = x0.x + 0.5 * dt * (kp.x + kv.x) + gx * dt + 0.5 * ax * (dt * dt);
-        y = x0.y + 0.5 * dt * (kp.y + kv.y) + gy * dt + 0.5 * ay * (dt * dt);
-        u = v0.x + 0.5 * dt * (ax + (double)ka.x);
-        v = v0.y + 0.5 * dt * (ay + (double)ka.y);
-        D.c_drho[s] = (R)dr;
-        D.c_acc[s] = mk2<R>((R)ax, (R)ay);
-        D.c_avg[s] = mk2<R>((R)gx, (R)gy);
-    } else if (stage < 3) {
-        const double f = stage < 2 ? 0.5 * dt : dt;
-        rho = stage < 2 ? r0 + dr * dt / 2 : r0 + dr * dt;
-        u = v0.x + f * ax + gx;
-        x = x0.x + f * u;
-        v = v0.y + f * ay + gy;
-        y = x0.y + f * v;
-        if (stage == 0) {
-            D.ks_r[s] = (R)dr;
-            D.ks_a[s] = mk2<R>((R)ax, (R)ay);
-            D.ks_v[s] = make_double2(u, v);
-        } else {
-            D.ks_r[s] = D.ks_r[s] + R(2) * (R)dr;
-            V2 ka = D.ks_a[s];
-            double2 kv = D.ks_v[s];
-            D.ks_a[s] = mk2<R>(ka.x + R(2) * (R)ax, ka.y + R(2) * (R)ay);
-            D.ks_v[s] = make_double2(kv.x + 2 * u, kv.y + 2 * v);
-        }
-    } else {
-        const V2 ka = D.ks_a[s];
-        const double2 kv = D.ks_v[s];
-        rho = r0 + ((double)D.ks_r[s] + dr) * dt / 6.0;
-        u = v0.x + ((double)ka.x + ax) * dt / 6.0 + gx;
-        x = x0.x + ((double)kv.x + u) * dt / 6.0 + 0.5 * dt * dt * ax;
-        v = v0.y + ((double)ka.y + ay) * dt / 6.0 + gy;
-        y = x0.y + ((double)kv.y + v) * dt / 6.0 + 0.5 * dt * dt * ay;
-        // rates of this last RHS become next step's K1
-        D.c_drho[s] = (R)dr;
-        D.c_acc[s] = mk2<R>((R)ax, (R)ay);
-        D.c_avg[s] = mk2<R>((R)gx, (R)gy);
-    }
-    // the neighbour lists stay exact while nobody moved more than half the skin
-    const double ddx = x - x0.x, ddy = y - x0.y;
-    if (ddx * ddx + ddy * ddy > P.skin_half2) atomicOr(status, ST_SKIN);
-    const bool final_stage = stage == 3 || stage == 11;
-    if (final_stage) {
+    stage_update<R>(D, s, stage, dt, x0, v0, r0, dr, ax, ay, gx, gy, x, y, u, v, rho);
+    check_skin(P, x0, x, y, status);
+    if (stage == 3 || stage == 11) {
         if (do_shift) apply_shift(P, D, s, x, y, rho);
-        if (!(isfinite(x) && isfinite(y) && isfinite(u) && isfinite(v) && isfinite(rho))) atomicOr(status, ST_NONFINITE);
-        D.pos0[s] = make_double2(x, y);
-        D.vel0[s] = make_double2(u, v);
-        D.rho0[s] = rho;
-        D.pos[s] = make_double2(x, y);
-        if (to_staging) {
-            const int i = D.id[s];
-            if (i < P.n_host) {
-                S.pos[i] = make_double2(x, y);
-                S.vel[i] = make_double2(u, v);
-                S.rho[i] = rho;
-                // the carried rates as k_unsort reads them back (rounded to R)
-                S.r_drho[i] = (double)(R)dr;
-                S.r_acc[i] = make_double2((double)(R)ax, (double)(R)ay);
-                S.r_avg[i] = make_double2((double)(R)gx, (double)(R)gy);
-            }
-        }
-    } else {
-        D.pos[s] = make_double2(x, y);
+        store_end<R>(P, D, Staging{}, s, x, y, u, v, rho, dr, ax, ay, gx, gy, 0, status);
     }
-    double p, c;
-    eos64(P, rho, p, c);
-    const double m = D.mass[s];
-    D.kin[s] = make_double4(u, v, rho, p);
-    D.aux[s] = mk4<R>((R)m, (R)(m / rho), (R)c, (R)D.smass[s]);
-    store_split(D, s, make_double2(x, y), make_double4(u, v, rho, p));
+    store_records<R>(P, D, s, make_double2(x, y), u, v, rho, D.mass[s], D.smass[s], false);
 }
 
 // Density re-initialisation by moving least squares (Reinitialize_particle_density:

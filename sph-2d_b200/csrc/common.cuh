@@ -147,6 +147,29 @@ __device__ __forceinline__ double4 load4(const double4* p) {
 }
 __device__ __forceinline__ float4 load4(const float4* p) { return *p; }
 
+// Lanes that share one particle in the neighbour loops (L = 1: a thread per
+// particle): the group's lanes take the list entries lane, lane + L, ... and add
+// their sums in a fixed butterfly order.
+template <int L>
+struct Lanes {
+    int lane;            // this thread's place in its group
+    unsigned below;      // the lanes of the group before this one, as a warp mask
+    unsigned group;      // the group as a warp mask
+    __device__ __forceinline__ Lanes() {
+        const int l = threadIdx.x & 31;
+        lane = L == 1 ? 0 : l & (L - 1);
+        group = L == 32 ? 0xffffffffu : ((1u << (L & 31)) - 1u) << (l & ~(L - 1));
+        below = group & ((1u << l) - 1u);
+    }
+    // the particle of this thread
+    static __device__ __forceinline__ int particle() { return (int)((blockIdx.x * blockDim.x + threadIdx.x) / L); }
+    template <typename T>
+    __device__ __forceinline__ void sum(T& v) const {
+#pragma unroll
+        for (int o = 1; o < L; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+};
+
 // Plain accumulator for the FP64 path.
 struct DSum {
     double s;

@@ -87,17 +87,21 @@ __device__ __noinline__ bool surface_test(const Params& P, const Sorted<R>& D, i
 #ifndef SPH_PASS_A_F32_MS_BLOCKS
 #define SPH_PASS_A_F32_MS_BLOCKS 7
 #endif
-template <typename R, bool HLREC, bool MS>
+template <typename R, bool HLREC, bool MS, int L = 1>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_BLOCKS : SPH_PASS_A_F32_BLOCKS) : (MS ? 4 : 5))
     k_pass_a(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D) {
     using V4 = typename VT<R>::V4;
     constexpr bool F32 = sizeof(R) == 4;
     constexpr bool HL = HLREC && F32;
     constexpr bool LO = HL && MS;        // the lo parts of u, v, rho, p
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= P.n_tot) return;
+    const Lanes<L> ln;
+    const int t = Lanes<L>::particle();
+    const bool live = t < P.n_tot;
+    if (L == 1 && !live) return;
+    const int a = live ? t : P.n_tot - 1;        // (every lane takes part in the ballots)
     const int ta = D.type[a];
-    const int nn = D.nnbr[a];
+    const int nn = live ? D.nnbr[a] : 0;
+    const int most = L == 1 ? nn : __reduce_max_sync(0xffffffffu, nn);
     const double2 xa = HL ? make_double2(0.0, 0.0) : D.pos[a];
     const double4 ka = HL ? make_double4(0.0, 0.0, __ldg(&D.kin[a].z), 0.0) : D.kin[a];
     const float4 xa_hl = HL ? D.xhl[a] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -119,8 +123,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
     // two-deep software pipeline: the list entry two iterations ahead, the
     // neighbour's position and records (kin, volume) one iteration ahead, so the
     // loads of the next neighbour are in flight while this one is evaluated
-    unsigned ent_n = nn > 0 ? __ldg(&D.nbr[a]) : 0u;
-    unsigned ent_nn = nn > 1 ? __ldg(&D.nbr[(size_t)P.nbr_stride + a]) : 0u;
+    unsigned ent_n = nn > ln.lane ? __ldg(&D.nbr[(size_t)ln.lane * P.nbr_stride + a]) : 0u;
+    unsigned ent_nn = nn > ln.lane + L ? __ldg(&D.nbr[(size_t)(ln.lane + L) * P.nbr_stride + a]) : 0u;
     double2 xb_n = make_double2(0.0, 0.0);
     double4 kb_n = make_double4(0.0, 0.0, 0.0, 0.0);
     float4 xbhl_n = make_float4(0.f, 0.f, 0.f, 0.f), kbh_n = xbhl_n, kbl_n = xbhl_n;
@@ -130,34 +134,46 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
         else { xb_n = __ldg(&D.pos[bb]); kb_n = load4(&D.kin[bb]); }
         vb_n = D.aux[bb].y;
     };
-    if (nn > 0) fetch((int)(ent_n & 0x7fffffffu));
-    for (int e = 0; e < nn; ++e) {
+    if (nn > ln.lane) fetch((int)(ent_n & 0x7fffffffu));
+    for (int e0 = 0; e0 < most; e0 += L) {
+        const int e = e0 + ln.lane;
         const unsigned ent = ent_n;
         const int b = (int)(ent & 0x7fffffffu);
         const double2 xb = xb_n;
         const double4 kb = kb_n;
         const float4 xbhl = xbhl_n, kbh = kbh_n, kbl = kbl_n;
         const R Vb = vb_n;
-        if (e + 1 < nn) {
+        if (e + L < nn) {
             ent_n = ent_nn;
             fetch((int)(ent_n & 0x7fffffffu));
-            if (e + 2 < nn) ent_nn = __ldg(&D.nbr[(size_t)(e + 2) * P.nbr_stride + a]);
+            if (e + 2 * L < nn) ent_nn = __ldg(&D.nbr[(size_t)(e + 2 * L) * P.nbr_stride + a]);
         }
         const double dxd = HL ? 0.0 : xa.x - xb.x, dyd = HL ? 0.0 : xa.y - xb.y;
         const float dxf = HL ? (xa_hl.x - xbhl.x) + (xa_hl.z - xbhl.z) : 0.f;
         const float dyf = HL ? (xa_hl.y - xbhl.y) + (xa_hl.w - xbhl.w) : 0.f;
         R d = R(0), inv_d = R(0);
         double s2 = 0.0;                 // FP64: the squared distance
-        if (F32) {
-            const R s = HL ? (R)(dxf * dxf + dyf * dyf) : (R)(dxd * dxd + dyd * dyd);
-            if (!(s <= r2cut) || s < r2min) continue;
-            inv_d = rsqrtf(s);
-            d = s * inv_d;
+        if constexpr (L > 1) {
+            static_assert(!F32, "the lanes of a group would reorder FP32 sums");
+            // the pair list in the order of the neighbour list
+            const bool in = in_support_s2(P, dxd, dyd, s2) && e < nn;
+            const unsigned hit = __ballot_sync(0xffffffffu, in) & ln.group;
+            const int at = np + __popc(hit & ln.below);
+            np += __popc(hit);
+            if (!in) continue;
+            D.pairs[(size_t)at * P.nbr_stride + a] = ent;
         } else {
-            if (!in_support_s2(P, dxd, dyd, s2)) continue;
+            if (F32) {
+                const R s = HL ? (R)(dxf * dxf + dyf * dyf) : (R)(dxd * dxd + dyd * dyd);
+                if (!(s <= r2cut) || s < r2min) continue;
+                inv_d = rsqrtf(s);
+                d = s * inv_d;
+            } else {
+                if (!in_support_s2(P, dxd, dyd, s2)) continue;
+            }
+            D.pairs[(size_t)np * P.nbr_stride + a] = ent;
+            ++np;
         }
-        D.pairs[(size_t)np * P.nbr_stride + a] = ent;
-        ++np;
         const R dx = HL ? (R)dxf : (R)dxd, dy = HL ? (R)dyf : (R)dyd;
         // grad_a W = g(d) (x_a - x_b)  (compute_kernel)
         R gs, wk;
@@ -223,6 +239,15 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
         g[6] += dv * gx; g[7] += dv * gy;
         if (P.muscl) { g[2] += dp * gx; g[3] += dp * gy; }
     }
+    if constexpr (L > 1) {
+        ln.sum(fra); ln.sum(b00); ln.sum(b01); ln.sum(b10); ln.sum(b11);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) ln.sum(g[c]);
+        if (MS) { ln.sum(xs0); ln.sum(xs1); }
+        // the pairs the other lanes wrote are visible to lane 0 (surface_test)
+        __syncwarp();
+        if (!live || ln.lane != 0) return;
+    }
     D.npairs[a] = np;
     fra = fra * (R)(1.0 / P.sv);
     // inverse of the 2x2 tensor in FP64 (matrix_inversion_less_three,
@@ -281,10 +306,31 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
     if (MS) D.avg[a] = mk2<R>(xs0, xs1);
 }
 
+// Lanes per particle of the FP64 pair loops, by particle count.  A thread per
+// particle leaves SMs idle below one wave (148 SMs x 3 to 5 blocks of 128) and
+// each thread then runs a chain of 21 to 40 neighbours of FP64 latency; lanes cut
+// the chain but repeat the loop's head and end.  Measured per launch, us, 1 / 2 / 4
+// lanes, MUSCL Taylor-Green: pass A 14.9 / 12.4 / 10.5 at 11,000 particles,
+// 15.3 / 12.7 / 14.6 at 24,000, 16.8 / 14.5 / 16.7 at 42,000, 20.4 / 21.9 / 22.7 at
+// 68,000; pass C 28 / 20 / 17, 31 / 23 / 25, 37 / 36 / 35, 56 / 49 / 53, and
+// 65 / 68 / 79 at 105,000 (8 and 16 lanes slower from 11,000 on).  The mixed path
+// keeps one lane: its FP32 sums depend on their order.
+constexpr int kLanes4Below = 17000, kLanes2BelowA = 60000, kLanes2BelowC = 90000;
+
+template <typename R, bool HLREC, int L>
+void launch_pass_a_lanes(const Params& P, const Sorted<R>& D, cudaStream_t st) {
+    const int nb = (int)(((long long)P.n_tot * L + 127) / 128);
+    if (P.ms) k_pass_a<R, HLREC, true, L><<<nb, 128, 0, st>>>(P, D);
+    else k_pass_a<R, HLREC, false, L><<<nb, 128, 0, st>>>(P, D);
+}
+
 template <typename R, bool HLREC>
-void launch_pass_a(const Params& P, const Sorted<R>& D, int nb, cudaStream_t st) {
-    if (P.ms) k_pass_a<R, HLREC, true><<<nb, 128, 0, st>>>(P, D);
-    else k_pass_a<R, HLREC, false><<<nb, 128, 0, st>>>(P, D);
+void launch_pass_a(const Params& P, const Sorted<R>& D, cudaStream_t st) {
+    if constexpr (sizeof(R) == 8 && HLREC) {
+        if (P.n_tot < kLanes4Below) { launch_pass_a_lanes<R, HLREC, 4>(P, D, st); return; }
+        if (P.n_tot < kLanes2BelowA) { launch_pass_a_lanes<R, HLREC, 2>(P, D, st); return; }
+    }
+    launch_pass_a_lanes<R, HLREC, 1>(P, D, st);
 }
 
 // Near-free-surface flags (Define_freesurface...f90:418-440): every pair

@@ -158,7 +158,7 @@ struct Side {
 // blocks without the prefetch 5.89).  ncu at 1024^2, 398 -> 270 M warp
 // instructions, 654 -> 431 us: FP64 pipe 50 % busy, L1 data stage 67 % (176 B of
 // records per neighbour), 58 % issue-active.
-template <typename R, bool MUSCL, bool MS, bool SHIFT>
+template <typename R, bool MUSCL, bool MS, bool SHIFT, int L = 1>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIFT_BLOCKS : SPH_PASS_C_F32_BLOCKS) : 3)
     k_pass_c(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D, const __grid_constant__ StageArgs G) {
     using V4 = typename VT<R>::V4;
@@ -171,10 +171,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
     // neighbour's FP64 position (and FP64 volume) instead of its hi/lo position
     // and takes the FP32 difference as the rounding of the FP64 one
     constexpr bool X64 = !HL || SHIFT;
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= P.n_tot) return;
+    const Lanes<L> ln;
+    const int t = Lanes<L>::particle();
+    const bool live = t < P.n_tot;
+    if (L == 1 && !live) return;
+    const int a = live ? t : P.n_tot - 1;        // (every lane takes part in the sums)
     const int ta = D.type[a];
-    const int nn = D.npairs[a];
+    const int nn = live ? D.npairs[a] : 0;
     const double2 xa = X64 ? D.pos[a] : make_double2(0.0, 0.0);
     float4 xa_hl = make_float4(0.f, 0.f, 0.f, 0.f);
     Side<R> S;
@@ -219,10 +222,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
     const double inv_h64 = P.inv_h, inv_h2_64 = P.inv_h2, inv_wdx = 1.0 / P.w_dx;
 
     // the pairs pass A found inside the support at this RHS
-    unsigned ent_n = nn > 0 ? __ldg(&D.pairs[a]) : 0u;
+    unsigned ent_n = nn > ln.lane ? __ldg(&D.pairs[(size_t)ln.lane * P.nbr_stride + a]) : 0u;
     // software pipeline: the pair entry two iterations ahead; the neighbour's
     // position and its records one iteration ahead
-    unsigned ent_nn = nn > 1 ? __ldg(&D.pairs[(size_t)P.nbr_stride + a]) : 0u;
+    unsigned ent_nn = nn > ln.lane + L ? __ldg(&D.pairs[(size_t)(ln.lane + L) * P.nbr_stride + a]) : 0u;
     double2 xb_n = make_double2(0.0, 0.0);
     float4 xbhl_n = make_float4(0.f, 0.f, 0.f, 0.f);
     double vd_n = 0.0;                 // FP64 volume, mixed SHIFT launch
@@ -234,14 +237,14 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         t.aux = load4(&D.aux[bb]); t.nb1 = load4(&D.nb1[bb]); t.nb2 = load4(&D.nb2[bb]);
         if (MUSCL) t.nb3 = load4(&D.nb3[bb]);
     };
-    if (nn > 0) {
+    if (nn > ln.lane) {
         const int b0 = (int)(ent_n & 0x7fffffffu);
         if (X64) xb_n = __ldg(&D.pos[b0]);
         else xbhl_n = __ldg(&D.xhl[b0]);
         if (VPRE) vd_n = __ldg(&D.vol64[b0]);
         load_records(b0, T_n);
     }
-    for (int e = 0; e < nn; ++e) {
+    for (int e = ln.lane; e < nn; e += L) {
         const unsigned ent = ent_n;
         const int b = (int)(ent & 0x7fffffffu);
         const bool a_is_i = (ent >> 31) != 0;
@@ -249,14 +252,14 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         const float4 xbhl = xbhl_n;
         const double vd_b = vd_n;
         const Side<R> T = T_n;
-        if (e + 1 < nn) {
+        if (e + L < nn) {
             ent_n = ent_nn;
             const int b1 = (int)(ent_n & 0x7fffffffu);
             if (X64) xb_n = __ldg(&D.pos[b1]);
             else xbhl_n = __ldg(&D.xhl[b1]);
             if (VPRE) vd_n = __ldg(&D.vol64[b1]);
             load_records(b1, T_n);
-            if (e + 2 < nn) ent_nn = __ldg(&D.pairs[(size_t)(e + 2) * P.nbr_stride + a]);
+            if (e + 2 * L < nn) ent_nn = __ldg(&D.pairs[(size_t)(e + 2 * L) * P.nbr_stride + a]);
         }
         // x_a - x_b: FP64, or hi/lo in FP32 (the mixed SHIFT launch: the FP32
         // rounding of the FP64 difference, which its shifting sum needs)
@@ -567,6 +570,12 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
             shx += f * dxd;
             shy += f * dyd;
         }
+    }
+    if constexpr (L > 1) {
+        ln.sum(cont.s); ln.sum(accx.s); ln.sum(accy.s);
+        if (!MUSCL && !MS) { ln.sum(xsx); ln.sum(xsy); }
+        if (SHIFT) { ln.sum(shx); ln.sum(shy); }
+        if (!live || ln.lane != 0) return;
     }
     // assembly (single_step_compute.f90:152-171, Solver :627-635)
     const R drho_a = (R)cont.val();

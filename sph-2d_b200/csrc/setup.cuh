@@ -751,4 +751,90 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
     D.nnbr[a] = cnt;
 }
 
+// The same lists with L lanes per particle: the lanes split the candidates of the
+// three rows, taken as one range, and a ballot gives each accepted one its place,
+// so the entries come in the same order.  For particle counts that leave most of
+// the GPU idle with a thread per particle, whose ~74 (Wendland C2) to ~140
+// (Gaussian) candidates are then a chain of dependent loads.
+template <typename R, int L>
+__global__ void __launch_bounds__(128) k_build_lists_lanes(Params P, Sorted<R> D, unsigned* status) {
+    constexpr bool F32 = sizeof(R) == 4;
+    const Lanes<L> ln;
+    const int g = Lanes<L>::particle();
+    const bool live = g < P.n_tot;
+    const int a = live ? g : P.n_tot - 1;
+    const int ta = D.type[a];
+    const double2 xa = D.pos0[a];
+    const float2 xa_h = F32 ? D.xh0[a] : make_float2(0.f, 0.f);
+    const int ida = D.id[a];
+    int lo[3] = {0, 0, 0}, len[3] = {0, 0, 0};
+    if (live && ta != SPH_TYPE_ILL && ta != 0) {
+        const int cx = (int)floor((xa.x - P.gx0) / P.cs), cy = (int)floor((xa.y - P.gy0) / P.cs);
+        const int x0 = max(cx - 1, 0), x1 = min(cx + 1, P.gnx - 1);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            const int gy = cy - 1 + r;
+            if (gy < 0 || gy > P.gny - 1) continue;
+            int b0 = -1, b1 = -1;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int gx = x0 + k;
+                if (gx > x1) continue;
+                const int st = D.cell_start[gy * P.gnx + gx], en = D.cell_end[gy * P.gnx + gx];
+                if (st < 0) continue;
+                if (b0 < 0) b0 = st;
+                b1 = en;
+            }
+            lo[r] = b0;
+            len[r] = b1 - b0;
+        }
+    }
+    const bool check_type = !(P.pair_rule == SPH_PAIRS_ONE_FLUID && ta == SPH_TYPE_WATER);
+    const int l01 = len[0] + len[1], total = l01 + len[2];
+    const int most = __reduce_max_sync(0xffffffffu, total);
+    int cnt = 0;
+#pragma unroll 2
+    for (int t0 = 0; t0 < most; t0 += L) {
+        const int t = t0 + ln.lane;
+        bool in = false;
+        unsigned v = 0u;
+        if (t < total) {
+            const int b = t < len[0] ? lo[0] + t : t < l01 ? lo[1] + (t - len[0]) : lo[2] + (t - l01);
+            v = (unsigned)b | (ida < __ldg(&D.id[b]) ? 0x80000000u : 0u);
+            if (F32) {
+                const float2 xb = __ldg(&D.xh0[b]);
+                const float dx = xa_h.x - xb.x, dy = xa_h.y - xb.y;
+                in = !(dx * dx + dy * dy > P.r2_list32);
+            } else {
+                const double2 xb = __ldg(&D.pos0[b]);
+                const double dx = xa.x - xb.x, dy = xa.y - xb.y;
+                in = !(dx * dx + dy * dy > P.r2_list);
+            }
+            in = in && b != a && (!check_type || pair_allowed(P.pair_rule, ta, D.type[b]));
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, in) & ln.group;
+        const int e = cnt + __popc(hit & ln.below);
+        if (in && e < P.max_nbr) D.nbr[(size_t)e * P.nbr_stride + a] = v;
+        cnt += __popc(hit);
+    }
+    if (!live || ln.lane != 0) return;
+    if (cnt > P.max_nbr) { atomicOr(status, ST_NBR_OVERFLOW); cnt = P.max_nbr; }
+    D.nnbr[a] = cnt;
+}
+
+// Measured, sort + lists in us per step, thread per particle against 8 lanes
+// (4, 16 and 32 within 3 us of it or slower): 36 -> 28 at 11,000 particles (100^2
+// Taylor-Green with images), 40 -> 37 at 42,000, 59 -> 47 at 49,000 (square D/30,
+// Gaussian), but 40 -> 43 at 68,000 and 72 -> 82 at 131,000: the GPU is full there.
+constexpr int kListLanes = 8, kListLanesBelow = 60000;
+template <typename R>
+void launch_lists(const Params& P, const Sorted<R>& D, unsigned* status, cudaStream_t st) {
+    if (P.n_tot < kListLanesBelow) {
+        const long long t = (long long)P.n_tot * kListLanes;
+        k_build_lists_lanes<R, kListLanes><<<(unsigned)((t + 127) / 128), 128, 0, st>>>(P, D, status);
+    } else {
+        k_build_lists<R><<<(P.n_tot + 127) / 128, 128, 0, st>>>(P, D, status);
+    }
+}
+
 }  // namespace sph

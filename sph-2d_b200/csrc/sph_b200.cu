@@ -410,7 +410,7 @@ int prepare(sph_handle* h, const StageArgs& first = StageArgs{}) {
     P.n_tot = h->n_host + n_img;
     k_place<<<blocks(std::max(P.n_tot, h->ncells), 256), 256, 0, h->stream>>>(P.n_tot, B, D.cell_start, D.cell_end);
     k_gather_sorted<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, h->S, D, B, first);
-    k_build_lists<R><<<blocks(P.n_tot, 128), 128, 0, h->stream>>>(P, D, h->d_status);
+    launch_lists<R>(P, D, h->d_status, h->stream);
     CK(cudaGetLastError());
     h->launches += periodic ? 6 : 5;
     h->sorted_valid = true;
@@ -429,23 +429,33 @@ StageArgs stage_args(sph_handle* h, int mode, int stage, double dt, int shift = 
     return g;
 }
 
-template <typename R>
-void launch_pass_c(const Params& P, const Sorted<R>& D, const StageArgs& G, bool shift, int nb, cudaStream_t st) {
+template <typename R, int L>
+void launch_pass_c_lanes(const Params& P, const Sorted<R>& D, const StageArgs& G, bool shift, cudaStream_t st) {
+    const int nb = blocks((long long)P.n_tot * L, 128);
     if (P.ms) {
-        if (shift) k_pass_c<R, false, true, true><<<nb, 128, 0, st>>>(P, D, G);
-        else k_pass_c<R, false, true, false><<<nb, 128, 0, st>>>(P, D, G);
+        if (shift) k_pass_c<R, false, true, true, L><<<nb, 128, 0, st>>>(P, D, G);
+        else k_pass_c<R, false, true, false, L><<<nb, 128, 0, st>>>(P, D, G);
         return;
     }
     // (the mixed Taylor-Green launches never carry the shifting sum)
     if constexpr (sizeof(R) == 8) {
         if (shift) {
-            if (P.muscl) k_pass_c<R, true, false, true><<<nb, 128, 0, st>>>(P, D, G);
-            else k_pass_c<R, false, false, true><<<nb, 128, 0, st>>>(P, D, G);
+            if (P.muscl) k_pass_c<R, true, false, true, L><<<nb, 128, 0, st>>>(P, D, G);
+            else k_pass_c<R, false, false, true, L><<<nb, 128, 0, st>>>(P, D, G);
             return;
         }
     }
-    if (P.muscl) k_pass_c<R, true, false, false><<<nb, 128, 0, st>>>(P, D, G);
-    else k_pass_c<R, false, false, false><<<nb, 128, 0, st>>>(P, D, G);
+    if (P.muscl) k_pass_c<R, true, false, false, L><<<nb, 128, 0, st>>>(P, D, G);
+    else k_pass_c<R, false, false, false, L><<<nb, 128, 0, st>>>(P, D, G);
+}
+
+template <typename R>
+void launch_pass_c(const Params& P, const Sorted<R>& D, const StageArgs& G, bool shift, cudaStream_t st) {
+    if constexpr (sizeof(R) == 8) {
+        if (P.n_tot < kLanes4Below) { launch_pass_c_lanes<R, 4>(P, D, G, shift, st); return; }
+        if (P.n_tot < kLanes2BelowC) { launch_pass_c_lanes<R, 2>(P, D, G, shift, st); return; }
+    }
+    launch_pass_c_lanes<R, 1>(P, D, G, shift, st);
 }
 
 // One RHS evaluation on the current stage state.  G: the stage that follows it,
@@ -475,13 +485,13 @@ int rhs(sph_handle* h, int last, const StageArgs& G = StageArgs{}, int keep_j = 
         if (rc) return rc;
     }
     tic(h, PH_A);
-    launch_pass_a<R, true>(P, D, nb, h->stream);
+    launch_pass_a<R, true>(P, D, h->stream);
     tic(h, PH_C);
     // the mixed Taylor-Green path forms the shifting sum in k_shift_gather after
     // pass C; the FP64 and moving-square launches form it inside pass C
     const bool sep = sizeof(R) == 4 && !P.ms;
     const bool sh = last && h->cfg.shifting;
-    launch_pass_c<R>(P, D, sh && sep ? StageArgs{} : G, sh && !sep, nb, h->stream);
+    launch_pass_c<R>(P, D, sh && sep ? StageArgs{} : G, sh && !sep, h->stream);
     if constexpr (sizeof(R) == 4) if (sh && sep) {
         // timed with the update: shifting is part of the step's second pass
         tic(h, PH_UPDATE);
@@ -1267,13 +1277,12 @@ template <typename R>
 void adj_pass_a(sph_handle* h, const Sorted<R>& V) {
     ++h->P.rhs_gen;
     const Params& P = h->P;
-    const int nb = blocks(P.n_tot, 128);
     if constexpr (sizeof(R) == 4) {
         k_resplit<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P.n_tot, V);
-        launch_pass_a<R, true>(P, V, nb, h->stream);
+        launch_pass_a<R, true>(P, V, h->stream);
         h->launches += 1;
     } else {
-        launch_pass_a<R, false>(P, V, nb, h->stream);
+        launch_pass_a<R, false>(P, V, h->stream);
     }
     launch_near<R>(P, V, h->stream);
     h->launches += P.free_surface ? 2 : 1;
@@ -1443,7 +1452,7 @@ void adj_rhs_ms_values(sph_handle* h, const Sorted<R>& V, int kept_j) {
             h->body_acc[1], X->A.gint, X->A.gsw);
         h->launches += 1;
     }
-    launch_pass_a<R, false>(P, V, blocks(P.n_tot, kAdjThreads), h->stream);
+    launch_pass_a<R, false>(P, V, h->stream);
     launch_near<R>(P, V, h->stream);
 }
 

@@ -596,6 +596,7 @@ constexpr int kAdjLanes = SPH_ADJ_LANES;     // 2 or 4
 template <typename R, bool MS = false, bool MUSCL = false, bool HLLC = false>
 __global__ void __launch_bounds__(kAdjThreads, MUSCL ? SPH_ADJ_C_MUSCL_MIN_BLOCKS : SPH_ADJ_C_MIN_BLOCKS) k_adj_c(Params P, Sorted<R> D, Adj A, const double* lr,
                                                         const double2* la, double* nu_part) {
+    stamp_phase(P.stamp);
     __shared__ double red[kAdjThreads];
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = t / kAdjLanes;
@@ -980,6 +981,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_a(Params P, Sorted<R> D, Ad
 //   s_a = sum_b phi(d) V_b r,  phi = (1 + R (W/W_dx)^4) G,  r = x_a - x_b.
 template <typename R>
 __global__ void k_shift_sum(Params P, Sorted<R> D, Adj A) {
+    stamp_phase(P.stamp);
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
     const double2 xa = D.pos[a];
@@ -1091,6 +1093,7 @@ __device__ __forceinline__ void shift_reverse(const Params& P, const Sorted<R>& 
 template <typename R>
 __global__ void k_adj_stage3(Params P, Sorted<R> D, Adj A, double dt, int shift, const double2* ox = nullptr,
                              const double* orho = nullptr) {
+    stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     const int i = D.id[s];
@@ -1206,6 +1209,7 @@ __device__ __forceinline__ void mls_pbar_to_d(const double (&pb)[6], double dx, 
 // density (lam) per slot.
 template <typename R>
 __global__ void k_adj_mls_end(Params P, Sorted<R> D, Adj A, int shift, double2* xe, double* lam) {
+    stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     const int i = D.id[s];
@@ -1561,7 +1565,8 @@ __global__ void k_adj_route(int n_src, int base, const int* cnt, const int* off,
 // The hi/lo records of the mixed path formed from the FP64 state of V (as the
 // forward's stages write them).
 template <typename R>
-__global__ void k_resplit(int n, Sorted<R> D) {
+__global__ void k_resplit(int n, Sorted<R> D, unsigned long long* stamp) {
+    stamp_phase(stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     store_split(D, s, D.pos[s], D.kin[s]);
@@ -1570,6 +1575,7 @@ __global__ void k_resplit(int n, Sorted<R> D) {
 // Stage state -> the arrays the RHS reads (positions, kinematic and auxiliary records).
 template <typename R>
 __global__ void k_adj_load(Params P, Sorted<R> D, const double2* pos, const double4* kin) {
+    stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     const double2 x = pos ? pos[s] : D.pos0[s];
@@ -1596,7 +1602,8 @@ struct SnapPtrs {
     double2 *pos, *vel, *r_acc, *r_avg;
     double *rho, *r_drho;
 };
-__global__ void k_snap_copy(int n, SnapPtrs dst, SnapPtrs src) {
+__global__ void k_snap_copy(int n, SnapPtrs dst, SnapPtrs src, unsigned long long* stamp) {
+    stamp_phase(stamp);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     dst.pos[i] = src.pos[i]; dst.vel[i] = src.vel[i]; dst.rho[i] = src.rho[i];
@@ -1622,7 +1629,9 @@ struct PrepDesc {
 // restoring, so no launch reads counts it is writing); each particle copies its
 // own entries only.  Arrays whose size is a multiple of 16 bytes move in 16-byte
 // words (the arrays and the slot offsets are 256-byte aligned).
-__global__ void k_prep_copy(const PrepDesc* d, int n_tot, unsigned* slot, int save, const int* cnt) {
+__global__ void k_prep_copy(const PrepDesc* d, int n_tot, unsigned* slot, int save, const int* cnt,
+                            unsigned long long* stamp) {
+    stamp_phase(stamp);
     const PrepDesc c = d[blockIdx.y];
     unsigned* s = slot + c.off;
     const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1998,6 +2007,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_ghost_water(Params P, Sorte
 template <typename R>
 __global__ void k_adj_stage_end_ms(Params P, Sorted<R> D, Adj A, double dt, int shift, const double2* ox = nullptr,
                                    const double* orho = nullptr) {
+    stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     const int i = D.id[s];

@@ -55,9 +55,22 @@ struct Params {
     int gnx, gny;
     // sizes
     int n_host, n_tot, max_nbr, nbr_stride;
+    unsigned long long* stamp;   // where the kernel that begins a timed phase writes its start (or null)
     int rhs_gen;             // number of the RHS being evaluated (see Sorted::surf_gen)
     double skin_half2;       // (skin/2)^2: allowed squared displacement since the list build
 };
+
+// Start of a timed phase: the first kernel launched after the host marked the
+// phase writes the device clock (nanoseconds, steps of 32) into its slot.  An
+// event between every two passes cost 5 us of GPU time each, a third of a small
+// step; this costs one thread a load.
+__device__ __forceinline__ void stamp_phase(unsigned long long* slot) {
+    if (slot == nullptr || blockIdx.x != 0 || blockIdx.y != 0 || threadIdx.x != 0) return;
+    if (*slot != 0ull) return;
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    *slot = t;
+}
 
 template <typename R> struct VT;
 template <> struct VT<double> { using V2 = double2; using V4 = double4; };

@@ -90,6 +90,7 @@ __device__ __noinline__ bool surface_test(const Params& P, const Sorted<R>& D, i
 template <typename R, bool HLREC, bool MS, int L = 1>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_BLOCKS : SPH_PASS_A_F32_BLOCKS) : (MS ? 4 : 5))
     k_pass_a(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D) {
+    stamp_phase(P.stamp);
     using V4 = typename VT<R>::V4;
     constexpr bool F32 = sizeof(R) == 4;
     constexpr bool HL = HLREC && F32;
@@ -326,11 +327,15 @@ void launch_pass_a_lanes(const Params& P, const Sorted<R>& D, cudaStream_t st) {
 
 template <typename R, bool HLREC>
 void launch_pass_a(const Params& P, const Sorted<R>& D, cudaStream_t st) {
-    if constexpr (sizeof(R) == 8 && HLREC) {
-        if (P.n_tot < kLanes4Below) { launch_pass_a_lanes<R, HLREC, 4>(P, D, st); return; }
-        if (P.n_tot < kLanes2BelowA) { launch_pass_a_lanes<R, HLREC, 2>(P, D, st); return; }
+    if constexpr (sizeof(R) == 8) {
+        // HLREC means nothing to FP64: one kernel for both, so that the adjoint's
+        // re-run forms the forward's bits
+        if (P.n_tot < kLanes4Below) launch_pass_a_lanes<R, true, 4>(P, D, st);
+        else if (P.n_tot < kLanes2BelowA) launch_pass_a_lanes<R, true, 2>(P, D, st);
+        else launch_pass_a_lanes<R, true, 1>(P, D, st);
+    } else {
+        launch_pass_a_lanes<R, HLREC, 1>(P, D, st);
     }
-    launch_pass_a_lanes<R, HLREC, 1>(P, D, st);
 }
 
 // Near-free-surface flags (Define_freesurface...f90:418-440): every pair

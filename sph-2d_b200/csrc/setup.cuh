@@ -69,7 +69,7 @@ struct SetupBuf {
     int4* blk;            // [image blocks] image sums (x: left/right, y: bottom/top of host
                           // particles, z: bottom/top of left/right images), then exclusive
     int* tot;             // [3] their totals
-    unsigned* done;       // [2] blocks finished (image count, cell scan); left at 0
+    unsigned* done;       // [3] blocks finished (image count, cell scan, diagnostics); left at 0
     unsigned* key;        // [cap] cell of particle i (id order), ncells = not binned
     int* rank;            // [cap] its arrival number in the cell
     int* cnt;             // [ncells + 1] particles per cell
@@ -150,6 +150,7 @@ __device__ __forceinline__ void image_counts(const Params& P, double2 x, bool il
 }
 
 __global__ void __launch_bounds__(kImgThreads) k_img_count(Params P, Staging S, SetupBuf B, HostBox* box, unsigned seq) {
+    stamp_phase(P.stamp);
     __shared__ unsigned long long sh[32];
     __shared__ int flag;
     const int i = blockIdx.x * kImgThreads + threadIdx.x;
@@ -223,6 +224,7 @@ __device__ __forceinline__ void put_image(const Params& P, const Staging& S, con
 // offsets for the reverse sweep.
 __global__ void __launch_bounds__(kImgThreads) k_img_emit(Params P, Staging S, SetupBuf B, int cap, int periodic,
                                                           int route, unsigned* status) {
+    stamp_phase(P.stamp);
     __shared__ unsigned long long sh[32];
     const int i = blockIdx.x * kImgThreads + threadIdx.x;
     const bool live = i < P.n_host;
@@ -277,7 +279,8 @@ __global__ void __launch_bounds__(kImgThreads) k_img_emit(Params P, Staging S, S
 
 // Exclusive scan of the cell counts within blocks of kScanCells cells; the last
 // block scans the block sums.
-__global__ void __launch_bounds__(kScanThreads) k_cell_scan(SetupBuf B) {
+__global__ void __launch_bounds__(kScanThreads) k_cell_scan(SetupBuf B, unsigned long long* stamp) {
+    stamp_phase(stamp);
     __shared__ int sh[32];
     __shared__ int flag;
     constexpr int per = kScanCells / kScanThreads;
@@ -629,6 +632,7 @@ __global__ void k_gather_sorted(Params P, Staging S, Sorted<R> D, SetupBuf B, St
 // sorted master state -> id order (host particles only; images are dropped)
 template <typename R>
 __global__ void k_unsort(Params P, Staging S, Sorted<R> D) {
+    stamp_phase(P.stamp);
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     int i = D.id[s];

@@ -93,9 +93,11 @@ struct sph_handle {
     int* d_cnt_id = nullptr;
     // timing
     bool timing = true;
-    std::vector<cudaEvent_t> ev_pool;
+    std::vector<cudaEvent_t> ev_pool;     // begin and end of each timed stretch
     size_t ev_used = 0;
-    std::vector<int> ev_phase;
+    unsigned long long* d_stamps = nullptr;   // [kStamps] start of each phase (0: not begun)
+    std::vector<int> stamp_of;            // phase of each used slot (-1: outside the phases)
+    bool timed_open = false;
     double t_ms[PH_COUNT] = {0};
     double t_total = 0;
     long long n_rhs = 0, n_steps = 0;
@@ -280,31 +282,63 @@ int status_to_code(unsigned st) {
     return SPH_OK;
 }
 
-// --- timing helpers ---------------------------------------------------------
-void tic(sph_handle* h, int phase) {
-    if (!h->timing) return;
+// --- timing -----------------------------------------------------------------
+// A stretch of work (a sph_step call, say) is timed by an event at either end;
+// inside it the phases are marked by the kernels that begin them (stamp_phase).
+// Both are read when the times are asked for.
+constexpr int kStamps = 8192;
+
+void mark_event(sph_handle* h) {
     if (h->ev_used >= h->ev_pool.size()) {
         cudaEvent_t e;
         cudaEventCreate(&e);
         h->ev_pool.push_back(e);
     }
-    cudaEventRecord(h->ev_pool[h->ev_used], h->stream);
-    h->ev_phase.push_back(phase);
-    h->ev_used++;
+    cudaEventRecord(h->ev_pool[h->ev_used++], h->stream);
+}
+
+// End of the stretch.
+void toc(sph_handle* h) {
+    if (!h->timed_open) return;
+    k_stamp<<<1, 1, 0, h->stream>>>(h->d_stamps + h->stamp_of.size());
+    h->stamp_of.push_back(-1);
+    h->P.stamp = nullptr;
+    mark_event(h);
+    h->timed_open = false;
 }
 
 void timing_flush(sph_handle* h) {
-    if (!h->timing || h->ev_used == 0) return;
-    cudaEventSynchronize(h->ev_pool[h->ev_used - 1]);
-    for (size_t k = 0; k + 1 < h->ev_used; ++k) {
+    toc(h);
+    if (h->stamp_of.empty()) return;
+    std::vector<unsigned long long> t(h->stamp_of.size());
+    cudaMemcpyAsync(t.data(), h->d_stamps, sizeof(t[0]) * t.size(), cudaMemcpyDeviceToHost, h->stream);
+    cudaMemsetAsync(h->d_stamps, 0, sizeof(t[0]) * t.size(), h->stream);
+    cudaStreamSynchronize(h->stream);
+    int ph = -1;
+    unsigned long long from = 0;
+    for (size_t k = 0; k < t.size(); ++k) {
+        if (t[k] == 0) continue;                  // a phase without launches
+        if (ph >= 0 && ph < PH_COUNT) h->t_ms[ph] += 1e-6 * (double)(t[k] - from);
+        ph = h->stamp_of[k];
+        from = t[k];
+    }
+    for (size_t k = 0; k + 1 < h->ev_used; k += 2) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, h->ev_pool[k], h->ev_pool[k + 1]);
-        int ph = h->ev_phase[k];
-        if (ph >= 0 && ph < PH_COUNT) h->t_ms[ph] += ms;
         h->t_total += ms;
     }
     h->ev_used = 0;
-    h->ev_phase.clear();
+    h->stamp_of.clear();
+}
+
+// Phase `phase` begins with the next launch (-1: none does).
+void tic(sph_handle* h, int phase) {
+    if (!h->timing) return;
+    if (h->timed_open && h->stamp_of.back() == phase) return;
+    if (h->stamp_of.size() + 2 > kStamps) timing_flush(h);
+    if (!h->timed_open) { mark_event(h); h->timed_open = true; }
+    h->P.stamp = h->d_stamps + h->stamp_of.size();
+    h->stamp_of.push_back(phase);
 }
 
 template <typename R> Sorted<R>& sorted(sph_handle* h);
@@ -396,7 +430,7 @@ int prepare(sph_handle* h, const StageArgs& first = StageArgs{}) {
     // (the routing of image adjoints is kept once an adjoint run exists)
     k_img_emit<<<nhb, kImgThreads, 0, h->stream>>>(P, h->S, B, h->cap_tot, periodic, h->adj != nullptr, h->d_status);
     tic(h, PH_SORT);
-    k_cell_scan<<<ncb, kScanThreads, 0, h->stream>>>(B);
+    k_cell_scan<<<ncb, kScanThreads, 0, h->stream>>>(B, P.stamp);
     CK(cudaGetLastError());
     int n_img = 0;
     if (periodic) {
@@ -529,12 +563,17 @@ int stage(sph_handle* h, int st, double dt, int use_carried, int do_shift) {
     return SPH_OK;
 }
 
-int read_status(sph_handle* h) {
-    unsigned st = 0;
-    CK(cudaMemcpyAsync(&st, h->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+// The status word the host box holds, cleared on the device when set.
+int take_status(sph_handle* h) {
+    const unsigned st = h->box->status;
     if (st) CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream));
     return status_to_code(st);
+}
+
+int read_status(sph_handle* h) {
+    CK(cudaMemcpyAsync((void*)&h->box->status, h->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    return take_status(h);
 }
 
 // Reinitialize_particle_density on the state after the integrator update of a
@@ -621,46 +660,44 @@ int run_steps(sph_handle* h, int nsteps, double dt) {
             if ((rc = rhs<R>(h, 1, stage_args(h, STAGE_END, stn, dt, h->cfg.shifting, to_staging)))) return rc;
             if (to_staging) h->staging_valid = true;
         }
-        tic(h, -1);
         h->step_count++;
         h->n_steps++;
-        if (h->ev_used > 4096) timing_flush(h);
     }
-    timing_flush(h);
-    return read_status(h);
+    toc(h);
+    return SPH_OK;
 }
 
+// The diagnostics of the current state; with_status: and the status of the work
+// before them, in the same wait (an error is returned, *result left as it was).
 template <typename R>
-int diagnostics(sph_handle* h, sph_diag* out) {
+int diagnostics(sph_handle* h, sph_diag* result, bool with_status) {
+    sph_diag d, *out = &d;
     memset(out, 0, sizeof(*out));
     if (!h->sorted_valid) {
         // state only in staging: sort it once to reduce over the same arrays
         int rc = prepare<R>(h);
+        toc(h);
         if (rc) return rc;
     }
     const Params& P = h->P;
-    const int nparts = 148 * 4;
-    k_diag_partial<R><<<nparts, kRedThreads, 0, h->stream>>>(P, sorted<R>(h), h->d_part, h->d_part + nparts);
-    k_diag_final<<<1, kRedThreads, 0, h->stream>>>(nparts, h->d_part, h->d_part + nparts, h->d_diag);
-    CK(cudaMemsetAsync(h->d_int, 0, sizeof(int), h->stream));
-    k_count_surface<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, sorted<R>(h), h->d_int);
-    h->launches += 3;
-    double v[2];
-    int nsurf = 0;
-    CK(cudaMemcpyAsync(v, h->d_diag, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(&nsurf, h->d_int, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    if (h->bf_pending) {
-        const double* fin = h->d_bf + (size_t)6 * blocks(h->cap_tot, kRedThreads);
-        CK(cudaMemcpyAsync(h->bf, fin, 6 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    }
+    const double* fin = h->bf_pending ? h->d_bf + (size_t)6 * blocks(h->cap_tot, kRedThreads) : nullptr;
+    k_diag<R><<<std::min(kDiagBlocks, blocks(P.n_tot, kRedThreads)), kRedThreads, 0, h->stream>>>(
+        P, sorted<R>(h), h->d_part, h->d_part + kDiagBlocks, h->d_int, h->B.done + 2, h->d_status, fin, h->d_box);
+    CK(cudaGetLastError());
+    h->launches += 1;
     CK(cudaStreamSynchronize(h->stream));
+    const int rc = with_status ? take_status(h) : SPH_OK;
+    if (fin)
+        for (int c = 0; c < 6; ++c) h->bf[c] = h->box->diag[2 + c];
     h->bf_pending = false;
-    out->kinetic_energy = v[0];
-    out->max_speed = v[1];
+    if (rc) return rc;
+    out->kinetic_energy = h->box->diag[0];
+    out->max_speed = h->box->diag[1];
     out->n_images = h->n_img;
-    out->n_surface = h->have_rhs ? nsurf : 0;
+    out->n_surface = h->have_rhs ? h->box->nsurf : 0;
     out->pair_count = h->last_pairs;
     for (int c = 0; c < 6; ++c) out->body_force[c] = h->bf[c];
+    *result = d;
     return SPH_OK;
 }
 
@@ -831,7 +868,8 @@ int snap_io(sph_handle* h, const Snap& s, int k, int n, bool save) {
     const size_t o = (size_t)k * n;
     const SnapPtrs slot{s.pos + o, s.vel + o, s.r_acc + o, s.r_avg + o, s.rho + o, s.r_drho + o};
     const SnapPtrs stg{h->S.pos, h->S.vel, h->S.r_acc, h->S.r_avg, h->S.rho, h->S.r_drho};
-    k_snap_copy<<<blocks(n, 256), 256, 0, h->stream>>>(n, save ? slot : stg, save ? stg : slot);
+    k_snap_copy<<<blocks(n, 256), 256, 0, h->stream>>>(n, save ? slot : stg, save ? stg : slot,
+                                                      h->P.stamp);
     CK(cudaGetLastError());
     h->launches += 1;
     if (!save) {
@@ -936,7 +974,7 @@ int prep_save(sph_handle* h, int j, bool lists = true) {
     const int nt = h->P.n_tot;
     const int* cnt = h->mixed ? h->D32.nnbr : h->D64.nnbr;
     k_prep_copy<<<dim3(blocks(nt, 256), X->n_prep - (lists ? 0 : 1)), 256, 0, h->stream>>>(
-        X->d_prep, nt, X->prep + (size_t)j * X->prep_words, 1, cnt);
+        X->d_prep, nt, X->prep + (size_t)j * X->prep_words, 1, cnt, nullptr);
     CK(cudaGetLastError());
     h->launches += 1;
     X->seg_nimg[j] = h->n_img;
@@ -957,7 +995,7 @@ int prep_restore(sph_handle* h, int j, bool lists = true) {
     tic(h, PH_SORT);
     unsigned* slot = X->prep + (size_t)j * X->prep_words;
     k_prep_copy<<<dim3(blocks(P.n_tot, 256), X->n_prep - (lists ? 0 : 1)), 256, 0, h->stream>>>(
-        X->d_prep, P.n_tot, slot, 0, (const int*)(slot + X->prep_nnbr_off));
+        X->d_prep, P.n_tot, slot, 0, (const int*)(slot + X->prep_nnbr_off), P.stamp);
     CK(cudaGetLastError());
     h->launches += 1;
     h->sorted_valid = true;
@@ -1109,7 +1147,7 @@ int adjoint_forward(sph_handle* h, const sph_adj_config* ac, double* loss) {
     for (int c = 0; c < X->nseg; ++c) {
         if ((rc = unsort<R>(h)) || (rc = snap_io(h, X->ck, c, n, true))) return rc;
         const int ns = std::min(X->every, X->nsteps - c * X->every);
-        if ((rc = run_steps<R>(h, ns, X->dt))) return rc;
+        if ((rc = run_steps<R>(h, ns, X->dt)) || (rc = read_status(h))) return rc;
     }
     if ((rc = unsort<R>(h)) || (rc = snap_io(h, X->ck, X->nseg, n, true))) return rc;
     double v = 0.0;
@@ -1237,7 +1275,6 @@ int step_keep(sph_handle* h, double dt, int j, bool full) {
             }
         }
         tic(h, -1);
-        if (h->ev_used > 4096) timing_flush(h);
         return SPH_OK;
     }
     // RK4: RHS k + 1 (k = 0, 1, 2) on stage state S(k+1) and the stage it feeds
@@ -1266,7 +1303,6 @@ int step_keep(sph_handle* h, double dt, int j, bool full) {
         h->n_steps++;
     }
     tic(h, -1);
-    if (h->ev_used > 4096) timing_flush(h);
     return SPH_OK;
 }
 
@@ -1278,7 +1314,7 @@ void adj_pass_a(sph_handle* h, const Sorted<R>& V) {
     ++h->P.rhs_gen;
     const Params& P = h->P;
     if constexpr (sizeof(R) == 4) {
-        k_resplit<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P.n_tot, V);
+        k_resplit<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P.n_tot, V, P.stamp);
         launch_pass_a<R, true>(P, V, h->stream);
         h->launches += 1;
     } else {
@@ -1424,7 +1460,6 @@ int adj_step(sph_handle* h, bool first, int j) {
     }
     CK(cudaGetLastError());
     tic(h, -1);
-    if (h->ev_used > 4096) timing_flush(h);
     return SPH_OK;
 }
 
@@ -1620,7 +1655,6 @@ int adj_step_ms(sph_handle* h, bool first, int j, int jstep) {
     h->launches += 2;
     CK(cudaGetLastError());
     tic(h, -1);
-    if (h->ev_used > 4096) timing_flush(h);
     return SPH_OK;
 }
 
@@ -1657,7 +1691,7 @@ int adjoint_backward(sph_handle* h, double dloss, double* g_vel0, double* g_rho0
         for (int j = s0; j < s1; ++j) {
             if ((rc = unsort<R>(h)) || (rc = snap_io(h, X->seg, j - s0, n, true))) return rc;
             if (stored) rc = step_keep<R>(h, X->dt, j - s0, j + 1 < s1);
-            else if (j + 1 < s1) rc = run_steps<R>(h, 1, X->dt);
+            else if (j + 1 < s1 && !(rc = run_steps<R>(h, 1, X->dt))) rc = read_status(h);
             if (rc) return rc;
         }
         for (int j = s1 - 1; j >= s0; --j) {
@@ -1669,7 +1703,7 @@ int adjoint_backward(sph_handle* h, double dloss, double* g_vel0, double* g_rho0
             if (rc) return rc;
         }
     }
-    timing_flush(h);
+    toc(h);
     if ((rc = read_status(h))) return rc;
     // gradients with respect to the state the forward started from (id order)
     if (g_vel0) {
@@ -1713,7 +1747,7 @@ void destroy(sph_handle* h) {
                     h->S.r_avg, h->S.lr_cnt, h->S.lr_off, h->S.tb_cnt, h->S.tb_off, h->B.blk, h->B.tot, h->B.done, h->B.key, h->B.rank,
                     h->B.cnt, h->B.pre, h->B.blkoff, h->B.perm, h->cub_tmp,
                     h->d_status, h->d_int, h->d_part, h->d_diag, h->d_xfer, h->d_export, h->d_off64, h->d_cnt_id,
-                    h->d_mls, h->d_ghost_ids};
+                    h->d_mls, h->d_ghost_ids, h->d_stamps};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
     if (h->copy_stream) { cudaStreamSynchronize(h->copy_stream); cudaStreamDestroy(h->copy_stream); }
@@ -1763,8 +1797,8 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     // set-up
     SetupBuf& B = h->B;
     B.ncells = h->ncells;
-    CK(dalloc(&B.blk, blocks(h->cap_host, kImgThreads))); CK(dalloc(&B.tot, 3)); CK(dalloc(&B.done, 2));
-    CK(cudaMemsetAsync(B.done, 0, 2 * sizeof(unsigned), h->stream));
+    CK(dalloc(&B.blk, blocks(h->cap_host, kImgThreads))); CK(dalloc(&B.tot, 3)); CK(dalloc(&B.done, 3));
+    CK(cudaMemsetAsync(B.done, 0, 3 * sizeof(unsigned), h->stream));
     CK(dalloc(&B.key, cap)); CK(dalloc(&B.rank, cap)); CK(dalloc(&B.perm, cap));
     CK(dalloc(&B.cnt, (size_t)h->ncells + 1)); CK(dalloc(&B.pre, (size_t)h->ncells + 1));
     CK(dalloc(&B.blkoff, blocks((long long)h->ncells + 1, kScanCells)));
@@ -1779,8 +1813,10 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
         CK(cudaMalloc(&h->cub_tmp, h->cub_bytes));
     }
     CK(dalloc(&h->d_status, 1)); CK(cudaMemset(h->d_status, 0, sizeof(unsigned)));
-    CK(dalloc(&h->d_int, 4));
-    CK(dalloc(&h->d_part, 2 * 148 * 4)); CK(dalloc(&h->d_diag, 2));
+    CK(dalloc(&h->d_stamps, kStamps));
+    CK(cudaMemsetAsync(h->d_stamps, 0, sizeof(unsigned long long) * kStamps, h->stream));
+    CK(dalloc(&h->d_int, kDiagBlocks));
+    CK(dalloc(&h->d_part, 2 * kDiagBlocks)); CK(dalloc(&h->d_diag, 2));
     CK(dalloc(&h->d_xfer, (size_t)6 * h->cap_host));
     if (cfg->mls_order) CK(dalloc(&h->d_mls, cap));
     if (h->mixed) rc = alloc_sorted(h->D32, cap, h->P.max_nbr, h->ncells);
@@ -2101,6 +2137,7 @@ int sph_find_particle_pair(sph_handle* h, long long pair_cap, int* pair_i, int* 
     if (pair_cap > 0 && (!pair_i || !pair_j)) return SPH_E_ARG;
     CK(cudaSetDevice(h->device));
     int rc = DISPATCH(h, prepare, h);
+    toc(h);
     if (rc) return rc;
     rc = read_status(h);
     if (rc) return rc;
@@ -2115,8 +2152,8 @@ int sph_rhs(sph_handle* h, double* drhodt, double* acc, double* avg_vel, int* fs
     h->bf_every_rhs = true;
     rc = DISPATCH(h, rhs, h, 0);
     h->bf_every_rhs = false;
+    toc(h);
     if (rc) return rc;
-    timing_flush(h);
     rc = read_status(h);
     if (rc) return rc;
     rc = DISPATCH(h, export_fields, h);
@@ -2160,14 +2197,16 @@ int sph_step(sph_handle* h, int nsteps, double dt, sph_diag* out) {
     CK(cudaSetDevice(h->device));
     int rc = DISPATCH(h, run_steps, h, nsteps, dt);
     if (rc) return rc;
-    if (out) return DISPATCH(h, diagnostics, h, out);
-    return SPH_OK;
+    // (without a sorted state the diagnostics sort it first: the status is that of the steps)
+    const bool together = out && h->sorted_valid;
+    if (!together && (rc = read_status(h))) return rc;
+    return out ? DISPATCH(h, diagnostics, h, out, together) : SPH_OK;
 }
 
 int sph_diagnostics(sph_handle* h, sph_diag* out) {
     if (!h || !out || h->n_host <= 0) return SPH_E_ARG;
     CK(cudaSetDevice(h->device));
-    return DISPATCH(h, diagnostics, h, out);
+    return DISPATCH(h, diagnostics, h, out, false);
 }
 
 int sph_adjoint_forward(sph_handle* h, const sph_adj_config* cfg, double* loss) {

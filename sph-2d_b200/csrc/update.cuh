@@ -22,6 +22,7 @@ __device__ __forceinline__ void apply_shift(const Params& P, const Sorted<R>& D,
 template <typename R>
 __global__ void k_stage(Params P, Sorted<R> D, int stage, double dt, int use_carried, int do_shift,
                         unsigned* status) {
+    stamp_phase(P.stamp);
     using V2 = typename VT<R>::V2;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
@@ -105,6 +106,7 @@ __device__ __forceinline__ bool chol_solve_e1(double (&A)[M * (M + 1) / 2], doub
 
 template <typename R, int M>
 __global__ void k_mls(Params P, Sorted<R> D, double* rho_new) {
+    stamp_phase(P.stamp);
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
     const double rho_a = D.kin[a].z;
@@ -171,6 +173,7 @@ __global__ void k_mls(Params P, Sorted<R> D, double* rho_new) {
 // Define_freesurface_and_Normailized_derivates.f90:87-91), in FP64.
 template <typename R>
 __global__ void k_mls1(Params P, Sorted<R> D, double* rho_new) {
+    stamp_phase(P.stamp);
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
     rho_new[a] = D.kin[a].z;
@@ -198,6 +201,7 @@ __global__ void k_mls1(Params P, Sorted<R> D, double* rho_new) {
 // step (when on) is applied, as the reference's driver calls the two in turn.
 template <typename R>
 __global__ void k_finish_mls(Params P, Sorted<R> D, const double* rho_new, int do_shift, unsigned* status) {
+    stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     if (!integrated(P, D.type[s]) || D.id[s] >= P.n_host) return;
@@ -310,6 +314,7 @@ template <typename R>
 __global__ void k_assign_ghosts(Params P, Sorted<R> D, const int* ghost_ids, int n_ghost, double t, double bvx,
                                 double bvy, double bax, double bay, double4* gint = nullptr,
                                 double* gsw = nullptr) {
+    stamp_phase(P.stamp);
     const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wg >= n_ghost) return;                       // whole warps
     const int s = D.slot_of[ghost_ids[wg]];
@@ -398,40 +403,57 @@ __global__ void k_ghost_refill(Sorted<R> D, const int* ghost_ids, int n_ghost) {
     D.rho0[s] = k.z;
 }
 
+// The end of a timed stretch of work.
+__global__ void k_stamp(unsigned long long* slot) { stamp_phase(slot); }
+
 // Kinetic energy and max |v| of the water host particles
-// (Sampling_subroutine.f90:346-356): deterministic two-level reduction in FP64.
+// (Sampling_subroutine.f90:346-356) in FP64 and the number of flagged surface
+// particles: block partials, then the last block to finish adds them in a fixed
+// order and writes the results, the status word and the last body force (bf, or
+// null) to the page-locked box the host reads after one wait.
 constexpr int kRedThreads = 256;
+constexpr int kDiagBlocks = 148 * 4;
 template <typename R>
-__global__ void k_diag_partial(Params P, Sorted<R> D, double* part_ke, double* part_max) {
+__global__ void __launch_bounds__(kRedThreads) k_diag(Params P, Sorted<R> D, double* part_ke, double* part_max,
+                                                      int* part_ns, unsigned* done, const unsigned* status,
+                                                      const double* bf, HostBox* box) {
     __shared__ double ske[kRedThreads], smx[kRedThreads];
+    __shared__ int sns[kRedThreads];
+    __shared__ int flag;
+    const int t = threadIdx.x;
+    auto reduce = [&](double ke, double mx, int ns) {
+        ske[t] = ke; smx[t] = mx; sns[t] = ns;
+        __syncthreads();
+        for (int w = kRedThreads / 2; w > 0; w >>= 1) {
+            if (t < w) { ske[t] += ske[t + w]; smx[t] = fmax(smx[t], smx[t + w]); sns[t] += sns[t + w]; }
+            __syncthreads();
+        }
+    };
     double ke = 0.0, mx = 0.0;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < P.n_tot; s += gridDim.x * blockDim.x) {
+    int ns = 0;
+    for (int s = blockIdx.x * blockDim.x + t; s < P.n_tot; s += gridDim.x * blockDim.x) {
+        ns += D.flags[s] & 1;
         if (D.type[s] != SPH_TYPE_WATER || D.id[s] >= P.n_host) continue;
         double2 v = D.vel0[s];
         double vv = v.x * v.x + v.y * v.y;
         ke += 0.5 * D.mass[s] * vv;
         mx = fmax(mx, sqrt(vv));
     }
-    ske[threadIdx.x] = ke; smx[threadIdx.x] = mx;
-    __syncthreads();
-    for (int w = kRedThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) { ske[threadIdx.x] += ske[threadIdx.x + w]; smx[threadIdx.x] = fmax(smx[threadIdx.x], smx[threadIdx.x + w]); }
-        __syncthreads();
+    reduce(ke, mx, ns);
+    if (t == 0) { part_ke[blockIdx.x] = ske[0]; part_max[blockIdx.x] = smx[0]; part_ns[blockIdx.x] = sns[0]; }
+    if (!last_block(done, &flag)) return;
+    ke = mx = 0.0;
+    ns = 0;
+    for (int i = t; i < (int)gridDim.x; i += kRedThreads) {
+        ke += __ldcg(&part_ke[i]); mx = fmax(mx, __ldcg(&part_max[i])); ns += __ldcg(&part_ns[i]);
     }
-    if (threadIdx.x == 0) { part_ke[blockIdx.x] = ske[0]; part_max[blockIdx.x] = smx[0]; }
-}
-
-__global__ void k_diag_final(int nparts, const double* part_ke, const double* part_max, double* out) {
-    __shared__ double ske[kRedThreads], smx[kRedThreads];
-    double ke = 0.0, mx = 0.0;
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) { ke += part_ke[i]; mx = fmax(mx, part_max[i]); }
-    ske[threadIdx.x] = ke; smx[threadIdx.x] = mx;
-    __syncthreads();
-    for (int w = kRedThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) { ske[threadIdx.x] += ske[threadIdx.x + w]; smx[threadIdx.x] = fmax(smx[threadIdx.x], smx[threadIdx.x + w]); }
-        __syncthreads();
+    reduce(ke, mx, ns);
+    if (t == 0) {
+        box->diag[0] = ske[0]; box->diag[1] = smx[0];
+        box->nsurf = sns[0];
+        box->status = *status;
     }
-    if (threadIdx.x == 0) { out[0] = ske[0]; out[1] = smx[0]; }
+    if (t < 6 && bf) box->diag[2 + t] = bf[t];
 }
 
 // Body force of the last RHS (Moving_Square.../Calculate_Body_Force.f90:53-142 and
@@ -503,14 +525,6 @@ __global__ void k_body_force_final(int nparts, const double* part, double* out) 
         if (threadIdx.x == 0) out[c] = sh[0];
         __syncthreads();
     }
-}
-
-// Count of flagged surface particles (diagnostics).
-template <typename R>
-__global__ void k_count_surface(Params P, Sorted<R> D, int* out) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= P.n_tot) return;
-    if (D.flags[s] & 1) atomicAdd(out, 1);
 }
 
 // --- find_particle_pair entry point ---------------------------------------

@@ -1875,12 +1875,12 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_ghost_lambda(Params P, Sort
             lp = pbar * inv; lu = ubar * inv; lv = vbar * inv; lm = A.sm[s] * inv;
             lw = -(lp * pint + lu * uint + lv * vint + lm * m);
             double a0 = 0.0, a1 = 0.0;
-            ghost_visit_warp(P, D, s, [&](int b, double dx, double dy, double q, double w) {
-                const double4 kb = D.kin[b];
+            ghost_visit_warp(P, D, s, [&](int b, double dx, double dy, double s2, double w) {
+                const double4 kb = load4(&D.kin[b]);
                 const double mb = D.mass[b];
-                const double Vb = mb / kb.z, W = w * Vb;
+                const double Vb = mb * rcp64(kb.z), W = w * Vb;
                 const double Wb = lp * (kb.w + kb.z * (gxe * dx + gye * dy)) + lu * kb.x + lv * kb.y + lm * mb + lw;
-                const double k = Wb * Vb * ghost_dw_over_d(P, q);
+                const double k = Wb * Vb * ghost_dw_over_d(P, s2);
                 const double cg = lp * kb.z * W;
                 xs0 += k * dx + cg * gxe;
                 xs1 += k * dy + cg * gye;
@@ -1919,8 +1919,7 @@ __device__ __forceinline__ void ghost_water_one(const Params& P, const Sorted<R>
     const double2 xj = D.pos[j], x0 = D.pos0[j];
     const int cx = (int)floor((x0.x - P.gx0) / P.cs), cy = (int)floor((x0.y - P.gy0) / P.cs);
     const double4 kj = D.kin[j];
-    const double mj = D.mass[j], Vj = mj / kj.z;
-    const double hg = P.ghost_h;
+    const double mj = D.mass[j], ij = rcp64(kj.z), Vj = mj * ij;
     double x0b = 0, x1b = 0, ub = 0, vb = 0, pb = 0, rb = 0;
     const int gx0 = max(cx - P.ghost_cells, 0), gx1 = min(cx + P.ghost_cells, P.gnx - 1);
     for (int gy = max(cy - P.ghost_cells, 0); gy <= min(cy + P.ghost_cells, P.gny - 1); ++gy) {
@@ -1934,23 +1933,14 @@ __device__ __forceinline__ void ghost_water_one(const Params& P, const Sorted<R>
         }
         if (lo < 0) continue;
         for (int s = lo + lane; s < hi; s += 32) {
-            if (D.type[s] != SPH_TYPE_FIX_GHOST || D.id[s] >= P.n_host) continue;
             const double2 x = D.pos[s];
             const double dx = x.x - xj.x, dy = x.y - xj.y;
-            const double d = sqrt(dx * dx + dy * dy);
-            if (!(d <= P.ghost_r)) continue;
-            const double4 lam = A.glam[s];
+            const double s2 = dx * dx + dy * dy;
+            if (D.type[s] != SPH_TYPE_FIX_GHOST || D.id[s] >= P.n_host || !(s2 <= P.ghost_r2)) continue;
+            const double4 lam = load4(&A.glam[s]);
             const double lw = A.glamw[s];
             if (lam.x == 0.0 && lam.y == 0.0 && lam.z == 0.0 && lam.w == 0.0 && lw == 0.0) continue;
-            const double q = d / hg;
-            double w;
-            if (P.kernel_model == SPH_KERNEL_GAUSSIAN) {
-                w = (exp(-(q * q)) - P.gauss_e9) * P.ghost_kf;
-            } else {
-                const double tq = 1.0 - q / 2.0;
-                const double t2 = tq * tq;
-                w = P.ghost_kf * (1.0 + 2.0 * q) * (t2 * t2);
-            }
+            const double w = ghost_w(P, s2);
             const bool body = D.itype[s] == SPH_TYPE_BODY;
             const double gxe = P.grav[0] + (body ? bax : 0.0), gye = P.grav[1] + (body ? bay : 0.0);
             const double ge = gxe * dx + gye * dy;
@@ -1958,8 +1948,8 @@ __device__ __forceinline__ void ghost_water_one(const Params& P, const Sorted<R>
             ub += lam.y * W; vb += lam.z * W; pb += lam.x * W;
             rb += lam.x * W * ge;
             const double Wb = lam.x * (kj.w + kj.z * ge) + lam.y * kj.x + lam.z * kj.y + lam.w * mj + lw;
-            rb -= Wb * W / kj.z;
-            const double k = Wb * Vj * ghost_dw_over_d(P, q);
+            rb -= Wb * W * ij;
+            const double k = Wb * Vj * ghost_dw_over_d(P, s2);
             const double cg = lam.x * kj.z * W;
             x0b -= k * dx + cg * gxe;
             x1b -= k * dy + cg * gye;

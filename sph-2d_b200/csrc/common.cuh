@@ -29,6 +29,7 @@ struct Params {
     // ghost assignment (moving-square driver)
     int ghost_assign, wall_bc, ghost_cells;
     double ghost_h, ghost_r, ghost_kf, shock_t, grav[2];
+    double ghost_r2, ghost_ih2;   // squared interpolation radius, 1 / ghost_h^2
     // kernel / pair search
     double h, r_cut, cut_min, kfactor, gauss_e9, q_zero;
     double s_cut, s_min;     // the support test on the squared distance: the largest s with

@@ -604,6 +604,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         if (G.mode == STAGE_MID) {
             D.pos_n[a] = D.pos[a]; D.kin_n[a] = D.kin[a]; D.aux_n[a] = D.aux[a];
             if (F32) { D.vol64_n[a] = D.vol64[a]; D.kh_n[a] = D.kh[a]; D.kl_n[a] = D.kl[a]; D.xhl_n[a] = D.xhl[a]; }
+        } else if (MS && G.to_staging && ta == SPH_TYPE_FIX_GHOST) {
+            // a ghost ends the step with what the ghost assignment gave it
+            const int i = D.id[a];
+            G.S.vel[i] = D.vel0[a]; G.S.rho[i] = D.rho0[a]; G.S.mass[i] = D.mass[a]; G.S.smass[i] = D.smass[a];
         }
         return;
     }

@@ -149,7 +149,20 @@ __device__ __forceinline__ void image_counts(const Params& P, double2 x, bool il
     tb = band_count(x.y, P.box_lo[1], P.box_hi[1], P.band);
 }
 
-__global__ void __launch_bounds__(kImgThreads) k_img_count(Params P, Staging S, SetupBuf B, HostBox* box, unsigned seq) {
+// Body_Motion_Solver (Moving_Square.../Body_Motion_Solver.f90:187-193): the body
+// particles (initial type SPH_TYPE_BODY) move by the step's displacement.  Applied
+// by the kernel that first reads the positions of a step.
+__device__ __forceinline__ double2 move_body(const Staging& S, int i, double2 disp) {
+    double2 x = S.pos[i];
+    if ((disp.x != 0.0 || disp.y != 0.0) && S.itype[i] == SPH_TYPE_BODY) {
+        x = make_double2(x.x + disp.x, x.y + disp.y);
+        S.pos[i] = x;
+    }
+    return x;
+}
+
+__global__ void __launch_bounds__(kImgThreads) k_img_count(Params P, Staging S, SetupBuf B, HostBox* box, unsigned seq,
+                                                           double2 disp) {
     stamp_phase(P.stamp);
     __shared__ unsigned long long sh[32];
     __shared__ int flag;
@@ -157,7 +170,7 @@ __global__ void __launch_bounds__(kImgThreads) k_img_count(Params P, Staging S, 
     for (int c = i; c <= B.ncells; c += gridDim.x * kImgThreads) B.cnt[c] = 0;
     int lr = 0, tb = 0;
     if (i < P.n_host) {
-        const double2 xy = S.pos[i];
+        const double2 xy = move_body(S, i, disp);
         const bool ill = S.type[i] == SPH_TYPE_ILL;
         const double2 w = wrap_position(P, xy);
         if (!ill && (w.x != xy.x || w.y != xy.y)) S.pos[i] = w;
@@ -223,14 +236,14 @@ __device__ __forceinline__ void put_image(const Params& P, const Staging& S, con
 // left/right images; the low side first).  route: also keep the counts and
 // offsets for the reverse sweep.
 __global__ void __launch_bounds__(kImgThreads) k_img_emit(Params P, Staging S, SetupBuf B, int cap, int periodic,
-                                                          int route, unsigned* status) {
+                                                          int route, unsigned* status, double2 disp) {
     stamp_phase(P.stamp);
     __shared__ unsigned long long sh[32];
     const int i = blockIdx.x * kImgThreads + threadIdx.x;
     const bool live = i < P.n_host;
     double2 x = make_double2(0.0, 0.0);
     int t = SPH_TYPE_ILL;
-    if (live) { x = S.pos[i]; t = S.type[i]; }
+    if (live) { x = move_body(S, i, disp); t = S.type[i]; }
     if (live) cell_key(P, B, i, x, t, status);
     if (!periodic) return;
     int lr, tb;

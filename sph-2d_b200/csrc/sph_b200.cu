@@ -103,7 +103,10 @@ struct sph_handle {
     long long n_rhs = 0, n_steps = 0;
     long long launches = 0;
     double bf[6] = {0, 0, 0, 0, 0, 0};   // body force of the last RHS
-    double* d_bf = nullptr;               // [6 * blocks(cap_tot) partials + 6]
+    double* d_bf = nullptr;               // [6] the force, then its block partials
+    int* d_body_ids = nullptr;            // host particles of the body, from sph_set_initial_type
+    int n_body = 0, cap_body = 0;
+    double body_disp[2] = {0.0, 0.0};     // displacement of the body the next set-up applies
     bool bf_every_rhs = false;            // sph_rhs also reports it
     bool bf_pending = false;              // the device copy is newer than bf (read on demand)
     struct AdjCtx* adj = nullptr;         // saved context of sph_adjoint_forward
@@ -263,6 +266,8 @@ int derive_params(const sph_config& c, Params& P) {
     P.wall_bc = c.wall_bc;
     P.ghost_h = (q ? (double)(float)c.ghost_h_factor : c.ghost_h_factor) * c.h;
     P.ghost_r = c.kernel_scale * P.ghost_h;
+    P.ghost_r2 = P.ghost_r * P.ghost_r;
+    P.ghost_ih2 = 1.0 / (P.ghost_h * P.ghost_h);
     P.ghost_kf = c.kernel_model == SPH_KERNEL_GAUSSIAN
                      ? 1.0 / (pi_k * (P.ghost_h * P.ghost_h) * (q ? (double)(1.0f - 10.0f * expf(-9.0f))
                                                                   : 1.0 - 10.0 * exp(-9.0)))
@@ -425,10 +430,13 @@ int prepare(sph_handle* h, const StageArgs& first = StageArgs{}) {
     tic(h, PH_IMAGES);
     const int nhb = blocks(h->n_host, kImgThreads), ncb = blocks(h->ncells + 1, kScanCells);
     const int periodic = h->cfg.periodic ? 1 : 0;
-    if (periodic) k_img_count<<<nhb, kImgThreads, 0, h->stream>>>(P, h->S, B, h->d_box, ++h->box_seq);
+    const double2 disp = make_double2(h->body_disp[0], h->body_disp[1]);
+    if (periodic) k_img_count<<<nhb, kImgThreads, 0, h->stream>>>(P, h->S, B, h->d_box, ++h->box_seq, disp);
     else CK(cudaMemsetAsync(B.cnt, 0, sizeof(int) * (size_t)(h->ncells + 1), h->stream));
     // (the routing of image adjoints is kept once an adjoint run exists)
-    k_img_emit<<<nhb, kImgThreads, 0, h->stream>>>(P, h->S, B, h->cap_tot, periodic, h->adj != nullptr, h->d_status);
+    k_img_emit<<<nhb, kImgThreads, 0, h->stream>>>(P, h->S, B, h->cap_tot, periodic, h->adj != nullptr, h->d_status,
+                                                    periodic ? make_double2(0.0, 0.0) : disp);
+    h->body_disp[0] = h->body_disp[1] = 0.0;
     tic(h, PH_SORT);
     k_cell_scan<<<ncb, kScanThreads, 0, h->stream>>>(B, P.stamp);
     CK(cudaGetLastError());
@@ -535,12 +543,11 @@ int rhs(sph_handle* h, int last, const StageArgs& G = StageArgs{}, int keep_j = 
     CK(cudaGetLastError());
     h->launches += 2;
     if (P.has_body && (last || h->bf_every_rhs)) {
-        const int nbf = blocks(P.n_tot, kRedThreads);      // <= blocks(cap_tot), the partial buffer size
-        double* fin = h->d_bf + (size_t)6 * blocks(h->cap_tot, kRedThreads);
-        k_body_force<R><<<nbf, kRedThreads, 0, h->stream>>>(P, D, h->d_bf);
-        k_body_force_final<<<1, kRedThreads, 0, h->stream>>>(nbf, h->d_bf, fin);
+        double* fin = h->d_bf;
+        k_body_force<R><<<blocks((long long)h->n_body * 32, kRedThreads), kRedThreads, 0, h->stream>>>(
+            P, D, h->d_body_ids, h->n_body, h->d_bf + 6, fin, h->B.done + 3);
         h->bf_pending = true;
-        h->launches += 2;
+        h->launches += 1;
         if (h->drag_acc && last) {
             k_drag_acc<<<1, 32, 0, h->stream>>>(fin, h->drag_w, h->drag_acc);
             h->launches += 1;
@@ -619,13 +626,8 @@ int step_begin(sph_handle* h, double dt) {
         }
     }
     if (h->P.ghost_assign && (h->body_vel[0] != 0.0 || h->body_vel[1] != 0.0)) {
-        int rc = unsort<R>(h);
-        if (rc) return rc;
-        k_translate_body<<<blocks(h->n_host, 256), 256, 0, h->stream>>>(h->n_host, h->S.itype, h->S.pos,
-                                                                          h->body_vel[0] * dt, h->body_vel[1] * dt);
-        CK(cudaGetLastError());
-        h->launches += 1;
-        h->sorted_valid = false;
+        h->body_disp[0] = h->body_vel[0] * dt;
+        h->body_disp[1] = h->body_vel[1] * dt;
     }
     return SPH_OK;
 }
@@ -654,9 +656,9 @@ int run_steps(sph_handle* h, int nsteps, double dt) {
                 (rc = reinit_density<R>(h, h->cfg.shifting)))
                 return rc;
         } else {
-            // the Taylor-Green driver's final stage keeps the id-order staging current
-            // (the moving-square ghost assignment changes the sorted state outside it)
-            const int to_staging = (!pc && !h->P.ms && !h->P.ghost_assign) ? 1 : 0;
+            // the final stage keeps the id-order staging current (the ghost assignment
+            // with a Taylor-Green solver changes the sorted state outside it)
+            const int to_staging = (h->P.ms || !h->P.ghost_assign) ? 1 : 0;
             if ((rc = rhs<R>(h, 1, stage_args(h, STAGE_END, stn, dt, h->cfg.shifting, to_staging)))) return rc;
             if (to_staging) h->staging_valid = true;
         }
@@ -680,7 +682,7 @@ int diagnostics(sph_handle* h, sph_diag* result, bool with_status) {
         if (rc) return rc;
     }
     const Params& P = h->P;
-    const double* fin = h->bf_pending ? h->d_bf + (size_t)6 * blocks(h->cap_tot, kRedThreads) : nullptr;
+    const double* fin = h->bf_pending ? h->d_bf : nullptr;
     k_diag<R><<<std::min(kDiagBlocks, blocks(P.n_tot, kRedThreads)), kRedThreads, 0, h->stream>>>(
         P, sorted<R>(h), h->d_part, h->d_part + kDiagBlocks, h->d_int, h->B.done + 2, h->d_status, fin, h->d_box);
     CK(cudaGetLastError());
@@ -991,6 +993,7 @@ int prep_restore(sph_handle* h, int j, bool lists = true) {
     P.n_host = h->n_host;
     h->n_img = X->seg_nimg[j];
     h->n_lr = X->seg_nlr[j];
+    h->body_disp[0] = h->body_disp[1] = 0.0;       // the saved state has the body moved
     P.n_tot = h->n_host + h->n_img;
     tic(h, PH_SORT);
     unsigned* slot = X->prep + (size_t)j * X->prep_words;
@@ -1732,6 +1735,31 @@ int adjoint_backward(sph_handle* h, double dloss, double* g_vel0, double* g_rho0
     return SPH_OK;
 }
 
+// The body of the body-force integral: the host particles whose initial type is
+// SPH_TYPE_BODY.
+int set_body(sph_handle* h, int n, const int* itype) {
+    std::vector<int> ids;
+    for (int i = 0; i < n; ++i)
+        if (itype[i] == SPH_TYPE_BODY) ids.push_back(i);
+    h->P.has_body = ids.empty() ? 0 : 1;
+    if (ids.empty()) { h->n_body = 0; return SPH_OK; }
+    if (!h->d_body_ids || (int)ids.size() > h->cap_body) {
+        CK(cudaStreamSynchronize(h->stream));
+        cudaFree(h->d_body_ids);
+        cudaFree(h->d_bf);
+        h->d_body_ids = nullptr;
+        h->d_bf = nullptr;
+        h->cap_body = 0;
+        CK(dalloc(&h->d_body_ids, ids.size()));
+        CK(dalloc(&h->d_bf, 6 + 6 * (size_t)blocks((long long)ids.size() * 32, kRedThreads)));
+        h->cap_body = (int)ids.size();
+    }
+    h->n_body = (int)ids.size();
+    CK(cudaMemcpyAsync(h->d_body_ids, ids.data(), sizeof(int) * ids.size(), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    return SPH_OK;
+}
+
 // Dispatch on the pair precision of the handle.
 #define DISPATCH(h, fn, ...) ((h)->mixed ? fn<float>(__VA_ARGS__) : fn<double>(__VA_ARGS__))
 
@@ -1747,7 +1775,7 @@ void destroy(sph_handle* h) {
                     h->S.r_avg, h->S.lr_cnt, h->S.lr_off, h->S.tb_cnt, h->S.tb_off, h->B.blk, h->B.tot, h->B.done, h->B.key, h->B.rank,
                     h->B.cnt, h->B.pre, h->B.blkoff, h->B.perm, h->cub_tmp,
                     h->d_status, h->d_int, h->d_part, h->d_diag, h->d_xfer, h->d_export, h->d_off64, h->d_cnt_id,
-                    h->d_mls, h->d_ghost_ids, h->d_stamps};
+                    h->d_mls, h->d_ghost_ids, h->d_stamps, h->d_body_ids};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
     if (h->copy_stream) { cudaStreamSynchronize(h->copy_stream); cudaStreamDestroy(h->copy_stream); }
@@ -1790,15 +1818,14 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     CK(dalloc(&h->S.mass, cap)); CK(dalloc(&h->S.smass, cap)); CK(dalloc(&h->S.type, cap));
     CK(dalloc(&h->S.itype, cap));
     CK(dalloc(&h->S.blabel, cap)); CK(cudaMemset(h->S.blabel, 0, sizeof(int) * (size_t)cap));
-    CK(dalloc(&h->d_bf, (size_t)6 * blocks(cap, kRedThreads) + 6));
     CK(dalloc(&h->S.r_drho, h->cap_host)); CK(dalloc(&h->S.r_acc, h->cap_host)); CK(dalloc(&h->S.r_avg, h->cap_host));
     CK(dalloc(&h->S.lr_cnt, cap)); CK(dalloc(&h->S.lr_off, cap));
     CK(dalloc(&h->S.tb_cnt, cap)); CK(dalloc(&h->S.tb_off, cap));
     // set-up
     SetupBuf& B = h->B;
     B.ncells = h->ncells;
-    CK(dalloc(&B.blk, blocks(h->cap_host, kImgThreads))); CK(dalloc(&B.tot, 3)); CK(dalloc(&B.done, 3));
-    CK(cudaMemsetAsync(B.done, 0, 3 * sizeof(unsigned), h->stream));
+    CK(dalloc(&B.blk, blocks(h->cap_host, kImgThreads))); CK(dalloc(&B.tot, 3)); CK(dalloc(&B.done, 4));
+    CK(cudaMemsetAsync(B.done, 0, 4 * sizeof(unsigned), h->stream));
     CK(dalloc(&B.key, cap)); CK(dalloc(&B.rank, cap)); CK(dalloc(&B.perm, cap));
     CK(dalloc(&B.cnt, (size_t)h->ncells + 1)); CK(dalloc(&B.pre, (size_t)h->ncells + 1));
     CK(dalloc(&B.blkoff, blocks((long long)h->ncells + 1, kScanCells)));
@@ -1944,12 +1971,8 @@ int sph_set_initial_type(sph_handle* h, int n, const int* initial_type) {
     int rc = h->mixed ? unsort<float>(h) : unsort<double>(h);
     if (rc) return rc;
     CK(cudaMemcpyAsync(h->S.itype, initial_type, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    int body = 0;
-    for (int i = 0; i < n; ++i) body |= initial_type[i] == SPH_TYPE_BODY;
-    h->P.has_body = body;
     h->sorted_valid = false;
-    return SPH_OK;
+    return set_body(h, n, initial_type);
 }
 
 int sph_set_boundary_labels(sph_handle* h, int n, const int* labels) {
@@ -2102,18 +2125,15 @@ int sph_restart_load(sph_handle* h, const void* buf, size_t bytes) {
         (rc = put(h->S.r_avg, 16)))
         return rc;
     std::vector<int> g;
-    int body = 0;
-    for (size_t i = 0; i < nn; ++i) {
+    for (size_t i = 0; i < nn; ++i)
         if (type[i] == SPH_TYPE_FIX_GHOST) g.push_back((int)i);
-        body |= itype[i] == SPH_TYPE_BODY;
-    }
     if (!h->d_ghost_ids) CK(dalloc(&h->d_ghost_ids, h->cap_host));
     h->n_ghost = (int)g.size();
     if (!g.empty())
         CK(cudaMemcpyAsync(h->d_ghost_ids, g.data(), sizeof(int) * g.size(), cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->n_host = n;
-    h->P.has_body = body;
+    if ((rc = set_body(h, n, itype))) return rc;
     for (int c = 0; c < 6; ++c) h->bf[c] = 0.0;
     h->bf_pending = false;
     h->staging_valid = true;

@@ -222,63 +222,59 @@ __global__ void k_finish_mls(Params P, Sorted<R> D, const double* rho_new, int d
     store_split(D, s, make_double2(x, y), make_double4(v.x, v.y, rho, p));
 }
 
-// Body_Motion_Solver (Moving_Square.../Body_Motion_Solver.f90:187-193): the body
-// particles (initial type SPH_TYPE_BODY) move by the step's displacement.
-__global__ void k_translate_body(int n, const int* itype, double2* pos, double dx, double dy) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || itype[i] != SPH_TYPE_BODY) return;
-    const double2 x = pos[i];
-    pos[i] = make_double2(x.x + dx, x.y + dy);
+// Ghost kernel value at squared distance s2.
+__device__ __forceinline__ double ghost_w(const Params& P, double s2) {
+    if (P.kernel_model == SPH_KERNEL_GAUSSIAN) return (exp(-(s2 * P.ghost_ih2)) - P.gauss_e9) * P.ghost_kf;
+    const double q = sqrt(s2 * P.ghost_ih2);
+    const double tq = 1.0 - 0.5 * q, t2 = tq * tq;
+    return P.ghost_kf * (1.0 + 2.0 * q) * (t2 * t2);
 }
-
-// (dw/dd) / d of the ghost kernel at q = d / h_g.
-__device__ __forceinline__ double ghost_dw_over_d(const Params& P, double q) {
-    const double hg2 = P.ghost_h * P.ghost_h;
-    if (P.kernel_model == SPH_KERNEL_GAUSSIAN) return -2.0 * exp(-(q * q)) * P.ghost_kf / hg2;
-    const double tq = 1.0 - q / 2.0;
-    return -5.0 * (tq * tq * tq) * P.ghost_kf / hg2;
+// (dw/dd) / d of it.
+__device__ __forceinline__ double ghost_dw_over_d(const Params& P, double s2) {
+    if (P.kernel_model == SPH_KERNEL_GAUSSIAN) return -2.0 * exp(-(s2 * P.ghost_ih2)) * P.ghost_kf * P.ghost_ih2;
+    const double tq = 1.0 - 0.5 * sqrt(s2 * P.ghost_ih2);
+    return -5.0 * (tq * tq * tq) * P.ghost_kf * P.ghost_ih2;
 }
 
 // The neighbours the ghost assignment interpolates from for ghost slot s: the
 // non-ghost particles within kernel_scale * 1.2 h, found over the window of s's
 // cell (the list-build cells, so the window reaches ghost_r plus half the skin).
-// The 32 lanes of a warp split the candidates of each window row (the slots of
-// a row's window cells are contiguous in the cell-sorted order); fn(b, dx, dy,
-// q, w) gets (dx, dy) = x_s - x_b, q = d / h_g and the kernel value w with the
-// ghost smoothing length h_g, on the lane that visits b.
+// Lane k finds the slot range of the window's row k (the slots of a row's window
+// cells are contiguous in the cell-sorted order), so the ranges are one round of
+// loads; then the 32 lanes split the candidates of each row.  fn(b, dx, dy, s2, w)
+// gets (dx, dy) = x_s - x_b, the squared distance and the kernel value with the
+// ghost smoothing length, on the lane that visits b.
 template <typename R, typename F>
 __device__ __forceinline__ void ghost_visit_warp(const Params& P, const Sorted<R>& D, int s, F&& fn) {
     const int lane = threadIdx.x & 31;
     const double2 x = D.pos[s];
     const int cx = (int)floor((x.x - P.gx0) / P.cs), cy = (int)floor((x.y - P.gy0) / P.cs);
-    const double hg = P.ghost_h;
     const int gx0 = max(cx - P.ghost_cells, 0), gx1 = min(cx + P.ghost_cells, P.gnx - 1);
-    for (int gy = max(cy - P.ghost_cells, 0); gy <= min(cy + P.ghost_cells, P.gny - 1); ++gy) {
-        const int row = gy * P.gnx;
-        int lo = -1, hi = -1;
-        for (int gx = gx0; gx <= gx1; ++gx) {
-            const int b0 = D.cell_start[row + gx];
-            if (b0 < 0) continue;
-            if (lo < 0) lo = b0;
-            hi = D.cell_end[row + gx];
-        }
-        if (lo < 0) continue;
-        for (int b = lo + lane; b < hi; b += 32) {
-            if (D.type[b] == SPH_TYPE_FIX_GHOST) continue;
-            const double2 xb = D.pos[b];
-            const double dx = x.x - xb.x, dy = x.y - xb.y;
-            const double d = sqrt(dx * dx + dy * dy);
-            if (!(d <= P.ghost_r)) continue;
-            const double q = d / hg;
-            double w;
-            if (P.kernel_model == SPH_KERNEL_GAUSSIAN) {
-                w = (exp(-(q * q)) - P.gauss_e9) * P.ghost_kf;
-            } else {
-                const double tq = 1.0 - q / 2.0;
-                const double t2 = tq * tq;
-                w = P.ghost_kf * (1.0 + 2.0 * q) * (t2 * t2);
+    const int gy0 = max(cy - P.ghost_cells, 0), gy1 = min(cy + P.ghost_cells, P.gny - 1);
+    for (int r0 = gy0; r0 <= gy1; r0 += 32) {
+        int lo = 0, hi = 0;
+        if (r0 + lane <= gy1) {
+            const int row = (r0 + lane) * P.gnx;
+            int first = -1;
+            for (int gx = gx0; gx <= gx1; ++gx) {
+                const int b0 = D.cell_start[row + gx], b1 = D.cell_end[row + gx];
+                if (b0 < 0) continue;
+                if (first < 0) first = b0;
+                hi = b1;
             }
-            fn(b, dx, dy, q, w);
+            lo = max(first, 0);
+        }
+        const int rows = min(gy1 - r0 + 1, 32);
+        for (int k = 0; k < rows; ++k) {
+            const int end = __shfl_sync(0xffffffffu, hi, k);
+            for (int b = __shfl_sync(0xffffffffu, lo, k) + lane; b < end; b += 32) {
+                const double2 xb = D.pos[b];
+                const int tb = D.type[b];
+                const double dx = x.x - xb.x, dy = x.y - xb.y;
+                const double s2 = dx * dx + dy * dy;
+                if (tb == SPH_TYPE_FIX_GHOST || !(s2 <= P.ghost_r2)) continue;
+                fn(b, dx, dy, s2, ghost_w(P, s2));
+            }
         }
     }
 }
@@ -324,9 +320,9 @@ __global__ void k_assign_ghosts(Params P, Sorted<R> D, const int* ghost_ids, int
     double sw = 0.0, sp = 0.0, su = 0.0, sv = 0.0, sm = 0.0;
     int cnt = 0;
     ghost_visit_warp(P, D, s, [&](int b, double dx, double dy, double, double w) {
-        const double4 kb = D.kin[b];
+        const double4 kb = load4(&D.kin[b]);
         const double mb = D.mass[b];
-        const double W = w * (mb / kb.z);
+        const double W = w * (mb * rcp64(kb.z));
         sw += W;
         sp += kb.w * W + kb.z * W * (gxe * dx + gye * dy);
         su += kb.x * W;
@@ -464,67 +460,81 @@ __global__ void __launch_bounds__(kRedThreads) k_diag(Params P, Sorted<R> D, dou
 //       or   sum_b rho_a V_b 2 (dim+2) nu ((v_a-v_b).(x_a-x_b)) / r^2 B_a^-1 grad_a W_ab
 // and the forces are sum_a V_a BFP_a, sum_a V_a BFV_a and their sum (no gravity).
 // Gathered from the body side: body particle b sums V_a times its terms over its
-// pair neighbours a (the pair set is symmetric), so only the body's threads loop.
+// pair neighbours a (the pair set is symmetric), one warp per body particle
+// (body_ids: the body's host particles) with the lanes on the pairs; the last
+// block adds the block partials (part, [6][blocks]) in a fixed order into out.
+// A thread per particle of the whole tank left a few warps with chains of up to
+// 45 neighbours, and a second launch for the sum: pass C and the force together
+// 84 -> 52 us per step at D/30 (FP64), 440 -> 389 us at D/100 (mixed).
 template <typename R>
-__global__ void k_body_force(Params P, Sorted<R> D, double* part) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    double f[6] = {0, 0, 0, 0, 0, 0};
-    if (b < P.n_tot && D.itype[b] == SPH_TYPE_BODY) {
+__global__ void __launch_bounds__(kRedThreads) k_body_force(Params P, Sorted<R> D, const int* body_ids, int n_body,
+                                                            double* part, double* out, unsigned* done) {
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int g = (blockIdx.x * kRedThreads + t) >> 5;
+    double f[4] = {0, 0, 0, 0};
+    if (g < n_body) {
+        const int b = D.slot_of[body_ids[g]];
         const int nn = D.npairs[b];
-        const double2 xb = D.pos[b];
-        const double4 kb = D.kin[b];
-        const double Vb = D.mass[b] / kb.z;
-        for (int e = 0; e < nn; ++e) {
-            const int a = (int)(D.pairs[(size_t)e * P.nbr_stride + b] & 0x7fffffffu);
-            const double2 xa = D.pos[a];
-            const double4 ka = D.kin[a];
-            const double4 bi = D.binv64[a];
-            const double Va = D.mass[a] / ka.z;
-            const double dx = xa.x - xb.x, dy = xa.y - xb.y;
-            const double r2 = dx * dx + dy * dy, d = sqrt(r2);
-            double w, gx, gy;
-            kernel_w_dw<double>(P, d, dx, dy, w, gx, gy);
-            const double n0 = bi.x * gx + bi.y * gy, n1 = bi.z * gx + bi.w * gy;
-            const double bp0 = -Vb * (ka.w + kb.w) * n0, bp1 = -Vb * (ka.w + kb.w) * n1;
-            const double du = ka.x - kb.x, dv = ka.y - kb.y;
-            double bv0, bv1;
-            if (P.laplacian == 1) {
-                const double fv = ka.z * Vb * 2 * P.nu * (dx * n0 + dy * n1) / r2;
-                bv0 = fv * du; bv1 = fv * dv;
-            } else {
-                const double fv = ka.z * Vb * 2 * (2 + 2) * P.nu * (du * dx + dv * dy) / r2;
-                bv0 = fv * n0; bv1 = fv * n1;
+        if (nn > 0) {
+            const double2 xb = D.pos[b];
+            const double4 kb = load4(&D.kin[b]);
+            const double Vb = D.mass[b] * rcp64(kb.z);
+            for (int e = lane; e < nn; e += 32) {
+                const int a = (int)(D.pairs[(size_t)e * P.nbr_stride + b] & 0x7fffffffu);
+                const double2 xa = D.pos[a];
+                const double4 ka = load4(&D.kin[a]), bi = load4(&D.binv64[a]);
+                const double Va = D.mass[a] * rcp64(ka.z);
+                const double dx = xa.x - xb.x, dy = xa.y - xb.y;
+                const double s2 = dx * dx + dy * dy;
+                // grad_a W = G (x_a - x_b)
+                double G;
+                if (P.kernel_model == SPH_KERNEL_GAUSSIAN) G = exp(-(s2 * P.inv_h2)) * P.gk;
+                else { const double tq = 1.0 - s2 * rsqrt64(s2) * P.half_inv_h; G = P.gk * (tq * tq * tq); }
+                const double gx = G * dx, gy = G * dy;
+                const double n0 = bi.x * gx + bi.y * gy, n1 = bi.z * gx + bi.w * gy;
+                const double fp = -Va * Vb * (ka.w + kb.w);
+                f[0] += fp * n0; f[1] += fp * n1;
+                const double du = ka.x - kb.x, dv = ka.y - kb.y;
+                const double fv = Va * ka.z * Vb * 2 * P.nu * rcp64(s2);
+                if (P.laplacian == 1) {
+                    const double l = fv * (dx * n0 + dy * n1);
+                    f[2] += l * du; f[3] += l * dv;
+                } else {
+                    const double l = fv * (2 + 2) * (du * dx + dv * dy);
+                    f[2] += l * n0; f[3] += l * n1;
+                }
             }
-            f[0] += Va * bp0; f[1] += Va * bp1; f[2] += Va * bv0; f[3] += Va * bv1;
-            f[4] += Va * (bp0 + bv0); f[5] += Va * (bp1 + bv1);
         }
     }
-    __shared__ double sh[6][kRedThreads];
-    for (int c = 0; c < 6; ++c) sh[c][threadIdx.x] = f[c];
+    __shared__ double sh[4][kRedThreads / 32];
+    __shared__ int flag;
+    auto reduce = [&]() {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            for (int o = 16; o > 0; o >>= 1) f[c] += __shfl_down_sync(0xffffffffu, f[c], o);
+            if (lane == 0) sh[c][w] = f[c];
+        }
+        __syncthreads();
+        if (t < 4) {
+            double v = 0.0;
+            for (int k = 0; k < kRedThreads / 32; ++k) v += sh[t][k];
+            f[0] = v;                       // thread c: component c
+        }
+    };
+    reduce();
+    if (t < 4) part[(size_t)t * gridDim.x + blockIdx.x] = f[0];
+    if (!last_block(done, &flag)) return;
+    for (int c = 0; c < 4; ++c) {
+        f[c] = 0.0;
+        for (int i = t; i < (int)gridDim.x; i += kRedThreads) f[c] += __ldcg(&part[(size_t)c * gridDim.x + i]);
+    }
+    reduce();
+    if (t < 4) {
+        out[t] = f[0];
+        sh[t][0] = f[0];
+    }
     __syncthreads();
-    for (int w = kRedThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int c = 0; c < 6; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int c = 0; c < 6; ++c) part[(size_t)c * gridDim.x + blockIdx.x] = sh[c][0];
-}
-
-__global__ void k_body_force_final(int nparts, const double* part, double* out) {
-    __shared__ double sh[kRedThreads];
-    for (int c = 0; c < 6; ++c) {
-        double s = 0.0;
-        for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += part[(size_t)c * nparts + i];
-        sh[threadIdx.x] = s;
-        __syncthreads();
-        for (int w = kRedThreads / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[c] = sh[0];
-        __syncthreads();
-    }
+    if (t < 2) out[4 + t] = sh[t][0] + sh[2 + t][0];
 }
 
 // --- find_particle_pair entry point ---------------------------------------

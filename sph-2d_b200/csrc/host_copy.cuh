@@ -1,0 +1,167 @@
+// host_copy.cuh -- copies between device buffers and the caller's arrays.
+//
+// The caller's arrays are ordinary (pageable) Fortran or numpy memory as a rule.
+// The driver copies such memory through a buffer of its own, one array after
+// another with a wait each, at 3 to 8 GB/s.  Here the pieces of all arrays of a
+// call go through page-locked chunks of the handle: the DMA of one chunk runs
+// while the one before it is copied to (from) the caller's memory, by up to four
+// threads when there is enough to share.  Page-locked arrays are copied
+// directly.  Every call returns when its copies are complete.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <atomic>
+#include <cstring>
+#include <initializer_list>
+#include <new>
+#include <system_error>
+#include <thread>
+#include <vector>
+
+namespace sph {
+
+struct HostSeg {
+    void* host;
+    void* dev;
+    size_t bytes;
+};
+
+class HostCopy {
+public:
+    ~HostCopy() { release(); }
+    void release() {
+        for (int t = 0; t < kLanes; ++t)
+            for (int k = 0; k < 2; ++k) {
+                if (lane_[t].ev[k]) cudaEventDestroy(lane_[t].ev[k]);
+                if (lane_[t].buf[k]) cudaFreeHost(lane_[t].buf[k]);
+                lane_[t].ev[k] = nullptr;
+                lane_[t].buf[k] = nullptr;
+            }
+    }
+    // Device to host (to_host) or host to device on `stream`; complete on return.
+    // Null host pointers are skipped.
+    cudaError_t copy(int device, cudaStream_t stream, std::initializer_list<HostSeg> segs, bool to_host) {
+        try {
+            return copy_segs(device, stream, segs, to_host);
+        } catch (const std::bad_alloc&) {
+            return cudaErrorMemoryAllocation;
+        }
+    }
+
+private:
+    cudaError_t copy_segs(int device, cudaStream_t stream, std::initializer_list<HostSeg> segs, bool to_host) {
+        std::vector<HostSeg> pieces;
+        size_t total = 0;
+        for (const HostSeg& s : segs) {
+            if (!s.host || s.bytes == 0) continue;
+            if (page_locked(s.host)) {
+                const cudaError_t e = to_host ? cudaMemcpyAsync(s.host, s.dev, s.bytes, cudaMemcpyDeviceToHost, stream)
+                                              : cudaMemcpyAsync(s.dev, s.host, s.bytes, cudaMemcpyHostToDevice, stream);
+                if (e != cudaSuccess) return e;
+                continue;
+            }
+            for (size_t o = 0; o < s.bytes; o += kChunk)
+                pieces.push_back({(char*)s.host + o, (char*)s.dev + o, s.bytes - o < kChunk ? s.bytes - o : kChunk});
+            total += s.bytes;
+        }
+        // small pieces share a chunk
+        std::vector<Chunk> chunks;
+        for (const HostSeg& p : pieces) {
+            if (chunks.empty() || chunks.back().bytes + pad(p.bytes) > kChunk) chunks.push_back(Chunk{});
+            chunks.back().segs.push_back(p);
+            chunks.back().bytes += pad(p.bytes);
+        }
+        int lanes = 1;
+        if (total >= kShare) {
+            const unsigned hw = std::thread::hardware_concurrency();
+            lanes = hw >= 8 ? kLanes : hw >= 4 ? 2 : 1;
+        }
+        for (int t = 0; t < lanes && !chunks.empty(); ++t)
+            for (int k = 0; k < 2; ++k) {
+                cudaError_t e = cudaSuccess;
+                if (!lane_[t].buf[k] && (e = cudaHostAlloc(&lane_[t].buf[k], kChunk, cudaHostAllocDefault)) != cudaSuccess)
+                    return e;
+                if (!lane_[t].ev[k] &&
+                    (e = cudaEventCreateWithFlags(&lane_[t].ev[k], cudaEventDisableTiming)) != cudaSuccess)
+                    return e;
+            }
+        std::atomic<int> err{cudaSuccess};
+        auto work = [&](int t) {
+            if (t > 0) cudaSetDevice(device);
+            const cudaError_t e = run_lane(lane_[t], stream, chunks, t, lanes, to_host);
+            if (e != cudaSuccess) err = e;
+        };
+        std::thread helper[kLanes];
+        int started = 1;
+        for (; started < lanes; ++started) {
+            try {
+                helper[started] = std::thread(work, started);
+            } catch (const std::system_error&) {
+                break;                       // no more threads: this one takes their chunks
+            }
+        }
+        work(0);
+        for (int t = started; t < lanes; ++t) work(t);
+        for (int t = 1; t < started; ++t) helper[t].join();
+        const cudaError_t e = cudaStreamSynchronize(stream);
+        return err != cudaSuccess ? (cudaError_t)err.load() : e;
+    }
+
+    static constexpr size_t kChunk = size_t(1) << 20;      // 1 MiB: 20 us of PCIe, 8 MiB held at most
+    static constexpr size_t kShare = size_t(4) << 20;      // a thread costs about 30 us to start
+    static constexpr int kLanes = 4;
+    struct Chunk {
+        std::vector<HostSeg> segs;
+        size_t bytes = 0;
+    };
+    struct Lane {
+        void* buf[2] = {nullptr, nullptr};
+        cudaEvent_t ev[2] = {nullptr, nullptr};
+    };
+    Lane lane_[kLanes];
+
+    static size_t pad(size_t b) { return (b + 255) & ~size_t(255); }
+    static bool page_locked(const void* p) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
+        return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
+    }
+    // Chunks t, t + lanes, ...: two buffers, the DMA of one while the other is
+    // copied by this thread.
+    static cudaError_t run_lane(Lane& l, cudaStream_t stream, const std::vector<Chunk>& chunks, int t, int lanes,
+                                bool to_host) {
+        cudaError_t e = cudaSuccess;
+        const Chunk* behind = nullptr;          // to host: the chunk whose DMA is in flight
+        int k = 0;
+        auto unpack = [&](const Chunk& c, int b) {
+            if ((e = cudaEventSynchronize(l.ev[b])) != cudaSuccess) return;
+            size_t o = 0;
+            for (const HostSeg& s : c.segs) {
+                memcpy(s.host, (char*)l.buf[b] + o, s.bytes);
+                o += pad(s.bytes);
+            }
+        };
+        bool used[2] = {false, false};
+        for (size_t i = t; i < chunks.size() && e == cudaSuccess; i += lanes, k ^= 1) {
+            const Chunk& c = chunks[i];
+            if (!to_host && used[k]) e = cudaEventSynchronize(l.ev[k]);      // its DMA must be done
+            size_t o = 0;
+            for (const HostSeg& s : c.segs) {
+                char* pin = (char*)l.buf[k] + o;
+                if (e != cudaSuccess) break;
+                if (!to_host) memcpy(pin, s.host, s.bytes);
+                e = to_host ? cudaMemcpyAsync(pin, s.dev, s.bytes, cudaMemcpyDeviceToHost, stream)
+                            : cudaMemcpyAsync(s.dev, pin, s.bytes, cudaMemcpyHostToDevice, stream);
+                o += pad(s.bytes);
+            }
+            if (e == cudaSuccess) e = cudaEventRecord(l.ev[k], stream);
+            used[k] = true;
+            if (to_host && behind && e == cudaSuccess) unpack(*behind, k ^ 1);
+            behind = &c;
+        }
+        if (to_host && behind && e == cudaSuccess) unpack(*behind, k ^ 1);
+        return e;
+    }
+};
+
+}  // namespace sph

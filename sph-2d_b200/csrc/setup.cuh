@@ -86,6 +86,7 @@ struct HostBox {
     unsigned status;
     int nsurf;
     double diag[8];
+    long long pair_last[2];       // offset and count of the last particle's pairs
 };
 
 __device__ __forceinline__ int band_count(double v, double lo, double hi, double band) {

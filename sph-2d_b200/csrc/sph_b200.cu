@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "adjoint.cuh"
+#include "host_copy.cuh"
 
 using namespace sph;
 
@@ -89,8 +90,10 @@ struct sph_handle {
     double* d_diag = nullptr;
     double* d_xfer = nullptr;       // column-major transfer scratch [cap_host * 6]
     double* d_export = nullptr;     // k_export output (lazy)
-    long long* d_off64 = nullptr;   // pair offsets (lazy)
-    int* d_cnt_id = nullptr;
+    long long* d_off64 = nullptr;   // pair offsets and counts (lazy)
+    void* d_pairs = nullptr;        // emitted pairs, kept up to kKeepPairs bytes
+    size_t cap_pairs = 0;
+    HostCopy copier;                // page-locked chunks for the caller's arrays
     // timing
     bool timing = true;
     std::vector<cudaEvent_t> ev_pool;     // begin and end of each timed stretch
@@ -703,51 +706,66 @@ int diagnostics(sph_handle* h, sph_diag* result, bool with_status) {
     return SPH_OK;
 }
 
-__global__ void k_to_ll(int n, const int* in, long long* out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = in[i];
+// Copies between device buffers and the caller's arrays, complete on return.
+int to_host(sph_handle* h, std::initializer_list<HostSeg> segs) {
+    CK(h->copier.copy(h->device, h->stream, segs, true));
+    return SPH_OK;
 }
+int from_host(sph_handle* h, std::initializer_list<HostSeg> segs) {
+    CK(h->copier.copy(h->device, h->stream, segs, false));
+    return SPH_OK;
+}
+HostSeg hin(const void* host, void* dev, size_t bytes) { return HostSeg{const_cast<void*>(host), dev, bytes}; }
 
-// find_particle_pair on the current (prepared) state.
+// find_particle_pair on the state prepare has just sorted; the status of that
+// comes with the pair count in one wait.
+constexpr size_t kKeepPairs = size_t(256) << 20;
 template <typename R>
 int find_pairs(sph_handle* h, long long pair_cap, int* pi, int* pj, double* w, double* dwdx, long long* total) {
     const Params& P = h->P;
     const int n = P.n_tot;
-    if (!h->d_cnt_id) CK(dalloc(&h->d_cnt_id, h->cap_tot));
     if (!h->d_off64) CK(dalloc(&h->d_off64, 2 * ((size_t)h->cap_tot + 1)));
     long long* cnt64 = h->d_off64 + (h->cap_tot + 1);
-    k_pair_count<R><<<blocks(n, 128), 128, 0, h->stream>>>(P, sorted<R>(h), h->d_cnt_id);
-    k_to_ll<<<blocks(n, 256), 256, 0, h->stream>>>(n, h->d_cnt_id, cnt64);
+    k_pair_count<R><<<blocks(n, 128), 128, 0, h->stream>>>(P, sorted<R>(h), cnt64);
     size_t bytes = 0;
     CK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, cnt64, h->d_off64, n, h->stream));
     if (bytes > h->cub_bytes) return SPH_E_CAPACITY;
     CK(cub::DeviceScan::ExclusiveSum(h->cub_tmp, bytes, cnt64, h->d_off64, n, h->stream));
-    long long last[2];
+    long long* last = h->box->pair_last;
     CK(cudaMemcpyAsync(&last[0], h->d_off64 + n - 1, sizeof(long long), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaMemcpyAsync(&last[1], cnt64 + n - 1, sizeof(long long), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    int rc = read_status(h);
+    if (rc) return rc;
     *total = last[0] + last[1];
     h->last_pairs = *total;
     if (pi == nullptr || pair_cap <= 0) return SPH_OK;
-    const long long m = std::min(*total, pair_cap);
-    int *dpi = nullptr, *dpj = nullptr;
-    double *dw = nullptr, *ddw = nullptr;
-    CK(dalloc(&dpi, m)); CK(dalloc(&dpj, m));
-    if (w) CK(dalloc(&dw, m));
-    if (dwdx) CK(dalloc(&ddw, 2 * m));
-    k_pair_emit<R><<<blocks(n, 128), 128, 0, h->stream>>>(P, sorted<R>(h), h->d_off64, m, dpi, dpj, dw, ddw);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(pi, dpi, sizeof(int) * m, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(pj, dpj, sizeof(int) * m, cudaMemcpyDeviceToHost, h->stream));
-    if (w) CK(cudaMemcpyAsync(w, dw, sizeof(double) * m, cudaMemcpyDeviceToHost, h->stream));
-    if (dwdx) {
-        CK(cudaMemcpyAsync(dwdx, ddw, sizeof(double) * m, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaMemcpyAsync(dwdx + pair_cap, ddw + m, sizeof(double) * m, cudaMemcpyDeviceToHost, h->stream));
+    const size_t m = (size_t)std::min(*total, pair_cap);
+    // w, dwdx, pair_i, pair_j of m pairs
+    const size_t need = std::max<size_t>(m, 1) * (sizeof(double) * 3 + sizeof(int) * 2);
+    if (need > h->cap_pairs) {
+        cudaFree(h->d_pairs);
+        h->d_pairs = nullptr;
+        h->cap_pairs = 0;
+        const size_t room = need <= kKeepPairs ? need + need / 8 : need;
+        CK(cudaMalloc(&h->d_pairs, room));
+        h->cap_pairs = room;
     }
-    CK(cudaStreamSynchronize(h->stream));
-    cudaFree(dpi); cudaFree(dpj);
-    if (dw) cudaFree(dw);
-    if (ddw) cudaFree(ddw);
+    double* dw = static_cast<double*>(h->d_pairs);
+    double* ddw = dw + m;
+    int* dpi = reinterpret_cast<int*>(ddw + 2 * m);
+    int* dpj = dpi + m;
+    k_pair_emit<R><<<blocks(n, 128), 128, 0, h->stream>>>(P, sorted<R>(h), h->d_off64, (long long)m, dpi, dpj,
+                                                          w ? dw : nullptr, dwdx ? ddw : nullptr);
+    CK(cudaGetLastError());
+    rc = to_host(h, {{pi, dpi, sizeof(int) * m}, {pj, dpj, sizeof(int) * m}, {w, dw, sizeof(double) * m},
+                     {dwdx, ddw, sizeof(double) * m},
+                     {dwdx ? dwdx + pair_cap : nullptr, ddw + m, sizeof(double) * m}});
+    if (h->cap_pairs > kKeepPairs) {
+        cudaFree(h->d_pairs);
+        h->d_pairs = nullptr;
+        h->cap_pairs = 0;
+    }
+    if (rc) return rc;
     return *total > pair_cap ? SPH_E_CAPACITY : SPH_OK;
 }
 
@@ -1130,7 +1148,7 @@ int adjoint_forward(sph_handle* h, const sph_adj_config* ac, double* loss) {
     if (h->P.mls_order && X->stage_slots < X->every) return SPH_E_CAPACITY;
     const int n = h->n_host;
     if (ac->loss == SPH_LOSS_VELOCITY_MISFIT) {
-        CK(cudaMemcpyAsync(h->d_xfer, ac->target_vel, sizeof(double) * 2 * n, cudaMemcpyHostToDevice, h->stream));
+        if ((rc = from_host(h, {hin(ac->target_vel, h->d_xfer, sizeof(double) * 2 * n)}))) return rc;
         k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, h->d_xfer, X->target);
         h->launches += 1;
     }
@@ -1709,19 +1727,12 @@ int adjoint_backward(sph_handle* h, double dloss, double* g_vel0, double* g_rho0
     toc(h);
     if ((rc = read_status(h))) return rc;
     // gradients with respect to the state the forward started from (id order)
-    if (g_vel0) {
-        k_deinterleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, A.lv, h->d_xfer);
-        CK(cudaMemcpyAsync(g_vel0, h->d_xfer, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-    }
-    if (g_pos0) {
-        k_deinterleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, A.lx, h->d_xfer);
-        CK(cudaMemcpyAsync(g_pos0, h->d_xfer, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-    }
-    if (g_rho0) CK(cudaMemcpyAsync(g_rho0, A.lrho, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
-    if (g_params) CK(cudaMemcpyAsync(g_params, A.nu_acc, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    double* gx = h->d_xfer + 2 * (size_t)n;
+    if (g_vel0) k_deinterleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, A.lv, h->d_xfer);
+    if (g_pos0) k_deinterleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, A.lx, gx);
+    if ((rc = to_host(h, {{g_vel0, h->d_xfer, sizeof(double) * 2 * n}, {g_pos0, gx, sizeof(double) * 2 * n},
+                          {g_rho0, A.lrho, sizeof(double) * n}, {g_params, A.nu_acc, sizeof(double)}})))
+        return rc;
     // the handle continues from the forward's final state
     if ((rc = snap_io(h, X->ck, X->nseg, n, false))) return rc;
     h->step_count = X->step0 + X->nsteps;
@@ -1774,7 +1785,7 @@ void destroy(sph_handle* h) {
                     h->S.r_drho, h->S.r_acc,
                     h->S.r_avg, h->S.lr_cnt, h->S.lr_off, h->S.tb_cnt, h->S.tb_off, h->B.blk, h->B.tot, h->B.done, h->B.key, h->B.rank,
                     h->B.cnt, h->B.pre, h->B.blkoff, h->B.perm, h->cub_tmp,
-                    h->d_status, h->d_int, h->d_part, h->d_diag, h->d_xfer, h->d_export, h->d_off64, h->d_cnt_id,
+                    h->d_status, h->d_int, h->d_part, h->d_diag, h->d_xfer, h->d_export, h->d_off64, h->d_pairs,
                     h->d_mls, h->d_ghost_ids, h->d_stamps, h->d_body_ids};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
@@ -1859,17 +1870,13 @@ int get_state_impl(sph_handle* h, int n, double* pos, double* vel, double* rho, 
     if (rc) return rc;
     // one pass packs x, v (column-major), rho and the pressure (status_equation
     // on the device) into the transfer buffer; the requested blocks are then
-    // copied back with a single wait at the end
+    // copied back
     k_snapshot<<<blocks(n, 256), 256, 0, h->stream>>>(h->P, n, h->S.pos, h->S.vel, h->S.rho, h->d_xfer);
     CK(cudaGetLastError());
     h->launches += 1;
     const size_t nn = (size_t)n;
-    if (pos) CK(cudaMemcpyAsync(pos, h->d_xfer, sizeof(double) * 2 * nn, cudaMemcpyDeviceToHost, h->stream));
-    if (vel) CK(cudaMemcpyAsync(vel, h->d_xfer + 2 * nn, sizeof(double) * 2 * nn, cudaMemcpyDeviceToHost, h->stream));
-    if (rho) CK(cudaMemcpyAsync(rho, h->d_xfer + 4 * nn, sizeof(double) * nn, cudaMemcpyDeviceToHost, h->stream));
-    if (press) CK(cudaMemcpyAsync(press, h->d_xfer + 5 * nn, sizeof(double) * nn, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    return SPH_OK;
+    return to_host(h, {{pos, h->d_xfer, sizeof(double) * 2 * nn}, {vel, h->d_xfer + 2 * nn, sizeof(double) * 2 * nn},
+                       {rho, h->d_xfer + 4 * nn, sizeof(double) * nn}, {press, h->d_xfer + 5 * nn, sizeof(double) * nn}});
 }
 
 }  // namespace
@@ -1908,16 +1915,17 @@ int sph_set_state(sph_handle* h, int n, const double* pos, const double* vel, co
     if (n > h->cap_host) return SPH_E_CAPACITY;
     CK(cudaSetDevice(h->device));
     h->n_host = n;
-    CK(cudaMemcpyAsync(h->d_xfer, pos, sizeof(double) * 2 * n, cudaMemcpyHostToDevice, h->stream));
+    const size_t nn = (size_t)n;
+    double* xv = h->d_xfer + 2 * nn;
+    int rc = from_host(h, {hin(pos, h->d_xfer, sizeof(double) * 2 * nn), hin(vel, xv, sizeof(double) * 2 * nn),
+                           hin(rho, h->S.rho, sizeof(double) * nn), hin(mass, h->S.mass, sizeof(double) * nn),
+                           hin(sps_mass, h->S.smass, sizeof(double) * nn), hin(type, h->S.type, sizeof(int) * nn)});
+    if (rc) return rc;
     k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, h->d_xfer, h->S.pos);
-    CK(cudaMemcpyAsync(h->d_xfer + 2 * (size_t)n, vel, sizeof(double) * 2 * n, cudaMemcpyHostToDevice, h->stream));
-    k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, h->d_xfer + 2 * (size_t)n, h->S.vel);
-    CK(cudaMemcpyAsync(h->S.rho, rho, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->S.mass, mass, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->S.smass, sps_mass ? sps_mass : mass, sizeof(double) * n, cudaMemcpyHostToDevice,
-                       h->stream));
-    CK(cudaMemcpyAsync(h->S.type, type, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->S.itype, type, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream));
+    k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, xv, h->S.vel);
+    if (!sps_mass)
+        CK(cudaMemcpyAsync(h->S.smass, h->S.mass, sizeof(double) * nn, cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->S.itype, h->S.type, sizeof(int) * nn, cudaMemcpyDeviceToDevice, h->stream));
     {
         // the ghost assignment works one warp per ghost over this list
         std::vector<int> g;
@@ -1934,14 +1942,13 @@ int sph_set_state(sph_handle* h, int n, const double* pos, const double* vel, co
     CK(cudaMemsetAsync(h->S.r_drho, 0, sizeof(double) * n, h->stream));
     CK(cudaMemsetAsync(h->S.r_acc, 0, sizeof(double2) * n, h->stream));
     CK(cudaMemsetAsync(h->S.r_avg, 0, sizeof(double2) * n, h->stream));
+    CK(cudaMemsetAsync(h->S.blabel, 0, sizeof(int) * (size_t)n, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->staging_valid = true;
     h->sorted_valid = false;
     h->have_rhs = false;
     h->step_count = 0;
     h->t_phys = 0.0;
-    CK(cudaMemsetAsync(h->S.blabel, 0, sizeof(int) * (size_t)n, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
     return SPH_OK;
 }
 
@@ -1950,15 +1957,14 @@ int sph_update_state(sph_handle* h, int n, const double* pos, const double* vel,
     CK(cudaSetDevice(h->device));
     int rc = h->mixed ? unsort<float>(h) : unsort<double>(h);
     if (rc) return rc;
-    CK(cudaMemcpyAsync(h->d_xfer, pos, sizeof(double) * 2 * n, cudaMemcpyHostToDevice, h->stream));
+    // complete on return: the caller owns (and may refill) its arrays afterwards
+    double* xv = h->d_xfer + 2 * (size_t)n;
+    if ((rc = from_host(h, {hin(pos, h->d_xfer, sizeof(double) * 2 * n), hin(vel, xv, sizeof(double) * 2 * n),
+                            hin(rho, h->S.rho, sizeof(double) * n)})))
+        return rc;
     k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, h->d_xfer, h->S.pos);
-    CK(cudaMemcpyAsync(h->d_xfer + 2 * (size_t)n, vel, sizeof(double) * 2 * n, cudaMemcpyHostToDevice, h->stream));
-    k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, h->d_xfer + 2 * (size_t)n, h->S.vel);
-    CK(cudaMemcpyAsync(h->S.rho, rho, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
+    k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, xv, h->S.vel);
     CK(cudaGetLastError());
-    // the copies from page-locked buffers run asynchronously: finish them before
-    // returning, since the caller owns (and may refill) its arrays afterwards
-    CK(cudaStreamSynchronize(h->stream));
     h->launches += 2;
     h->staging_valid = true;
     h->sorted_valid = false;
@@ -2159,8 +2165,6 @@ int sph_find_particle_pair(sph_handle* h, long long pair_cap, int* pair_i, int* 
     int rc = DISPATCH(h, prepare, h);
     toc(h);
     if (rc) return rc;
-    rc = read_status(h);
-    if (rc) return rc;
     return DISPATCH(h, find_pairs, h, pair_cap, pair_i, pair_j, w, dwdx, pair_number);
 }
 
@@ -2176,20 +2180,16 @@ int sph_rhs(sph_handle* h, double* drhodt, double* acc, double* avg_vel, int* fs
     if (rc) return rc;
     rc = read_status(h);
     if (rc) return rc;
-    rc = DISPATCH(h, export_fields, h);
-    if (rc) return rc;
+    if (!h->d_export) CK(dalloc(&h->d_export, (size_t)kExportFields * h->cap_host));
+    if (h->mixed) k_export_rhs<float><<<blocks(h->P.n_tot, 256), 256, 0, h->stream>>>(h->P, h->D32, h->d_export);
+    else k_export_rhs<double><<<blocks(h->P.n_tot, 256), 256, 0, h->stream>>>(h->P, h->D64, h->d_export);
+    CK(cudaGetLastError());
     const size_t n = (size_t)h->n_host;
-    std::vector<double> buf(7 * n);
-    CK(cudaMemcpyAsync(buf.data(), h->d_export, sizeof(double) * 7 * n, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    for (size_t i = 0; i < n; ++i) {
-        if (drhodt) drhodt[i] = buf[i];
-        if (acc) { acc[i] = buf[n + i]; acc[n + i] = buf[2 * n + i]; }
-        if (avg_vel) { avg_vel[i] = buf[3 * n + i]; avg_vel[n + i] = buf[4 * n + i]; }
-        if (fs) fs[i] = (int)buf[5 * n + i];
-        if (near_fs) near_fs[i] = (int)buf[6 * n + i];
-    }
-    return SPH_OK;
+    double* x = h->d_export;
+    int* flag = reinterpret_cast<int*>(x + 5 * n);
+    return to_host(h, {{drhodt, x, sizeof(double) * n}, {acc, x + n, sizeof(double) * 2 * n},
+                       {avg_vel, x + 3 * n, sizeof(double) * 2 * n}, {fs, flag, sizeof(int) * n},
+                       {near_fs, flag + n, sizeof(int) * n}});
 }
 
 int sph_get_field(sph_handle* h, int field, double* out) {
@@ -2206,10 +2206,7 @@ int sph_get_field(sph_handle* h, int field, double* out) {
     int rc = DISPATCH(h, export_fields, h);
     if (rc) return rc;
     const size_t n = (size_t)h->n_host;
-    CK(cudaMemcpyAsync(out, h->d_export + first * n, sizeof(double) * count * n, cudaMemcpyDeviceToHost,
-                       h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    return SPH_OK;
+    return to_host(h, {{out, h->d_export + first * n, sizeof(double) * count * n}});
 }
 
 int sph_step(sph_handle* h, int nsteps, double dt, sph_diag* out) {

@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(kRedThreads) k_body_force(Params P, Sorted<R> 
 // --- find_particle_pair entry point ---------------------------------------
 // Pairs are emitted once, by their pair_i (lower id), sorted by (i, j).
 template <typename R>
-__global__ void k_pair_count(Params P, Sorted<R> D, int* cnt_id) {
+__global__ void k_pair_count(Params P, Sorted<R> D, long long* cnt_id) {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
     const int nn = D.nnbr[a];
@@ -620,6 +620,24 @@ __global__ void k_snapshot(Params P, int n, const double2* pos, const double2* v
     out[2 * (size_t)n + i] = v.x; out[3 * (size_t)n + i] = v.y;
     out[4 * (size_t)n + i] = r;
     out[5 * (size_t)n + i] = p;
+}
+
+// What sph_rhs returns, in id order (host particles) and in the layout of its
+// arrays: drho [n], acc [2n], avg [2n] as doubles, then fs [n], near [n] as ints.
+template <typename R>
+__global__ void k_export_rhs(Params P, Sorted<R> D, double* out) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= P.n_tot) return;
+    const int i = D.id[s];
+    if (i >= P.n_host) return;
+    const size_t n = (size_t)P.n_host;
+    const auto a = D.acc[s], g = D.avg[s];
+    out[i] = (double)D.drho[s];
+    out[n + i] = (double)a.x; out[2 * n + i] = (double)a.y;
+    out[3 * n + i] = (double)g.x; out[4 * n + i] = (double)g.y;
+    int* flag = reinterpret_cast<int*>(out + 5 * n);
+    flag[i] = D.flags[s] & 1;
+    flag[n + i] = (D.flags[s] >> 1) & 1;
 }
 
 // Per-particle outputs of the last RHS in id order (host particles), as doubles.

@@ -596,6 +596,7 @@ constexpr int kAdjLanes = SPH_ADJ_LANES;     // 2 or 4
 template <typename R, bool MS = false, bool MUSCL = false, bool HLLC = false>
 __global__ void __launch_bounds__(kAdjThreads, MUSCL ? SPH_ADJ_C_MUSCL_MIN_BLOCKS : SPH_ADJ_C_MIN_BLOCKS) k_adj_c(Params P, Sorted<R> D, Adj A, const double* lr,
                                                         const double2* la, double* nu_part) {
+    pdl_begin();
     stamp_phase(P.stamp);
     __shared__ double red[kAdjThreads];
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -703,6 +704,7 @@ __device__ __forceinline__ double block_sum(double s, double* red32) {
 }
 
 __global__ void k_adj_nu_sum(int nparts, const double* part, double* acc) {
+    pdl_begin();
     __shared__ double red[32];
     double s = 0.0;
     for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += part[i];
@@ -715,6 +717,7 @@ __global__ void k_adj_nu_sum(int nparts, const double* part, double* acc) {
 // and B^-1 in shgr / shbi.
 template <typename R>
 __global__ void k_adj_point(Params P, Sorted<R> D, Adj A, int shift) {
+    pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
     const int ta = D.type[a];
@@ -872,6 +875,7 @@ __device__ __forceinline__ void rev_rawsum(double r0, double r1, double id, doub
 template <typename R, bool MS = false, bool MUSCL = false>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_a(Params P, Sorted<R> D, Adj A, int stage, double dt,
                                                        const double2* lg) {
+    pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int c0 = t / kAdjLanes, lane = t & (kAdjLanes - 1);
     // every lane of the warp takes part in the shuffles below
@@ -981,6 +985,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_a(Params P, Sorted<R> D, Ad
 //   s_a = sum_b phi(d) V_b r,  phi = (1 + R (W/W_dx)^4) G,  r = x_a - x_b.
 template <typename R>
 __global__ void k_shift_sum(Params P, Sorted<R> D, Adj A) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
@@ -1007,6 +1012,7 @@ __global__ void k_shift_sum(Params P, Sorted<R> D, Adj A) {
 // neighbours b (their sums, through r and V_c = m_c / rho_c) to sx, sr.
 template <typename R>
 __global__ void k_adj_shift(Params P, Sorted<R> D, Adj A) {
+    pdl_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.n_tot) return;
     const double2 xc = D.pos[c];
@@ -1093,6 +1099,7 @@ __device__ __forceinline__ void shift_reverse(const Params& P, const Sorted<R>& 
 template <typename R>
 __global__ void k_adj_stage3(Params P, Sorted<R> D, Adj A, double dt, int shift, const double2* ox = nullptr,
                              const double* orho = nullptr) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
@@ -1209,6 +1216,7 @@ __device__ __forceinline__ void mls_pbar_to_d(const double (&pb)[6], double dx, 
 // density (lam) per slot.
 template <typename R>
 __global__ void k_adj_mls_end(Params P, Sorted<R> D, Adj A, int shift, double2* xe, double* lam) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
@@ -1235,6 +1243,7 @@ __device__ __forceinline__ bool mls_in(const Params& P, double px, double py, do
 // rho_a' (14), the adjoint of rho_a through a's own term (15, moving square).
 template <typename R, int M>
 __global__ void k_adj_mls_own(Params P, Sorted<R> V, const double* lam, double* cy, double2* xown) {
+    pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
     double* o = cy + (size_t)16 * a;
@@ -1357,6 +1366,7 @@ __global__ void k_adj_mls_own(Params P, Sorted<R> V, const double* lam, double* 
 template <typename R, int M>
 __global__ void k_adj_mls_nbr(Params P, Sorted<R> V, const double* lam, const double* cy, const double2* xown,
                               const double2* xe, double2* ox, double* orho, double2* gm) {
+    pdl_begin();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= P.n_tot) return;
     const double2 xq = V.pos[q];
@@ -1426,6 +1436,7 @@ __global__ void k_adj_mls_nbr(Params P, Sorted<R> V, const double* lam, const do
 // them, after k_adj_c has formed the latter.
 template <typename R>
 __global__ void k_adj_add_ghost_rm(Params P, Sorted<R> D, Adj A, const double2* gm) {
+    pdl_begin();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot || D.type[s] == SPH_TYPE_WATER) return;
     const double2 g = gm[s];
@@ -1448,6 +1459,7 @@ __global__ void k_adj_add_ghost_rm(Params P, Sorted<R> D, Adj A, const double2* 
 template <typename R>
 __global__ void k_adj_mls1_end(Params P, Sorted<R> D, const double2* xe, const double* lam, double2* ox,
                                double* orho) {
+    pdl_begin();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     ox[s] = xe[s];
@@ -1458,6 +1470,7 @@ __global__ void k_adj_mls1_end(Params P, Sorted<R> D, const double2* xe, const d
 // (cy[16 a ..]: mode 12 = 2 for an owner, S_w 13, rho_a' 14).
 template <typename R>
 __global__ void k_adj_mls1_own(Params P, Sorted<R> V, double* cy) {
+    pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
     double* o = cy + (size_t)16 * a;
@@ -1489,6 +1502,7 @@ __global__ void k_adj_mls1_own(Params P, Sorted<R> V, double* cy) {
 // list, added to sx and sr (after k_adj_c has formed the RHS's own).
 template <typename R>
 __global__ void k_adj_mls1_nbr(Params P, Sorted<R> V, Adj A, const double* lam, const double* cy) {
+    pdl_begin();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= P.n_tot) return;
     const int tq = V.type[q];
@@ -1531,6 +1545,7 @@ __global__ void k_adj_mls1_nbr(Params P, Sorted<R> V, Adj A, const double* lam, 
 // Sorted step-start adjoints -> id order; the K1 adjoint goes to the previous step.
 template <typename R>
 __global__ void k_adj_scatter(Params P, Sorted<R> D, Adj A, int first) {
+    pdl_begin();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     const int i = D.id[s];
@@ -1548,6 +1563,7 @@ __global__ void k_adj_scatter(Params P, Sorted<R> D, Adj A, int first) {
 // state, shifted by a period): bottom/top images first, since their sources
 // include left/right images, then left/right images to the host particles.
 __global__ void k_adj_route(int n_src, int base, const int* cnt, const int* off, Adj A) {
+    pdl_begin();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_src) return;
     const int c = cnt[s];
@@ -1566,6 +1582,7 @@ __global__ void k_adj_route(int n_src, int base, const int* cnt, const int* off,
 // forward's stages write them).
 template <typename R>
 __global__ void k_resplit(int n, Sorted<R> D, unsigned long long* stamp) {
+    pdl_begin();
     stamp_phase(stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
@@ -1575,6 +1592,7 @@ __global__ void k_resplit(int n, Sorted<R> D, unsigned long long* stamp) {
 // Stage state -> the arrays the RHS reads (positions, kinematic and auxiliary records).
 template <typename R>
 __global__ void k_adj_load(Params P, Sorted<R> D, const double2* pos, const double4* kin) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
@@ -1603,6 +1621,7 @@ struct SnapPtrs {
     double *rho, *r_drho;
 };
 __global__ void k_snap_copy(int n, SnapPtrs dst, SnapPtrs src, unsigned long long* stamp) {
+    pdl_begin();
     stamp_phase(stamp);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -1631,6 +1650,7 @@ struct PrepDesc {
 // words (the arrays and the slot offsets are 256-byte aligned).
 __global__ void k_prep_copy(const PrepDesc* d, int n_tot, unsigned* slot, int save, const int* cnt,
                             unsigned long long* stamp) {
+    pdl_begin();
     stamp_phase(stamp);
     const PrepDesc c = d[blockIdx.y];
     unsigned* s = slot + c.off;
@@ -1666,6 +1686,7 @@ __global__ void k_prep_copy(const PrepDesc* d, int n_tot, unsigned* slot, int sa
 // Copy of the stage state (positions and records) into the stage store.
 template <typename R>
 __global__ void k_keep_stage(int n, Sorted<R> D, double2* pos, double4* kin, typename VT<R>::V4* aux) {
+    pdl_begin();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     pos[s] = D.pos[s]; kin[s] = D.kin[s]; aux[s] = D.aux[s];
@@ -1674,6 +1695,7 @@ __global__ void k_keep_stage(int n, Sorted<R> D, double2* pos, double4* kin, typ
 // Loss of the final state (id order, host water particles): per-block partials.
 __global__ void k_adj_loss(int n, int kind, const int* type, const double2* vel, const double* mass,
                            const double2* target, double* part) {
+    pdl_begin();
     __shared__ double red[256];
     double s = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1700,6 +1722,7 @@ __global__ void k_adj_loss(int n, int kind, const int* type, const double2* vel,
 // whose terms enter step by step in the reverse sweep).
 __global__ void k_adj_seed(int n, int kind, double dloss, const int* type, const double2* vel, const double* mass,
                            const double2* target, Adj A) {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double2 g = make_double2(0, 0);
@@ -1736,6 +1759,7 @@ __global__ void k_adj_seed(int n, int kind, double dloss, const int* type, const
 // particles k_mark_body_nbrs flagged (nflag == 2) have terms.
 template <typename R>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_drag(Params P, Sorted<R> D, Adj A, double w, double* nu_part) {
+    pdl_begin();
     __shared__ double red[kAdjThreads];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double nu_sum = 0.0;
@@ -1817,6 +1841,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_drag(Params P, Sorted<R> D,
 // cleared before and the ghost flags written after this kernel's use).
 template <typename R>
 __global__ void k_mark_body_nbrs(Params P, Sorted<R> D) {
+    pdl_begin();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= P.n_tot || D.itype[b] != SPH_TYPE_BODY) return;
     const int nn = D.npairs[b];
@@ -1843,6 +1868,7 @@ template <typename R>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_ghost_lambda(Params P, Sorted<R> D, Adj A,
                                                                   const int* ghost_ids, int n_ghost, double t,
                                                                   double bax, double bay, double* part) {
+    pdl_begin();
     __shared__ double red[4][kAdjThreads / 32];
     const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1975,6 +2001,7 @@ __device__ __forceinline__ void ghost_water_one(const Params& P, const Sorted<R>
 template <typename R>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_ghost_water(Params P, Sorted<R> D, Adj A, double bax,
                                                                  double bay) {
+    pdl_begin();
     // a fixed grid of warps strides over the slots; only the flagged ones work
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < P.n_tot; j += nw) {
@@ -1997,6 +2024,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_ghost_water(Params P, Sorte
 template <typename R>
 __global__ void k_adj_stage_end_ms(Params P, Sorted<R> D, Adj A, double dt, int shift, const double2* ox = nullptr,
                                    const double* orho = nullptr) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
@@ -2035,6 +2063,7 @@ __global__ void k_adj_stage_end_ms(Params P, Sorted<R> D, Adj A, double dt, int 
 // first step's fresh RHS, pred = 0), the plain accumulation.
 template <typename R>
 __global__ void k_adj_stage_ms(Params P, Sorted<R> D, Adj A, int pred, double dt) {
+    pdl_begin();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     const double2 sx = A.sx[s], su = A.su[s];
@@ -2062,6 +2091,7 @@ __global__ void k_adj_stage_ms(Params P, Sorted<R> D, Adj A, int pred, double dt
 // (the body moves by u_body dt at the step start, so dL/du_body += dt times this).
 template <typename R>
 __global__ void k_adj_body_pos(Params P, Sorted<R> D, Adj A, double* part) {
+    pdl_begin();
     __shared__ double red[2][256];
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     double x = 0.0, y = 0.0;
@@ -2080,6 +2110,7 @@ __global__ void k_adj_body_pos(Params P, Sorted<R> D, Adj A, double* part) {
 
 // out[q] += scale * sum_i part[q nparts + i], q < nq, in block order.
 __global__ void k_adj_motion_sum(int nparts, int nq, const double* part, double scale, double* out) {
+    pdl_begin();
     __shared__ double red[32];
     for (int q = 0; q < nq; ++q) {
         double s = 0.0;
@@ -2091,6 +2122,7 @@ __global__ void k_adj_motion_sum(int nparts, int nq, const double* part, double 
 
 // Drag loss accumulation of the forward run: acc += w * F_x.
 __global__ void k_drag_acc(const double* force, double w, double* acc) {
+    pdl_begin();
     if (threadIdx.x == 0 && blockIdx.x == 0) acc[0] += w * force[4];
 }
 

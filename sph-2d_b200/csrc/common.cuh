@@ -73,6 +73,43 @@ __device__ __forceinline__ void stamp_phase(unsigned long long* slot) {
     *slot = t;
 }
 
+// Programmatic dependent launch: every kernel of the library begins with
+// pdl_begin and is launched with `launch`.  The next kernel of the stream may then
+// be brought in as soon as this one's blocks have ended, while their writes and
+// the launch are still being settled, and waits there for both
+// (griddepcontrol.wait), so the order of the work is the stream's as before.  What
+// goes is 1 to 2 us between two kernels, where a kernel of a small step takes 5 to
+// 8: plain 100^2 1079 -> 795 us per 10 steps, adjoint 256^2 61.9 -> 54.6 ms, 401^2
+// mixed 1956 -> 1815 us per 5.
+//
+// For launches up to kPdlThreads threads: above, the time between kernels no
+// longer shows.  Letting the next kernel in early (griddepcontrol.launch_dependents
+// at the top) was slower: 893 us in the first case, and pass A of 256^2 rose from
+// 5.9 to 7.9 ms: its blocks gather on the SMs that have room while the kernel
+// before still fills the others; without the size limit 2048^2 took 57.6 instead
+// of 34.4 ms.
+constexpr unsigned kPdlThreads = 500000;
+__host__ __device__ constexpr bool pdl_small(unsigned blocks, unsigned threads) {
+    return (unsigned long long)blocks * threads <= kPdlThreads;
+}
+__device__ __forceinline__ void pdl_begin() {
+    if (pdl_small(gridDim.x * gridDim.y, blockDim.x)) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... Params_, typename... Args>
+inline void launch(void (*kernel)(Params_...), dim3 grid, dim3 block, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.stream = st;
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = a;
+    c.numAttrs = pdl_small(grid.x * grid.y, block.x) ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, static_cast<Params_>(args)...);     // (errors: cudaGetLastError at the callers)
+}
+
 template <typename R> struct VT;
 template <> struct VT<double> { using V2 = double2; using V4 = double4; };
 template <> struct VT<float> { using V2 = float2; using V4 = float4; };
@@ -154,9 +191,10 @@ __device__ __forceinline__ double rsqrt64(double x) {
 
 // One 32-byte record: a single 256-bit load for FP64 (cudaMalloc'd arrays of
 // 32-byte elements, so every element is 32-byte aligned), 128-bit for FP32.
+// (volatile: never moved above pdl_begin.)
 __device__ __forceinline__ double4 load4(const double4* p) {
     double4 v;
-    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ float4 load4(const float4* p) { return *p; }

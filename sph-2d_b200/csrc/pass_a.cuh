@@ -90,6 +90,7 @@ __device__ __noinline__ bool surface_test(const Params& P, const Sorted<R>& D, i
 template <typename R, bool HLREC, bool MS, int L = 1>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_BLOCKS : SPH_PASS_A_F32_BLOCKS) : (MS ? 4 : 5))
     k_pass_a(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D) {
+    pdl_begin();
     stamp_phase(P.stamp);
     using V4 = typename VT<R>::V4;
     constexpr bool F32 = sizeof(R) == 4;
@@ -321,8 +322,8 @@ constexpr int kLanes4Below = 17000, kLanes2BelowA = 60000, kLanes2BelowC = 90000
 template <typename R, bool HLREC, int L>
 void launch_pass_a_lanes(const Params& P, const Sorted<R>& D, cudaStream_t st) {
     const int nb = (int)(((long long)P.n_tot * L + 127) / 128);
-    if (P.ms) k_pass_a<R, HLREC, true, L><<<nb, 128, 0, st>>>(P, D);
-    else k_pass_a<R, HLREC, false, L><<<nb, 128, 0, st>>>(P, D);
+    if (P.ms) launch(k_pass_a<R, HLREC, true, L>, nb, 128, st, P, D);
+    else launch(k_pass_a<R, HLREC, false, L>, nb, 128, st, P, D);
 }
 
 template <typename R, bool HLREC>
@@ -345,6 +346,7 @@ void launch_pass_a(const Params& P, const Sorted<R>& D, cudaStream_t st) {
 // RHS have no surface particle and every thread returns at once.
 template <typename R>
 __global__ void k_near(Params P, Sorted<R> D) {
+    pdl_begin();
     if (*D.surf_gen != P.rhs_gen) return;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < P.n_tot; a += gridDim.x * blockDim.x) {
         if (!(D.flags[a] & 1)) continue;
@@ -362,7 +364,7 @@ void launch_near(const Params& P, const Sorted<R>& D, cudaStream_t st) {
     int nb = (P.n_tot + 127) / 128;
     if (nb > 148 * 8) nb = 148 * 8;
     if (nb == 0) return;
-    k_near<R><<<nb, 128, 0, st>>>(P, D);
+    launch(k_near<R>, nb, 128, st, P, D);
 }
 
 }  // namespace sph

@@ -161,6 +161,7 @@ struct Side {
 template <typename R, bool MUSCL, bool MS, bool SHIFT, int L = 1>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIFT_BLOCKS : SPH_PASS_C_F32_BLOCKS) : 3)
     k_pass_c(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D, const __grid_constant__ StageArgs G) {
+    pdl_begin();
     stamp_phase(P.stamp);
     using V4 = typename VT<R>::V4;
     using A = typename Acc<R>::T;
@@ -639,6 +640,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
 template <typename R>
 __global__ void __launch_bounds__(128, 12) k_shift_gather(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D,
                                                         const __grid_constant__ StageArgs G) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;

@@ -164,6 +164,7 @@ __device__ __forceinline__ double2 move_body(const Staging& S, int i, double2 di
 
 __global__ void __launch_bounds__(kImgThreads) k_img_count(Params P, Staging S, SetupBuf B, HostBox* box, unsigned seq,
                                                            double2 disp) {
+    pdl_begin();
     stamp_phase(P.stamp);
     __shared__ unsigned long long sh[32];
     __shared__ int flag;
@@ -238,6 +239,7 @@ __device__ __forceinline__ void put_image(const Params& P, const Staging& S, con
 // offsets for the reverse sweep.
 __global__ void __launch_bounds__(kImgThreads) k_img_emit(Params P, Staging S, SetupBuf B, int cap, int periodic,
                                                           int route, unsigned* status, double2 disp) {
+    pdl_begin();
     stamp_phase(P.stamp);
     __shared__ unsigned long long sh[32];
     const int i = blockIdx.x * kImgThreads + threadIdx.x;
@@ -294,6 +296,7 @@ __global__ void __launch_bounds__(kImgThreads) k_img_emit(Params P, Staging S, S
 // Exclusive scan of the cell counts within blocks of kScanCells cells; the last
 // block scans the block sums.
 __global__ void __launch_bounds__(kScanThreads) k_cell_scan(SetupBuf B, unsigned long long* stamp) {
+    pdl_begin();
     stamp_phase(stamp);
     __shared__ int sh[32];
     __shared__ int flag;
@@ -322,6 +325,7 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(SetupBuf B, unsigned
 
 // Cell ranges (-1 for an empty cell), and each particle at its arrival place.
 __global__ void k_place(int n_tot, SetupBuf B, int* cell_start, int* cell_end) {
+    pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < B.ncells) {
         const int n = B.cnt[t], st = B.blkoff[t >> kScanShift] + B.pre[t];
@@ -593,6 +597,7 @@ __device__ __forceinline__ void shift_by(const Params& P, double2 sh, double g0,
 // number of lower ids in the cell (about 8 reads that the warp shares).
 template <typename R>
 __global__ void k_gather_sorted(Params P, Staging S, Sorted<R> D, SetupBuf B, StageArgs G) {
+    pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.n_tot) return;
     const int i = (int)B.perm[t];
@@ -646,6 +651,7 @@ __global__ void k_gather_sorted(Params P, Staging S, Sorted<R> D, SetupBuf B, St
 // sorted master state -> id order (host particles only; images are dropped)
 template <typename R>
 __global__ void k_unsort(Params P, Staging S, Sorted<R> D) {
+    pdl_begin();
     stamp_phase(P.stamp);
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
@@ -683,6 +689,7 @@ __device__ __forceinline__ bool pair_allowed(int rule, int ti, int tj) {
 constexpr int kListStage = 32;
 template <typename R>
 __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsigned* status) {
+    pdl_begin();
     __shared__ unsigned stage[kListStage][128];
     const int tid = threadIdx.x;
     int a = blockIdx.x * blockDim.x + tid;
@@ -776,6 +783,7 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
 // (Gaussian) candidates are then a chain of dependent loads.
 template <typename R, int L>
 __global__ void __launch_bounds__(128) k_build_lists_lanes(Params P, Sorted<R> D, unsigned* status) {
+    pdl_begin();
     constexpr bool F32 = sizeof(R) == 4;
     const Lanes<L> ln;
     const int g = Lanes<L>::particle();
@@ -849,9 +857,9 @@ template <typename R>
 void launch_lists(const Params& P, const Sorted<R>& D, unsigned* status, cudaStream_t st) {
     if (P.n_tot < kListLanesBelow) {
         const long long t = (long long)P.n_tot * kListLanes;
-        k_build_lists_lanes<R, kListLanes><<<(unsigned)((t + 127) / 128), 128, 0, st>>>(P, D, status);
+        launch(k_build_lists_lanes<R, kListLanes>, (unsigned)((t + 127) / 128), 128, st, P, D, status);
     } else {
-        k_build_lists<R><<<(P.n_tot + 127) / 128, 128, 0, st>>>(P, D, status);
+        launch(k_build_lists<R>, (P.n_tot + 127) / 128, 128, st, P, D, status);
     }
 }
 

@@ -308,7 +308,7 @@ void mark_event(sph_handle* h) {
 // End of the stretch.
 void toc(sph_handle* h) {
     if (!h->timed_open) return;
-    k_stamp<<<1, 1, 0, h->stream>>>(h->d_stamps + h->stamp_of.size());
+    launch(k_stamp, 1, 1, h->stream, h->d_stamps + h->stamp_of.size());
     h->stamp_of.push_back(-1);
     h->P.stamp = nullptr;
     mark_event(h);
@@ -398,7 +398,7 @@ int unsort(sph_handle* h) {
     if (h->staging_valid) return SPH_OK;
     if (!h->sorted_valid) return SPH_E_ARG;
     Params P = h->P;
-    k_unsort<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, h->S, sorted<R>(h));
+    launch(k_unsort<R>, blocks(P.n_tot, 256), 256, h->stream, P, h->S, sorted<R>(h));
     CK(cudaGetLastError());
     h->launches += 1;
     h->staging_valid = true;
@@ -434,14 +434,14 @@ int prepare(sph_handle* h, const StageArgs& first = StageArgs{}) {
     const int nhb = blocks(h->n_host, kImgThreads), ncb = blocks(h->ncells + 1, kScanCells);
     const int periodic = h->cfg.periodic ? 1 : 0;
     const double2 disp = make_double2(h->body_disp[0], h->body_disp[1]);
-    if (periodic) k_img_count<<<nhb, kImgThreads, 0, h->stream>>>(P, h->S, B, h->d_box, ++h->box_seq, disp);
+    if (periodic) launch(k_img_count, nhb, kImgThreads, h->stream, P, h->S, B, h->d_box, ++h->box_seq, disp);
     else CK(cudaMemsetAsync(B.cnt, 0, sizeof(int) * (size_t)(h->ncells + 1), h->stream));
     // (the routing of image adjoints is kept once an adjoint run exists)
-    k_img_emit<<<nhb, kImgThreads, 0, h->stream>>>(P, h->S, B, h->cap_tot, periodic, h->adj != nullptr, h->d_status,
+    launch(k_img_emit, nhb, kImgThreads, h->stream, P, h->S, B, h->cap_tot, periodic, h->adj != nullptr, h->d_status,
                                                     periodic ? make_double2(0.0, 0.0) : disp);
     h->body_disp[0] = h->body_disp[1] = 0.0;
     tic(h, PH_SORT);
-    k_cell_scan<<<ncb, kScanThreads, 0, h->stream>>>(B, P.stamp);
+    launch(k_cell_scan, ncb, kScanThreads, h->stream, B, P.stamp);
     CK(cudaGetLastError());
     int n_img = 0;
     if (periodic) {
@@ -453,8 +453,8 @@ int prepare(sph_handle* h, const StageArgs& first = StageArgs{}) {
     }
     h->n_img = n_img;
     P.n_tot = h->n_host + n_img;
-    k_place<<<blocks(std::max(P.n_tot, h->ncells), 256), 256, 0, h->stream>>>(P.n_tot, B, D.cell_start, D.cell_end);
-    k_gather_sorted<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, h->S, D, B, first);
+    launch(k_place, blocks(std::max(P.n_tot, h->ncells), 256), 256, h->stream, P.n_tot, B, D.cell_start, D.cell_end);
+    launch(k_gather_sorted<R>, blocks(P.n_tot, 256), 256, h->stream, P, h->S, D, B, first);
     launch_lists<R>(P, D, h->d_status, h->stream);
     CK(cudaGetLastError());
     h->launches += periodic ? 6 : 5;
@@ -478,20 +478,20 @@ template <typename R, int L>
 void launch_pass_c_lanes(const Params& P, const Sorted<R>& D, const StageArgs& G, bool shift, cudaStream_t st) {
     const int nb = blocks((long long)P.n_tot * L, 128);
     if (P.ms) {
-        if (shift) k_pass_c<R, false, true, true, L><<<nb, 128, 0, st>>>(P, D, G);
-        else k_pass_c<R, false, true, false, L><<<nb, 128, 0, st>>>(P, D, G);
+        if (shift) launch(k_pass_c<R, false, true, true, L>, nb, 128, st, P, D, G);
+        else launch(k_pass_c<R, false, true, false, L>, nb, 128, st, P, D, G);
         return;
     }
     // (the mixed Taylor-Green launches never carry the shifting sum)
     if constexpr (sizeof(R) == 8) {
         if (shift) {
-            if (P.muscl) k_pass_c<R, true, false, true, L><<<nb, 128, 0, st>>>(P, D, G);
-            else k_pass_c<R, false, false, true, L><<<nb, 128, 0, st>>>(P, D, G);
+            if (P.muscl) launch(k_pass_c<R, true, false, true, L>, nb, 128, st, P, D, G);
+            else launch(k_pass_c<R, false, false, true, L>, nb, 128, st, P, D, G);
             return;
         }
     }
-    if (P.muscl) k_pass_c<R, true, false, false, L><<<nb, 128, 0, st>>>(P, D, G);
-    else k_pass_c<R, false, false, false, L><<<nb, 128, 0, st>>>(P, D, G);
+    if (P.muscl) launch(k_pass_c<R, true, false, false, L>, nb, 128, st, P, D, G);
+    else launch(k_pass_c<R, false, false, false, L>, nb, 128, st, P, D, G);
 }
 
 template <typename R>
@@ -519,8 +519,7 @@ int rhs(sph_handle* h, int last, const StageArgs& G = StageArgs{}, int keep_j = 
         // Assign_boundary_particles at the start of single_step_compute (MS Single_step_compute.f90:73)
         tic(h, PH_UPDATE);
         if (h->n_ghost > 0) {
-            k_assign_ghosts<R><<<blocks((long long)h->n_ghost * 32, 128), 128, 0, h->stream>>>(
-                P, D, h->d_ghost_ids, h->n_ghost, h->t_phys, h->body_vel[0], h->body_vel[1], h->body_acc[0],
+            launch(k_assign_ghosts<R>, blocks((long long)h->n_ghost * 32, 128), 128, h->stream, P, D, h->d_ghost_ids, h->n_ghost, h->t_phys, h->body_vel[0], h->body_vel[1], h->body_acc[0],
                 h->body_acc[1], gint, gsw);
             h->launches += 1;
         }
@@ -540,19 +539,18 @@ int rhs(sph_handle* h, int last, const StageArgs& G = StageArgs{}, int keep_j = 
     if constexpr (sizeof(R) == 4) if (sh && sep) {
         // timed with the update: shifting is part of the step's second pass
         tic(h, PH_UPDATE);
-        k_shift_gather<R><<<nb, 128, 0, h->stream>>>(P, D, G);
+        launch(k_shift_gather<R>, nb, 128, h->stream, P, D, G);
         h->launches += 1;
     }
     CK(cudaGetLastError());
     h->launches += 2;
     if (P.has_body && (last || h->bf_every_rhs)) {
         double* fin = h->d_bf;
-        k_body_force<R><<<blocks((long long)h->n_body * 32, kRedThreads), kRedThreads, 0, h->stream>>>(
-            P, D, h->d_body_ids, h->n_body, h->d_bf + 6, fin, h->B.done + 3);
+        launch(k_body_force<R>, blocks((long long)h->n_body * 32, kRedThreads), kRedThreads, h->stream, P, D, h->d_body_ids, h->n_body, h->d_bf + 6, fin, h->B.done + 3);
         h->bf_pending = true;
         h->launches += 1;
         if (h->drag_acc && last) {
-            k_drag_acc<<<1, 32, 0, h->stream>>>(fin, h->drag_w, h->drag_acc);
+            launch(k_drag_acc, 1, 32, h->stream, fin, h->drag_w, h->drag_acc);
             h->launches += 1;
         }
     }
@@ -566,7 +564,7 @@ template <typename R>
 int stage(sph_handle* h, int st, double dt, int use_carried, int do_shift) {
     const Params& P = h->P;
     tic(h, PH_UPDATE);
-    k_stage<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, sorted<R>(h), st, dt, use_carried, do_shift,
+    launch(k_stage<R>, blocks(P.n_tot, 256), 256, h->stream, P, sorted<R>(h), st, dt, use_carried, do_shift,
                                                              h->d_status);
     CK(cudaGetLastError());
     h->launches += 1;
@@ -595,9 +593,9 @@ int reinit_density(sph_handle* h, int do_shift) {
     const int nb = blocks(P.n_tot, 128);
     tic(h, PH_UPDATE);
     // (order 1 formed its densities on the step's last RHS: mls1_on_last_rhs)
-    if (P.mls_order == 6) k_mls<R, 6><<<nb, 128, 0, h->stream>>>(P, D, h->d_mls);
-    else if (P.mls_order == 3) k_mls<R, 3><<<nb, 128, 0, h->stream>>>(P, D, h->d_mls);
-    k_finish_mls<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, D, h->d_mls, do_shift, h->d_status);
+    if (P.mls_order == 6) launch(k_mls<R, 6>, nb, 128, h->stream, P, D, h->d_mls);
+    else if (P.mls_order == 3) launch(k_mls<R, 3>, nb, 128, h->stream, P, D, h->d_mls);
+    launch(k_finish_mls<R>, blocks(P.n_tot, 256), 256, h->stream, P, D, h->d_mls, do_shift, h->d_status);
     CK(cudaGetLastError());
     h->launches += P.mls_order == 1 ? 1 : 2;
     return SPH_OK;
@@ -609,7 +607,7 @@ template <typename R>
 int mls1_on_last_rhs(sph_handle* h) {
     const Params& P = h->P;
     tic(h, PH_UPDATE);
-    k_mls1<R><<<blocks(P.n_tot, 128), 128, 0, h->stream>>>(P, sorted<R>(h), h->d_mls);
+    launch(k_mls1<R>, blocks(P.n_tot, 128), 128, h->stream, P, sorted<R>(h), h->d_mls);
     CK(cudaGetLastError());
     h->launches += 1;
     return SPH_OK;
@@ -686,8 +684,7 @@ int diagnostics(sph_handle* h, sph_diag* result, bool with_status) {
     }
     const Params& P = h->P;
     const double* fin = h->bf_pending ? h->d_bf : nullptr;
-    k_diag<R><<<std::min(kDiagBlocks, blocks(P.n_tot, kRedThreads)), kRedThreads, 0, h->stream>>>(
-        P, sorted<R>(h), h->d_part, h->d_part + kDiagBlocks, h->d_int, h->B.done + 2, h->d_status, fin, h->d_box);
+    launch(k_diag<R>, std::min(kDiagBlocks, blocks(P.n_tot, kRedThreads)), kRedThreads, h->stream, P, sorted<R>(h), h->d_part, h->d_part + kDiagBlocks, h->d_int, h->B.done + 2, h->d_status, fin, h->d_box);
     CK(cudaGetLastError());
     h->launches += 1;
     CK(cudaStreamSynchronize(h->stream));
@@ -726,7 +723,7 @@ int find_pairs(sph_handle* h, long long pair_cap, int* pi, int* pj, double* w, d
     const int n = P.n_tot;
     if (!h->d_off64) CK(dalloc(&h->d_off64, 2 * ((size_t)h->cap_tot + 1)));
     long long* cnt64 = h->d_off64 + (h->cap_tot + 1);
-    k_pair_count<R><<<blocks(n, 128), 128, 0, h->stream>>>(P, sorted<R>(h), cnt64);
+    launch(k_pair_count<R>, blocks(n, 128), 128, h->stream, P, sorted<R>(h), cnt64);
     size_t bytes = 0;
     CK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, cnt64, h->d_off64, n, h->stream));
     if (bytes > h->cub_bytes) return SPH_E_CAPACITY;
@@ -754,7 +751,7 @@ int find_pairs(sph_handle* h, long long pair_cap, int* pi, int* pj, double* w, d
     double* ddw = dw + m;
     int* dpi = reinterpret_cast<int*>(ddw + 2 * m);
     int* dpj = dpi + m;
-    k_pair_emit<R><<<blocks(n, 128), 128, 0, h->stream>>>(P, sorted<R>(h), h->d_off64, (long long)m, dpi, dpj,
+    launch(k_pair_emit<R>, blocks(n, 128), 128, h->stream, P, sorted<R>(h), h->d_off64, (long long)m, dpi, dpj,
                                                           w ? dw : nullptr, dwdx ? ddw : nullptr);
     CK(cudaGetLastError());
     rc = to_host(h, {{pi, dpi, sizeof(int) * m}, {pj, dpj, sizeof(int) * m}, {w, dw, sizeof(double) * m},
@@ -774,7 +771,7 @@ int export_fields(sph_handle* h) {
     if (!h->have_rhs || !h->sorted_valid) return SPH_E_ARG;
     if (!h->d_export) CK(dalloc(&h->d_export, (size_t)kExportFields * h->cap_host));
     const Params& P = h->P;
-    k_export<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, sorted<R>(h), h->d_export);
+    launch(k_export<R>, blocks(P.n_tot, 256), 256, h->stream, P, sorted<R>(h), h->d_export);
     CK(cudaGetLastError());
     return SPH_OK;
 }
@@ -888,7 +885,7 @@ int snap_io(sph_handle* h, const Snap& s, int k, int n, bool save) {
     const size_t o = (size_t)k * n;
     const SnapPtrs slot{s.pos + o, s.vel + o, s.r_acc + o, s.r_avg + o, s.rho + o, s.r_drho + o};
     const SnapPtrs stg{h->S.pos, h->S.vel, h->S.r_acc, h->S.r_avg, h->S.rho, h->S.r_drho};
-    k_snap_copy<<<blocks(n, 256), 256, 0, h->stream>>>(n, save ? slot : stg, save ? stg : slot,
+    launch(k_snap_copy, blocks(n, 256), 256, h->stream, n, save ? slot : stg, save ? stg : slot,
                                                       h->P.stamp);
     CK(cudaGetLastError());
     h->launches += 1;
@@ -993,8 +990,7 @@ int prep_save(sph_handle* h, int j, bool lists = true) {
     if (!X->prep) return SPH_OK;
     const int nt = h->P.n_tot;
     const int* cnt = h->mixed ? h->D32.nnbr : h->D64.nnbr;
-    k_prep_copy<<<dim3(blocks(nt, 256), X->n_prep - (lists ? 0 : 1)), 256, 0, h->stream>>>(
-        X->d_prep, nt, X->prep + (size_t)j * X->prep_words, 1, cnt, nullptr);
+    launch(k_prep_copy, dim3(blocks(nt, 256), X->n_prep - (lists ? 0 : 1)), 256, h->stream, X->d_prep, nt, X->prep + (size_t)j * X->prep_words, 1, cnt, nullptr);
     CK(cudaGetLastError());
     h->launches += 1;
     X->seg_nimg[j] = h->n_img;
@@ -1015,8 +1011,7 @@ int prep_restore(sph_handle* h, int j, bool lists = true) {
     P.n_tot = h->n_host + h->n_img;
     tic(h, PH_SORT);
     unsigned* slot = X->prep + (size_t)j * X->prep_words;
-    k_prep_copy<<<dim3(blocks(P.n_tot, 256), X->n_prep - (lists ? 0 : 1)), 256, 0, h->stream>>>(
-        X->d_prep, P.n_tot, slot, 0, (const int*)(slot + X->prep_nnbr_off), P.stamp);
+    launch(k_prep_copy, dim3(blocks(P.n_tot, 256), X->n_prep - (lists ? 0 : 1)), 256, h->stream, X->d_prep, P.n_tot, slot, 0, (const int*)(slot + X->prep_nnbr_off), P.stamp);
     CK(cudaGetLastError());
     h->launches += 1;
     h->sorted_valid = true;
@@ -1149,7 +1144,7 @@ int adjoint_forward(sph_handle* h, const sph_adj_config* ac, double* loss) {
     const int n = h->n_host;
     if (ac->loss == SPH_LOSS_VELOCITY_MISFIT) {
         if ((rc = from_host(h, {hin(ac->target_vel, h->d_xfer, sizeof(double) * 2 * n)}))) return rc;
-        k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, h->d_xfer, X->target);
+        launch(k_interleave, blocks(n, 256), 256, h->stream, n, h->d_xfer, X->target);
         h->launches += 1;
     }
     X->step0 = h->step_count;
@@ -1176,11 +1171,11 @@ int adjoint_forward(sph_handle* h, const sph_adj_config* ac, double* loss) {
         CK(cudaMemcpyAsync(&v, X->drag_acc, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     } else {
         const int nparts = 148 * 4;
-        k_adj_loss<<<nparts, 256, 0, h->stream>>>(n, X->loss, h->S.type, h->S.vel, h->S.mass, X->target,
+        launch(k_adj_loss, nparts, 256, h->stream, n, X->loss, h->S.type, h->S.vel, h->S.mass, X->target,
                                                  X->loss_part);
         h->launches += 2;
         CK(cudaMemsetAsync(h->d_diag, 0, sizeof(double), h->stream));
-        k_adj_nu_sum<<<1, 1024, 0, h->stream>>>(nparts, X->loss_part, h->d_diag);
+        launch(k_adj_nu_sum, 1, 1024, h->stream, nparts, X->loss_part, h->d_diag);
         CK(cudaMemcpyAsync(&v, h->d_diag, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     }
     CK(cudaStreamSynchronize(h->stream));
@@ -1239,7 +1234,7 @@ template <typename R>
 int keep_stage(sph_handle* h, int j, int k) {
     Sorted<R> V = stage_view<R>(h, j, k);
     const int nt = h->P.n_tot;
-    k_keep_stage<R><<<blocks(nt, 256), 256, 0, h->stream>>>(nt, sorted<R>(h), V.pos, V.kin, V.aux);
+    launch(k_keep_stage<R>, blocks(nt, 256), 256, h->stream, nt, sorted<R>(h), V.pos, V.kin, V.aux);
     CK(cudaGetLastError());
     h->launches += 1;
     return SPH_OK;
@@ -1335,7 +1330,7 @@ void adj_pass_a(sph_handle* h, const Sorted<R>& V) {
     ++h->P.rhs_gen;
     const Params& P = h->P;
     if constexpr (sizeof(R) == 4) {
-        k_resplit<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P.n_tot, V, P.stamp);
+        launch(k_resplit<R>, blocks(P.n_tot, 256), 256, h->stream, P.n_tot, V, P.stamp);
         launch_pass_a<R, true>(P, V, h->stream);
         h->launches += 1;
     } else {
@@ -1365,22 +1360,22 @@ int adj_rhs(sph_handle* h, const Sorted<R>& V, int k, int stage, bool shift = fa
     }
     tic(h, PH_ADJ);
     if (P.muscl)
-        k_adj_c<R, false, true><<<nbc, kAdjThreads, 0, h->stream>>>(P, V, A, A.lr[k], A.la[k],
+        launch(k_adj_c<R, false, true>, nbc, kAdjThreads, h->stream, P, V, A, A.lr[k], A.la[k],
                                                                      A.nu_part + (size_t)k * nbc);
     else
-        k_adj_c<R><<<nbc, kAdjThreads, 0, h->stream>>>(P, V, A, A.lr[k], A.la[k], A.nu_part + (size_t)k * nbc);
+        launch(k_adj_c<R>, nbc, kAdjThreads, h->stream, P, V, A, A.lr[k], A.la[k], A.nu_part + (size_t)k * nbc);
     if (shift) {
-        k_adj_shift<R><<<nb, kAdjThreads, 0, h->stream>>>(P, V, A);
+        launch(k_adj_shift<R>, nb, kAdjThreads, h->stream, P, V, A);
         h->launches += 1;
     }
     if (mls1) {
-        k_adj_mls1_own<R><<<blocks(P.n_tot, 128), 128, 0, h->stream>>>(P, V, X->mls_cy);
-        k_adj_mls1_nbr<R><<<blocks(P.n_tot, 128), 128, 0, h->stream>>>(P, V, A, X->mls_lam, X->mls_cy);
+        launch(k_adj_mls1_own<R>, blocks(P.n_tot, 128), 128, h->stream, P, V, X->mls_cy);
+        launch(k_adj_mls1_nbr<R>, blocks(P.n_tot, 128), 128, h->stream, P, V, A, X->mls_lam, X->mls_cy);
         h->launches += 2;
     }
-    k_adj_point<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, V, A, shift ? 1 : 0);
-    if (P.muscl) k_adj_a<R, false, true><<<nbc, kAdjThreads, 0, h->stream>>>(P, V, A, stage, X->dt, nullptr);
-    else k_adj_a<R><<<nbc, kAdjThreads, 0, h->stream>>>(P, V, A, stage, X->dt, nullptr);
+    launch(k_adj_point<R>, blocks(P.n_tot, 256), 256, h->stream, P, V, A, shift ? 1 : 0);
+    if (P.muscl) launch(k_adj_a<R, false, true>, nbc, kAdjThreads, h->stream, P, V, A, stage, X->dt, nullptr);
+    else launch(k_adj_a<R>, nbc, kAdjThreads, h->stream, P, V, A, stage, X->dt, nullptr);
     CK(cudaGetLastError());
     h->launches += 3;
     return SPH_OK;
@@ -1421,7 +1416,7 @@ int adj_step(sph_handle* h, bool first, int j) {
             adj_pass_a<R>(h, V);
         }
         tic(h, PH_ADJ);
-        k_shift_sum<R><<<nb, 256, 0, h->stream>>>(P, V, A);
+        launch(k_shift_sum<R>, nb, 256, h->stream, P, V, A);
         h->launches += 1;
     }
     tic(h, PH_ADJ);
@@ -1431,51 +1426,51 @@ int adj_step(sph_handle* h, bool first, int j) {
     if (mls1) {
         // the shift's reverse; the positions pass through to the last stage, the
         // re-initialised densities' adjoint waits for the last RHS's reverse
-        k_adj_mls_end<R><<<nb, 256, 0, h->stream>>>(P, D, A, shift ? 1 : 0, X->mls_xe, X->mls_lam);
-        k_adj_mls1_end<R><<<nb, 256, 0, h->stream>>>(P, D, X->mls_xe, X->mls_lam, X->mls_x, X->mls_r);
-        k_adj_stage3<R><<<nb, 256, 0, h->stream>>>(P, D, A, dt, 0, X->mls_x, X->mls_r);
+        launch(k_adj_mls_end<R>, nb, 256, h->stream, P, D, A, shift ? 1 : 0, X->mls_xe, X->mls_lam);
+        launch(k_adj_mls1_end<R>, nb, 256, h->stream, P, D, X->mls_xe, X->mls_lam, X->mls_x, X->mls_r);
+        launch(k_adj_stage3<R>, nb, 256, h->stream, P, D, A, dt, 0, X->mls_x, X->mls_r);
         h->launches += 3;
     } else if (mls) {
         // the shift's reverse, then that of the re-initialisation on the state the
         // last stage produced (stage slot state 3) over the step's lists
         const Sorted<R> V3 = stage_view<R>(h, j, 3);
         const int nbo = blocks(P.n_tot, 128);
-        k_adj_mls_end<R><<<nb, 256, 0, h->stream>>>(P, D, A, shift ? 1 : 0, X->mls_xe, X->mls_lam);
+        launch(k_adj_mls_end<R>, nb, 256, h->stream, P, D, A, shift ? 1 : 0, X->mls_xe, X->mls_lam);
         if (P.mls_order == 6) {
-            k_adj_mls_own<R, 6><<<nbo, 128, 0, h->stream>>>(P, V3, X->mls_lam, X->mls_cy, X->mls_xo);
-            k_adj_mls_nbr<R, 6><<<nbo, 128, 0, h->stream>>>(P, V3, X->mls_lam, X->mls_cy, X->mls_xo, X->mls_xe,
+            launch(k_adj_mls_own<R, 6>, nbo, 128, h->stream, P, V3, X->mls_lam, X->mls_cy, X->mls_xo);
+            launch(k_adj_mls_nbr<R, 6>, nbo, 128, h->stream, P, V3, X->mls_lam, X->mls_cy, X->mls_xo, X->mls_xe,
                                                              X->mls_x, X->mls_r, nullptr);
         } else {
-            k_adj_mls_own<R, 3><<<nbo, 128, 0, h->stream>>>(P, V3, X->mls_lam, X->mls_cy, X->mls_xo);
-            k_adj_mls_nbr<R, 3><<<nbo, 128, 0, h->stream>>>(P, V3, X->mls_lam, X->mls_cy, X->mls_xo, X->mls_xe,
+            launch(k_adj_mls_own<R, 3>, nbo, 128, h->stream, P, V3, X->mls_lam, X->mls_cy, X->mls_xo);
+            launch(k_adj_mls_nbr<R, 3>, nbo, 128, h->stream, P, V3, X->mls_lam, X->mls_cy, X->mls_xo, X->mls_xe,
                                                              X->mls_x, X->mls_r, nullptr);
         }
-        k_adj_stage3<R><<<nb, 256, 0, h->stream>>>(P, D, A, dt, 0, X->mls_x, X->mls_r);
+        launch(k_adj_stage3<R>, nb, 256, h->stream, P, D, A, dt, 0, X->mls_x, X->mls_r);
         h->launches += 4;
     } else {
         // the step end's shift reads the last RHS's flags, B^-1 and grad rho (kept:
         // from pass-A slot 3 j + 2; else the re-run above left them in the arrays)
-        k_adj_stage3<R><<<nb, 256, 0, h->stream>>>(P, kept ? pa_view<R>(h, D, 3 * j + 2) : D, A, dt,
-                                                     shift ? 1 : 0);
+        launch(k_adj_stage3<R>, nb, 256, h->stream, P, kept ? pa_view<R>(h, D, 3 * j + 2) : D, A, dt,
+                                                     shift ? 1 : 0, nullptr, nullptr);
         h->launches += 1;
     }
     for (int k = 2; k >= 0; --k)
         if ((rc = adj_rhs<R>(h, view(k), k + 1, k, shift && k == 2, kept, mls1 && k == 2))) return rc;
     if (first) {
         // the fresh K1 of the first step was evaluated on the step-start state
-        k_adj_load<R><<<nb, 256, 0, h->stream>>>(P, D, nullptr, nullptr);
+        launch(k_adj_load<R>, nb, 256, h->stream, P, D, nullptr, nullptr);
         h->launches += 1;
         if ((rc = adj_rhs<R>(h, D, 0, -1))) return rc;
     }
     tic(h, PH_ADJ);
     const int nba = blocks((long long)P.n_tot * kAdjLanes, kAdjThreads);
-    k_adj_nu_sum<<<1, 1024, 0, h->stream>>>((first ? 4 : 3) * nba, A.nu_part + (first ? 0 : nba), A.nu_acc);
-    k_adj_scatter<R><<<nb, 256, 0, h->stream>>>(P, D, A, first ? 1 : 0);
+    launch(k_adj_nu_sum, 1, 1024, h->stream, (first ? 4 : 3) * nba, A.nu_part + (first ? 0 : nba), A.nu_acc);
+    launch(k_adj_scatter<R>, nb, 256, h->stream, P, D, A, first ? 1 : 0);
     h->launches += 2;
     if (h->cfg.periodic) {
         const int n_src = h->n_host + h->n_lr;
-        k_adj_route<<<blocks(n_src, 256), 256, 0, h->stream>>>(n_src, n_src, h->S.tb_cnt, h->S.tb_off, A);
-        k_adj_route<<<blocks(h->n_host, 256), 256, 0, h->stream>>>(h->n_host, h->n_host, h->S.lr_cnt, h->S.lr_off,
+        launch(k_adj_route, blocks(n_src, 256), 256, h->stream, n_src, n_src, h->S.tb_cnt, h->S.tb_off, A);
+        launch(k_adj_route, blocks(h->n_host, 256), 256, h->stream, h->n_host, h->n_host, h->S.lr_cnt, h->S.lr_off,
                                                                      A);
         h->launches += 2;
     }
@@ -1496,15 +1491,14 @@ void adj_rhs_ms_values(sph_handle* h, const Sorted<R>& V, int kept_j) {
     const bool ghosts = P.ghost_assign && h->n_ghost > 0;
     if (kept_j >= 0) {
         if (ghosts) {
-            k_ghost_refill<R><<<blocks(h->n_ghost, 256), 256, 0, h->stream>>>(V, h->d_ghost_ids, h->n_ghost);
+            launch(k_ghost_refill<R>, blocks(h->n_ghost, 256), 256, h->stream, V, h->d_ghost_ids, h->n_ghost);
             h->launches += 1;
         }
         return;
     }
     tic(h, PH_A);
     if (ghosts) {
-        k_assign_ghosts<R><<<blocks((long long)h->n_ghost * 32, 128), 128, 0, h->stream>>>(
-            P, V, h->d_ghost_ids, h->n_ghost, h->t_phys, h->body_vel[0], h->body_vel[1], h->body_acc[0],
+        launch(k_assign_ghosts<R>, blocks((long long)h->n_ghost * 32, 128), 128, h->stream, P, V, h->d_ghost_ids, h->n_ghost, h->t_phys, h->body_vel[0], h->body_vel[1], h->body_acc[0],
             h->body_acc[1], X->A.gint, X->A.gsw);
         h->launches += 1;
     }
@@ -1543,41 +1537,41 @@ int adj_rhs_ms(sph_handle* h, const Sorted<R>& V, int k, int pred, bool drag, in
     tic(h, PH_ADJ);
     CK(cudaMemsetAsync(V.nflag, 0, (size_t)P.n_tot, h->stream));
     if (P.hllc)
-        k_adj_c<R, true, false, true><<<nbc, kAdjThreads, 0, h->stream>>>(P, V, A, A.lr[k], A.la[k],
+        launch(k_adj_c<R, true, false, true>, nbc, kAdjThreads, h->stream, P, V, A, A.lr[k], A.la[k],
                                                                           A.nu_part + (size_t)k * nbc);
     else
-        k_adj_c<R, true><<<nbc, kAdjThreads, 0, h->stream>>>(P, V, A, A.lr[k], A.la[k], A.nu_part + (size_t)k * nbc);
+        launch(k_adj_c<R, true>, nbc, kAdjThreads, h->stream, P, V, A, A.lr[k], A.la[k], A.nu_part + (size_t)k * nbc);
     if (shift) {
-        k_adj_shift<R><<<nb, kAdjThreads, 0, h->stream>>>(P, V, A);
+        launch(k_adj_shift<R>, nb, kAdjThreads, h->stream, P, V, A);
         h->launches += 1;
     }
     if (gm) {
-        k_adj_add_ghost_rm<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, V, A, gm);
+        launch(k_adj_add_ghost_rm<R>, blocks(P.n_tot, 256), 256, h->stream, P, V, A, gm);
         h->launches += 1;
     }
     if (mls1) {
-        k_adj_mls1_own<R><<<blocks(P.n_tot, 128), 128, 0, h->stream>>>(P, V, X->mls_cy);
-        k_adj_mls1_nbr<R><<<blocks(P.n_tot, 128), 128, 0, h->stream>>>(P, V, A, X->mls_lam, X->mls_cy);
+        launch(k_adj_mls1_own<R>, blocks(P.n_tot, 128), 128, h->stream, P, V, X->mls_cy);
+        launch(k_adj_mls1_nbr<R>, blocks(P.n_tot, 128), 128, h->stream, P, V, A, X->mls_lam, X->mls_cy);
         h->launches += 2;
     }
     if (drag) {
         double* part = A.nu_part + (size_t)4 * nbc;
-        k_mark_body_nbrs<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, V);
-        k_adj_drag<R><<<nb, kAdjThreads, 0, h->stream>>>(P, V, A, X->dloss * X->dt, part);
-        k_adj_nu_sum<<<1, 1024, 0, h->stream>>>(nb, part, A.nu_acc);
+        launch(k_mark_body_nbrs<R>, blocks(P.n_tot, 256), 256, h->stream, P, V);
+        launch(k_adj_drag<R>, nb, kAdjThreads, h->stream, P, V, A, X->dloss * X->dt, part);
+        launch(k_adj_nu_sum, 1, 1024, h->stream, nb, part, A.nu_acc);
         h->launches += 3;
     }
-    k_adj_point<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, V, A, shift ? 1 : 0);
-    k_adj_a<R, true><<<nbc, kAdjThreads, 0, h->stream>>>(P, V, A, 0, X->dt, A.lg[k]);
+    launch(k_adj_point<R>, blocks(P.n_tot, 256), 256, h->stream, P, V, A, shift ? 1 : 0);
+    launch(k_adj_a<R, true>, nbc, kAdjThreads, h->stream, P, V, A, 0, X->dt, A.lg[k]);
     if (ghosts) {
         const int ngb = blocks((long long)h->n_ghost * 32, kAdjThreads);
-        k_adj_ghost_lambda<R><<<ngb, kAdjThreads, 0, h->stream>>>(P, V, A, h->d_ghost_ids, h->n_ghost, h->t_phys,
+        launch(k_adj_ghost_lambda<R>, ngb, kAdjThreads, h->stream, P, V, A, h->d_ghost_ids, h->n_ghost, h->t_phys,
                                                                   h->body_acc[0], h->body_acc[1], A.mo_part);
-        k_adj_motion_sum<<<1, 1024, 0, h->stream>>>(ngb, 4, A.mo_part, 1.0, A.g_motion + 4 * (size_t)jstep);
-        k_adj_ghost_water<R><<<148 * 8, kAdjThreads, 0, h->stream>>>(P, V, A, h->body_acc[0], h->body_acc[1]);
+        launch(k_adj_motion_sum, 1, 1024, h->stream, ngb, 4, A.mo_part, 1.0, A.g_motion + 4 * (size_t)jstep);
+        launch(k_adj_ghost_water<R>, 148 * 8, kAdjThreads, h->stream, P, V, A, h->body_acc[0], h->body_acc[1]);
         h->launches += 3;
     }
-    k_adj_stage_ms<R><<<blocks(P.n_tot, 256), 256, 0, h->stream>>>(P, V, A, pred, X->dt);
+    launch(k_adj_stage_ms<R>, blocks(P.n_tot, 256), 256, h->stream, P, V, A, pred, X->dt);
     CK(cudaGetLastError());
     h->launches += 5;
     return SPH_OK;
@@ -1619,7 +1613,7 @@ int adj_step_ms(sph_handle* h, bool first, int j, int jstep) {
         adj_rhs_ms_values<R>(h, V, kept ? j : -1);
         tic(h, PH_ADJ);
         if (shift) {
-            k_shift_sum<R><<<nb, 256, 0, h->stream>>>(P, V, A);
+            launch(k_shift_sum<R>, nb, 256, h->stream, P, V, A);
             h->launches += 1;
         }
     }
@@ -1627,30 +1621,30 @@ int adj_step_ms(sph_handle* h, bool first, int j, int jstep) {
     const bool mls1 = mls && P.mls_order == 1;
     if (mls1) {
         // as in adj_step: the densities' adjoint goes to the corrector RHS's reverse
-        k_adj_mls_end<R><<<nb, 256, 0, h->stream>>>(P, D, A, shift ? 1 : 0, X->mls_xe, X->mls_lam);
-        k_adj_mls1_end<R><<<nb, 256, 0, h->stream>>>(P, D, X->mls_xe, X->mls_lam, X->mls_x, X->mls_r);
-        k_adj_stage_end_ms<R><<<nb, 256, 0, h->stream>>>(P, D, A, dt, 0, X->mls_x, X->mls_r);
+        launch(k_adj_mls_end<R>, nb, 256, h->stream, P, D, A, shift ? 1 : 0, X->mls_xe, X->mls_lam);
+        launch(k_adj_mls1_end<R>, nb, 256, h->stream, P, D, X->mls_xe, X->mls_lam, X->mls_x, X->mls_r);
+        launch(k_adj_stage_end_ms<R>, nb, 256, h->stream, P, D, A, dt, 0, X->mls_x, X->mls_r);
         h->launches += 3;
     } else if (mls) {
         // the shift's reverse, then that of the re-initialisation on the corrected
         // state (stage slot state 3) over the step's lists
         const Sorted<R> V3 = stage_view<R>(h, j, 3);
         const int nbo = blocks(P.n_tot, 128);
-        k_adj_mls_end<R><<<nb, 256, 0, h->stream>>>(P, D, A, shift ? 1 : 0, X->mls_xe, X->mls_lam);
+        launch(k_adj_mls_end<R>, nb, 256, h->stream, P, D, A, shift ? 1 : 0, X->mls_xe, X->mls_lam);
         if (P.mls_order == 6) {
-            k_adj_mls_own<R, 6><<<nbo, 128, 0, h->stream>>>(P, V3, X->mls_lam, X->mls_cy, X->mls_xo);
-            k_adj_mls_nbr<R, 6><<<nbo, 128, 0, h->stream>>>(P, V3, X->mls_lam, X->mls_cy, X->mls_xo, X->mls_xe,
+            launch(k_adj_mls_own<R, 6>, nbo, 128, h->stream, P, V3, X->mls_lam, X->mls_cy, X->mls_xo);
+            launch(k_adj_mls_nbr<R, 6>, nbo, 128, h->stream, P, V3, X->mls_lam, X->mls_cy, X->mls_xo, X->mls_xe,
                                                              X->mls_x, X->mls_r, X->mls_gm);
         } else {
-            k_adj_mls_own<R, 3><<<nbo, 128, 0, h->stream>>>(P, V3, X->mls_lam, X->mls_cy, X->mls_xo);
-            k_adj_mls_nbr<R, 3><<<nbo, 128, 0, h->stream>>>(P, V3, X->mls_lam, X->mls_cy, X->mls_xo, X->mls_xe,
+            launch(k_adj_mls_own<R, 3>, nbo, 128, h->stream, P, V3, X->mls_lam, X->mls_cy, X->mls_xo);
+            launch(k_adj_mls_nbr<R, 3>, nbo, 128, h->stream, P, V3, X->mls_lam, X->mls_cy, X->mls_xo, X->mls_xe,
                                                              X->mls_x, X->mls_r, X->mls_gm);
         }
-        k_adj_stage_end_ms<R><<<nb, 256, 0, h->stream>>>(P, D, A, dt, 0, X->mls_x, X->mls_r);
+        launch(k_adj_stage_end_ms<R>, nb, 256, h->stream, P, D, A, dt, 0, X->mls_x, X->mls_r);
         h->launches += 4;
     } else {
-        k_adj_stage_end_ms<R><<<nb, 256, 0, h->stream>>>(P, shift && kept ? pa_view<R>(h, D, j) : D, A, dt,
-                                                          shift ? 1 : 0);
+        launch(k_adj_stage_end_ms<R>, nb, 256, h->stream, P, shift && kept ? pa_view<R>(h, D, j) : D, A, dt,
+                                                          shift ? 1 : 0, nullptr, nullptr);
         h->launches += 1;
     }
     if ((rc = adj_rhs_ms<R>(h, V, 1, 1, X->loss == SPH_LOSS_DRAG, jstep, kept ? j : -1, pre, shift,
@@ -1658,21 +1652,21 @@ int adj_step_ms(sph_handle* h, bool first, int j, int jstep) {
         return rc;
     if (first) {
         // the fresh K1 of the first step was evaluated on the step-start state
-        k_adj_load<R><<<nb, 256, 0, h->stream>>>(P, D, nullptr, nullptr);
+        launch(k_adj_load<R>, nb, 256, h->stream, P, D, nullptr, nullptr);
         h->launches += 1;
         if ((rc = adj_rhs_ms<R>(h, D, 0, 0, false, jstep))) return rc;
     }
     tic(h, PH_ADJ);
     const int nba = blocks((long long)P.n_tot * kAdjLanes, kAdjThreads);
-    k_adj_nu_sum<<<1, 1024, 0, h->stream>>>((first ? 2 : 1) * nba, A.nu_part + (first ? 0 : nba), A.nu_acc);
+    launch(k_adj_nu_sum, 1, 1024, h->stream, (first ? 2 : 1) * nba, A.nu_part + (first ? 0 : nba), A.nu_acc);
     // with library ghost assignment the body moved by u_body dt at the step start:
     // dL/du_body += dt sum_body dL/dx
     if (P.ghost_assign) {
-        k_adj_body_pos<R><<<nb, 256, 0, h->stream>>>(P, D, A, A.mo_part);
-        k_adj_motion_sum<<<1, 1024, 0, h->stream>>>(nb, 2, A.mo_part, dt, A.g_motion + 4 * (size_t)jstep);
+        launch(k_adj_body_pos<R>, nb, 256, h->stream, P, D, A, A.mo_part);
+        launch(k_adj_motion_sum, 1, 1024, h->stream, nb, 2, A.mo_part, dt, A.g_motion + 4 * (size_t)jstep);
         h->launches += 2;
     }
-    k_adj_scatter<R><<<nb, 256, 0, h->stream>>>(P, D, A, first ? 1 : 0);
+    launch(k_adj_scatter<R>, nb, 256, h->stream, P, D, A, first ? 1 : 0);
     h->launches += 2;
     CK(cudaGetLastError());
     tic(h, -1);
@@ -1698,7 +1692,7 @@ int adjoint_backward(sph_handle* h, double dloss, double* g_vel0, double* g_rho0
     if (ms) CK(cudaMemsetAsync(A.g_motion, 0, sizeof(double) * 4 * (size_t)X->nsteps, h->stream));
     // seed from the final state
     if ((rc = unsort<R>(h)) || (rc = snap_io(h, X->ck, X->nseg, n, false))) return rc;
-    k_adj_seed<<<blocks(n, 256), 256, 0, h->stream>>>(n, X->loss, dloss, h->S.type, h->S.vel, h->S.mass, X->target,
+    launch(k_adj_seed, blocks(n, 256), 256, h->stream, n, X->loss, dloss, h->S.type, h->S.vel, h->S.mass, X->target,
                                                      A);
     h->launches += 1;
     CK(cudaMemsetAsync(A.nu_acc, 0, sizeof(double), h->stream));
@@ -1728,8 +1722,8 @@ int adjoint_backward(sph_handle* h, double dloss, double* g_vel0, double* g_rho0
     if ((rc = read_status(h))) return rc;
     // gradients with respect to the state the forward started from (id order)
     double* gx = h->d_xfer + 2 * (size_t)n;
-    if (g_vel0) k_deinterleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, A.lv, h->d_xfer);
-    if (g_pos0) k_deinterleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, A.lx, gx);
+    if (g_vel0) launch(k_deinterleave, blocks(n, 256), 256, h->stream, n, A.lv, h->d_xfer);
+    if (g_pos0) launch(k_deinterleave, blocks(n, 256), 256, h->stream, n, A.lx, gx);
     if ((rc = to_host(h, {{g_vel0, h->d_xfer, sizeof(double) * 2 * n}, {g_pos0, gx, sizeof(double) * 2 * n},
                           {g_rho0, A.lrho, sizeof(double) * n}, {g_params, A.nu_acc, sizeof(double)}})))
         return rc;
@@ -1871,7 +1865,7 @@ int get_state_impl(sph_handle* h, int n, double* pos, double* vel, double* rho, 
     // one pass packs x, v (column-major), rho and the pressure (status_equation
     // on the device) into the transfer buffer; the requested blocks are then
     // copied back
-    k_snapshot<<<blocks(n, 256), 256, 0, h->stream>>>(h->P, n, h->S.pos, h->S.vel, h->S.rho, h->d_xfer);
+    launch(k_snapshot, blocks(n, 256), 256, h->stream, h->P, n, h->S.pos, h->S.vel, h->S.rho, h->d_xfer);
     CK(cudaGetLastError());
     h->launches += 1;
     const size_t nn = (size_t)n;
@@ -1921,8 +1915,8 @@ int sph_set_state(sph_handle* h, int n, const double* pos, const double* vel, co
                            hin(rho, h->S.rho, sizeof(double) * nn), hin(mass, h->S.mass, sizeof(double) * nn),
                            hin(sps_mass, h->S.smass, sizeof(double) * nn), hin(type, h->S.type, sizeof(int) * nn)});
     if (rc) return rc;
-    k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, h->d_xfer, h->S.pos);
-    k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, xv, h->S.vel);
+    launch(k_interleave, blocks(n, 256), 256, h->stream, n, h->d_xfer, h->S.pos);
+    launch(k_interleave, blocks(n, 256), 256, h->stream, n, xv, h->S.vel);
     if (!sps_mass)
         CK(cudaMemcpyAsync(h->S.smass, h->S.mass, sizeof(double) * nn, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->S.itype, h->S.type, sizeof(int) * nn, cudaMemcpyDeviceToDevice, h->stream));
@@ -1962,8 +1956,8 @@ int sph_update_state(sph_handle* h, int n, const double* pos, const double* vel,
     if ((rc = from_host(h, {hin(pos, h->d_xfer, sizeof(double) * 2 * n), hin(vel, xv, sizeof(double) * 2 * n),
                             hin(rho, h->S.rho, sizeof(double) * n)})))
         return rc;
-    k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, h->d_xfer, h->S.pos);
-    k_interleave<<<blocks(n, 256), 256, 0, h->stream>>>(n, xv, h->S.vel);
+    launch(k_interleave, blocks(n, 256), 256, h->stream, n, h->d_xfer, h->S.pos);
+    launch(k_interleave, blocks(n, 256), 256, h->stream, n, xv, h->S.vel);
     CK(cudaGetLastError());
     h->launches += 2;
     h->staging_valid = true;
@@ -2033,7 +2027,7 @@ int sph_snapshot_begin(sph_handle* h, int n, double* pos, double* vel, double* r
     if (!h->d_snap) CK(dalloc(&h->d_snap, (size_t)6 * h->cap_host));
     rc = h->mixed ? unsort<float>(h) : unsort<double>(h);
     if (rc) return rc;
-    k_snapshot<<<blocks(n, 256), 256, 0, h->stream>>>(h->P, n, h->S.pos, h->S.vel, h->S.rho, h->d_snap);
+    launch(k_snapshot, blocks(n, 256), 256, h->stream, h->P, n, h->S.pos, h->S.vel, h->S.rho, h->d_snap);
     CK(cudaGetLastError());
     h->launches += 1;
     CK(cudaEventRecord(h->snap_ready, h->stream));
@@ -2181,8 +2175,8 @@ int sph_rhs(sph_handle* h, double* drhodt, double* acc, double* avg_vel, int* fs
     rc = read_status(h);
     if (rc) return rc;
     if (!h->d_export) CK(dalloc(&h->d_export, (size_t)kExportFields * h->cap_host));
-    if (h->mixed) k_export_rhs<float><<<blocks(h->P.n_tot, 256), 256, 0, h->stream>>>(h->P, h->D32, h->d_export);
-    else k_export_rhs<double><<<blocks(h->P.n_tot, 256), 256, 0, h->stream>>>(h->P, h->D64, h->d_export);
+    if (h->mixed) launch(k_export_rhs<float>, blocks(h->P.n_tot, 256), 256, h->stream, h->P, h->D32, h->d_export);
+    else launch(k_export_rhs<double>, blocks(h->P.n_tot, 256), 256, h->stream, h->P, h->D64, h->d_export);
     CK(cudaGetLastError());
     const size_t n = (size_t)h->n_host;
     double* x = h->d_export;

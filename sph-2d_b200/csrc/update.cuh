@@ -22,6 +22,7 @@ __device__ __forceinline__ void apply_shift(const Params& P, const Sorted<R>& D,
 template <typename R>
 __global__ void k_stage(Params P, Sorted<R> D, int stage, double dt, int use_carried, int do_shift,
                         unsigned* status) {
+    pdl_begin();
     stamp_phase(P.stamp);
     using V2 = typename VT<R>::V2;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -106,6 +107,7 @@ __device__ __forceinline__ bool chol_solve_e1(double (&A)[M * (M + 1) / 2], doub
 
 template <typename R, int M>
 __global__ void k_mls(Params P, Sorted<R> D, double* rho_new) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
@@ -173,6 +175,7 @@ __global__ void k_mls(Params P, Sorted<R> D, double* rho_new) {
 // Define_freesurface_and_Normailized_derivates.f90:87-91), in FP64.
 template <typename R>
 __global__ void k_mls1(Params P, Sorted<R> D, double* rho_new) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
@@ -201,6 +204,7 @@ __global__ void k_mls1(Params P, Sorted<R> D, double* rho_new) {
 // step (when on) is applied, as the reference's driver calls the two in turn.
 template <typename R>
 __global__ void k_finish_mls(Params P, Sorted<R> D, const double* rho_new, int do_shift, unsigned* status) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
@@ -310,6 +314,7 @@ template <typename R>
 __global__ void k_assign_ghosts(Params P, Sorted<R> D, const int* ghost_ids, int n_ghost, double t, double bvx,
                                 double bvy, double bax, double bay, double4* gint = nullptr,
                                 double* gsw = nullptr) {
+    pdl_begin();
     stamp_phase(P.stamp);
     const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wg >= n_ghost) return;                       // whole warps
@@ -388,6 +393,7 @@ __global__ void k_assign_ghosts(Params P, Sorted<R> D, const int* ghost_ids, int
 // state that already holds the assigned ghosts (FP64 records: aux.x = m exactly).
 template <typename R>
 __global__ void k_ghost_refill(Sorted<R> D, const int* ghost_ids, int n_ghost) {
+    pdl_begin();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n_ghost) return;
     const int s = D.slot_of[ghost_ids[g]];
@@ -400,7 +406,7 @@ __global__ void k_ghost_refill(Sorted<R> D, const int* ghost_ids, int n_ghost) {
 }
 
 // The end of a timed stretch of work.
-__global__ void k_stamp(unsigned long long* slot) { stamp_phase(slot); }
+__global__ void k_stamp(unsigned long long* slot) { pdl_begin(); stamp_phase(slot); }
 
 // Kinetic energy and max |v| of the water host particles
 // (Sampling_subroutine.f90:346-356) in FP64 and the number of flagged surface
@@ -413,6 +419,7 @@ template <typename R>
 __global__ void __launch_bounds__(kRedThreads) k_diag(Params P, Sorted<R> D, double* part_ke, double* part_max,
                                                       int* part_ns, unsigned* done, const unsigned* status,
                                                       const double* bf, HostBox* box) {
+    pdl_begin();
     __shared__ double ske[kRedThreads], smx[kRedThreads];
     __shared__ int sns[kRedThreads];
     __shared__ int flag;
@@ -469,6 +476,7 @@ __global__ void __launch_bounds__(kRedThreads) k_diag(Params P, Sorted<R> D, dou
 template <typename R>
 __global__ void __launch_bounds__(kRedThreads) k_body_force(Params P, Sorted<R> D, const int* body_ids, int n_body,
                                                             double* part, double* out, unsigned* done) {
+    pdl_begin();
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const int g = (blockIdx.x * kRedThreads + t) >> 5;
     double f[4] = {0, 0, 0, 0};
@@ -541,6 +549,7 @@ __global__ void __launch_bounds__(kRedThreads) k_body_force(Params P, Sorted<R> 
 // Pairs are emitted once, by their pair_i (lower id), sorted by (i, j).
 template <typename R>
 __global__ void k_pair_count(Params P, Sorted<R> D, long long* cnt_id) {
+    pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
     const int nn = D.nnbr[a];
@@ -559,6 +568,7 @@ __global__ void k_pair_count(Params P, Sorted<R> D, long long* cnt_id) {
 template <typename R>
 __global__ void k_pair_emit(Params P, Sorted<R> D, const long long* off_id, long long cap, int* pi, int* pj,
                             double* w, double* dwdx) {
+    pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= P.n_tot) return;
     const int nn = D.nnbr[a];
@@ -597,10 +607,12 @@ __global__ void k_pair_emit(Params P, Sorted<R> D, const long long* off_id, long
 
 // --- column-major (n,2) <-> interleaved conversions -----------------------
 __global__ void k_interleave(int n, const double* colmaj, double2* out) {
+    pdl_begin();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = make_double2(colmaj[i], colmaj[n + i]);
 }
 __global__ void k_deinterleave(int n, const double2* in, double* colmaj) {
+    pdl_begin();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) { double2 v = in[i]; colmaj[i] = v.x; colmaj[n + i] = v.y; }
 }
@@ -610,6 +622,7 @@ __global__ void k_deinterleave(int n, const double2* in, double* colmaj) {
 // [5n, 6n) pressure from the equation of state.
 __global__ void k_snapshot(Params P, int n, const double2* pos, const double2* vel, const double* rho,
                            double* out) {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double2 x = pos[i], v = vel[i];
@@ -626,6 +639,7 @@ __global__ void k_snapshot(Params P, int n, const double2* pos, const double2* v
 // arrays: drho [n], acc [2n], avg [2n] as doubles, then fs [n], near [n] as ints.
 template <typename R>
 __global__ void k_export_rhs(Params P, Sorted<R> D, double* out) {
+    pdl_begin();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     const int i = D.id[s];
@@ -646,6 +660,7 @@ __global__ void k_export_rhs(Params P, Sorted<R> D, double* out) {
 constexpr int kExportFields = 23;
 template <typename R>
 __global__ void k_export(Params P, Sorted<R> D, double* out) {
+    pdl_begin();
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n_tot) return;
     int i = D.id[s];

@@ -24,6 +24,7 @@ struct HostSeg {
     void* host;
     void* dev;
     size_t bytes;
+    bool joined = false;      // the device range goes on where the segment before it ends
 };
 
 class HostCopy {
@@ -61,15 +62,21 @@ private:
                 continue;
             }
             for (size_t o = 0; o < s.bytes; o += kChunk)
-                pieces.push_back({(char*)s.host + o, (char*)s.dev + o, s.bytes - o < kChunk ? s.bytes - o : kChunk});
+                pieces.push_back({(char*)s.host + o, (char*)s.dev + o, s.bytes - o < kChunk ? s.bytes - o : kChunk,
+                                  s.joined || o > 0});
             total += s.bytes;
         }
-        // small pieces share a chunk
+        // small pieces share a chunk, and joined ones a DMA
         std::vector<Chunk> chunks;
         for (const HostSeg& p : pieces) {
-            if (chunks.empty() || chunks.back().bytes + pad(p.bytes) > kChunk) chunks.push_back(Chunk{});
-            chunks.back().segs.push_back(p);
-            chunks.back().bytes += pad(p.bytes);
+            if (chunks.empty() || pad(chunks.back().bytes) + p.bytes > kChunk) chunks.push_back(Chunk{});
+            Chunk& c = chunks.back();
+            const bool next = p.joined && !c.dma.empty() && c.dma.back().dev + c.dma.back().bytes == p.dev;
+            const size_t at = next ? c.bytes : pad(c.bytes);
+            if (next) c.dma.back().bytes += p.bytes;
+            else c.dma.push_back({(char*)p.dev, at, p.bytes});
+            c.piece.push_back({(char*)p.host, at, p.bytes});
+            c.bytes = at + p.bytes;
         }
         int lanes = 1;
         if (total >= kShare) {
@@ -110,8 +117,17 @@ private:
     static constexpr size_t kChunk = size_t(1) << 20;      // 1 MiB: 20 us of PCIe, 8 MiB held at most
     static constexpr size_t kShare = size_t(4) << 20;      // a thread costs about 30 us to start
     static constexpr int kLanes = 4;
+    struct Part {
+        char* host;
+        size_t off, bytes;     // place in the chunk
+    };
+    struct Dma {
+        char* dev;
+        size_t off, bytes;
+    };
     struct Chunk {
-        std::vector<HostSeg> segs;
+        std::vector<Part> piece;
+        std::vector<Dma> dma;
         size_t bytes = 0;
     };
     struct Lane {
@@ -135,24 +151,19 @@ private:
         int k = 0;
         auto unpack = [&](const Chunk& c, int b) {
             if ((e = cudaEventSynchronize(l.ev[b])) != cudaSuccess) return;
-            size_t o = 0;
-            for (const HostSeg& s : c.segs) {
-                memcpy(s.host, (char*)l.buf[b] + o, s.bytes);
-                o += pad(s.bytes);
-            }
+            for (const Part& q : c.piece) memcpy(q.host, (char*)l.buf[b] + q.off, q.bytes);
         };
         bool used[2] = {false, false};
         for (size_t i = t; i < chunks.size() && e == cudaSuccess; i += lanes, k ^= 1) {
             const Chunk& c = chunks[i];
             if (!to_host && used[k]) e = cudaEventSynchronize(l.ev[k]);      // its DMA must be done
-            size_t o = 0;
-            for (const HostSeg& s : c.segs) {
-                char* pin = (char*)l.buf[k] + o;
+            char* pin = (char*)l.buf[k];
+            if (!to_host && e == cudaSuccess)
+                for (const Part& q : c.piece) memcpy(pin + q.off, q.host, q.bytes);
+            for (const Dma& d : c.dma) {
                 if (e != cudaSuccess) break;
-                if (!to_host) memcpy(pin, s.host, s.bytes);
-                e = to_host ? cudaMemcpyAsync(pin, s.dev, s.bytes, cudaMemcpyDeviceToHost, stream)
-                            : cudaMemcpyAsync(s.dev, pin, s.bytes, cudaMemcpyHostToDevice, stream);
-                o += pad(s.bytes);
+                e = to_host ? cudaMemcpyAsync(pin + d.off, d.dev, d.bytes, cudaMemcpyDeviceToHost, stream)
+                            : cudaMemcpyAsync(d.dev, pin + d.off, d.bytes, cudaMemcpyHostToDevice, stream);
             }
             if (e == cudaSuccess) e = cudaEventRecord(l.ev[k], stream);
             used[k] = true;

@@ -712,7 +712,9 @@ int from_host(sph_handle* h, std::initializer_list<HostSeg> segs) {
     CK(h->copier.copy(h->device, h->stream, segs, false));
     return SPH_OK;
 }
-HostSeg hin(const void* host, void* dev, size_t bytes) { return HostSeg{const_cast<void*>(host), dev, bytes}; }
+HostSeg hin(const void* host, void* dev, size_t bytes, bool joined = false) {
+    return HostSeg{const_cast<void*>(host), dev, bytes, joined};
+}
 
 // find_particle_pair on the state prepare has just sorted; the status of that
 // comes with the pair count in one wait.
@@ -1869,8 +1871,10 @@ int get_state_impl(sph_handle* h, int n, double* pos, double* vel, double* rho, 
     CK(cudaGetLastError());
     h->launches += 1;
     const size_t nn = (size_t)n;
-    return to_host(h, {{pos, h->d_xfer, sizeof(double) * 2 * nn}, {vel, h->d_xfer + 2 * nn, sizeof(double) * 2 * nn},
-                       {rho, h->d_xfer + 4 * nn, sizeof(double) * nn}, {press, h->d_xfer + 5 * nn, sizeof(double) * nn}});
+    return to_host(h, {{pos, h->d_xfer, sizeof(double) * 2 * nn, false},
+                       {vel, h->d_xfer + 2 * nn, sizeof(double) * 2 * nn, true},
+                       {rho, h->d_xfer + 4 * nn, sizeof(double) * nn, true},
+                       {press, h->d_xfer + 5 * nn, sizeof(double) * nn, true}});
 }
 
 }  // namespace
@@ -1952,14 +1956,14 @@ int sph_update_state(sph_handle* h, int n, const double* pos, const double* vel,
     int rc = h->mixed ? unsort<float>(h) : unsort<double>(h);
     if (rc) return rc;
     // complete on return: the caller owns (and may refill) its arrays afterwards
-    double* xv = h->d_xfer + 2 * (size_t)n;
-    if ((rc = from_host(h, {hin(pos, h->d_xfer, sizeof(double) * 2 * n), hin(vel, xv, sizeof(double) * 2 * n),
-                            hin(rho, h->S.rho, sizeof(double) * n)})))
+    const size_t nn = (size_t)n;
+    if ((rc = from_host(h, {hin(pos, h->d_xfer, sizeof(double) * 2 * nn),
+                            hin(vel, h->d_xfer + 2 * nn, sizeof(double) * 2 * nn, true),
+                            hin(rho, h->d_xfer + 4 * nn, sizeof(double) * nn, true)})))
         return rc;
-    launch(k_interleave, blocks(n, 256), 256, h->stream, n, h->d_xfer, h->S.pos);
-    launch(k_interleave, blocks(n, 256), 256, h->stream, n, xv, h->S.vel);
+    launch(k_upload, blocks(n, 256), 256, h->stream, n, h->d_xfer, h->S.pos, h->S.vel, h->S.rho);
     CK(cudaGetLastError());
-    h->launches += 2;
+    h->launches += 1;
     h->staging_valid = true;
     h->sorted_valid = false;
     return SPH_OK;
@@ -2181,9 +2185,9 @@ int sph_rhs(sph_handle* h, double* drhodt, double* acc, double* avg_vel, int* fs
     const size_t n = (size_t)h->n_host;
     double* x = h->d_export;
     int* flag = reinterpret_cast<int*>(x + 5 * n);
-    return to_host(h, {{drhodt, x, sizeof(double) * n}, {acc, x + n, sizeof(double) * 2 * n},
-                       {avg_vel, x + 3 * n, sizeof(double) * 2 * n}, {fs, flag, sizeof(int) * n},
-                       {near_fs, flag + n, sizeof(int) * n}});
+    return to_host(h, {{drhodt, x, sizeof(double) * n, false}, {acc, x + n, sizeof(double) * 2 * n, true},
+                       {avg_vel, x + 3 * n, sizeof(double) * 2 * n, true}, {fs, flag, sizeof(int) * n, true},
+                       {near_fs, flag + n, sizeof(int) * n, true}});
 }
 
 int sph_get_field(sph_handle* h, int field, double* out) {

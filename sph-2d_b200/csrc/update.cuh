@@ -611,6 +611,16 @@ __global__ void k_interleave(int n, const double* colmaj, double2* out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = make_double2(colmaj[i], colmaj[n + i]);
 }
+// pos, vel (column-major) and rho, one after another, into the id-order arrays.
+__global__ void k_upload(int n, const double* in, double2* pos, double2* vel, double* rho) {
+    pdl_begin();
+    const size_t nn = (size_t)n;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    pos[i] = make_double2(in[i], in[nn + i]);
+    vel[i] = make_double2(in[2 * nn + i], in[3 * nn + i]);
+    rho[i] = in[4 * nn + i];
+}
 __global__ void k_deinterleave(int n, const double2* in, double* colmaj) {
     pdl_begin();
     int i = blockIdx.x * blockDim.x + threadIdx.x;

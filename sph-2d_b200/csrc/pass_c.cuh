@@ -157,8 +157,14 @@ struct Side {
 // records loaded one iteration ahead (kept: 168 registers, 3 blocks per SM; 4
 // blocks without the prefetch 5.89).  ncu at 1024^2, 398 -> 270 M warp
 // instructions, 654 -> 431 us: FP64 pipe 50 % busy, L1 data stage 67 % (176 B of
-// records per neighbour), 58 % issue-active.
-template <typename R, bool MUSCL, bool MS, bool SHIFT, int L = 1>
+// records per neighbour), 58 % issue-active, the rest waits on results (1.9 cycles
+// an instruction at 3 warps a scheduler).  So branches inside the pair cost more
+// than the work they skip, as they end the stretch the compiler can interleave:
+// with the stages in this kernel 6.24 ms, 5.86 with the viscosity and the
+// near-surface case as selects, 5.06 with the kernel model fixed at compile time
+// (KM; FP64 launches).  In the mixed path it is the other way round (3.06 -> 3.27
+// ms): there the branch keeps the neighbour's loads early, and KM is 0.
+template <typename R, bool MUSCL, bool MS, bool SHIFT, int L = 1, int KM = 0>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIFT_BLOCKS : SPH_PASS_C_F32_BLOCKS) : 3)
     k_pass_c(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D, const __grid_constant__ StageArgs G) {
     pdl_begin();
@@ -201,6 +207,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
     typename VT<R>::V2 avg_a = mk2<R>(R(0), R(0));
     if (MS) avg_a = D.avg[a];
 
+    const bool gauss = KM ? KM == SPH_KERNEL_GAUSSIAN : P.kernel_model == SPH_KERNEL_GAUSSIAN;
     const R hbar = (R)P.h;
     const R inv_h = (R)P.inv_h;
     const R gk = (R)P.gk;
@@ -319,7 +326,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         {
             const R q = d * inv_h;
             const R kf = (R)P.kfactor;
-            if (P.kernel_model == SPH_KERNEL_GAUSSIAN) {
+            if (gauss) {
                 const R ex = exp(-(q * q));
                 w = (ex - (R)P.gauss_e9) * kf;
                 g = ex * gk;
@@ -373,7 +380,12 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
             const R bR = min(R(3) * (max(dU, R(0))), cbar);
             const R Ps = Pbar + R(0.5) * bR * rbar * dU;
             PA = near_a ? Pbar : Ps;
-            if (!near_a) { wa0 -= sU * e0; wa1 -= sU * e1; }
+            if constexpr (F32) {
+                if (!near_a) { wa0 -= sU * e0; wa1 -= sU * e1; }
+            } else {
+                const R sn = near_a ? R(0) : sU;
+                wa0 -= sn * e0; wa1 -= sn * e1;
+            }
         } else if (near_a) {
             PA = Pbar;
         } else if (HL) {
@@ -481,7 +493,12 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         // artificial viscosity (:392-417)
         const R inv_r2 = inv_d * inv_d;
         const R vx = du * xij0 + dv * xij1;
-        if (vx < R(0)) {
+        if constexpr (!F32) {
+            const R phi1 = hbar * min(vx, R(0)) * rcp(d * d + fh2);
+            const R mp = (Vb * rho_b) * ((beta * phi1 - alpha * cbar) * phi1 * inv_rbar);
+            tx -= mp * nd0;
+            ty -= mp * nd1;
+        } else if (vx < R(0)) {
             const R phi1 = fast_quot(hbar * vx, d * d + fh2);
             const R Pi = (-alpha * cbar * phi1 + beta * (phi1 * phi1)) * inv_rbar;
             tx += mb * (-Pi * nd0);
@@ -552,7 +569,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
                 const double d0 = (double)d;
                 const double dd2 = fma(fma(-d0, d0, dxd * dxd + dyd * dyd), 0.5 * (double)inv_d, d0);
                 const double q = dd2 * inv_h64;
-                if (P.kernel_model == SPH_KERNEL_GAUSSIAN) {
+                if (gauss) {
                     const double ex = exp(-(q * q));
                     wd = (ex - P.gauss_e9) * P.kfactor;
                     gd = -2.0 * P.kfactor * ex * inv_h2_64;

@@ -474,33 +474,41 @@ StageArgs stage_args(sph_handle* h, int mode, int stage, double dt, int shift = 
     return g;
 }
 
-template <typename R, int L>
+template <typename R, int L, int KM>
 void launch_pass_c_lanes(const Params& P, const Sorted<R>& D, const StageArgs& G, bool shift, cudaStream_t st) {
     const int nb = blocks((long long)P.n_tot * L, 128);
     if (P.ms) {
-        if (shift) launch(k_pass_c<R, false, true, true, L>, nb, 128, st, P, D, G);
-        else launch(k_pass_c<R, false, true, false, L>, nb, 128, st, P, D, G);
+        if (shift) launch(k_pass_c<R, false, true, true, L, KM>, nb, 128, st, P, D, G);
+        else launch(k_pass_c<R, false, true, false, L, KM>, nb, 128, st, P, D, G);
         return;
     }
     // (the mixed Taylor-Green launches never carry the shifting sum)
     if constexpr (sizeof(R) == 8) {
         if (shift) {
-            if (P.muscl) launch(k_pass_c<R, true, false, true, L>, nb, 128, st, P, D, G);
-            else launch(k_pass_c<R, false, false, true, L>, nb, 128, st, P, D, G);
+            if (P.muscl) launch(k_pass_c<R, true, false, true, L, KM>, nb, 128, st, P, D, G);
+            else launch(k_pass_c<R, false, false, true, L, KM>, nb, 128, st, P, D, G);
             return;
         }
     }
-    if (P.muscl) launch(k_pass_c<R, true, false, false, L>, nb, 128, st, P, D, G);
-    else launch(k_pass_c<R, false, false, false, L>, nb, 128, st, P, D, G);
+    if (P.muscl) launch(k_pass_c<R, true, false, false, L, KM>, nb, 128, st, P, D, G);
+    else launch(k_pass_c<R, false, false, false, L, KM>, nb, 128, st, P, D, G);
+}
+
+template <int KM>
+void launch_pass_c64(const Params& P, const Sorted<double>& D, const StageArgs& G, bool shift, cudaStream_t st) {
+    if (P.n_tot < kLanes4Below) launch_pass_c_lanes<double, 4, KM>(P, D, G, shift, st);
+    else if (P.n_tot < kLanes2BelowC) launch_pass_c_lanes<double, 2, KM>(P, D, G, shift, st);
+    else launch_pass_c_lanes<double, 1, KM>(P, D, G, shift, st);
 }
 
 template <typename R>
 void launch_pass_c(const Params& P, const Sorted<R>& D, const StageArgs& G, bool shift, cudaStream_t st) {
     if constexpr (sizeof(R) == 8) {
-        if (P.n_tot < kLanes4Below) { launch_pass_c_lanes<R, 4>(P, D, G, shift, st); return; }
-        if (P.n_tot < kLanes2BelowC) { launch_pass_c_lanes<R, 2>(P, D, G, shift, st); return; }
+        if (P.kernel_model == SPH_KERNEL_GAUSSIAN) launch_pass_c64<SPH_KERNEL_GAUSSIAN>(P, D, G, shift, st);
+        else launch_pass_c64<SPH_KERNEL_WENDLAND2>(P, D, G, shift, st);
+    } else {
+        launch_pass_c_lanes<R, 1, 0>(P, D, G, shift, st);
     }
-    launch_pass_c_lanes<R, 1>(P, D, G, shift, st);
 }
 
 // One RHS evaluation on the current stage state.  G: the stage that follows it,

@@ -219,15 +219,23 @@ __device__ __forceinline__ void cell_key(const Params& P, const SetupBuf& B, int
     B.rank[o] = atomicAdd(&B.cnt[key], 1);
 }
 
-// One image of host particle i with id o.
-__device__ __forceinline__ void put_image(const Params& P, const Staging& S, const SetupBuf& B, int i, int o, double2 x,
-                                          int cap, unsigned* status) {
+// What an image takes from its source, read once for all its images (up to eight
+// in a thin box) and before their stores: the loads of an image used to wait for
+// the previous image's stores.  images 14.4 -> 12.6 us per step at 100^2, 206 ->
+// 169 us at 2048^2.
+struct ImageSource {
+    double2 vel;
+    double rho, mass, smass;
+};
+// One image with id o.
+__device__ __forceinline__ void put_image(const Params& P, const Staging& S, const SetupBuf& B, const ImageSource& q, int o,
+                                          double2 x, int cap, unsigned* status) {
     if (o >= cap) return;                       // the host sees the total and stops
     S.pos[o] = x;
-    S.vel[o] = S.vel[i];
-    S.rho[o] = S.rho[i];
-    S.mass[o] = S.mass[i];
-    S.smass[o] = S.smass[i];
+    S.vel[o] = q.vel;
+    S.rho[o] = q.rho;
+    S.mass[o] = q.mass;
+    S.smass[o] = q.smass;
     S.type[o] = SPH_TYPE_PERIODIC;
     S.itype[o] = SPH_TYPE_PERIODIC;
     cell_key(P, B, o, x, SPH_TYPE_PERIODIC, status);
@@ -269,6 +277,7 @@ __global__ void __launch_bounds__(kImgThreads) k_img_emit(Params P, Staging S, S
         }
     }
     if (lr == 0 && tb == 0) return;
+    const ImageSource src = {S.vel[i], S.rho[i], S.mass[i], S.smass[i]};
     const double Lx = P.box_hi[0] - P.box_lo[0], Ly = P.box_hi[1] - P.box_lo[1];
     // sides of each axis in order: low side (shift +L), high side (-L)
     const bool xlo = x.x <= (P.box_lo[0] + P.band) && x.x >= P.box_lo[0];
@@ -283,13 +292,13 @@ __global__ void __launch_bounds__(kImgThreads) k_img_emit(Params P, Staging S, S
         double2 y = x;
         if (sx >= 0) {
             y.x = x.x + (sx == 0 ? Lx : -Lx);
-            put_image(P, S, B, i, o, y, cap, status);
+            put_image(P, S, B, src, o, y, cap, status);
             ++o;
         }
         int q = first_tb + (sx < 0 ? o_tb : o_lt + k * tb);
         if (sx >= 0) ++k;
-        if (ylo) { put_image(P, S, B, i, q, make_double2(y.x, y.y + Ly), cap, status); ++q; }
-        if (yhi) put_image(P, S, B, i, q, make_double2(y.x, y.y + (-Ly)), cap, status);
+        if (ylo) { put_image(P, S, B, src, q, make_double2(y.x, y.y + Ly), cap, status); ++q; }
+        if (yhi) put_image(P, S, B, src, q, make_double2(y.x, y.y + (-Ly)), cap, status);
     }
 }
 
@@ -310,6 +319,10 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(SetupBuf B, unsigned
 #pragma unroll
     for (int k = 0; k < per; ++k)
         if (c0 + k <= B.ncells) { B.pre[c0 + k] = run; run += v[k]; }
+    if (gridDim.x == 1) {            // one block's offset is 0: nothing to scan
+        if (threadIdx.x == 0) B.blkoff[0] = 0;
+        return;
+    }
     if (threadIdx.x == 0) B.blkoff[blockIdx.x] = total;
     if (!last_block(&B.done[1], &flag)) return;
     int sum = 0;
@@ -678,6 +691,14 @@ __device__ __forceinline__ bool pair_allowed(int rule, int ti, int tj) {
     return true;
 }
 
+// Whether pair_allowed can refuse a pair of a particle of type ti: with the
+// one-fluid rule not for water, with the other rule only for the boundary types.
+// Where it cannot, no candidate's type is read: sort + lists 189 -> 172 us per step
+// for the square at D/100, 35 -> 30 us at D/30.
+__device__ __forceinline__ bool pair_may_fail(int rule, int ti) {
+    return rule == SPH_PAIRS_ONE_FLUID ? ti != SPH_TYPE_WATER : ti == -2 || ti == -3 || ti == -201;
+}
+
 // --- 5. neighbour lists ----------------------------------------------------
 // Every particle b != a in the 3x3 cells with |x_a - x_b|^2 <= (support*(1+skin))^2
 // and an allowed type pair.  The exact support test is repeated at every RHS on
@@ -687,7 +708,9 @@ __device__ __forceinline__ bool pair_allowed(int rule, int ti, int tj) {
 // ([entry][thread], conflict-free) and written out row by row after the scan, so
 // the stores of a warp are coalesced; longer lists write the rest directly.
 constexpr int kListStage = 32;
-template <typename R>
+// ONE: the one-fluid rule, known to the compiler (the square's rule in the same code
+// cost the Taylor-Green lists 3 %: 748 -> 769 us per step at 2048^2, 737 this way).
+template <typename R, bool ONE>
 __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsigned* status) {
     pdl_begin();
     __shared__ unsigned stage[kListStage][128];
@@ -713,8 +736,8 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
         int ida = D.id[a];
         int cx = (int)floor((xa.x - P.gx0) / P.cs), cy = (int)floor((xa.y - P.gy0) / P.cs);
         int x0 = max(cx - 1, 0), x1 = min(cx + 1, P.gnx - 1);
-        // with the one-fluid rule every pair of a water particle is allowed
-        const bool check_type = !(P.pair_rule == SPH_PAIRS_ONE_FLUID && ta == SPH_TYPE_WATER);
+        const int rule = ONE ? (int)SPH_PAIRS_ONE_FLUID : P.pair_rule;
+        const bool check_type = pair_may_fail(rule, ta);
         for (int gy = max(cy - 1, 0); gy <= min(cy + 1, P.gny - 1); ++gy) {
             // the cells x0..x1 of a row are consecutive keys, so their particles
             // form one contiguous range of the sorted order
@@ -743,7 +766,7 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (b + k == a) continue;
-                    if (check_type && !pair_allowed(P.pair_rule, ta, tb[k])) continue;
+                    if (check_type && !pair_allowed(rule, ta, tb[k])) continue;
                     if (F32) {
                         const float dx = xa_h.x - xbh[k].x, dy = xa_h.y - xbh[k].y;
                         if (dx * dx + dy * dy > P.r2_list32) continue;
@@ -756,7 +779,7 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
             }
             for (; b < b1; ++b) {
                 if (b == a) continue;
-                if (check_type && !pair_allowed(P.pair_rule, ta, D.type[b])) continue;
+                if (check_type && !pair_allowed(rule, ta, D.type[b])) continue;
                 if (F32) {
                     const float2 xbh = xh[b];
                     const float dx = xa_h.x - xbh.x, dy = xa_h.y - xbh.y;
@@ -815,7 +838,7 @@ __global__ void __launch_bounds__(128) k_build_lists_lanes(Params P, Sorted<R> D
             len[r] = b1 - b0;
         }
     }
-    const bool check_type = !(P.pair_rule == SPH_PAIRS_ONE_FLUID && ta == SPH_TYPE_WATER);
+    const bool check_type = pair_may_fail(P.pair_rule, ta);
     const int l01 = len[0] + len[1], total = l01 + len[2];
     const int most = __reduce_max_sync(0xffffffffu, total);
     int cnt = 0;
@@ -859,7 +882,8 @@ void launch_lists(const Params& P, const Sorted<R>& D, unsigned* status, cudaStr
         const long long t = (long long)P.n_tot * kListLanes;
         launch(k_build_lists_lanes<R, kListLanes>, (unsigned)((t + 127) / 128), 128, st, P, D, status);
     } else {
-        launch(k_build_lists<R>, (P.n_tot + 127) / 128, 128, st, P, D, status);
+        launch(P.pair_rule == SPH_PAIRS_ONE_FLUID ? k_build_lists<R, true> : k_build_lists<R, false>,
+               (P.n_tot + 127) / 128, 128, st, P, D, status);
     }
 }
 

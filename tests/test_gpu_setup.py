@@ -65,3 +65,13 @@ def test_images_follow_a_particle_through_the_boundary(lib, oracle):
             sim.set_state(p, case.vel, case.rho, case.mass, case.type)
             out.append(sim.find_particle_pair(20 * n))
     assert np.array_equal(out[0]["pair_i"], out[1]["pair_i"]) and np.array_equal(out[0]["pair_j"], out[1]["pair_j"])
+
+
+@pytest.mark.parametrize("side", [40, 260])
+def test_pairs_of_typed_particles_under_the_same_boundary_rule(lib, oracle, side):
+    """Every type the rule tells apart, on both list builders (8 lanes per particle at
+    40^2, a thread at 260^2): only the boundary types look at their candidates' types."""
+    case = S.make_tgv(side, jitter=0.1, seed=7)
+    case.cfg.pair_rule = S.PAIRS_NO_SAME_BND
+    typ = np.random.default_rng(side).choice(np.array([2, -2, -3, -201, -102], case.type.dtype), case.n)
+    _check(oracle, case, case.pos, typ)

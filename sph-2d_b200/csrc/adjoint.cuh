@@ -139,7 +139,8 @@ struct PSide {
     bool water, near;
 };
 
-template <typename R, bool MS = false, bool MUSCL = false>
+// BI: with B^-1, which only the particle whose sum is differentiated needs.
+template <typename R, bool MS = false, bool MUSCL = false, bool BI = true>
 __device__ __forceinline__ PSide load_side(const Sorted<R>& D, int s) {
     PSide o;
     o.x = D.pos[s];
@@ -155,7 +156,7 @@ __device__ __forceinline__ PSide load_side(const Sorted<R>& D, int s) {
     const double gs = grad_scale<R>();
     o.t0 = (double)n1.x; o.t1 = (double)n1.y; o.t2 = (double)n1.z; o.g0 = gs * n1.w;
     o.g1 = gs * D.nb2[s].x;
-    o.bi = load4(&D.binv64[s]);
+    if (BI) o.bi = load4(&D.binv64[s]);
     o.water = D.type[s] == SPH_TYPE_WATER;
     o.near = (D.flags[s] & 2) != 0;
     o.ax = o.ay = 0.0;
@@ -574,13 +575,67 @@ __device__ __forceinline__ void rev_pair(const Params& P, const PSide& A, const 
     o.Vb = Vbb;
 }
 
-// Reverse of pass C for the RHS whose rate adjoints are (lr, la).  Four
-// consecutive lanes share a particle c: lane bit 0 picks the role (0: the
-// derivative of c's own sum, 1: the derivatives of the neighbours' sums with
-// respect to c's inputs), lane bit 1 the pairs (even or odd list positions).
-// Each lane inlines one pair reverse, so the register count stays low and a
-// small particle count still fills the GPU; the four partial sums are combined
-// by shuffles in a fixed order.
+// The part of k_adj_c's sums that one lane forms, over the pairs e0, e0 + 2, ... of c.
+// ROLE 0: the derivative of c's own sum; 1: the derivatives of the neighbours' sums
+// with respect to c's inputs.
+template <typename R, bool MS, bool MUSCL, bool HLLC, int ROLE, int NV>
+__device__ __forceinline__ void adj_c_pairs(const Params& P, const Sorted<R>& D, const double* lr, const double2* la,
+                                            int c, int e0, double (&v)[NV], double& nu_sum) {
+    const int nn = D.npairs[c];
+    double l_r = 0.0;
+    double2 l_a = make_double2(0.0, 0.0);
+    if (ROLE == 0) {
+        l_r = lr[c];
+        l_a = la[c];
+        if (D.type[c] != SPH_TYPE_WATER || (l_r == 0.0 && l_a.x == 0.0 && l_a.y == 0.0)) return;
+    }
+    const PSide Sc = load_side<R, MS, MUSCL, ROLE == 0>(D, c);
+    unsigned next = e0 < nn ? D.pairs[(size_t)e0 * P.nbr_stride + c] : 0u;
+    for (int e = e0; e < nn; e += 2) {
+        const unsigned ent = next;
+        if (e + 2 < nn) next = D.pairs[(size_t)(e + 2) * P.nbr_stride + c];
+        const int b = (int)(ent & 0x7fffffffu);
+        const bool c_lower = (ent >> 31) != 0;  // c has the lower id of the pair
+        // all of b's loads are issued before the first branch on one of them
+        if (ROLE == 1) {
+            l_r = lr[b];
+            l_a = la[b];
+        }
+        const PSide Sb = load_side<R, MS, MUSCL, ROLE == 1>(D, b);
+        if (ROLE == 1 && (!Sb.water || (l_r == 0.0 && l_a.x == 0.0 && l_a.y == 0.0))) continue;
+        PBar o;
+        if (ROLE == 0) {
+            rev_pair<MS, MUSCL, HLLC>(P, Sc, Sb, l_r, l_a.x, l_a.y, o, c_lower);
+            v[0] += o.x0; v[1] += o.x1; v[2] += o.u; v[3] += o.v;
+            v[4] += o.pa; v[5] += o.ca; v[6] += o.ra;
+            v[13] += o.bi0; v[14] += o.bi1; v[15] += o.bi2; v[16] += o.bi3;
+            nu_sum += o.nu;
+            if (MS) { v[17] += o.avg0; v[18] += o.avg1; }
+            if (MUSCL) {
+                v[17] += o.gpa0; v[18] += o.gpa1; v[19] += o.gua0; v[20] += o.gua1; v[21] += o.gva0; v[22] += o.gva1;
+            }
+        } else {
+            rev_pair<MS, MUSCL, HLLC>(P, Sb, Sc, l_r, l_a.x, l_a.y, o, !c_lower);
+            v[0] -= o.x0; v[1] -= o.x1; v[2] -= o.u; v[3] -= o.v;
+            v[4] += o.pb; v[5] += o.cb; v[6] += o.rb; v[7] += o.Vb;
+            if (MS) { v[17] -= o.avg0; v[18] -= o.avg1; v[19] += o.mb; }
+            if (MUSCL) {
+                v[17] += o.gpb0; v[18] += o.gpb1; v[19] += o.gub0; v[20] += o.gub1; v[21] += o.gvb0; v[22] += o.gvb1;
+            }
+        }
+        v[8] += o.t0; v[9] += o.t1; v[10] += o.t2; v[11] += o.g0; v[12] += o.g1;
+    }
+}
+
+// Reverse of pass C for the RHS whose rate adjoints are (lr, la).  Four lanes share
+// a particle c: two neighbouring lanes of a warp take its even and odd list
+// positions, and two warps the two roles of adj_c_pairs, so that each warp runs
+// the code of one role, c's side stays in registers and a small particle count
+// still fills the GPU.  Partial sums: over the two lanes, then over the roles.
+// Bound by FP64 latency at 3 blocks per SM (the chain list entry -> records ->
+// one long reverse); with the roles on neighbouring lanes both sides and their
+// reciprocals were re-read for every pair, behind two branches: the reverse phase
+// 31.1 -> 28.0 ms per 64 steps at 256^2 (31.6 with 2 blocks and no spill).
 #ifndef SPH_ADJ_LANES
 #define SPH_ADJ_LANES 4
 #endif
@@ -591,6 +646,7 @@ __device__ __forceinline__ void rev_pair(const Params& P, const PSide& A, const 
 #define SPH_ADJ_C_MUSCL_MIN_BLOCKS 2 // the limiter reverses need more than 168
 #endif
 constexpr int kAdjLanes = SPH_ADJ_LANES;     // 2 or 4
+constexpr int kAdjCLanes = 4;                // of k_adj_c: 2 roles x 2 lanes
 // HLLC: the moving-square HLLC solver (a variant of its own, so that the
 // modified solver's reverse carries none of its registers).
 template <typename R, bool MS = false, bool MUSCL = false, bool HLLC = false>
@@ -599,63 +655,34 @@ __global__ void __launch_bounds__(kAdjThreads, MUSCL ? SPH_ADJ_C_MUSCL_MIN_BLOCK
     pdl_begin();
     stamp_phase(P.stamp);
     __shared__ double red[kAdjThreads];
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = t / kAdjLanes;
-    const int role = t & 1, par = (t >> 1) & (kAdjLanes / 2 - 1);
-    double nu_sum = 0.0;
-    // every lane of the warp takes part in the shuffles below
-    const bool live = c < P.n_tot;
     // 0-16 as below; MS: 17-18 avg, 19 mass; MUSCL: 17-22 grad p, u, v
     constexpr int NV = MS ? 20 : (MUSCL ? 23 : 17);
-    double v[23];
+    constexpr int NC = kAdjThreads / kAdjCLanes;    // particles of a block
+    __shared__ double part[NV][NC];
+    const int role = (threadIdx.x >> 5) & 1;
+    const int slot = (int)(threadIdx.x >> 6) * 16 + (int)((threadIdx.x & 31) >> 1);
+    const int c = (int)blockIdx.x * NC + slot;
+    const bool live = c < P.n_tot;
+    double nu_sum = 0.0;
+    double v[NV];
 #pragma unroll
-    for (int q = 0; q < 23; ++q) v[q] = 0.0;
+    for (int q = 0; q < NV; ++q) v[q] = 0.0;
     if (live) {
-        const int nn = D.npairs[c];
-        // both roles run the same instructions: the two sides are loaded by
-        // index (c's records stay in L1), not branched on
-        const double sg = role ? -1.0 : 1.0;
-        for (int e = par; e < nn; e += kAdjLanes / 2) {
-            const unsigned ent = D.pairs[(size_t)e * P.nbr_stride + c];
-            const int b = (int)(ent & 0x7fffffffu);
-            const int acc_at = role ? b : c;         // the particle whose sum is differentiated
-            const bool c_lower = (ent >> 31) != 0;  // c has the lower id of the pair
-            const int other = role ? c : b;
-            if (D.type[acc_at] != SPH_TYPE_WATER) continue;
-            const double l_r = lr[acc_at];
-            const double2 l_a = la[acc_at];
-            if (l_r == 0.0 && l_a.x == 0.0 && l_a.y == 0.0) continue;
-            const PSide Sa = load_side<R, MS, MUSCL>(D, acc_at);
-            const PSide Sb = load_side<R, MS, MUSCL>(D, other);
-            PBar o;
-            rev_pair<MS, MUSCL, HLLC>(P, Sa, Sb, l_r, l_a.x, l_a.y, o, role ? !c_lower : c_lower);
-            v[0] += sg * o.x0; v[1] += sg * o.x1; v[2] += sg * o.u; v[3] += sg * o.v;
-            v[4] += role ? o.pb : o.pa;
-            v[5] += role ? o.cb : o.ca;
-            v[6] += role ? o.rb : o.ra;
-            v[7] += role ? o.Vb : 0.0;
-            v[8] += o.t0; v[9] += o.t1; v[10] += o.t2; v[11] += o.g0; v[12] += o.g1;
-            if (!role) {
-                v[13] += o.bi0; v[14] += o.bi1; v[15] += o.bi2; v[16] += o.bi3;
-                nu_sum += o.nu;
-            }
-            if (MS) {
-                v[17] += sg * o.avg0; v[18] += sg * o.avg1;
-                v[19] += role ? o.mb : 0.0;
-            }
-            if (MUSCL) {
-                v[17] += role ? o.gpb0 : o.gpa0; v[18] += role ? o.gpb1 : o.gpa1;
-                v[19] += role ? o.gub0 : o.gua0; v[20] += role ? o.gub1 : o.gua1;
-                v[21] += role ? o.gvb0 : o.gva0; v[22] += role ? o.gvb1 : o.gva1;
-            }
-        }
+        if (role == 0) adj_c_pairs<R, MS, MUSCL, HLLC, 0>(P, D, lr, la, c, threadIdx.x & 1, v, nu_sum);
+        else adj_c_pairs<R, MS, MUSCL, HLLC, 1>(P, D, lr, la, c, threadIdx.x & 1, v, nu_sum);
     }
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        v[q] += __shfl_xor_sync(0xffffffffu, v[q], 1);
-        if (kAdjLanes == 4) v[q] += __shfl_xor_sync(0xffffffffu, v[q], 2);
+    for (int q = 0; q < NV; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], 1);
+    const bool first = (threadIdx.x & 1) == 0;
+    if (role == 1 && first) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) part[q][slot] = v[q];
     }
-    if (live && (t & (kAdjLanes - 1)) == 0) {
+    red[threadIdx.x] = nu_sum;
+    __syncthreads();
+    if (live && role == 0 && first) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) v[q] += part[q][slot];
         const double4 k = D.kin[c];
         const double rho = k.z, ir = 1.0 / rho, V = D.mass[c] * ir;
         A.irho[c] = ir;
@@ -677,8 +704,6 @@ __global__ void __launch_bounds__(kAdjThreads, MUSCL ? SPH_ADJ_C_MUSCL_MIN_BLOCK
             A.ggv[c] = make_double2(v[21], v[22]);
         }
     }
-    red[threadIdx.x] = nu_sum;
-    __syncthreads();
     for (int w = kAdjThreads / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();

@@ -1055,7 +1055,7 @@ int adj_prepare_ctx(sph_handle* h, const sph_adj_config* ac) {
             (rc = adj_alloc(X, &A.sr, nt)) || (rc = adj_alloc(X, &A.gbinv, nt)) || (rc = adj_alloc(X, &A.ggr, nt)) ||
             (rc = adj_alloc(X, &A.gtau, nt)) || (rc = adj_alloc(X, &A.mu1, nt)) || (rc = adj_alloc(X, &A.mu2, nt)) ||
             (rc = adj_alloc(X, &A.mu3, nt)) ||
-            (rc = adj_alloc(X, &A.nu_part, (size_t)5 * blocks((long long)nt * kAdjLanes, kAdjThreads))) ||
+            (rc = adj_alloc(X, &A.nu_part, (size_t)5 * blocks((long long)nt * kAdjCLanes, kAdjThreads))) ||
             (rc = adj_alloc(X, &A.nu_acc, 1)) || (rc = adj_alloc(X, &A.irho, nt)) || (rc = adj_alloc(X, &A.ssum, nt)) || (rc = adj_alloc(X, &A.ggp, nt)) ||
             (rc = adj_alloc(X, &A.ggu, nt)) || (rc = adj_alloc(X, &A.ggv, nt)) || (rc = adj_alloc(X, &A.mu4, nt)) ||
             (rc = adj_alloc(X, &A.smu, nt)) || (rc = adj_alloc(X, &A.shgr, nt)) || (rc = adj_alloc(X, &A.shbi, nt)) || (rc = adj_alloc(X, &A.lx, nt)) || (rc = adj_alloc(X, &A.lv, nt)) ||
@@ -1363,7 +1363,7 @@ int adj_rhs(sph_handle* h, const Sorted<R>& V, int k, int stage, bool shift = fa
     AdjCtx* X = h->adj;
     Adj& A = X->A;
     const int nb = blocks(P.n_tot, kAdjThreads);
-    const int nbc = blocks((long long)P.n_tot * kAdjLanes, kAdjThreads);
+    const int nbc = blocks((long long)P.n_tot * kAdjCLanes, kAdjThreads);
     if (!shift && !kept) {
         tic(h, PH_A);
         adj_pass_a<R>(h, V);
@@ -1534,7 +1534,7 @@ int adj_rhs_ms(sph_handle* h, const Sorted<R>& V, int k, int pred, bool drag, in
     AdjCtx* X = h->adj;
     Adj A = X->A;
     const int nb = blocks(P.n_tot, kAdjThreads);
-    const int nbc = blocks((long long)P.n_tot * kAdjLanes, kAdjThreads);
+    const int nbc = blocks((long long)P.n_tot * kAdjCLanes, kAdjThreads);
     const bool ghosts = P.ghost_assign && h->n_ghost > 0;
     if (kept_j >= 0) {
         // the segment re-run left this RHS's assigned ghosts in the stage slot and

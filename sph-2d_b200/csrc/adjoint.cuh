@@ -636,17 +636,20 @@ __device__ __forceinline__ void adj_c_pairs(const Params& P, const Sorted<R>& D,
 // one long reverse); with the roles on neighbouring lanes both sides and their
 // reciprocals were re-read for every pair, behind two branches: the reverse phase
 // 31.1 -> 28.0 ms per 64 steps at 256^2 (31.6 with 2 blocks and no spill).
-#ifndef SPH_ADJ_LANES
-#define SPH_ADJ_LANES 4
-#endif
 #ifndef SPH_ADJ_C_MIN_BLOCKS
 #define SPH_ADJ_C_MIN_BLOCKS 3       // 168 registers: 3 blocks of 128 per SM
 #endif
 #ifndef SPH_ADJ_C_MUSCL_MIN_BLOCKS
 #define SPH_ADJ_C_MUSCL_MIN_BLOCKS 2 // the limiter reverses need more than 168
 #endif
-constexpr int kAdjLanes = SPH_ADJ_LANES;     // 2 or 4
-constexpr int kAdjCLanes = 4;                // of k_adj_c: 2 roles x 2 lanes
+// Lanes per particle of the kernels that walk pair lists (k_adj_c: 2 roles x 2 lanes).
+constexpr int kAdjLanes = 4;
+// Sum over a particle's kAdjLanes lanes, in every one of them.
+__device__ __forceinline__ double adj_lane_sum(double v, unsigned lanes = 0xffffffffu) {
+    v += __shfl_xor_sync(lanes, v, 1);
+    v += __shfl_xor_sync(lanes, v, 2);
+    return v;
+}
 // HLLC: the moving-square HLLC solver (a variant of its own, so that the
 // modified solver's reverse carries none of its registers).
 template <typename R, bool MS = false, bool MUSCL = false, bool HLLC = false>
@@ -657,7 +660,7 @@ __global__ void __launch_bounds__(kAdjThreads, MUSCL ? SPH_ADJ_C_MUSCL_MIN_BLOCK
     __shared__ double red[kAdjThreads];
     // 0-16 as below; MS: 17-18 avg, 19 mass; MUSCL: 17-22 grad p, u, v
     constexpr int NV = MS ? 20 : (MUSCL ? 23 : 17);
-    constexpr int NC = kAdjThreads / kAdjCLanes;    // particles of a block
+    constexpr int NC = kAdjThreads / kAdjLanes;    // particles of a block
     __shared__ double part[NV][NC];
     const int role = (threadIdx.x >> 5) & 1;
     const int slot = (int)(threadIdx.x >> 6) * 16 + (int)((threadIdx.x & 31) >> 1);
@@ -920,8 +923,10 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_a(Params P, Sorted<R> D, Ad
         lac = make_double2(g.x + l.x, g.y + l.y);
     }
     const int nn = live ? D.npairs[c] : 0;
+    unsigned next = lane < nn ? D.pairs[(size_t)lane * P.nbr_stride + c] : 0u;
     for (int e = lane; e < nn; e += kAdjLanes) {
-        const int b = (int)(D.pairs[(size_t)e * P.nbr_stride + c] & 0x7fffffffu);
+        const int b = (int)(next & 0x7fffffffu);
+        if (e + kAdjLanes < nn) next = D.pairs[(size_t)(e + kAdjLanes) * P.nbr_stride + c];
         const double2 xb = D.pos[b];
         const double4 kb = D.kin[b];
         const double r0 = xc.x - xb.x, r1 = xc.y - xb.y;
@@ -982,8 +987,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_a(Params P, Sorted<R> D, Ad
     for (int q = 0; q < 8; ++q) {
         if (!MS && q == 6) continue;
         if (!MUSCL && q == 7) continue;
-        v[q] += __shfl_xor_sync(0xffffffffu, v[q], 1);
-        if (kAdjLanes == 4) v[q] += __shfl_xor_sync(0xffffffffu, v[q], 2);
+        v[q] = adj_lane_sum(v[q]);
     }
     if (!live || lane != 0) return;
     x0b = v[0]; x1b = v[1]; ub = v[2]; vb = v[3]; rb = v[4]; Vb = v[5]; mb_ = v[6]; pb_ = v[7];
@@ -1008,28 +1012,37 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_a(Params P, Sorted<R> D, Ad
 // (the forward forms it in the last pass C of a step, k_pass_c<..., SHIFT>, or
 // in k_shift_gather on the mixed Taylor-Green path):
 //   s_a = sum_b phi(d) V_b r,  phi = (1 + R (W/W_dx)^4) G,  r = x_a - x_b.
+// kAdjLanes lanes per particle (a thread each: 21.9 us at 68,000 particles, and
+// k_adj_shift 27.3; with the prefetch in k_adj_a the three took the reverse phase
+// from 28.0 to 26.5 ms per 64 steps at 256^2).
 template <typename R>
 __global__ void k_shift_sum(Params P, Sorted<R> D, Adj A) {
     pdl_begin();
     stamp_phase(P.stamp);
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= P.n_tot) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = t & (kAdjLanes - 1);
+    const bool live = t / kAdjLanes < P.n_tot;
+    const int a = live ? t / kAdjLanes : 0;
     const double2 xa = D.pos[a];
     const double iwdx = 1.0 / P.w_dx;
     double s0 = 0.0, s1 = 0.0;
-    const int nn = D.npairs[a];
-    for (int e = 0; e < nn; ++e) {
-        const int b = (int)(D.pairs[(size_t)e * P.nbr_stride + a] & 0x7fffffffu);
+    const int nn = live ? D.npairs[a] : 0;
+    unsigned next = lane < nn ? D.pairs[(size_t)lane * P.nbr_stride + a] : 0u;
+    for (int e = lane; e < nn; e += kAdjLanes) {
+        const int b = (int)(next & 0x7fffffffu);
+        if (e + kAdjLanes < nn) next = D.pairs[(size_t)(e + kAdjLanes) * P.nbr_stride + a];
         const double2 xb = D.pos[b];
+        const double Vb = D.mass[b] * rcp64(D.kin[b].z);
         const double r0 = xa.x - xb.x, r1 = xa.y - xb.y;
         const double d2 = r0 * r0 + r1 * r1, d = d2 * rsqrt64(d2);
         double G, dG, W;
         kernel_gw(P, d, G, dG, W);
         const double q = W * iwdx, q2 = q * q;
-        const double f = (1.0 + P.shift_R * (q2 * q2)) * G * (D.mass[b] / D.kin[b].z);
+        const double f = (1.0 + P.shift_R * (q2 * q2)) * G * Vb;
         s0 += f * r0; s1 += f * r1;
     }
-    A.ssum[a] = make_double2(s0, s1);
+    s0 = adj_lane_sum(s0); s1 = adj_lane_sum(s1);
+    if (live && lane == 0) A.ssum[a] = make_double2(s0, s1);
 }
 
 // Reverse of the shifting sums with their adjoints mu (smu): particle c adds
@@ -1038,19 +1051,24 @@ __global__ void k_shift_sum(Params P, Sorted<R> D, Adj A) {
 template <typename R>
 __global__ void k_adj_shift(Params P, Sorted<R> D, Adj A) {
     pdl_begin();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.n_tot) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = t & (kAdjLanes - 1);
+    const bool live = t / kAdjLanes < P.n_tot;
+    const int c = live ? t / kAdjLanes : 0;
     const double2 xc = D.pos[c];
     const double2 mc = A.smu[c];
     const double Vc = D.mass[c] * A.irho[c];
     const double iwdx = 1.0 / P.w_dx;
     double x0b = 0, x1b = 0, Vb_ = 0;
-    const int nn = D.npairs[c];
-    for (int e = 0; e < nn; ++e) {
-        const int b = (int)(D.pairs[(size_t)e * P.nbr_stride + c] & 0x7fffffffu);
+    const int nn = live ? D.npairs[c] : 0;
+    unsigned next = lane < nn ? D.pairs[(size_t)lane * P.nbr_stride + c] : 0u;
+    for (int e = lane; e < nn; e += kAdjLanes) {
+        const int b = (int)(next & 0x7fffffffu);
+        if (e + kAdjLanes < nn) next = D.pairs[(size_t)(e + kAdjLanes) * P.nbr_stride + c];
         const double2 mb = A.smu[b];
-        if (mc.x == 0.0 && mc.y == 0.0 && mb.x == 0.0 && mb.y == 0.0) continue;
         const double2 xb = D.pos[b];
+        const double Vb = D.mass[b] * A.irho[b];
+        if (mc.x == 0.0 && mc.y == 0.0 && mb.x == 0.0 && mb.y == 0.0) continue;
         const double r0 = xc.x - xb.x, r1 = xc.y - xb.y;
         const double d2 = r0 * r0 + r1 * r1, id = rsqrt64(d2), d = d2 * id;
         double G, dG, W;
@@ -1059,7 +1077,6 @@ __global__ void k_adj_shift(Params P, Sorted<R> D, Adj A) {
         const double phi = (1.0 + P.shift_R * q4) * G;
         // dphi/dd: dW/dd = G d
         const double dphi = 4.0 * P.shift_R * q2 * q * (G * d * iwdx) * G + (1.0 + P.shift_R * q4) * dG;
-        const double Vb = D.mass[b] * A.irho[b];
         // own sum: mu_c . V_b phi r, r = x_c - x_b
         const double rm = r0 * mc.x + r1 * mc.y;
         x0b += Vb * (phi * mc.x + dphi * rm * r0 * id);
@@ -1070,6 +1087,8 @@ __global__ void k_adj_shift(Params P, Sorted<R> D, Adj A) {
         x1b -= Vc * (phi * mb.y - dphi * rmb * r1 * id);
         Vb_ += phi * rmb;
     }
+    x0b = adj_lane_sum(x0b); x1b = adj_lane_sum(x1b); Vb_ = adj_lane_sum(Vb_);
+    if (!live || lane != 0) return;
     const double2 sx = A.sx[c];
     A.sx[c] = make_double2(sx.x + x0b, sx.y + x1b);
     A.sr[c] -= Vc * A.irho[c] * Vb_;
@@ -1786,7 +1805,13 @@ template <typename R>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_drag(Params P, Sorted<R> D, Adj A, double w, double* nu_part) {
     pdl_begin();
     __shared__ double red[kAdjThreads];
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    // kAdjLanes lanes per particle: the body particles' lists were one thread's work
+    // each (here, in k_mark_body_nbrs, k_shift_sum and k_adj_shift together: reverse
+    // phase of the D/25 square 8.2 -> 6.4 ms per 32 steps).  A particle's lanes take
+    // the same branch, so their shuffles stay together
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = t / kAdjLanes, lane = t & (kAdjLanes - 1);
+    const unsigned group = 0xfu << (threadIdx.x & 28);
     double nu_sum = 0.0;
     if (c < P.n_tot && (D.itype[c] == SPH_TYPE_BODY || D.nflag[c] == 2)) {
         const bool cbody = D.itype[c] == SPH_TYPE_BODY;
@@ -1797,7 +1822,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_drag(Params P, Sorted<R> D,
         double x0b = 0, x1b = 0, ub = 0, pb = 0, rb = 0, Vb_ = 0;
         double4 gb = make_double4(0, 0, 0, 0);
         const int nn = D.npairs[c];
-        for (int e = 0; e < nn; ++e) {
+        for (int e = lane; e < nn; e += kAdjLanes) {
             const int b = (int)(D.pairs[(size_t)e * P.nbr_stride + c] & 0x7fffffffu);
             const bool bbody = D.itype[b] == SPH_TYPE_BODY;
             if (!bbody && !cbody) continue;
@@ -1841,7 +1866,11 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_drag(Params P, Sorted<R> D,
                 Vb_ += w * Va * Tin;
             }
         }
-        if (nn > 0) {
+        x0b = adj_lane_sum(x0b, group); x1b = adj_lane_sum(x1b, group); ub = adj_lane_sum(ub, group);
+        pb = adj_lane_sum(pb, group); rb = adj_lane_sum(rb, group); Vb_ = adj_lane_sum(Vb_, group);
+        gb.x = adj_lane_sum(gb.x, group); gb.y = adj_lane_sum(gb.y, group);
+        gb.z = adj_lane_sum(gb.z, group); gb.w = adj_lane_sum(gb.w, group);
+        if (nn > 0 && lane == 0) {
             double dp, dc;
             eos_deriv(P, kc.z, dp, dc);
             const double2 sx = A.sx[c], su = A.su[c];
@@ -1867,10 +1896,11 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_drag(Params P, Sorted<R> D,
 template <typename R>
 __global__ void k_mark_body_nbrs(Params P, Sorted<R> D) {
     pdl_begin();
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = t / kAdjLanes;
     if (b >= P.n_tot || D.itype[b] != SPH_TYPE_BODY) return;
     const int nn = D.npairs[b];
-    for (int e = 0; e < nn; ++e) D.nflag[(int)(D.pairs[(size_t)e * P.nbr_stride + b] & 0x7fffffffu)] = 2;
+    for (int e = t & (kAdjLanes - 1); e < nn; e += kAdjLanes) D.nflag[(int)(D.pairs[(size_t)e * P.nbr_stride + b] & 0x7fffffffu)] = 2;
 }
 
 // Reverse of k_assign_ghosts, ghost side, one warp per ghost as in the forward
@@ -1966,49 +1996,35 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_ghost_lambda(Params P, Sort
 template <typename R>
 __device__ __forceinline__ void ghost_water_one(const Params& P, const Sorted<R>& D, const Adj& A, int j, double bax,
                                                 double bay) {
-    const int lane = threadIdx.x & 31;
-    const double2 xj = D.pos[j], x0 = D.pos0[j];
-    const int cx = (int)floor((x0.x - P.gx0) / P.cs), cy = (int)floor((x0.y - P.gy0) / P.cs);
+    const double2 xj = D.pos[j];
     const double4 kj = D.kin[j];
     const double mj = D.mass[j], ij = rcp64(kj.z), Vj = mj * ij;
     double x0b = 0, x1b = 0, ub = 0, vb = 0, pb = 0, rb = 0;
-    const int gx0 = max(cx - P.ghost_cells, 0), gx1 = min(cx + P.ghost_cells, P.gnx - 1);
-    for (int gy = max(cy - P.ghost_cells, 0); gy <= min(cy + P.ghost_cells, P.gny - 1); ++gy) {
-        const int row = gy * P.gnx;
-        int lo = -1, hi = -1;
-        for (int gx = gx0; gx <= gx1; ++gx) {
-            const int b0 = D.cell_start[row + gx];
-            if (b0 < 0) continue;
-            if (lo < 0) lo = b0;
-            hi = D.cell_end[row + gx];
-        }
-        if (lo < 0) continue;
-        for (int s = lo + lane; s < hi; s += 32) {
-            const double2 x = D.pos[s];
-            const double dx = x.x - xj.x, dy = x.y - xj.y;
-            const double s2 = dx * dx + dy * dy;
-            if (D.type[s] != SPH_TYPE_FIX_GHOST || D.id[s] >= P.n_host || !(s2 <= P.ghost_r2)) continue;
-            const double4 lam = load4(&A.glam[s]);
-            const double lw = A.glamw[s];
-            if (lam.x == 0.0 && lam.y == 0.0 && lam.z == 0.0 && lam.w == 0.0 && lw == 0.0) continue;
-            const double w = ghost_w(P, s2);
-            const bool body = D.itype[s] == SPH_TYPE_BODY;
-            const double gxe = P.grav[0] + (body ? bax : 0.0), gye = P.grav[1] + (body ? bay : 0.0);
-            const double ge = gxe * dx + gye * dy;
-            const double W = w * Vj;
-            ub += lam.y * W; vb += lam.z * W; pb += lam.x * W;
-            rb += lam.x * W * ge;
-            const double Wb = lam.x * (kj.w + kj.z * ge) + lam.y * kj.x + lam.z * kj.y + lam.w * mj + lw;
-            rb -= Wb * W * ij;
-            const double k = Wb * Vj * ghost_dw_over_d(P, s2);
-            const double cg = lam.x * kj.z * W;
-            x0b -= k * dx + cg * gxe;
-            x1b -= k * dy + cg * gye;
-        }
-    }
+    window_visit_warp(P, D, D.pos0[j], [&](int s) {
+        const double2 x = D.pos[s];
+        const double dx = x.x - xj.x, dy = x.y - xj.y;
+        const double s2 = dx * dx + dy * dy;
+        if (D.type[s] != SPH_TYPE_FIX_GHOST || D.id[s] >= P.n_host || !(s2 <= P.ghost_r2)) return;
+        const double4 lam = load4(&A.glam[s]);
+        const double lw = A.glamw[s];
+        if (lam.x == 0.0 && lam.y == 0.0 && lam.z == 0.0 && lam.w == 0.0 && lw == 0.0) return;
+        const double w = ghost_w(P, s2);
+        const bool body = D.itype[s] == SPH_TYPE_BODY;
+        const double gxe = P.grav[0] + (body ? bax : 0.0), gye = P.grav[1] + (body ? bay : 0.0);
+        const double ge = gxe * dx + gye * dy;
+        const double W = w * Vj;
+        ub += lam.y * W; vb += lam.z * W; pb += lam.x * W;
+        rb += lam.x * W * ge;
+        const double Wb = lam.x * (kj.w + kj.z * ge) + lam.y * kj.x + lam.z * kj.y + lam.w * mj + lw;
+        rb -= Wb * W * ij;
+        const double k = Wb * Vj * ghost_dw_over_d(P, s2);
+        const double cg = lam.x * kj.z * W;
+        x0b -= k * dx + cg * gxe;
+        x1b -= k * dy + cg * gye;
+    });
     x0b = warp_sum(x0b); x1b = warp_sum(x1b); ub = warp_sum(ub); vb = warp_sum(vb);
     pb = warp_sum(pb); rb = warp_sum(rb);
-    if (lane != 0) return;
+    if ((threadIdx.x & 31) != 0) return;
     double dp, dc;
     eos_deriv(P, kj.z, dp, dc);
     const double2 sx = A.sx[j], su = A.su[j];
@@ -2027,11 +2043,16 @@ template <typename R>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_ghost_water(Params P, Sorted<R> D, Adj A, double bax,
                                                                  double bay) {
     pdl_begin();
-    // a fixed grid of warps strides over the slots; only the flagged ones work
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < P.n_tot; j += nw) {
-        if (D.nflag[j] == 0 || D.type[j] == SPH_TYPE_FIX_GHOST) continue;    // whole warps
-        ghost_water_one(P, D, A, j, bax, bay);
+    // (one slot per round of loads and the window's rows one after the other: reverse
+    // phase of the D/25 square 6.38 ms per 32 steps, 6.12 this way)
+    // warp w owns the slots w, w + nw, w + 2 nw, ... (the flagged ones are close
+    // together); its lanes look at 32 of them at a time
+    const int nw = (gridDim.x * blockDim.x) >> 5, lane = threadIdx.x & 31;
+    for (int j0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j0 < P.n_tot; j0 += 32 * nw) {
+        const int j = j0 + lane * nw;
+        const bool work = j < P.n_tot && D.nflag[j] != 0 && D.type[j] != SPH_TYPE_FIX_GHOST;
+        for (unsigned m = __ballot_sync(0xffffffffu, work); m; m &= m - 1)
+            ghost_water_one(P, D, A, j0 + (__ffs(m) - 1) * nw, bax, bay);
     }
 }
 

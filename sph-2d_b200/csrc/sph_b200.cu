@@ -1055,7 +1055,7 @@ int adj_prepare_ctx(sph_handle* h, const sph_adj_config* ac) {
             (rc = adj_alloc(X, &A.sr, nt)) || (rc = adj_alloc(X, &A.gbinv, nt)) || (rc = adj_alloc(X, &A.ggr, nt)) ||
             (rc = adj_alloc(X, &A.gtau, nt)) || (rc = adj_alloc(X, &A.mu1, nt)) || (rc = adj_alloc(X, &A.mu2, nt)) ||
             (rc = adj_alloc(X, &A.mu3, nt)) ||
-            (rc = adj_alloc(X, &A.nu_part, (size_t)5 * blocks((long long)nt * kAdjCLanes, kAdjThreads))) ||
+            (rc = adj_alloc(X, &A.nu_part, (size_t)5 * blocks((long long)nt * kAdjLanes, kAdjThreads))) ||
             (rc = adj_alloc(X, &A.nu_acc, 1)) || (rc = adj_alloc(X, &A.irho, nt)) || (rc = adj_alloc(X, &A.ssum, nt)) || (rc = adj_alloc(X, &A.ggp, nt)) ||
             (rc = adj_alloc(X, &A.ggu, nt)) || (rc = adj_alloc(X, &A.ggv, nt)) || (rc = adj_alloc(X, &A.mu4, nt)) ||
             (rc = adj_alloc(X, &A.smu, nt)) || (rc = adj_alloc(X, &A.shgr, nt)) || (rc = adj_alloc(X, &A.shbi, nt)) || (rc = adj_alloc(X, &A.lx, nt)) || (rc = adj_alloc(X, &A.lv, nt)) ||
@@ -1362,8 +1362,7 @@ int adj_rhs(sph_handle* h, const Sorted<R>& V, int k, int stage, bool shift = fa
     const Params& P = h->P;
     AdjCtx* X = h->adj;
     Adj& A = X->A;
-    const int nb = blocks(P.n_tot, kAdjThreads);
-    const int nbc = blocks((long long)P.n_tot * kAdjCLanes, kAdjThreads);
+    const int nbc = blocks((long long)P.n_tot * kAdjLanes, kAdjThreads);
     if (!shift && !kept) {
         tic(h, PH_A);
         adj_pass_a<R>(h, V);
@@ -1375,7 +1374,7 @@ int adj_rhs(sph_handle* h, const Sorted<R>& V, int k, int stage, bool shift = fa
     else
         launch(k_adj_c<R>, nbc, kAdjThreads, h->stream, P, V, A, A.lr[k], A.la[k], A.nu_part + (size_t)k * nbc);
     if (shift) {
-        launch(k_adj_shift<R>, nb, kAdjThreads, h->stream, P, V, A);
+        launch(k_adj_shift<R>, nbc, kAdjThreads, h->stream, P, V, A);
         h->launches += 1;
     }
     if (mls1) {
@@ -1426,7 +1425,7 @@ int adj_step(sph_handle* h, bool first, int j) {
             adj_pass_a<R>(h, V);
         }
         tic(h, PH_ADJ);
-        launch(k_shift_sum<R>, nb, 256, h->stream, P, V, A);
+        launch(k_shift_sum<R>, blocks((long long)P.n_tot * kAdjLanes, 256), 256, h->stream, P, V, A);
         h->launches += 1;
     }
     tic(h, PH_ADJ);
@@ -1533,8 +1532,7 @@ int adj_rhs_ms(sph_handle* h, const Sorted<R>& V, int k, int pred, bool drag, in
     const Params& P = h->P;
     AdjCtx* X = h->adj;
     Adj A = X->A;
-    const int nb = blocks(P.n_tot, kAdjThreads);
-    const int nbc = blocks((long long)P.n_tot * kAdjCLanes, kAdjThreads);
+    const int nbc = blocks((long long)P.n_tot * kAdjLanes, kAdjThreads);
     const bool ghosts = P.ghost_assign && h->n_ghost > 0;
     if (kept_j >= 0) {
         // the segment re-run left this RHS's assigned ghosts in the stage slot and
@@ -1552,7 +1550,7 @@ int adj_rhs_ms(sph_handle* h, const Sorted<R>& V, int k, int pred, bool drag, in
     else
         launch(k_adj_c<R, true>, nbc, kAdjThreads, h->stream, P, V, A, A.lr[k], A.la[k], A.nu_part + (size_t)k * nbc);
     if (shift) {
-        launch(k_adj_shift<R>, nb, kAdjThreads, h->stream, P, V, A);
+        launch(k_adj_shift<R>, nbc, kAdjThreads, h->stream, P, V, A);
         h->launches += 1;
     }
     if (gm) {
@@ -1566,9 +1564,9 @@ int adj_rhs_ms(sph_handle* h, const Sorted<R>& V, int k, int pred, bool drag, in
     }
     if (drag) {
         double* part = A.nu_part + (size_t)4 * nbc;
-        launch(k_mark_body_nbrs<R>, blocks(P.n_tot, 256), 256, h->stream, P, V);
-        launch(k_adj_drag<R>, nb, kAdjThreads, h->stream, P, V, A, X->dloss * X->dt, part);
-        launch(k_adj_nu_sum, 1, 1024, h->stream, nb, part, A.nu_acc);
+        launch(k_mark_body_nbrs<R>, nbc, kAdjThreads, h->stream, P, V);
+        launch(k_adj_drag<R>, nbc, kAdjThreads, h->stream, P, V, A, X->dloss * X->dt, part);
+        launch(k_adj_nu_sum, 1, 1024, h->stream, nbc, part, A.nu_acc);
         h->launches += 3;
     }
     launch(k_adj_point<R>, blocks(P.n_tot, 256), 256, h->stream, P, V, A, shift ? 1 : 0);
@@ -1623,7 +1621,7 @@ int adj_step_ms(sph_handle* h, bool first, int j, int jstep) {
         adj_rhs_ms_values<R>(h, V, kept ? j : -1);
         tic(h, PH_ADJ);
         if (shift) {
-            launch(k_shift_sum<R>, nb, 256, h->stream, P, V, A);
+            launch(k_shift_sum<R>, blocks((long long)P.n_tot * kAdjLanes, 256), 256, h->stream, P, V, A);
             h->launches += 1;
         }
     }

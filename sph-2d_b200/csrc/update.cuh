@@ -240,19 +240,14 @@ __device__ __forceinline__ double ghost_dw_over_d(const Params& P, double s2) {
     return -5.0 * (tq * tq * tq) * P.ghost_kf * P.ghost_ih2;
 }
 
-// The neighbours the ghost assignment interpolates from for ghost slot s: the
-// non-ghost particles within kernel_scale * 1.2 h, found over the window of s's
-// cell (the list-build cells, so the window reaches ghost_r plus half the skin).
-// Lane k finds the slot range of the window's row k (the slots of a row's window
-// cells are contiguous in the cell-sorted order), so the ranges are one round of
-// loads; then the 32 lanes split the candidates of each row.  fn(b, dx, dy, s2, w)
-// gets (dx, dy) = x_s - x_b, the squared distance and the kernel value with the
-// ghost smoothing length, on the lane that visits b.
+// The slots of the ghost assignment's window around the list-build cell of x0: fn(b)
+// on the lane that visits b.  Lane k finds the slot range of the window's row k
+// (the slots of a row's window cells are contiguous in the cell-sorted order), so
+// the ranges are one round of loads; then the 32 lanes split each row.
 template <typename R, typename F>
-__device__ __forceinline__ void ghost_visit_warp(const Params& P, const Sorted<R>& D, int s, F&& fn) {
+__device__ __forceinline__ void window_visit_warp(const Params& P, const Sorted<R>& D, double2 x0, F&& fn) {
     const int lane = threadIdx.x & 31;
-    const double2 x = D.pos[s];
-    const int cx = (int)floor((x.x - P.gx0) / P.cs), cy = (int)floor((x.y - P.gy0) / P.cs);
+    const int cx = (int)floor((x0.x - P.gx0) / P.cs), cy = (int)floor((x0.y - P.gy0) / P.cs);
     const int gx0 = max(cx - P.ghost_cells, 0), gx1 = min(cx + P.ghost_cells, P.gnx - 1);
     const int gy0 = max(cy - P.ghost_cells, 0), gy1 = min(cy + P.ghost_cells, P.gny - 1);
     for (int r0 = gy0; r0 <= gy1; r0 += 32) {
@@ -271,16 +266,27 @@ __device__ __forceinline__ void ghost_visit_warp(const Params& P, const Sorted<R
         const int rows = min(gy1 - r0 + 1, 32);
         for (int k = 0; k < rows; ++k) {
             const int end = __shfl_sync(0xffffffffu, hi, k);
-            for (int b = __shfl_sync(0xffffffffu, lo, k) + lane; b < end; b += 32) {
-                const double2 xb = D.pos[b];
-                const int tb = D.type[b];
-                const double dx = x.x - xb.x, dy = x.y - xb.y;
-                const double s2 = dx * dx + dy * dy;
-                if (tb == SPH_TYPE_FIX_GHOST || !(s2 <= P.ghost_r2)) continue;
-                fn(b, dx, dy, s2, ghost_w(P, s2));
-            }
+            for (int b = __shfl_sync(0xffffffffu, lo, k) + lane; b < end; b += 32) fn(b);
         }
     }
+}
+
+// The neighbours the ghost assignment interpolates from for ghost slot s: the
+// non-ghost particles within kernel_scale * 1.2 h, found over the window of s's
+// cell (the list-build cells, so the window reaches ghost_r plus half the skin).
+// fn(b, dx, dy, s2, w) gets (dx, dy) = x_s - x_b, the squared distance and the
+// kernel value with the ghost smoothing length, on the lane that visits b.
+template <typename R, typename F>
+__device__ __forceinline__ void ghost_visit_warp(const Params& P, const Sorted<R>& D, int s, F&& fn) {
+    const double2 x = D.pos[s];
+    window_visit_warp(P, D, x, [&](int b) {
+        const double2 xb = D.pos[b];
+        const int tb = D.type[b];
+        const double dx = x.x - xb.x, dy = x.y - xb.y;
+        const double s2 = dx * dx + dy * dy;
+        if (tb == SPH_TYPE_FIX_GHOST || !(s2 <= P.ghost_r2)) return;
+        fn(b, dx, dy, s2, ghost_w(P, s2));
+    });
 }
 
 // Sum over the warp, lane 0's association order, broadcast to every lane (so

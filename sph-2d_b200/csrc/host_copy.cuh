@@ -31,13 +31,21 @@ class HostCopy {
 public:
     ~HostCopy() { release(); }
     void release() {
-        for (int t = 0; t < kLanes; ++t)
-            for (int k = 0; k < 2; ++k) {
+        for (int t = 0; t < kLanes; ++t) {
+            for (int k = 0; k < 2; ++k)
                 if (lane_[t].ev[k]) cudaEventDestroy(lane_[t].ev[k]);
-                if (lane_[t].buf[k]) cudaFreeHost(lane_[t].buf[k]);
-                lane_[t].ev[k] = nullptr;
-                lane_[t].buf[k] = nullptr;
-            }
+            if (lane_[t].buf[0]) cudaFreeHost(lane_[t].buf[0]);
+            lane_[t] = Lane{};
+        }
+    }
+    // The first lane's chunks with `extra` zeroed bytes of page-locked memory behind
+    // them, which the caller may use until release().
+    cudaError_t reserve(size_t extra, void** mem) {
+        const cudaError_t e = open(lane_[0], extra);
+        if (e != cudaSuccess) return e;
+        *mem = (char*)lane_[0].buf[0] + 2 * kChunk;
+        memset(*mem, 0, extra);
+        return cudaSuccess;
     }
     // Device to host (to_host) or host to device on `stream`; complete on return.
     // Null host pointers are skipped.
@@ -83,15 +91,10 @@ private:
             const unsigned hw = std::thread::hardware_concurrency();
             lanes = hw >= 8 ? kLanes : hw >= 4 ? 2 : 1;
         }
-        for (int t = 0; t < lanes && !chunks.empty(); ++t)
-            for (int k = 0; k < 2; ++k) {
-                cudaError_t e = cudaSuccess;
-                if (!lane_[t].buf[k] && (e = cudaHostAlloc(&lane_[t].buf[k], kChunk, cudaHostAllocDefault)) != cudaSuccess)
-                    return e;
-                if (!lane_[t].ev[k] &&
-                    (e = cudaEventCreateWithFlags(&lane_[t].ev[k], cudaEventDisableTiming)) != cudaSuccess)
-                    return e;
-            }
+        for (int t = 0; t < lanes && t < (int)chunks.size(); ++t) {
+            const cudaError_t e = open(lane_[t], 0);
+            if (e != cudaSuccess) return e;
+        }
         std::atomic<int> err{cudaSuccess};
         auto work = [&](int t) {
             if (t > 0) cudaSetDevice(device);
@@ -135,6 +138,17 @@ private:
         cudaEvent_t ev[2] = {nullptr, nullptr};
     };
     Lane lane_[kLanes];
+    // One allocation per lane: each takes 0.8 to 2.6 ms whatever its size.
+    static cudaError_t open(Lane& l, size_t extra) {
+        cudaError_t e = cudaSuccess;
+        if (!l.buf[0]) {
+            if ((e = cudaHostAlloc(&l.buf[0], 2 * kChunk + extra, cudaHostAllocDefault)) != cudaSuccess) return e;
+            l.buf[1] = (char*)l.buf[0] + kChunk;
+        }
+        for (int k = 0; k < 2 && e == cudaSuccess; ++k)
+            if (!l.ev[k]) e = cudaEventCreateWithFlags(&l.ev[k], cudaEventDisableTiming);
+        return e;
+    }
 
     static size_t pad(size_t b) { return (b + 255) & ~size_t(255); }
     static bool page_locked(const void* p) {

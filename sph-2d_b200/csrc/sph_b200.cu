@@ -1299,6 +1299,10 @@ int step_keep(sph_handle* h, double dt, int j, bool full) {
     // corrector; the Runge-Kutta RHS 2-4) fill its pass-A slots, and its reverse
     // step re-runs no pass A, so it needs no neighbour lists
     const bool keep_pa = h->adj->pa && full && !first && !mls;
+    // the final stage as run_steps takes it: inside the last RHS, staging kept current
+    const int stn = h->cfg.integrator == SPH_INTEGRATOR_EULER_PC ? 11 : 3;
+    const int to_staging = !mls && (h->P.ms || !h->P.ghost_assign) ? 1 : 0;
+    const StageArgs end = mls ? StageArgs{} : stage_args(h, STAGE_END, stn, dt, h->cfg.shifting, to_staging);
     int rc = step_begin<R>(h, dt);
     if (rc || (rc = prepare<R>(h)) || (rc = prep_save(h, j, !keep_pa))) return rc;
     h->adj->seg_ntot[j] = h->P.n_tot;
@@ -1313,19 +1317,19 @@ int step_keep(sph_handle* h, double dt, int j, bool full) {
             const size_t o = (size_t)j * X->cap_tot;
             {
                 PaSwap<R> sw(h, j);
-                if ((rc = rhs<R>(h, 1, StageArgs{}, j, X->pa_gint + o, X->pa_gsw + o)) ||
-                    (rc = stage<R>(h, 11, dt, 0, h->cfg.shifting)))
-                    return rc;
+                if ((rc = rhs<R>(h, 1, end, j, X->pa_gint + o, X->pa_gsw + o))) return rc;
             }
+            if (to_staging) h->staging_valid = true;
             X->seg_kept[j] = 1;
             h->step_count++;
             h->n_steps++;
         } else {
             if ((rc = keep_stage<R>(h, j, 0))) return rc;
             if (full) {
-                if ((rc = rhs<R>(h, 1)) || (mls1 && (rc = mls1_on_last_rhs<R>(h))) ||
-                    (rc = stage<R>(h, 11, dt, 0, mls ? 0 : h->cfg.shifting)))
+                if ((rc = rhs<R>(h, 1, end)) || (mls1 && (rc = mls1_on_last_rhs<R>(h))) ||
+                    (mls && (rc = stage<R>(h, 11, dt, 0, 0))))
                     return rc;
+                if (to_staging) h->staging_valid = true;
                 // the re-initialisation reads the corrected state (stage slot state 3)
                 if (mls && ((rc = keep_stage<R>(h, j, 3)) || (rc = reinit_density<R>(h, h->cfg.shifting))))
                     return rc;
@@ -1340,23 +1344,22 @@ int step_keep(sph_handle* h, double dt, int j, bool full) {
     // write pass A's outputs into pass-A slot 3 j + k when the step is kept
     h->adj->seg_kept[j] = keep_pa ? 1 : 0;
     if ((rc = stage<R>(h, 0, dt, first ? 0 : 1, 0)) || (rc = keep_stage<R>(h, j, 0))) return rc;
-    {
-        PaSwap<R> sw(h, 3 * j, keep_pa);
-        if ((rc = rhs<R>(h, 0)) || (rc = stage<R>(h, 1, dt, 0, 0))) return rc;
+    for (int k = 0; k < 2; ++k) {
+        {
+            PaSwap<R> sw(h, 3 * j + k, keep_pa);
+            if ((rc = rhs<R>(h, 0, stage_args(h, STAGE_MID, k + 1, dt)))) return rc;
+        }
+        swap_stage_state(sorted<R>(h));          // (the end of sw took the RHS's exchange back)
+        if ((rc = keep_stage<R>(h, j, k + 1))) return rc;
     }
-    if ((rc = keep_stage<R>(h, j, 1))) return rc;
-    {
-        PaSwap<R> sw(h, 3 * j + 1, keep_pa);
-        if ((rc = rhs<R>(h, 0)) || (rc = stage<R>(h, 2, dt, 0, 0))) return rc;
-    }
-    if ((rc = keep_stage<R>(h, j, 2))) return rc;
     if (full) {
         {
             PaSwap<R> sw(h, 3 * j + 2, keep_pa);
-            if ((rc = rhs<R>(h, 1)) || (mls1 && (rc = mls1_on_last_rhs<R>(h))) ||
-                (rc = stage<R>(h, 3, dt, 0, mls ? 0 : h->cfg.shifting)))
+            if ((rc = rhs<R>(h, 1, end)) || (mls1 && (rc = mls1_on_last_rhs<R>(h))) ||
+                (mls && (rc = stage<R>(h, 3, dt, 0, 0))))
                 return rc;
         }
+        if (to_staging) h->staging_valid = true;
         if (mls && ((rc = keep_stage<R>(h, j, 3)) || (rc = reinit_density<R>(h, h->cfg.shifting)))) return rc;
         h->step_count++;
         h->n_steps++;

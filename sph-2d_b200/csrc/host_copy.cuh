@@ -34,16 +34,19 @@ public:
         for (int t = 0; t < kLanes; ++t) {
             for (int k = 0; k < 2; ++k)
                 if (lane_[t].ev[k]) cudaEventDestroy(lane_[t].ev[k]);
-            if (lane_[t].buf[0]) cudaFreeHost(lane_[t].buf[0]);
-            lane_[t] = Lane{};
         }
+        for (void** b : {&first_, &rest_}) {
+            if (*b) cudaFreeHost(*b);
+            *b = nullptr;
+        }
+        for (Lane& l : lane_) l = Lane{};
     }
     // The first lane's chunks with `extra` zeroed bytes of page-locked memory behind
     // them, which the caller may use until release().
     cudaError_t reserve(size_t extra, void** mem) {
-        const cudaError_t e = open(lane_[0], extra);
+        const cudaError_t e = open(1, extra);
         if (e != cudaSuccess) return e;
-        *mem = (char*)lane_[0].buf[0] + 2 * kChunk;
+        *mem = (char*)first_ + 2 * kChunk;
         memset(*mem, 0, extra);
         return cudaSuccess;
     }
@@ -91,8 +94,8 @@ private:
             const unsigned hw = std::thread::hardware_concurrency();
             lanes = hw >= 8 ? kLanes : hw >= 4 ? 2 : 1;
         }
-        for (int t = 0; t < lanes && t < (int)chunks.size(); ++t) {
-            const cudaError_t e = open(lane_[t], 0);
+        if (!chunks.empty()) {
+            const cudaError_t e = open(lanes, 0);
             if (e != cudaSuccess) return e;
         }
         std::atomic<int> err{cudaSuccess};
@@ -138,15 +141,23 @@ private:
         cudaEvent_t ev[2] = {nullptr, nullptr};
     };
     Lane lane_[kLanes];
-    // One allocation per lane: each takes 0.8 to 2.6 ms whatever its size.
-    static cudaError_t open(Lane& l, size_t extra) {
+    // Page-locked memory: one allocation for the first lane, one for the others, since
+    // each takes 0.8 to 2.6 ms whatever its size.
+    void* first_ = nullptr;
+    void* rest_ = nullptr;
+    cudaError_t open(int lanes, size_t extra) {
         cudaError_t e = cudaSuccess;
-        if (!l.buf[0]) {
-            if ((e = cudaHostAlloc(&l.buf[0], 2 * kChunk + extra, cudaHostAllocDefault)) != cudaSuccess) return e;
-            l.buf[1] = (char*)l.buf[0] + kChunk;
-        }
-        for (int k = 0; k < 2 && e == cudaSuccess; ++k)
-            if (!l.ev[k]) e = cudaEventCreateWithFlags(&l.ev[k], cudaEventDisableTiming);
+        if (!first_ && (e = cudaHostAlloc(&first_, 2 * kChunk + extra, cudaHostAllocDefault)) != cudaSuccess) return e;
+        if (lanes > 1 && !rest_ &&
+            (e = cudaHostAlloc(&rest_, (kLanes - 1) * 2 * kChunk, cudaHostAllocDefault)) != cudaSuccess)
+            return e;
+        for (int t = 0; t < lanes; ++t)
+            for (int k = 0; k < 2; ++k) {
+                lane_[t].buf[k] = t == 0 ? (char*)first_ + k * kChunk : (char*)rest_ + (2 * (t - 1) + k) * kChunk;
+                if (!lane_[t].ev[k] &&
+                    (e = cudaEventCreateWithFlags(&lane_[t].ev[k], cudaEventDisableTiming)) != cudaSuccess)
+                    return e;
+            }
         return e;
     }
 

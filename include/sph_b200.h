@@ -149,7 +149,11 @@ typedef struct sph_diag {
                                  Single_step_compute.f90:228-243); zero without body particles */
 } sph_diag;
 
-/* per-pass device times (CUDA events) accumulated since the last reset, ms */
+/* device times accumulated since the last reset, ms: phases from time stamps that
+ * their first kernel writes, the total from CUDA events.  The surface tests run
+ * inside passes A and C (surface_ms is 0); the stages of the integrator run in the
+ * set-up's gather (sort_ms) and at the end of pass C, or of the shifting gather
+ * (update_ms). */
 typedef struct sph_timings {
     double sort_ms, pass_a_ms, surface_ms, pass_c_ms, update_ms, images_ms, total_ms;
     long long rhs_evaluations, steps;

@@ -59,7 +59,8 @@ __device__ __forceinline__ double2 wrap_position(const Params& P, double2 x) {
 // image counts and offsets by two library scans with a host wait each, a library
 // radix sort and separate key and range passes (18 launches), same slot order:
 // images + sort + lists 166 -> 59 us per step at 100^2 (FP64), 195 -> 85 us at
-// 401^2 and 1.11 -> 0.98 ms at 2048^2 (mixed).
+// 401^2 and 1.11 -> 0.98 ms at 2048^2 (mixed); 29, 62 us and 0.91 ms with the lanes,
+// the dependent launches and the shared reads below.
 constexpr int kImgThreads = 1024;         // host particles per block
 constexpr int kScanThreads = 1024;        // cell scan: kScanCells cells per block
 constexpr int kScanShift = 12, kScanCells = 1 << kScanShift;

@@ -6,8 +6,8 @@
 // and the halo exchanges of exchange_buffer_domain_information are gone).
 //
 // Per time step (time_iteration.f90:781-1073):
-//   prepare: periodic wrap + images (id order), cell keys, radix sort,
-//            cell ranges, neighbour lists with a skin, neighbour records
+//   prepare: periodic wrap + images (id order), counting sort by cell, gather
+//            with the neighbour records, neighbour lists with a skin
 //   RHS    : pass A (renormalisation, gradients, SPS, surface test) -> pass C
 //            (near-surface flags, fused forces)
 //   stages : the first in the gather, the others in the kernel that ends each

@@ -700,6 +700,14 @@ __device__ __forceinline__ bool pair_may_fail(int rule, int ti) {
     return rule == SPH_PAIRS_ONE_FLUID ? ti != SPH_TYPE_WATER : ti == -2 || ti == -3 || ti == -201;
 }
 
+// Cell column (row) of coordinate v, for a scan of the columns c - 1 .. c + 1 of n.  A
+// particle off the grid (not binned, reported as ST_DOMAIN) still comes here, and a
+// coordinate of 1e300 or an infinity saturates the conversion to int, so that c + 1
+// overflows: clamped to [-2, n + 1] first, where the scan meets no column (NaN: -2).
+__device__ __forceinline__ int scan_cell(double v, double lo, double cs, int n) {
+    return (int)fmin(fmax(floor((v - lo) / cs), -2.0), n + 1.0);
+}
+
 // --- 5. neighbour lists ----------------------------------------------------
 // Every particle b != a in the 3x3 cells with |x_a - x_b|^2 <= (support*(1+skin))^2
 // and an allowed type pair.  The exact support test is repeated at every RHS on
@@ -735,7 +743,7 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
         double2 xa = D.pos0[a];
         const float2 xa_h = F32 ? xh[a] : make_float2(0.f, 0.f);
         int ida = D.id[a];
-        int cx = (int)floor((xa.x - P.gx0) / P.cs), cy = (int)floor((xa.y - P.gy0) / P.cs);
+        const int cx = scan_cell(xa.x, P.gx0, P.cs, P.gnx), cy = scan_cell(xa.y, P.gy0, P.cs, P.gny);
         int x0 = max(cx - 1, 0), x1 = min(cx + 1, P.gnx - 1);
         const int rule = ONE ? (int)SPH_PAIRS_ONE_FLUID : P.pair_rule;
         const bool check_type = pair_may_fail(rule, ta);
@@ -819,7 +827,7 @@ __global__ void __launch_bounds__(128) k_build_lists_lanes(Params P, Sorted<R> D
     const int ida = D.id[a];
     int lo[3] = {0, 0, 0}, len[3] = {0, 0, 0};
     if (live && ta != SPH_TYPE_ILL && ta != 0) {
-        const int cx = (int)floor((xa.x - P.gx0) / P.cs), cy = (int)floor((xa.y - P.gy0) / P.cs);
+        const int cx = scan_cell(xa.x, P.gx0, P.cs, P.gnx), cy = scan_cell(xa.y, P.gy0, P.cs, P.gny);
         const int x0 = max(cx - 1, 0), x1 = min(cx + 1, P.gnx - 1);
 #pragma unroll
         for (int r = 0; r < 3; ++r) {

@@ -2010,6 +2010,8 @@ int sph_set_initial_type(sph_handle* h, int n, const int* initial_type) {
     int rc = h->mixed ? unsort<float>(h) : unsort<double>(h);
     if (rc) return rc;
     CK(cudaMemcpyAsync(h->S.itype, initial_type, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream));
+    // (complete on return, body or not: the caller owns its array afterwards)
+    CK(cudaStreamSynchronize(h->stream));
     h->sorted_valid = false;
     return set_body(h, n, initial_type);
 }

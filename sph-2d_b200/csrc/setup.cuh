@@ -83,7 +83,7 @@ struct SetupBuf {
 // Totals the host waits for (page-locked, mapped): written by the device, seq last.
 struct HostBox {
     int tot[3];
-    volatile unsigned seq;
+    volatile unsigned seq;        // (the host reads it with acquire order, then tot)
     unsigned status;
     int nsurf;
     double diag[8];

@@ -439,15 +439,17 @@ int unsort(sph_handle* h) {
 }
 
 // Wait for the image totals of set-up number seq (k_img_count writes them to
-// mapped memory while the kernels behind it run).  The stream is queried now and
-// then, so a failed launch ends the wait.
+// mapped memory while the kernels behind it run): an acquire load, so the totals
+// read after it are those the device wrote before seq.  The stream is queried now
+// and then, so a failed launch ends the wait.
 int wait_totals(sph_handle* h, unsigned seq) {
-    for (unsigned spin = 1; h->box->seq != seq; ++spin) {
+    auto posted = [&] { return __atomic_load_n(&h->box->seq, __ATOMIC_ACQUIRE) == seq; };
+    for (unsigned spin = 1; !posted(); ++spin) {
         if ((spin & 0xfff) != 0) continue;
         const cudaError_t e = cudaStreamQuery(h->stream);
         if (e == cudaErrorNotReady) continue;
         CK(e);
-        if (h->box->seq != seq) return SPH_E_CUDA;      // everything queued has run without it
+        if (!posted()) return SPH_E_CUDA;      // everything queued has run without it
     }
     return SPH_OK;
 }

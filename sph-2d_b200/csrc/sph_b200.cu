@@ -145,7 +145,8 @@ struct sph_handle {
     long long n_rhs = 0, n_steps = 0;
     long long launches = 0;
     double bf[6] = {0, 0, 0, 0, 0, 0};   // body force of the last RHS
-    double* d_bf = nullptr;               // [6] the force, then its block partials
+    double* d_bf = nullptr;               // [6] the force of the last RHS that formed it
+    double* d_bf_part = nullptr;          // its block partials, sized by the body
     int* d_body_ids = nullptr;            // host particles of the body, from sph_set_initial_type
     int n_body = 0, cap_body = 0;
     double body_disp[2] = {0.0, 0.0};     // displacement of the body the next set-up applies
@@ -589,7 +590,7 @@ int rhs(sph_handle* h, int last, const StageArgs& G = StageArgs{}, int keep_j = 
     h->launches += 2;
     if (P.has_body && (last || h->bf_every_rhs)) {
         double* fin = h->d_bf;
-        launch(k_body_force<R>, blocks((long long)h->n_body * 32, kRedThreads), kRedThreads, h->stream, P, D, h->d_body_ids, h->n_body, h->d_bf + 6, fin, h->B.done + 3);
+        launch(k_body_force<R>, blocks((long long)h->n_body * 32, kRedThreads), kRedThreads, h->stream, P, D, h->d_body_ids, h->n_body, h->d_bf_part, fin, h->B.done + 3);
         h->bf_pending = true;
         h->launches += 1;
         if (h->drag_acc && last) {
@@ -1797,12 +1798,12 @@ int set_body(sph_handle* h, int n, const int* itype) {
     if (!h->d_body_ids || (int)ids.size() > h->cap_body) {
         CK(cudaStreamSynchronize(h->stream));
         cudaFree(h->d_body_ids);
-        cudaFree(h->d_bf);
+        cudaFree(h->d_bf_part);
         h->d_body_ids = nullptr;
-        h->d_bf = nullptr;
+        h->d_bf_part = nullptr;
         h->cap_body = 0;
         CK(dalloc(&h->d_body_ids, ids.size()));
-        CK(dalloc(&h->d_bf, 6 + 6 * (size_t)blocks((long long)ids.size() * 32, kRedThreads)));
+        CK(dalloc(&h->d_bf_part, 4 * (size_t)blocks((long long)ids.size() * 32, kRedThreads)));
         h->cap_body = (int)ids.size();
     }
     h->n_body = (int)ids.size();
@@ -1819,7 +1820,7 @@ void destroy(sph_handle* h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->adj) { adj_free_all(h->adj); delete h->adj; }
-    void* ptrs[] = {h->d_bf, h->d_export, h->d_off64, h->d_pairs, h->d_ghost_ids, h->d_body_ids};
+    void* ptrs[] = {h->d_bf_part, h->d_export, h->d_off64, h->d_pairs, h->d_ghost_ids, h->d_body_ids};
     for (void* p : ptrs) if (p) cudaFree(p);
     h->mem.release();
     for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
@@ -1877,7 +1878,7 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     char* tmp = nullptr;
     m.add(&tmp, h->cub_bytes);
     m.add(&h->d_status, 1); m.add(&h->d_stamps, kStamps); m.add(&h->d_int, kDiagBlocks);
-    m.add(&h->d_part, 2 * kDiagBlocks); m.add(&h->d_diag, 2);
+    m.add(&h->d_part, 2 * kDiagBlocks); m.add(&h->d_diag, 2); m.add(&h->d_bf, 6);
     m.add(&h->d_xfer, (size_t)6 * h->cap_host);
     if (cfg->mls_order) m.add(&h->d_mls, cap);
     if (h->mixed) add_sorted(m, h->D32, cap, h->P.max_nbr, h->ncells);

@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kRedThreads) k_diag(Params P, Sorted<R> D, dou
 // Gathered from the body side: body particle b sums V_a times its terms over its
 // pair neighbours a (the pair set is symmetric), one warp per body particle
 // (body_ids: the body's host particles) with the lanes on the pairs; the last
-// block adds the block partials (part, [6][blocks]) in a fixed order into out.
+// block adds the block partials (part, [4][blocks]) in a fixed order into out.
 // A thread per particle of the whole tank left a few warps with chains of up to
 // 45 neighbours, and a second launch for the sum: pass C and the force together
 // 84 -> 52 us per step at D/30 (FP64), 440 -> 389 us at D/100 (mixed).

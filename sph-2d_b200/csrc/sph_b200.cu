@@ -146,9 +146,9 @@ struct sph_handle {
     long long launches = 0;
     double bf[6] = {0, 0, 0, 0, 0, 0};   // body force of the last RHS
     double* d_bf = nullptr;               // [6] the force of the last RHS that formed it
-    double* d_bf_part = nullptr;          // its block partials, sized by the body
+    double* d_bf_part = nullptr;          // its block partials
     int* d_body_ids = nullptr;            // host particles of the body, from sph_set_initial_type
-    int n_body = 0, cap_body = 0;
+    int n_body = 0;
     double body_disp[2] = {0.0, 0.0};     // displacement of the body the next set-up applies
     bool bf_every_rhs = false;            // sph_rhs also reports it
     bool bf_pending = false;              // the device copy is newer than bf (read on demand)
@@ -1788,27 +1788,18 @@ int adjoint_backward(sph_handle* h, double dloss, double* g_vel0, double* g_rho0
 }
 
 // The body of the body-force integral: the host particles whose initial type is
-// SPH_TYPE_BODY.
+// SPH_TYPE_BODY.  (No allocation: a failed one would leave a body without its
+// buffers to the next step.)
 int set_body(sph_handle* h, int n, const int* itype) {
     std::vector<int> ids;
     for (int i = 0; i < n; ++i)
         if (itype[i] == SPH_TYPE_BODY) ids.push_back(i);
-    h->P.has_body = ids.empty() ? 0 : 1;
-    if (ids.empty()) { h->n_body = 0; return SPH_OK; }
-    if (!h->d_body_ids || (int)ids.size() > h->cap_body) {
-        CK(cudaStreamSynchronize(h->stream));
-        cudaFree(h->d_body_ids);
-        cudaFree(h->d_bf_part);
-        h->d_body_ids = nullptr;
-        h->d_bf_part = nullptr;
-        h->cap_body = 0;
-        CK(dalloc(&h->d_body_ids, ids.size()));
-        CK(dalloc(&h->d_bf_part, 4 * (size_t)blocks((long long)ids.size() * 32, kRedThreads)));
-        h->cap_body = (int)ids.size();
-    }
+    h->P.has_body = 0;
     h->n_body = (int)ids.size();
+    if (ids.empty()) return SPH_OK;
     CK(cudaMemcpyAsync(h->d_body_ids, ids.data(), sizeof(int) * ids.size(), cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    h->P.has_body = 1;
     return SPH_OK;
 }
 
@@ -1820,7 +1811,7 @@ void destroy(sph_handle* h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->adj) { adj_free_all(h->adj); delete h->adj; }
-    void* ptrs[] = {h->d_bf_part, h->d_export, h->d_off64, h->d_pairs, h->d_ghost_ids, h->d_body_ids};
+    void* ptrs[] = {h->d_export, h->d_off64, h->d_pairs, h->d_ghost_ids};
     for (void* p : ptrs) if (p) cudaFree(p);
     h->mem.release();
     for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
@@ -1879,6 +1870,8 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     m.add(&tmp, h->cub_bytes);
     m.add(&h->d_status, 1); m.add(&h->d_stamps, kStamps); m.add(&h->d_int, kDiagBlocks);
     m.add(&h->d_part, 2 * kDiagBlocks); m.add(&h->d_diag, 2); m.add(&h->d_bf, 6);
+    m.add(&h->d_body_ids, h->cap_host);
+    m.add(&h->d_bf_part, 4 * (size_t)blocks((long long)h->cap_host * 32, kRedThreads));
     m.add(&h->d_xfer, (size_t)6 * h->cap_host);
     if (cfg->mls_order) m.add(&h->d_mls, cap);
     if (h->mixed) add_sorted(m, h->D32, cap, h->P.max_nbr, h->ncells);

@@ -36,3 +36,18 @@ def test_pending_body_force_survives_a_new_body(lib, dx):
             out.append(np.array(got))
     assert (np.abs(out[0]).max(axis=1) > 0.0).all()
     assert np.array_equal(out[0], out[1])
+
+
+def test_setting_a_body_takes_no_device_memory(lib):
+    """The buffers of the body force are the handle's from its start, so that no call in
+    between can fail half-way for want of memory: a million body particles, free memory
+    the same before and after."""
+    import torch
+    case = S.make_tgv(1000)
+    with S.Simulation(case.cfg, case.n) as sim:
+        sim.set_state(case.pos, case.vel, case.rho, case.mass, case.type)
+        sim.set_initial_type(case.type)
+        before, _ = torch.cuda.mem_get_info()
+        sim.set_initial_type(np.full(case.n, S.TYPE_BODY, np.int32))
+        after, _ = torch.cuda.mem_get_info()
+    assert after == before

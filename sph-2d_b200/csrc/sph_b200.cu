@@ -221,6 +221,7 @@ int derive_params(const sph_config& c, Params& P) {
     P.h = c.h;
     const double hbar = (c.h + c.h) / 2.0;
     P.r_cut = c.kernel_scale * hbar;
+    if (!std::isfinite(P.r_cut)) return SPH_E_CONFIG;     // (the search for s_cut below would not end)
     if (q) {
         float e9 = expf(-9.0f);
         P.gauss_e9 = (double)e9;

@@ -420,10 +420,10 @@ void add_sorted(Slab& m, Sorted<R>& D, int cap, int max_nbr, int ncells) {
 }
 
 template <typename R>
-int clear_sorted(Sorted<R>& D, int cap) {
-    CK(cudaMemset(D.surf_gen, 0, sizeof(int)));
-    CK(cudaMemset(D.nb3, 0, sizeof(*D.nb3) * (size_t)cap));
-    CK(cudaMemset(D.flags, 0, (size_t)cap));
+int clear_sorted(Sorted<R>& D, int cap, cudaStream_t st) {
+    CK(cudaMemsetAsync(D.surf_gen, 0, sizeof(int), st));
+    CK(cudaMemsetAsync(D.nb3, 0, sizeof(*D.nb3) * (size_t)cap, st));
+    CK(cudaMemsetAsync(D.flags, 0, (size_t)cap, st));
     return SPH_OK;
 }
 
@@ -1880,13 +1880,15 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     rc = [&] { CK(m.commit()); return (int)SPH_OK; }();
     if (rc) { destroy(h); return rc; }
     h->cub_tmp = tmp;
-    CK(cudaMemset(h->S.blabel, 0, sizeof(int) * (size_t)cap));
-    CK(cudaMemset(h->d_status, 0, sizeof(unsigned)));
+    // (every clear in the handle's stream: it does not wait for the default stream, and
+    // the caller may have work queued there)
+    CK(cudaMemsetAsync(h->S.blabel, 0, sizeof(int) * (size_t)cap, h->stream));
+    CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream));
     CK(cudaMemsetAsync(B.done, 0, 4 * sizeof(unsigned), h->stream));
     CK(cudaMemsetAsync(h->d_stamps, 0, sizeof(unsigned long long) * kStamps, h->stream));
     CK(h->copier.reserve(sizeof(HostBox), (void**)&h->box));
     CK(cudaHostGetDevicePointer((void**)&h->d_box, h->box, 0));
-    rc = h->mixed ? clear_sorted(h->D32, cap) : clear_sorted(h->D64, cap);
+    rc = h->mixed ? clear_sorted(h->D32, cap, h->stream) : clear_sorted(h->D64, cap, h->stream);
     if (rc) { destroy(h); return rc; }
     *out = h;
     return SPH_OK;

@@ -2003,8 +2003,8 @@ __device__ __forceinline__ void ghost_water_one(const Params& P, const Sorted<R>
     window_visit_warp(P, D, D.pos0[j], [&](int s) {
         const double2 x = D.pos[s];
         const double dx = x.x - xj.x, dy = x.y - xj.y;
-        const double s2 = dx * dx + dy * dy;
-        if (D.type[s] != SPH_TYPE_FIX_GHOST || D.id[s] >= P.n_host || !(s2 <= P.ghost_r2)) return;
+        const double s2 = dist2(dx, dy);
+        if (D.type[s] != SPH_TYPE_FIX_GHOST || D.id[s] >= P.n_host || !(s2 <= P.ghost_s_cut)) return;
         const double4 lam = load4(&A.glam[s]);
         const double lw = A.glamw[s];
         if (lam.x == 0.0 && lam.y == 0.0 && lam.z == 0.0 && lam.w == 0.0 && lw == 0.0) return;

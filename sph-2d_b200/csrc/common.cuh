@@ -29,7 +29,7 @@ struct Params {
     // ghost assignment (moving-square driver)
     int ghost_assign, wall_bc, ghost_cells;
     double ghost_h, ghost_r, ghost_kf, shock_t, grav[2];
-    double ghost_r2, ghost_ih2;   // squared interpolation radius, 1 / ghost_h^2
+    double ghost_s_cut, ghost_ih2;   // the largest s with sqrt(s) <= ghost_r, 1 / ghost_h^2
     // kernel / pair search
     double h, r_cut, cut_min, kfactor, gauss_e9, q_zero;
     double s_cut, s_min;     // the support test on the squared distance: the largest s with
@@ -143,13 +143,15 @@ __device__ __forceinline__ void eos64(const Params& P, double rho, double& p, do
     c = P.sqrt_c0 * pw3(r);
 }
 
+// A squared distance rounded as the reference rounds it.
+__device__ __forceinline__ double dist2(double dx, double dy) { return __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)); }
+
 // Exact replica of the reference's support test
 //   distance = sqrt(dot(dx,dx));  distance <= kernel_scale*h  .and.  distance >= 1.0E-7
 // (find_particle_pair.f90:79-87) with the products and the sum rounded
 // separately (no FMA), so the pair set is bit-identical to the CPU's.
 __device__ __forceinline__ bool in_support(const Params& P, double dx, double dy, double& d) {
-    double s = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-    d = __dsqrt_rn(s);
+    d = __dsqrt_rn(dist2(dx, dy));
     return d <= P.r_cut && d >= P.cut_min;
 }
 
@@ -158,7 +160,7 @@ __device__ __forceinline__ bool in_support(const Params& P, double dx, double dy
 // d >= cut_min is s >= s_min for the bounds derive_params finds; the pair set is
 // the same, bit for bit.  s2: the squared distance.
 __device__ __forceinline__ bool in_support_s2(const Params& P, double dx, double dy, double& s2) {
-    s2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+    s2 = dist2(dx, dy);
     return s2 <= P.s_cut && s2 >= P.s_min;
 }
 

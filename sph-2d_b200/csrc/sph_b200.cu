@@ -177,6 +177,16 @@ struct sph_handle {
 
 namespace {
 
+// The largest s with sqrt(s) <= r: sqrt is monotonic and correctly rounded, so the
+// test sqrt(s) <= r is s <= this, bit for bit.
+double largest_square(double r) {
+    double s = r * r;
+    if (!(r > 0.0) || !std::isfinite(r)) return s;
+    while (sqrt(s) > r) s = nextafter(s, 0.0);
+    while (sqrt(nextafter(s, HUGE_VAL)) <= r) s = nextafter(s, HUGE_VAL);
+    return s;
+}
+
 // --- configuration -> kernel parameters (mirrors the oracle's constants) ---
 int derive_params(const sph_config& c, Params& P) {
     if (c.kernel_model != SPH_KERNEL_GAUSSIAN && c.kernel_model != SPH_KERNEL_WENDLAND2) return SPH_E_CONFIG;
@@ -221,7 +231,7 @@ int derive_params(const sph_config& c, Params& P) {
     P.h = c.h;
     const double hbar = (c.h + c.h) / 2.0;
     P.r_cut = c.kernel_scale * hbar;
-    if (!std::isfinite(P.r_cut)) return SPH_E_CONFIG;     // (the search for s_cut below would not end)
+    if (!std::isfinite(P.r_cut)) return SPH_E_CONFIG;
     if (q) {
         float e9 = expf(-9.0f);
         P.gauss_e9 = (double)e9;
@@ -253,9 +263,7 @@ int derive_params(const sph_config& c, Params& P) {
     P.inv_h2 = P.inv_h * P.inv_h;
     P.gk = (c.kernel_model == SPH_KERNEL_GAUSSIAN ? -2.0 : -5.0) * P.kfactor / (c.h * c.h);
     // in_support's bounds on the squared distance (see in_support_s2)
-    P.s_cut = P.r_cut * P.r_cut;
-    while (sqrt(P.s_cut) > P.r_cut) P.s_cut = nextafter(P.s_cut, 0.0);
-    while (sqrt(nextafter(P.s_cut, HUGE_VAL)) <= P.r_cut) P.s_cut = nextafter(P.s_cut, HUGE_VAL);
+    P.s_cut = largest_square(P.r_cut);
     P.s_min = P.cut_min * P.cut_min;
     while (sqrt(P.s_min) < P.cut_min) P.s_min = nextafter(P.s_min, HUGE_VAL);
     while (sqrt(nextafter(P.s_min, 0.0)) >= P.cut_min) P.s_min = nextafter(P.s_min, 0.0);
@@ -310,7 +318,7 @@ int derive_params(const sph_config& c, Params& P) {
     P.wall_bc = c.wall_bc;
     P.ghost_h = (q ? (double)(float)c.ghost_h_factor : c.ghost_h_factor) * c.h;
     P.ghost_r = c.kernel_scale * P.ghost_h;
-    P.ghost_r2 = P.ghost_r * P.ghost_r;
+    P.ghost_s_cut = largest_square(P.ghost_r);
     P.ghost_ih2 = 1.0 / (P.ghost_h * P.ghost_h);
     P.ghost_kf = c.kernel_model == SPH_KERNEL_GAUSSIAN
                      ? 1.0 / (pi_k * (P.ghost_h * P.ghost_h) * (q ? (double)(1.0f - 10.0f * expf(-9.0f))

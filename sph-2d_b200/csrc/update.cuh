@@ -283,8 +283,8 @@ __device__ __forceinline__ void ghost_visit_warp(const Params& P, const Sorted<R
         const double2 xb = D.pos[b];
         const int tb = D.type[b];
         const double dx = x.x - xb.x, dy = x.y - xb.y;
-        const double s2 = dx * dx + dy * dy;
-        if (tb == SPH_TYPE_FIX_GHOST || !(s2 <= P.ghost_r2)) return;
+        const double s2 = dist2(dx, dy);
+        if (tb == SPH_TYPE_FIX_GHOST || !(s2 <= P.ghost_s_cut)) return;
         fn(b, dx, dy, s2, ghost_w(P, s2));
     });
 }

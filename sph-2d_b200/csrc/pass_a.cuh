@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
     const int nn = live ? D.nnbr[a] : 0;
     const int most = L == 1 ? nn : __reduce_max_sync(0xffffffffu, nn);
     const double2 xa = HL ? make_double2(0.0, 0.0) : D.pos[a];
-    const double4 ka = HL ? make_double4(0.0, 0.0, __ldg(&D.kin[a].z), 0.0) : D.kin[a];
+    const double4 ka = HL ? make_double4(0.0, 0.0, load(&D.kin[a].z), 0.0) : D.kin[a];
     const float4 xa_hl = HL ? D.xhl[a] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 kah = HL ? D.kh[a] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 kal = LO ? D.kl[a] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -125,15 +125,15 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
     // two-deep software pipeline: the list entry two iterations ahead, the
     // neighbour's position and records (kin, volume) one iteration ahead, so the
     // loads of the next neighbour are in flight while this one is evaluated
-    unsigned ent_n = nn > ln.lane ? __ldg(&D.nbr[(size_t)ln.lane * P.nbr_stride + a]) : 0u;
-    unsigned ent_nn = nn > ln.lane + L ? __ldg(&D.nbr[(size_t)(ln.lane + L) * P.nbr_stride + a]) : 0u;
+    unsigned ent_n = nn > ln.lane ? load(&D.nbr[(size_t)ln.lane * P.nbr_stride + a]) : 0u;
+    unsigned ent_nn = nn > ln.lane + L ? load(&D.nbr[(size_t)(ln.lane + L) * P.nbr_stride + a]) : 0u;
     double2 xb_n = make_double2(0.0, 0.0);
     double4 kb_n = make_double4(0.0, 0.0, 0.0, 0.0);
     float4 xbhl_n = make_float4(0.f, 0.f, 0.f, 0.f), kbh_n = xbhl_n, kbl_n = xbhl_n;
     R vb_n = R(0);
     auto fetch = [&](int bb) {
-        if (HL) { xbhl_n = __ldg(&D.xhl[bb]); kbh_n = __ldg(&D.kh[bb]); if (LO) kbl_n = __ldg(&D.kl[bb]); }
-        else { xb_n = __ldg(&D.pos[bb]); kb_n = load4(&D.kin[bb]); }
+        if (HL) { xbhl_n = load(&D.xhl[bb]); kbh_n = load(&D.kh[bb]); if (LO) kbl_n = load(&D.kl[bb]); }
+        else { xb_n = load(&D.pos[bb]); kb_n = load4(&D.kin[bb]); }
         vb_n = D.aux[bb].y;
     };
     if (nn > ln.lane) fetch((int)(ent_n & 0x7fffffffu));
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (MS ? SPH_PASS_A_F32_MS_
         if (e + L < nn) {
             ent_n = ent_nn;
             fetch((int)(ent_n & 0x7fffffffu));
-            if (e + 2 * L < nn) ent_nn = __ldg(&D.nbr[(size_t)(e + 2 * L) * P.nbr_stride + a]);
+            if (e + 2 * L < nn) ent_nn = load(&D.nbr[(size_t)(e + 2 * L) * P.nbr_stride + a]);
         }
         const double dxd = HL ? 0.0 : xa.x - xb.x, dyd = HL ? 0.0 : xa.y - xb.y;
         const float dxf = HL ? (xa_hl.x - xbhl.x) + (xa_hl.z - xbhl.z) : 0.f;

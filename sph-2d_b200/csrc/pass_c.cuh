@@ -231,10 +231,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
     const double inv_h64 = P.inv_h, inv_h2_64 = P.inv_h2, inv_wdx = 1.0 / P.w_dx;
 
     // the pairs pass A found inside the support at this RHS
-    unsigned ent_n = nn > ln.lane ? __ldg(&D.pairs[(size_t)ln.lane * P.nbr_stride + a]) : 0u;
+    unsigned ent_n = nn > ln.lane ? load(&D.pairs[(size_t)ln.lane * P.nbr_stride + a]) : 0u;
     // software pipeline: the pair entry two iterations ahead; the neighbour's
     // position and its records one iteration ahead
-    unsigned ent_nn = nn > ln.lane + L ? __ldg(&D.pairs[(size_t)(ln.lane + L) * P.nbr_stride + a]) : 0u;
+    unsigned ent_nn = nn > ln.lane + L ? load(&D.pairs[(size_t)(ln.lane + L) * P.nbr_stride + a]) : 0u;
     double2 xb_n = make_double2(0.0, 0.0);
     float4 xbhl_n = make_float4(0.f, 0.f, 0.f, 0.f);
     double vd_n = 0.0;                 // FP64 volume, mixed SHIFT launch
@@ -248,9 +248,9 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
     };
     if (nn > ln.lane) {
         const int b0 = (int)(ent_n & 0x7fffffffu);
-        if (X64) xb_n = __ldg(&D.pos[b0]);
-        else xbhl_n = __ldg(&D.xhl[b0]);
-        if (VPRE) vd_n = __ldg(&D.vol64[b0]);
+        if (X64) xb_n = load(&D.pos[b0]);
+        else xbhl_n = load(&D.xhl[b0]);
+        if (VPRE) vd_n = load(&D.vol64[b0]);
         load_records(b0, T_n);
     }
     for (int e = ln.lane; e < nn; e += L) {
@@ -264,11 +264,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
         if (e + L < nn) {
             ent_n = ent_nn;
             const int b1 = (int)(ent_n & 0x7fffffffu);
-            if (X64) xb_n = __ldg(&D.pos[b1]);
-            else xbhl_n = __ldg(&D.xhl[b1]);
-            if (VPRE) vd_n = __ldg(&D.vol64[b1]);
+            if (X64) xb_n = load(&D.pos[b1]);
+            else xbhl_n = load(&D.xhl[b1]);
+            if (VPRE) vd_n = load(&D.vol64[b1]);
             load_records(b1, T_n);
-            if (e + 2 * L < nn) ent_nn = __ldg(&D.pairs[(size_t)(e + 2 * L) * P.nbr_stride + a]);
+            if (e + 2 * L < nn) ent_nn = load(&D.pairs[(size_t)(e + 2 * L) * P.nbr_stride + a]);
         }
         // x_a - x_b: FP64, or hi/lo in FP32 (the mixed SHIFT launch: the FP32
         // rounding of the FP64 difference, which its shifting sum needs)
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
                     wd = P.kfactor * (1.0 + 2.0 * q) * (t2 * t2);
                     gd = -5.0 * P.kfactor * (t2 * t) * inv_h2_64;
                 }
-                Vd = VPRE ? vd_b : __ldg(&D.vol64[b]);
+                Vd = VPRE ? vd_b : load(&D.vol64[b]);
             } else {
                 wd = (double)w; gd = (double)g; Vd = (double)Vb;
             }
@@ -671,14 +671,14 @@ __global__ void __launch_bounds__(128, 12) k_shift_gather(const __grid_constant_
     const double inv_h64 = P.inv_h, inv_h2_64 = P.inv_h2, inv_wdx = 1.0 / P.w_dx;
     double shx = 0.0, shy = 0.0;
     // the pair entry two iterations ahead, the neighbour's position and volume one ahead
-    unsigned ent_n = nn > 0 ? __ldg(&D.pairs[a]) : 0u;
-    unsigned ent_nn = nn > 1 ? __ldg(&D.pairs[(size_t)P.nbr_stride + a]) : 0u;
+    unsigned ent_n = nn > 0 ? load(&D.pairs[a]) : 0u;
+    unsigned ent_nn = nn > 1 ? load(&D.pairs[(size_t)P.nbr_stride + a]) : 0u;
     double2 xb_n = make_double2(0.0, 0.0);
     double vd_n = 0.0;
     if (nn > 0) {
         const int b0 = (int)(ent_n & 0x7fffffffu);
-        xb_n = __ldg(&D.pos[b0]);
-        vd_n = __ldg(&D.vol64[b0]);
+        xb_n = load(&D.pos[b0]);
+        vd_n = load(&D.vol64[b0]);
     }
     for (int e = 0; e < nn; ++e) {
         const double2 xb = xb_n;
@@ -686,9 +686,9 @@ __global__ void __launch_bounds__(128, 12) k_shift_gather(const __grid_constant_
         if (e + 1 < nn) {
             ent_n = ent_nn;
             const int b1 = (int)(ent_n & 0x7fffffffu);
-            xb_n = __ldg(&D.pos[b1]);
-            vd_n = __ldg(&D.vol64[b1]);
-            if (e + 2 < nn) ent_nn = __ldg(&D.pairs[(size_t)(e + 2) * P.nbr_stride + a]);
+            xb_n = load(&D.pos[b1]);
+            vd_n = load(&D.vol64[b1]);
+            if (e + 2 < nn) ent_nn = load(&D.pairs[(size_t)(e + 2) * P.nbr_stride + a]);
         }
         const double dxd = xa.x - xb.x, dyd = xa.y - xb.y;
         const double s2 = dxd * dxd + dyd * dyd;

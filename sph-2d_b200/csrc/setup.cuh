@@ -767,10 +767,10 @@ __global__ void __launch_bounds__(128) k_build_lists(Params P, Sorted<R> D, unsi
                 int tb[4], ib[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    if (F32) xbh[k] = __ldg(&xh[b + k]);
-                    else xb[k] = __ldg(&D.pos0[b + k]);
-                    ib[k] = __ldg(&D.id[b + k]);
-                    tb[k] = check_type ? __ldg(&D.type[b + k]) : 0;
+                    if (F32) xbh[k] = load(&xh[b + k]);
+                    else xb[k] = load(&D.pos0[b + k]);
+                    ib[k] = load(&D.id[b + k]);
+                    tb[k] = check_type ? load(&D.type[b + k]) : 0;
                 }
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -858,13 +858,13 @@ __global__ void __launch_bounds__(128) k_build_lists_lanes(Params P, Sorted<R> D
         unsigned v = 0u;
         if (t < total) {
             const int b = t < len[0] ? lo[0] + t : t < l01 ? lo[1] + (t - len[0]) : lo[2] + (t - l01);
-            v = (unsigned)b | (ida < __ldg(&D.id[b]) ? 0x80000000u : 0u);
+            v = (unsigned)b | (ida < load(&D.id[b]) ? 0x80000000u : 0u);
             if (F32) {
-                const float2 xb = __ldg(&D.xh0[b]);
+                const float2 xb = load(&D.xh0[b]);
                 const float dx = xa_h.x - xb.x, dy = xa_h.y - xb.y;
                 in = !(dx * dx + dy * dy > P.r2_list32);
             } else {
-                const double2 xb = __ldg(&D.pos0[b]);
+                const double2 xb = load(&D.pos0[b]);
                 const double dx = xa.x - xb.x, dy = xa.y - xb.y;
                 in = !(dx * dx + dy * dy > P.r2_list);
             }

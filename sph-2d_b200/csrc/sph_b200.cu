@@ -792,19 +792,21 @@ int find_pairs(sph_handle* h, long long pair_cap, int* pi, int* pj, double* w, d
     h->last_pairs = *total;
     if (pi == nullptr || pair_cap <= 0) return SPH_OK;
     const size_t m = (size_t)std::min(*total, pair_cap);
-    // w, dwdx, pair_i, pair_j of m pairs
-    const size_t need = std::max<size_t>(m, 1) * (sizeof(double) * 3 + sizeof(int) * 2);
+    // w, dwdx (those the caller wants), pair_i, pair_j of m pairs
+    const size_t nw = w ? m : 0, ndw = dwdx ? 2 * m : 0;
+    const size_t need = std::max<size_t>(sizeof(double) * (nw + ndw) + sizeof(int) * 2 * m, 1);
     if (need > h->cap_pairs) {
         cudaFree(h->d_pairs);
         h->d_pairs = nullptr;
         h->cap_pairs = 0;
-        const size_t room = need <= kKeepPairs ? need + need / 8 : need;
+        // (an eighth more, for a count that grows a little, within what is kept)
+        const size_t room = need <= kKeepPairs ? std::min(need + need / 8, kKeepPairs) : need;
         CK(cudaMalloc(&h->d_pairs, room));
         h->cap_pairs = room;
     }
     double* dw = static_cast<double*>(h->d_pairs);
-    double* ddw = dw + m;
-    int* dpi = reinterpret_cast<int*>(ddw + 2 * m);
+    double* ddw = dw + nw;
+    int* dpi = reinterpret_cast<int*>(ddw + ndw);
     int* dpj = dpi + m;
     launch(k_pair_emit<R>, blocks(n, 128), 128, h->stream, P, sorted<R>(h), h->d_off64, (long long)m, dpi, dpj,
                                                           w ? dw : nullptr, dwdx ? ddw : nullptr);

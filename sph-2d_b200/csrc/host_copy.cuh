@@ -14,7 +14,6 @@
 #include <cstring>
 #include <initializer_list>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -53,11 +52,15 @@ public:
     // Device to host (to_host) or host to device on `stream`; complete on return.
     // Null host pointers are skipped.
     cudaError_t copy(int device, cudaStream_t stream, std::initializer_list<HostSeg> segs, bool to_host) {
+        cudaError_t e;
         try {
-            return copy_segs(device, stream, segs, to_host);
-        } catch (const std::bad_alloc&) {
-            return cudaErrorMemoryAllocation;
+            e = copy_segs(device, stream, segs, to_host);
+        } catch (...) {
+            e = cudaErrorMemoryAllocation;
         }
+        // after a failure too: what was queued before it is at the caller's memory
+        if (e != cudaSuccess) cudaStreamSynchronize(stream);
+        return e;
     }
 
 private:
@@ -109,8 +112,8 @@ private:
         for (; started < lanes; ++started) {
             try {
                 helper[started] = std::thread(work, started);
-            } catch (const std::system_error&) {
-                break;                       // no more threads: this one takes their chunks
+            } catch (...) {
+                break;       // no more threads (or no memory for one): this one takes their chunks
             }
         }
         work(0);

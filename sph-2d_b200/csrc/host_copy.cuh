@@ -5,8 +5,8 @@
 // another with a wait each, at 3 to 8 GB/s.  Here the pieces of all arrays of a
 // call go through page-locked chunks of the handle: the DMA of one chunk runs
 // while the one before it is copied to (from) the caller's memory, by up to four
-// threads when there is enough to share.  Page-locked arrays are copied
-// directly.  Every call returns when its copies are complete.
+// threads when there is enough to share.  Page-locked arrays (and managed or
+// device ones) are copied directly.  Every call returns when its copies are complete.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -69,9 +69,9 @@ private:
         size_t total = 0;
         for (const HostSeg& s : segs) {
             if (!s.host || s.bytes == 0) continue;
-            if (page_locked(s.host)) {
-                const cudaError_t e = to_host ? cudaMemcpyAsync(s.host, s.dev, s.bytes, cudaMemcpyDeviceToHost, stream)
-                                              : cudaMemcpyAsync(s.dev, s.host, s.bytes, cudaMemcpyHostToDevice, stream);
+            if (known(s.host)) {
+                const cudaError_t e = cudaMemcpyAsync(to_host ? s.host : s.dev, to_host ? s.dev : s.host, s.bytes,
+                                                      cudaMemcpyDefault, stream);
                 if (e != cudaSuccess) return e;
                 continue;
             }
@@ -165,10 +165,12 @@ private:
     }
 
     static size_t pad(size_t b) { return (b + 255) & ~size_t(255); }
-    static bool page_locked(const void* p) {
+    // Page-locked, managed or device memory: the runtime can copy it directly, and
+    // device memory is not the CPU's to touch.
+    static bool known(const void* p) {
         cudaPointerAttributes a;
         if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
-        return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
+        return a.type != cudaMemoryTypeUnregistered;
     }
     // Chunks t, t + lanes, ...: two buffers, the DMA of one while the other is
     // copied by this thread.

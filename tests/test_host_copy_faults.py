@@ -21,3 +21,9 @@ def program(tmp_path_factory):
 def test_failures_leave_nothing_in_flight(program):
     out = subprocess.run([program], capture_output=True, text=True, timeout=300)
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout[-2000:] + out.stderr[-2000:]
+
+
+def test_device_arrays_are_left_to_the_runtime(program):
+    """A caller's array in device memory is copied by the runtime, never by the CPU."""
+    out = subprocess.run([program, "device"], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0 and out.stdout.strip() == "ok", (out.returncode, out.stdout[-2000:], out.stderr[-2000:])

@@ -10,12 +10,19 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
+#include <cstdlib>
 #include <cstring>
 #include <initializer_list>
 #include <new>
 #include <thread>
 #include <vector>
+
+// Bytes in large copies after which the helper threads get memory of their own (see kShare).
+#ifndef SPH_COPY_PAYBACK
+#define SPH_COPY_PAYBACK (size_t(64) << 20)
+#endif
 
 namespace sph {
 
@@ -34,18 +41,46 @@ public:
             for (int k = 0; k < 2; ++k)
                 if (lane_[t].ev[k]) cudaEventDestroy(lane_[t].ev[k]);
         }
-        for (void** b : {&first_, &rest_}) {
-            if (*b) cudaFreeHost(*b);
-            *b = nullptr;
+        if (first_ && registered_) {
+            cudaHostUnregister(first_);
+            free(first_);
+        } else if (first_) {
+            cudaFreeHost(first_);
         }
+        if (rest_) cudaFreeHost(rest_);
+        first_ = rest_ = nullptr;
+        registered_ = false;
+        chunk_ = kChunk;
+        moved_ = 0;
         for (Lane& l : lane_) l = Lane{};
     }
-    // The first lane's chunks with `extra` zeroed bytes of page-locked memory behind
-    // them, which the caller may use until release().
-    cudaError_t reserve(size_t extra, void** mem) {
-        const cudaError_t e = open(1, extra);
+    // The first lane's chunks, for an owner whose usual copies are of `usual` bytes,
+    // with `extra` zeroed bytes of page-locked memory behind them, which the caller
+    // may use until release().
+    //
+    // A small owner takes small chunks, of ordinary memory that is page-locked
+    // afterwards: to lock and unlock 0.25 / 0.5 / 1 MiB so takes 0.73 / 1.00 / 1.48 ms,
+    // to allocate and free locked memory 1.6 to 2.8 ms whatever the size.  A new
+    // handle of 2,209 particles with its first upload and its end: 3.8 ms with a
+    // full-size block, 1.4 ms.
+    cudaError_t reserve(size_t usual, size_t extra, void** mem) {
+        if (first_) return cudaErrorInvalidValue;
+        const size_t c = (usual + kPage - 1) & ~(kPage - 1);
+        const size_t bytes = (2 * std::max(c, kLeast) + extra + kPage - 1) & ~(kPage - 1);
+        if (bytes <= kRegister) {
+            void* p = aligned_alloc(kPage, bytes);
+            if (p && cudaHostRegister(p, bytes, cudaHostRegisterMapped) == cudaSuccess) {
+                first_ = p;
+                registered_ = true;
+                chunk_ = std::max(c, kLeast);
+            } else {
+                cudaGetLastError();
+                free(p);               // (not to be had: a block of full-size chunks)
+            }
+        }
+        const cudaError_t e = open_first(extra);
         if (e != cudaSuccess) return e;
-        *mem = (char*)first_ + 2 * kChunk;
+        *mem = (char*)first_ + 2 * chunk_;
         memset(*mem, 0, extra);
         return cudaSuccess;
     }
@@ -65,7 +100,7 @@ public:
 
 private:
     cudaError_t copy_segs(int device, cudaStream_t stream, std::initializer_list<HostSeg> segs, bool to_host) {
-        std::vector<HostSeg> pieces;
+        std::vector<HostSeg> pageable, pieces;
         size_t total = 0;
         for (const HostSeg& s : segs) {
             if (!s.host || s.bytes == 0) continue;
@@ -75,15 +110,23 @@ private:
                 if (e != cudaSuccess) return e;
                 continue;
             }
-            for (size_t o = 0; o < s.bytes; o += kChunk)
-                pieces.push_back({(char*)s.host + o, (char*)s.dev + o, s.bytes - o < kChunk ? s.bytes - o : kChunk,
-                                  s.joined || o > 0});
+            pageable.push_back(s);
             total += s.bytes;
         }
+        int lanes = 1;
+        size_t chunk = chunk_;
+        if (total > 0) {
+            const cudaError_t e = open(total, lanes, chunk);
+            if (e != cudaSuccess) return e;
+        }
+        for (const HostSeg& s : pageable)
+            for (size_t o = 0; o < s.bytes; o += chunk)
+                pieces.push_back({(char*)s.host + o, (char*)s.dev + o, std::min(s.bytes - o, chunk),
+                                  s.joined || o > 0});
         // small pieces share a chunk, and joined ones a DMA
         std::vector<Chunk> chunks;
         for (const HostSeg& p : pieces) {
-            if (chunks.empty() || pad(chunks.back().bytes) + p.bytes > kChunk) chunks.push_back(Chunk{});
+            if (chunks.empty() || pad(chunks.back().bytes) + p.bytes > chunk) chunks.push_back(Chunk{});
             Chunk& c = chunks.back();
             const bool next = p.joined && !c.dma.empty() && c.dma.back().dev + c.dma.back().bytes == p.dev;
             const size_t at = next ? c.bytes : pad(c.bytes);
@@ -91,15 +134,6 @@ private:
             else c.dma.push_back({(char*)p.dev, at, p.bytes});
             c.piece.push_back({(char*)p.host, at, p.bytes});
             c.bytes = at + p.bytes;
-        }
-        int lanes = 1;
-        if (total >= kShare) {
-            const unsigned hw = std::thread::hardware_concurrency();
-            lanes = hw >= 8 ? kLanes : hw >= 4 ? 2 : 1;
-        }
-        if (!chunks.empty()) {
-            const cudaError_t e = open(lanes, 0);
-            if (e != cudaSuccess) return e;
         }
         std::atomic<int> err{cudaSuccess};
         auto work = [&](int t) {
@@ -123,9 +157,19 @@ private:
         return err != cudaSuccess ? (cudaError_t)err.load() : e;
     }
 
-    static constexpr size_t kChunk = size_t(1) << 20;      // 1 MiB: 20 us of PCIe, 8 MiB held at most
-    static constexpr size_t kShare = size_t(4) << 20;      // a thread costs about 30 us to start
+    // Chunk and lanes, us for 1.0 / 3.2 / 31 / 210 MB to the host, 16 cores: 1 lane with
+    // chunks of 128 KiB 87 / 295 / 2760 / 21150, 256 KiB 71 / 241 / 2220 / 19320, 1 MiB
+    // 74 / 228 / 1930 / 17210; with 1 MiB 2 lanes 84 / 182 / 1440 / 9150, 3 lanes
+    // 93 / 165 / 1130 / 6980, 4 lanes 104 / 165 / 1270 / 5680, 6 lanes 140 / 179 / 1490 /
+    // 5650, 8 lanes 183 / 194 / 1360 / 5840 (a thread costs about 10 us to start).
+    // The lanes share the first lane's block at first (4 with 256 KiB: 88 / 186 / 1885 /
+    // 10080, and the first touch of the caller's new pages is shared too); memory of
+    // their own takes 4 to 5.5 ms once and saves up to 20 us a MB: they get it when
+    // this owner has moved SPH_COPY_PAYBACK bytes in such copies.
+    static constexpr size_t kChunk = size_t(1) << 20;      // 8 MiB held at most
+    static constexpr size_t kShare = size_t(4) << 20;
     static constexpr int kLanes = 4;
+    static constexpr size_t kPage = 4096, kLeast = size_t(64) << 10, kRegister = size_t(1) << 20;
     struct Part {
         char* host;
         size_t off, bytes;     // place in the chunk
@@ -144,19 +188,36 @@ private:
         cudaEvent_t ev[2] = {nullptr, nullptr};
     };
     Lane lane_[kLanes];
-    // Page-locked memory: one allocation for the first lane, one for the others, since
-    // each takes 0.8 to 2.6 ms whatever its size.
+    // Page-locked memory: one block for the first lane, one for the others, since an
+    // allocation takes 1 to 2.8 ms up to 2 MiB.
     void* first_ = nullptr;
     void* rest_ = nullptr;
-    cudaError_t open(int lanes, size_t extra) {
-        cudaError_t e = cudaSuccess;
-        if (!first_ && (e = cudaHostAlloc(&first_, 2 * kChunk + extra, cudaHostAllocDefault)) != cudaSuccess) return e;
-        if (lanes > 1 && !rest_ &&
-            (e = cudaHostAlloc(&rest_, (kLanes - 1) * 2 * kChunk, cudaHostAllocDefault)) != cudaSuccess)
-            return e;
+    bool registered_ = false;      // first_ is ordinary memory, locked
+    size_t chunk_ = kChunk;
+    size_t moved_ = 0;             // bytes of the copies of kShare and more
+    cudaError_t open_first(size_t extra) {
+        return first_ ? cudaSuccess : cudaHostAlloc(&first_, 2 * chunk_ + extra, cudaHostAllocDefault);
+    }
+    // The lanes and chunks for a copy of `total` bytes.
+    cudaError_t open(size_t total, int& lanes, size_t& chunk) {
+        cudaError_t e = open_first(0);
+        if (e != cudaSuccess) return e;
+        if (total >= kShare) {
+            moved_ += total;
+            if (!rest_ && moved_ >= SPH_COPY_PAYBACK &&
+                cudaHostAlloc(&rest_, (kLanes - 1) * 2 * chunk_, cudaHostAllocDefault) != cudaSuccess) {
+                cudaGetLastError();
+                rest_ = nullptr;       // (as before, then)
+            }
+            const unsigned hw = std::thread::hardware_concurrency();
+            lanes = hw >= 8 ? kLanes : hw >= 4 ? 2 : 1;
+            if (!rest_ && chunk_ < kChunk) lanes = 1;       // (a small block is not worth sharing)
+            else if (!rest_ && lanes > 1) chunk = chunk_ / kLanes;
+        }
         for (int t = 0; t < lanes; ++t)
             for (int k = 0; k < 2; ++k) {
-                lane_[t].buf[k] = t == 0 ? (char*)first_ + k * kChunk : (char*)rest_ + (2 * (t - 1) + k) * kChunk;
+                const int b = 2 * t + k;
+                lane_[t].buf[k] = b < 2 || chunk != chunk_ ? (char*)first_ + b * chunk : (char*)rest_ + (b - 2) * chunk;
                 if (!lane_[t].ev[k] &&
                     (e = cudaEventCreateWithFlags(&lane_[t].ev[k], cudaEventDisableTiming)) != cudaSuccess)
                     return e;

@@ -1896,7 +1896,8 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream));
     CK(cudaMemsetAsync(B.done, 0, 4 * sizeof(unsigned), h->stream));
     CK(cudaMemsetAsync(h->d_stamps, 0, sizeof(unsigned long long) * kStamps, h->stream));
-    CK(h->copier.reserve(sizeof(HostBox), (void**)&h->box));
+    // (usual copies: a whole state, 60 bytes a particle in seven arrays)
+    CK(h->copier.reserve((size_t)60 * n_capacity + 7 * 256, sizeof(HostBox), (void**)&h->box));
     CK(cudaHostGetDevicePointer((void**)&h->d_box, h->box, 0));
     rc = h->mixed ? clear_sorted(h->D32, cap, h->stream) : clear_sorted(h->D64, cap, h->stream);
     if (rc) { destroy(h); return rc; }

@@ -12,6 +12,7 @@
 #include <set>
 #include <vector>
 
+#define SPH_COPY_PAYBACK (size_t(16) << 20)     // the helper threads come with the second 9 MiB copy
 #include "../sph-2d_b200/csrc/host_copy.cuh"
 
 namespace {
@@ -19,7 +20,7 @@ std::recursive_mutex mu;
 std::vector<std::function<void()>> queue;      // work queued and not yet done
 size_t done = 0;                               // items of the queue that ran
 std::set<const void*> locked, device;          // page-locked and device arrays (start address)
-int memcpys, fail_memcpy = -1, fail_alloc = -1, allocs;
+int memcpys, fail_memcpy = -1, fail_alloc = -1, allocs, registers;
 long news, fail_new = -1;
 bool armed = false;                            // operator new counts and may fail
 thread_local bool inside = false;              // (not in this file's own calls)
@@ -68,7 +69,7 @@ cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
     return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
-cudaError_t cudaHostRegister(void*, size_t, unsigned) { return allocs++ == fail_alloc ? cudaErrorMemoryAllocation : cudaSuccess; }
+cudaError_t cudaHostRegister(void*, size_t, unsigned) { ++registers; return allocs == fail_alloc ? cudaErrorMemoryAllocation : cudaSuccess; }
 cudaError_t cudaHostUnregister(void*) { return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
@@ -87,7 +88,7 @@ void reset() {
     run_to(queue.size());
     queue.clear();
     done = 0;
-    memcpys = allocs = 0;
+    memcpys = allocs = registers = 0;
     fail_memcpy = fail_alloc = -1;
     news = 0;
     fail_new = -1;
@@ -107,7 +108,7 @@ int main(int argc, char** argv) {
     std::vector<char> host_a(small), host_b(big);
     locked.insert(host_a.data());
     cudaStream_t st = (cudaStream_t)1;
-    for (int dir = 0; dir < 2 && !only_device; ++dir) {
+    for (int dir = 0; dir < 2 && argc == 1; ++dir) {
         const bool to_host = dir == 1;
         std::vector<char>&src_a = to_host ? dev_a : host_a, &src_b = to_host ? dev_b : host_b;
         std::vector<char>&dst_a = to_host ? host_a : dev_a, &dst_b = to_host ? host_b : dev_b;
@@ -122,18 +123,22 @@ int main(int argc, char** argv) {
             sph::HostCopy c;
             expect(call(c) == cudaSuccess && right() && pending() == 0, "plain copy", dir);
         }
-        for (int k = 0; k < 24; ++k) {          // the k-th copy fails
+        for (int k = 0; k < 48; ++k) {          // the k / 2-th copy fails, in a first call and in a later one
             reset();
             sph::HostCopy c;
-            fail_memcpy = k;
+            if (k & 1) call(c);
+            reset();
+            fail_memcpy = k / 2;
             const cudaError_t e = call(c);
             expect(e != cudaSuccess || right(), "copy failure", k);
             expect(pending() == 0, "copies in flight after a copy failed", k);
         }
-        for (int k = 0; k < 3; ++k) {           // page-locked memory is refused
+        for (int k = 0; k < 4; ++k) {           // page-locked memory is refused
             reset();
             sph::HostCopy c;
-            fail_alloc = k;
+            if (k & 1) call(c);
+            reset();
+            fail_alloc = k / 2;
             const cudaError_t e = call(c);
             expect(e != cudaSuccess || right(), "allocation failure", k);
             expect(pending() == 0, "copies in flight after an allocation failed", k);
@@ -152,6 +157,46 @@ int main(int argc, char** argv) {
             expect(e != cudaSuccess || right(), "no memory", k);
             expect(pending() == 0, "copies in flight without memory", k);
         }
+    }
+    if (argc > 1 && argv[1][0] == 'r') {
+        // what a new owner takes, and that its copies are right with it
+        for (size_t usual : {size_t(1000), size_t(130000), size_t(400000), size_t(600000), size_t(10) << 20}) {
+            for (int refuse = 0; refuse < 2; ++refuse) {
+                reset();
+                sph::HostCopy c;
+                void* mem = nullptr;
+                fail_alloc = refuse ? 0 : -1;
+                const bool small_owner = usual <= 500000;
+                const cudaError_t e = c.reserve(usual, 200, &mem);
+                expect(registers == (small_owner ? 1 : 0), "blocks of ordinary memory locked", (long)usual);
+                expect(allocs == (small_owner && !refuse ? 0 : 1), "blocks of locked memory", (long)usual);
+                fail_alloc = -1;
+                if (refuse) {
+                    expect(e != cudaSuccess, "refused memory", (long)usual);
+                    continue;
+                }
+                expect(e == cudaSuccess && mem, "reserve", (long)usual);
+                for (int k = 0; k < 200; ++k) expect(((char*)mem)[k] == 0, "zeroed", k);
+                memset(mem, 0x5a, 200);
+                const int before = allocs;
+                for (int n = 0; n < 3; ++n) {
+                    for (size_t m : {size_t(1), size_t(4096), size_t(131073), size_t(700001), big}) {
+                        for (int dir = 0; dir < 2; ++dir) {
+                            std::vector<char>&src = dir ? dev_b : host_b, &dst = dir ? host_b : dev_b;
+                            src = want_b;
+                            memset(dst.data(), 0, big);
+                            expect(c.copy(0, st, {{host_b.data(), dev_b.data(), m}}, dir == 1) == cudaSuccess, "copy", (long)m);
+                            expect(!memcmp(dst.data(), want_b.data(), m) && (m == big || dst[m] == 0), "bytes", (long)m);
+                            if (m == big && n == 0 && dir == 0) expect(allocs == before, "first large copy takes memory", (long)usual);
+                        }
+                    }
+                }
+                expect(allocs == before + 1, "later large copies: one block more", (long)usual);
+                for (int k = 0; k < 200; ++k) expect(((char*)mem)[k] == 0x5a, "the owner's memory", k);
+            }
+        }
+        if (!bad) printf("ok\n");
+        return bad;
     }
     if (only_device) {
         // the caller's array is on the device: the runtime copies it, the CPU does not touch it

@@ -2306,6 +2306,7 @@ int sph_adjoint_motion_gradient(sph_handle* h, double* g_motion) {
 
 int sph_get_timings(sph_handle* h, sph_timings* out) {
     if (!h || !out) return SPH_E_ARG;
+    CK(cudaSetDevice(h->device));
     timing_flush(h);
     out->sort_ms = h->t_ms[PH_SORT];
     out->pass_a_ms = h->t_ms[PH_A];
@@ -2323,6 +2324,7 @@ int sph_get_timings(sph_handle* h, sph_timings* out) {
 
 int sph_reset_timings(sph_handle* h) {
     if (!h) return SPH_E_ARG;
+    CK(cudaSetDevice(h->device));
     timing_flush(h);
     for (double& t : h->t_ms) t = 0;
     h->t_total = 0;

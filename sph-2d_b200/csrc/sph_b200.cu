@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <vector>
 
@@ -138,7 +139,9 @@ struct sph_handle {
     std::vector<cudaEvent_t> ev_pool;     // begin and end of each timed stretch
     size_t ev_used = 0;
     unsigned long long* d_stamps = nullptr;   // [kStamps] start of each phase (0: not begun)
+    // (the three vectors have their full room from sph_init on: no step allocates)
     std::vector<int> stamp_of;            // phase of each used slot (-1: outside the phases)
+    std::vector<unsigned long long> stamp_buf;    // [kStamps] host copy of the stamps
     bool timed_open = false;
     double t_ms[PH_COUNT] = {0};
     double t_total = 0;
@@ -367,13 +370,15 @@ void toc(sph_handle* h) {
 void timing_flush(sph_handle* h) {
     toc(h);
     if (h->stamp_of.empty()) return;
-    std::vector<unsigned long long> t(h->stamp_of.size());
-    cudaMemcpyAsync(t.data(), h->d_stamps, sizeof(t[0]) * t.size(), cudaMemcpyDeviceToHost, h->stream);
-    cudaMemsetAsync(h->d_stamps, 0, sizeof(t[0]) * t.size(), h->stream);
+    const size_t n = h->stamp_of.size();
+    unsigned long long* t = h->stamp_buf.data();
+    memset(t, 0, sizeof(t[0]) * n);
+    cudaMemcpyAsync(t, h->d_stamps, sizeof(t[0]) * n, cudaMemcpyDeviceToHost, h->stream);
+    cudaMemsetAsync(h->d_stamps, 0, sizeof(t[0]) * n, h->stream);
     cudaStreamSynchronize(h->stream);
     int ph = -1;
     unsigned long long from = 0;
-    for (size_t k = 0; k < t.size(); ++k) {
+    for (size_t k = 0; k < n; ++k) {
         if (t[k] == 0) continue;                  // a phase without launches
         if (ph >= 0 && ph < PH_COUNT) h->t_ms[ph] += 1e-6 * (double)(t[k] - from);
         ph = h->stamp_of[k];
@@ -1802,14 +1807,18 @@ int adjoint_backward(sph_handle* h, double dloss, double* g_vel0, double* g_rho0
 // SPH_TYPE_BODY.  (No allocation: a failed one would leave a body without its
 // buffers to the next step.)
 int set_body(sph_handle* h, int n, const int* itype) {
-    std::vector<int> ids;
-    for (int i = 0; i < n; ++i)
-        if (itype[i] == SPH_TYPE_BODY) ids.push_back(i);
+    // (no exception from here: this runs inside C entry points)
+    std::unique_ptr<int[]> ids(new (std::nothrow) int[n]);
     h->P.has_body = 0;
-    h->n_body = (int)ids.size();
-    if (ids.empty()) return SPH_OK;
-    CK(cudaMemcpyAsync(h->d_body_ids, ids.data(), sizeof(int) * ids.size(), cudaMemcpyHostToDevice, h->stream));
+    h->n_body = 0;
+    if (!ids) return SPH_E_CAPACITY;
+    int m = 0;
+    for (int i = 0; i < n; ++i)
+        if (itype[i] == SPH_TYPE_BODY) ids[m++] = i;
+    if (m == 0) return SPH_OK;
+    CK(cudaMemcpyAsync(h->d_body_ids, ids.get(), sizeof(int) * m, cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    h->n_body = m;
     h->P.has_body = 1;
     return SPH_OK;
 }
@@ -1842,6 +1851,14 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     h->cfg = *cfg;
     int rc = derive_params(*cfg, h->P);
     if (rc) { delete h; return rc; }
+    try {
+        h->stamp_of.reserve(kStamps);
+        h->ev_pool.reserve(kStamps);           // two a stretch, which marks at least one phase and its end
+        h->stamp_buf.resize(kStamps);
+    } catch (const std::bad_alloc&) {
+        delete h;
+        return SPH_E_CAPACITY;
+    }
     CK(cudaGetDevice(&h->device));
     h->mixed = cfg->precision == SPH_PREC_MIXED;
     h->cap_host = n_capacity;

@@ -207,7 +207,10 @@ __global__ void __launch_bounds__(kImgThreads) k_img_count(Params P, Staging S, 
 
 // Cell key (row-major cells of edge >= list radius) and arrival number of id o.
 // Particles that are not binned (Assign_boundary_particles.f90:82) or off the
-// grid go past the last cell.
+// grid go past the last cell; there may be many (a host that marks what has left the
+// domain), so the threads of a warp that are here together take their numbers with one
+// atomic: with an atomic each on that one counter the images of 2^20 particles took
+// 48 / 375 / 640 us a step with none / half / nine tenths not binned.
 __device__ __forceinline__ void cell_key(const Params& P, const SetupBuf& B, int o, double2 x, int t, unsigned* status) {
     unsigned key = (unsigned)B.ncells;
     if (t != SPH_TYPE_ILL && t != 0) {
@@ -217,7 +220,15 @@ __device__ __forceinline__ void cell_key(const Params& P, const SetupBuf& B, int
         else atomicOr(status, ST_DOMAIN);
     }
     B.key[o] = key;
-    B.rank[o] = atomicAdd(&B.cnt[key], 1);
+    if (key < (unsigned)B.ncells) {
+        B.rank[o] = atomicAdd(&B.cnt[key], 1);
+    } else {
+        const unsigned here = __activemask();
+        const int lane = threadIdx.x & 31, first = __ffs(here) - 1;
+        int base = 0;
+        if (lane == first) base = atomicAdd(&B.cnt[key], __popc(here));
+        B.rank[o] = __shfl_sync(here, base, first) + __popc(here & ((1u << lane) - 1u));
+    }
 }
 
 // What an image takes from its source, read once for all its images (up to eight

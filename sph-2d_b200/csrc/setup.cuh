@@ -164,13 +164,14 @@ __device__ __forceinline__ double2 move_body(const Staging& S, int i, double2 di
 }
 
 __global__ void __launch_bounds__(kImgThreads) k_img_count(Params P, Staging S, SetupBuf B, HostBox* box, unsigned seq,
-                                                           double2 disp) {
+                                                           double2 disp, int clear) {
     pdl_begin();
     stamp_phase(P.stamp);
     __shared__ unsigned long long sh[32];
     __shared__ int flag;
     const int i = blockIdx.x * kImgThreads + threadIdx.x;
-    for (int c = i; c <= B.ncells; c += gridDim.x * kImgThreads) B.cnt[c] = 0;
+    if (clear)
+        for (int c = i; c <= B.ncells; c += gridDim.x * kImgThreads) B.cnt[c] = 0;
     int lr = 0, tb = 0;
     if (i < P.n_host) {
         const double2 xy = move_body(S, i, disp);
@@ -328,9 +329,11 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(SetupBuf B, unsigned
     for (int k = 0; k < per; ++k) { v[k] = c0 + k <= B.ncells ? B.cnt[c0 + k] : 0; s += v[k]; }
     int total;
     int run = block_scan<int>(s, sh, total);
+    if (total != 0) {                // (nobody reads the offsets of empty cells)
 #pragma unroll
-    for (int k = 0; k < per; ++k)
-        if (c0 + k <= B.ncells) { B.pre[c0 + k] = run; run += v[k]; }
+        for (int k = 0; k < per; ++k)
+            if (c0 + k <= B.ncells) { B.pre[c0 + k] = run; run += v[k]; }
+    }
     if (gridDim.x == 1) {            // one block's offset is 0: nothing to scan
         if (threadIdx.x == 0) B.blkoff[0] = 0;
         return;
@@ -348,18 +351,25 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(SetupBuf B, unsigned
     }
 }
 
-// Cell ranges (-1 for an empty cell), and each particle at its arrival place.
+// Cell ranges (-1 for an empty cell), and each particle at its arrival place.  SPARSE:
+// the ranges were set to -1 before, and the first particle of a cell writes its.
+template <bool SPARSE>
 __global__ void k_place(int n_tot, SetupBuf B, int* cell_start, int* cell_end) {
     pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < B.ncells) {
+    if (!SPARSE && t < B.ncells) {
         const int n = B.cnt[t], st = B.blkoff[t >> kScanShift] + B.pre[t];
         cell_start[t] = n ? st : -1;
         cell_end[t] = n ? st + n : -1;
     }
     if (t < n_tot) {
         const unsigned k = B.key[t];
-        B.perm[B.blkoff[k >> kScanShift] + B.pre[k] + B.rank[t]] = (unsigned)t;
+        const int st = B.blkoff[k >> kScanShift] + B.pre[k], r = B.rank[t];
+        B.perm[st + r] = (unsigned)t;
+        if (SPARSE && r == 0 && k < (unsigned)B.ncells) {
+            cell_start[k] = st;
+            cell_end[k] = st + B.cnt[k];
+        }
     }
 }
 

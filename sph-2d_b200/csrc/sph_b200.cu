@@ -469,6 +469,16 @@ int wait_totals(sph_handle* h, unsigned seq) {
     return SPH_OK;
 }
 
+// Whether the grid's cells outnumber the particles so far that the set-up clears its
+// tables with memsets and lets the particles write the ranges of their cells: 6 bytes
+// a cell instead of 24, for about 10 us of launches.  us per step (FP64 Taylor-Green),
+// a pass over the cells / this: 10,000 particles 89 / 94 with 64 cells a particle,
+// 112 / 102 with 256, 213 / 135 with 1000; 40,000 particles 169 / 169, 237 / 208,
+// 463 / 333; 250,000 particles 619 / 619 with 16 and 699 / 671 with 64.
+bool sparse_grid(int ncells, int n_host) {
+    return ncells > (1 << 20) && ncells / 16 > n_host;
+}
+
 // Step-start set-up: wrap + periodic images, sort, cell ranges, lists, records.
 // first: the step's first stage, applied to the carried rates by the gather
 // (mode STAGE_MID), or none.
@@ -484,8 +494,10 @@ int prepare(sph_handle* h, const StageArgs& first = StageArgs{}) {
     const int nhb = blocks(h->n_host, kImgThreads), ncb = blocks(h->ncells + 1, kScanCells);
     const int periodic = h->cfg.periodic ? 1 : 0;
     const double2 disp = make_double2(h->body_disp[0], h->body_disp[1]);
-    if (periodic) launch(k_img_count, nhb, kImgThreads, h->stream, P, h->S, B, h->d_box, ++h->box_seq, disp);
-    else CK(cudaMemsetAsync(B.cnt, 0, sizeof(int) * (size_t)(h->ncells + 1), h->stream));
+    const bool sparse = sparse_grid(h->ncells, h->n_host);
+    if (!periodic || sparse) CK(cudaMemsetAsync(B.cnt, 0, sizeof(int) * (size_t)(h->ncells + 1), h->stream));
+    if (periodic)
+        launch(k_img_count, nhb, kImgThreads, h->stream, P, h->S, B, h->d_box, ++h->box_seq, disp, sparse ? 0 : 1);
     // (the routing of image adjoints is kept once an adjoint run exists)
     launch(k_img_emit, nhb, kImgThreads, h->stream, P, h->S, B, h->cap_tot, periodic, h->adj != nullptr, h->d_status,
                                                     periodic ? make_double2(0.0, 0.0) : disp);
@@ -503,7 +515,14 @@ int prepare(sph_handle* h, const StageArgs& first = StageArgs{}) {
     }
     h->n_img = n_img;
     P.n_tot = h->n_host + n_img;
-    launch(k_place, blocks(std::max(P.n_tot, h->ncells), 256), 256, h->stream, P.n_tot, B, D.cell_start, D.cell_end);
+    if (sparse) {
+        CK(cudaMemsetAsync(D.cell_start, 0xff, sizeof(int) * (size_t)h->ncells, h->stream));
+        CK(cudaMemsetAsync(D.cell_end, 0xff, sizeof(int) * (size_t)h->ncells, h->stream));
+        launch(k_place<true>, blocks(P.n_tot, 256), 256, h->stream, P.n_tot, B, D.cell_start, D.cell_end);
+    } else {
+        launch(k_place<false>, blocks(std::max(P.n_tot, h->ncells), 256), 256, h->stream, P.n_tot, B, D.cell_start,
+               D.cell_end);
+    }
     launch(k_gather_sorted<R>, blocks(P.n_tot, 256), 256, h->stream, P, h->S, D, B, first);
     launch_lists<R>(P, D, h->d_status, h->stream);
     CK(cudaGetLastError());

@@ -504,6 +504,7 @@ __global__ void __launch_bounds__(kRedThreads) k_body_force(Params P, Sorted<R> 
                 double G;
                 if (P.kernel_model == SPH_KERNEL_GAUSSIAN) G = exp(-(s2 * P.inv_h2)) * P.gk;
                 else { const double tq = 1.0 - s2 * rsqrt64(s2) * P.half_inv_h; G = P.gk * (tq * tq * tq); }
+                if (s2 * P.inv_h2 <= P.q_zero * P.q_zero) G = 0.0;      // (compute_kernel)
                 const double gx = G * dx, gy = G * dy;
                 const double n0 = bi.x * gx + bi.y * gy, n1 = bi.z * gx + bi.w * gy;
                 const double fp = -Va * Vb * (ka.w + kb.w);

@@ -14,11 +14,12 @@
 //   Shift_particle_position.f90:78-103
 //   assembly: single_step_compute.f90:152-171
 //
-// Every pair quantity is evaluated in the reference's own orientation
-// (pair_i = the particle with the lower id, bit 31 of the list entry), so the
-// flux seen by the two particles of a pair is computed by the same sequence
-// of operations; each thread then keeps the pair_i or pair_j contribution that
-// belongs to its particle.  The physical terms are summed per pair and then
+// The flux seen by the two particles of a pair comes from the same bits: either in
+// the reference's own orientation (pair_i = the particle with the lower id, bit 31
+// of the list entry; the moving-square launches and the mixed ones without MUSCL),
+// or in the particle's own frame, where negation is exact and only the MUSCL
+// limiter looks at the orientation (AB, the other launches).  Each thread keeps the
+// contribution that belongs to its particle.  The physical terms are summed per pair and then
 // accumulated (the reference sums each term over all pairs first); the two
 // orders agree to round-off.
 //
@@ -651,9 +652,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (SHIFT ? SPH_PASS_C_SHIF
 // stalls on their loads; here it runs at full occupancy.  Particles the shift
 // does not move (not water, or near the free surface) get 0.  12 blocks of 128
 // per SM (40 registers): 0.32 -> 0.29 ms per step at 2048^2 against 44 registers
-// at 11 blocks; at 16 blocks (32 registers, 48 B spilled) it was slower.  With
-// the step's last stage behind the sum (StageArgs) 0.45 ms, against 0.29 and 0.30
-// for two passes; 10 blocks 0.49, 8 blocks without spills 0.57.
+// at 11 blocks; at 16 blocks (32 registers) it was slower.  With the step's last
+// stage behind the sum (StageArgs; 120 B of spill stores) 0.45
+// ms, against 0.29 and 0.30 for two passes; 10 blocks 0.49, 8 blocks without spills
+// 0.57.
 template <typename R>
 __global__ void __launch_bounds__(128, 12) k_shift_gather(const __grid_constant__ Params P, const __grid_constant__ Sorted<R> D,
                                                         const __grid_constant__ StageArgs G) {

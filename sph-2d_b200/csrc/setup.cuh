@@ -51,7 +51,8 @@ __device__ __forceinline__ double2 wrap_position(const Params& P, double2 x) {
 //   k_img_emit    writes the images at their offsets, the cell key of every
 //                 particle and its arrival number in its cell
 //   k_cell_scan   exclusive scan of the cell counts (last block: of the block sums)
-//   k_place       cell ranges; particle -> slot, unordered inside a cell
+//   k_place       cell ranges (on a grid of mostly empty cells, sparse_grid, only those
+//                 that hold particles); particle -> slot, unordered inside a cell
 //   k_gather_sorted  orders each cell by id while it copies the arrays: the same
 //                 order as a stable sort of the keys
 //   k_build_lists
@@ -70,7 +71,7 @@ struct SetupBuf {
     int4* blk;            // [image blocks] image sums (x: left/right, y: bottom/top of host
                           // particles, z: bottom/top of left/right images), then exclusive
     int* tot;             // [3] their totals
-    unsigned* done;       // [3] blocks finished (image count, cell scan, diagnostics); left at 0
+    unsigned* done;       // [4] blocks finished (image count, cell scan, diagnostics, body force); left at 0
     unsigned* key;        // [cap] cell of particle i (id order), ncells = not binned
     int* rank;            // [cap] its arrival number in the cell
     int* cnt;             // [ncells + 1] particles per cell
@@ -575,7 +576,6 @@ struct StageArgs {
     int mode;             // STAGE_NONE, STAGE_MID (into the other copy), STAGE_END
     int stage;
     double dt;
-    int shift;            // STAGE_END: apply the step's shift
     int to_staging;       // STAGE_END: also write the id-order state
     unsigned* status;
     Staging S;
@@ -733,7 +733,8 @@ __device__ __forceinline__ int scan_cell(double v, double lo, double cs, int n) 
 // Every particle b != a in the 3x3 cells with |x_a - x_b|^2 <= (support*(1+skin))^2
 // and an allowed type pair.  The exact support test is repeated at every RHS on
 // the current positions, so the list only has to be a superset of the pairs of
-// the whole step; k_stage checks the displacement bound that guarantees it.
+// the whole step; every stage checks the displacement bound that guarantees it
+// (check_skin).
 // The first kListStage entries of each list are staged in shared memory
 // ([entry][thread], conflict-free) and written out row by row after the scan, so
 // the stores of a warp are coalesced; longer lists write the rest directly.

@@ -19,11 +19,6 @@
 #include <thread>
 #include <vector>
 
-// Bytes in large copies after which the helper threads get memory of their own (see kShare).
-#ifndef SPH_COPY_PAYBACK
-#define SPH_COPY_PAYBACK (size_t(64) << 20)
-#endif
-
 namespace sph {
 
 struct HostSeg {
@@ -51,12 +46,11 @@ public:
         first_ = rest_ = nullptr;
         registered_ = false;
         chunk_ = kChunk;
-        moved_ = 0;
         for (Lane& l : lane_) l = Lane{};
     }
-    // The first lane's chunks, for an owner whose usual copies are of `usual` bytes,
-    // with `extra` zeroed bytes of page-locked memory behind them, which the caller
-    // may use until release().
+    // The chunks for an owner whose usual copies are of `usual` bytes, with `extra`
+    // zeroed bytes of page-locked memory behind the first lane's, which the caller may
+    // use until release().
     //
     // A small owner takes small chunks, of ordinary memory that is page-locked
     // afterwards: to lock and unlock 0.25 / 0.5 / 1 MiB so takes 0.73 / 1.00 / 1.48 ms,
@@ -80,6 +74,7 @@ public:
         }
         const cudaError_t e = open_first(extra);
         if (e != cudaSuccess) return e;
+        if (usual >= kShare) open_rest();
         *mem = (char*)first_ + 2 * chunk_;
         memset(*mem, 0, extra);
         return cudaSuccess;
@@ -114,19 +109,18 @@ private:
             total += s.bytes;
         }
         int lanes = 1;
-        size_t chunk = chunk_;
         if (total > 0) {
-            const cudaError_t e = open(total, lanes, chunk);
+            const cudaError_t e = open(total, lanes);
             if (e != cudaSuccess) return e;
         }
         for (const HostSeg& s : pageable)
-            for (size_t o = 0; o < s.bytes; o += chunk)
-                pieces.push_back({(char*)s.host + o, (char*)s.dev + o, std::min(s.bytes - o, chunk),
+            for (size_t o = 0; o < s.bytes; o += chunk_)
+                pieces.push_back({(char*)s.host + o, (char*)s.dev + o, std::min(s.bytes - o, chunk_),
                                   s.joined || o > 0});
         // small pieces share a chunk, and joined ones a DMA
         std::vector<Chunk> chunks;
         for (const HostSeg& p : pieces) {
-            if (chunks.empty() || pad(chunks.back().bytes) + p.bytes > chunk) chunks.push_back(Chunk{});
+            if (chunks.empty() || pad(chunks.back().bytes) + p.bytes > chunk_) chunks.push_back(Chunk{});
             Chunk& c = chunks.back();
             const bool next = p.joined && !c.dma.empty() && c.dma.back().dev + c.dma.back().bytes == p.dev;
             const size_t at = next ? c.bytes : pad(c.bytes);
@@ -162,10 +156,9 @@ private:
     // 74 / 228 / 1930 / 17210; with 1 MiB 2 lanes 84 / 182 / 1440 / 9150, 3 lanes
     // 93 / 165 / 1130 / 6980, 4 lanes 104 / 165 / 1270 / 5680, 6 lanes 140 / 179 / 1490 /
     // 5650, 8 lanes 183 / 194 / 1360 / 5840 (a thread costs about 10 us to start).
-    // The lanes share the first lane's block at first (4 with 256 KiB: 88 / 186 / 1885 /
-    // 10080, and the first touch of the caller's new pages is shared too); memory of
-    // their own takes 4 to 5.5 ms once and saves up to 20 us a MB: they get it when
-    // this owner has moved SPH_COPY_PAYBACK bytes in such copies.
+    // The other lanes would pay from 2 MB on, but their page-locked memory takes 4 to
+    // 5.5 ms once: they begin at 4 MiB.  An owner whose usual copies are that large
+    // gets it from reserve, not in its first copy.
     static constexpr size_t kChunk = size_t(1) << 20;      // 8 MiB held at most
     static constexpr size_t kShare = size_t(4) << 20;
     static constexpr int kLanes = 4;
@@ -194,30 +187,27 @@ private:
     void* rest_ = nullptr;
     bool registered_ = false;      // first_ is ordinary memory, locked
     size_t chunk_ = kChunk;
-    size_t moved_ = 0;             // bytes of the copies of kShare and more
     cudaError_t open_first(size_t extra) {
         return first_ ? cudaSuccess : cudaHostAlloc(&first_, 2 * chunk_ + extra, cudaHostAllocDefault);
     }
-    // The lanes and chunks for a copy of `total` bytes.
-    cudaError_t open(size_t total, int& lanes, size_t& chunk) {
+    void open_rest() {
+        if (!rest_ && cudaHostAlloc(&rest_, (kLanes - 1) * 2 * chunk_, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            rest_ = nullptr;           // (one lane, then)
+        }
+    }
+    // The lanes for a copy of `total` bytes.
+    cudaError_t open(size_t total, int& lanes) {
         cudaError_t e = open_first(0);
         if (e != cudaSuccess) return e;
         if (total >= kShare) {
-            moved_ += total;
-            if (!rest_ && moved_ >= SPH_COPY_PAYBACK &&
-                cudaHostAlloc(&rest_, (kLanes - 1) * 2 * chunk_, cudaHostAllocDefault) != cudaSuccess) {
-                cudaGetLastError();
-                rest_ = nullptr;       // (as before, then)
-            }
+            open_rest();
             const unsigned hw = std::thread::hardware_concurrency();
-            lanes = hw >= 8 ? kLanes : hw >= 4 ? 2 : 1;
-            if (!rest_ && chunk_ < kChunk) lanes = 1;       // (a small block is not worth sharing)
-            else if (!rest_ && lanes > 1) chunk = chunk_ / kLanes;
+            if (rest_) lanes = hw >= 8 ? kLanes : hw >= 4 ? 2 : 1;
         }
         for (int t = 0; t < lanes; ++t)
             for (int k = 0; k < 2; ++k) {
-                const int b = 2 * t + k;
-                lane_[t].buf[k] = b < 2 || chunk != chunk_ ? (char*)first_ + b * chunk : (char*)rest_ + (b - 2) * chunk;
+                lane_[t].buf[k] = t == 0 ? (char*)first_ + k * chunk_ : (char*)rest_ + (2 * (t - 1) + k) * chunk_;
                 if (!lane_[t].ev[k] &&
                     (e = cudaEventCreateWithFlags(&lane_[t].ev[k], cudaEventDisableTiming)) != cudaSuccess)
                     return e;

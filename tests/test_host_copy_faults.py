@@ -30,7 +30,8 @@ def test_device_arrays_are_left_to_the_runtime(program):
 
 
 def test_what_a_new_handle_takes(program):
-    """A small owner locks a little ordinary memory, a large one takes one block, the
-    helper threads' block comes after the first large copies; all copies right."""
+    """A small owner locks a little ordinary memory, others take one block and the helper
+    threads' block with the first large copy, an owner of large states takes both at
+    once; all copies right."""
     out = subprocess.run([program, "reserve"], capture_output=True, text=True, timeout=300)
     assert out.returncode == 0 and out.stdout.strip() == "ok", (out.returncode, out.stdout[-2000:], out.stderr[-2000:])

@@ -210,9 +210,10 @@ __global__ void __launch_bounds__(kImgThreads) k_img_count(Params P, Staging S, 
 // Cell key (row-major cells of edge >= list radius) and arrival number of id o.
 // Particles that are not binned (Assign_boundary_particles.f90:82) or off the
 // grid go past the last cell; there may be many (a host that marks what has left the
-// domain), so the threads of a warp that are here together take their numbers with one
-// atomic: with an atomic each on that one counter the images of 2^20 particles took
+// domain), so with MANY the threads of a warp that are here together take their numbers
+// with one atomic: with an atomic each on that one counter the images of 2^20 particles took
 // 48 / 375 / 640 us a step with none / half / nine tenths not binned.
+template <bool MANY>
 __device__ __forceinline__ void cell_key(const Params& P, const SetupBuf& B, int o, double2 x, int t, unsigned* status) {
     unsigned key = (unsigned)B.ncells;
     if (t != SPH_TYPE_ILL && t != 0) {
@@ -222,7 +223,7 @@ __device__ __forceinline__ void cell_key(const Params& P, const SetupBuf& B, int
         else atomicOr(status, ST_DOMAIN);
     }
     B.key[o] = key;
-    if (key < (unsigned)B.ncells) {
+    if (!MANY || key < (unsigned)B.ncells) {
         B.rank[o] = atomicAdd(&B.cnt[key], 1);
     } else {
         const unsigned here = __activemask();
@@ -252,7 +253,7 @@ __device__ __forceinline__ void put_image(const Params& P, const Staging& S, con
     S.smass[o] = q.smass;
     S.type[o] = SPH_TYPE_PERIODIC;
     S.itype[o] = SPH_TYPE_PERIODIC;
-    cell_key(P, B, o, x, SPH_TYPE_PERIODIC, status);
+    cell_key<false>(P, B, o, x, SPH_TYPE_PERIODIC, status);
 }
 
 // periodic: emit the images, numbered as the reference appends them (left/right
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(kImgThreads) k_img_emit(Params P, Staging S, S
     double2 x = make_double2(0.0, 0.0);
     int t = SPH_TYPE_ILL;
     if (live) { x = move_body(S, i, disp); t = S.type[i]; }
-    if (live) cell_key(P, B, i, x, t, status);
+    if (live) cell_key<true>(P, B, i, x, t, status);
     if (!periodic) return;
     int lr, tb;
     image_counts(P, x, t == SPH_TYPE_ILL, lr, tb);
@@ -724,9 +725,9 @@ __device__ __forceinline__ bool pair_may_fail(int rule, int ti) {
 // Cell column (row) of coordinate v, for a scan of the columns c - 1 .. c + 1 of n.  A
 // particle off the grid (not binned, reported as ST_DOMAIN) still comes here, and a
 // coordinate of 1e300 or an infinity saturates the conversion to int, so that c + 1
-// overflows: clamped to [-2, n + 1] first, where the scan meets no column (NaN: -2).
+// would overflow: clamped to [-2, n + 1], where the scan meets no column.
 __device__ __forceinline__ int scan_cell(double v, double lo, double cs, int n) {
-    return (int)fmin(fmax(floor((v - lo) / cs), -2.0), n + 1.0);
+    return min(max(__double2int_rd((v - lo) / cs), -2), n + 1);
 }
 
 // --- 5. neighbour lists ----------------------------------------------------

@@ -5,7 +5,7 @@
 // another with a wait each, at 3 to 8 GB/s.  Here the pieces of all arrays of a
 // call go through page-locked chunks of the handle: the DMA of one chunk runs
 // while the one before it is copied to (from) the caller's memory, by up to four
-// threads when there is enough to share.  Page-locked arrays (and managed or
+// threads from 4 MiB on.  Page-locked arrays (and managed or
 // device ones) are copied directly.  Every call returns when its copies are complete.
 #pragma once
 #include <cuda_runtime.h>

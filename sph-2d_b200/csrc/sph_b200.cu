@@ -61,7 +61,7 @@ cudaError_t dalloc(T** p, size_t count) {
 // Creating a handle is allocation calls only (0.1 to 0.4 ms each for 1 MiB and more):
 // with some eighty of them 8.7 to 13 ms to create and 7 ms to free at 14,000 particles
 // (moving square D/30), 25 and 25 ms at 2048^2; with one 1.5 to 3.3 and 1.1 ms, 4.3
-// and 6.4 ms.
+// and 6.4 ms (and HostCopy::reserve's page-locked memory at the larger size).
 class Slab {
 public:
     template <typename T>

@@ -43,7 +43,8 @@ public:
             cudaFreeHost(first_);
         }
         if (rest_) cudaFreeHost(rest_);
-        first_ = rest_ = nullptr;
+        if (grown_) cudaFreeHost(grown_);
+        first_ = rest_ = grown_ = nullptr;
         registered_ = false;
         chunk_ = kChunk;
         for (Lane& l : lane_) l = Lane{};
@@ -54,7 +55,9 @@ public:
     //
     // A small owner takes small chunks, of ordinary memory that is page-locked
     // afterwards: to lock and unlock 0.25 / 0.5 / 1 MiB so takes 0.73 / 1.00 / 1.48 ms,
-    // to allocate and free locked memory 1.6 to 2.8 ms whatever the size.  A new
+    // to allocate and free locked memory 1.6 to 2.8 ms whatever the size.  Its first
+    // copy of more than both (a pair list) takes the full-size block: with the small
+    // chunks those copies stayed 20 us (a tenth) slower.  A new
     // handle of 2,209 particles with its first upload and its end: 3.8 ms with a
     // full-size block, 1.4 ms.
     cudaError_t reserve(size_t usual, size_t extra, void** mem) {
@@ -185,6 +188,7 @@ private:
     // allocation takes 1 to 2.8 ms up to 2 MiB.
     void* first_ = nullptr;
     void* rest_ = nullptr;
+    void* grown_ = nullptr;        // a small owner's full-size chunks
     bool registered_ = false;      // first_ is ordinary memory, locked
     size_t chunk_ = kChunk;
     cudaError_t open_first(size_t extra) {
@@ -200,6 +204,14 @@ private:
     cudaError_t open(size_t total, int& lanes) {
         cudaError_t e = open_first(0);
         if (e != cudaSuccess) return e;
+        if (chunk_ < kChunk && total > 2 * chunk_) {
+            if (cudaHostAlloc(&grown_, 2 * kChunk, cudaHostAllocDefault) == cudaSuccess) {
+                chunk_ = kChunk;
+            } else {
+                cudaGetLastError();
+                grown_ = nullptr;      // (the small ones, then)
+            }
+        }
         if (total >= kShare) {
             open_rest();
             const unsigned hw = std::thread::hardware_concurrency();
@@ -207,7 +219,7 @@ private:
         }
         for (int t = 0; t < lanes; ++t)
             for (int k = 0; k < 2; ++k) {
-                lane_[t].buf[k] = t == 0 ? (char*)first_ + k * chunk_ : (char*)rest_ + (2 * (t - 1) + k) * chunk_;
+                lane_[t].buf[k] = t == 0 ? (char*)(grown_ ? grown_ : first_) + k * chunk_ : (char*)rest_ + (2 * (t - 1) + k) * chunk_;
                 if (!lane_[t].ev[k] &&
                     (e = cudaEventCreateWithFlags(&lane_[t].ev[k], cudaEventDisableTiming)) != cudaSuccess)
                     return e;

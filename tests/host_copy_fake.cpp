@@ -132,6 +132,15 @@ int main(int argc, char** argv) {
             expect(e != cudaSuccess || right(), "copy failure", k);
             expect(pending() == 0, "copies in flight after a copy failed", k);
         }
+        for (int k = 0; k < 3; ++k) {           // a small owner's larger blocks are refused
+            reset();
+            sph::HostCopy c;
+            void* mem;
+            c.reserve(1000, 64, &mem);
+            fail_alloc = k;
+            const cudaError_t e = call(c);
+            expect(e == cudaSuccess && right() && pending() == 0, "refused block of a small owner", k);
+        }
         for (int k = 0; k < 4; ++k) {           // page-locked memory is refused
             reset();
             sph::HostCopy c;
@@ -191,7 +200,7 @@ int main(int argc, char** argv) {
                         }
                     }
                 }
-                expect(allocs == before + (large_owner ? 0 : 1), "the large copies' block", (long)usual);
+                expect(allocs == before + (large_owner ? 0 : small_owner ? 2 : 1), "the large copies' blocks", (long)usual);
                 for (int k = 0; k < 200; ++k) expect(((char*)mem)[k] == 0x5a, "the owner's memory", k);
             }
         }

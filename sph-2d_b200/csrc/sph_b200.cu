@@ -1862,22 +1862,9 @@ void destroy(sph_handle* h) {
     delete h;
 }
 
-int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
-    int ndev = 0;
-    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) return SPH_E_NODEVICE;
-    sph_handle* h = new (std::nothrow) sph_handle();
-    if (!h) return SPH_E_CAPACITY;
-    h->cfg = *cfg;
-    int rc = derive_params(*cfg, h->P);
-    if (rc) { delete h; return rc; }
-    try {
-        h->stamp_of.reserve(kStamps);
-        h->ev_pool.reserve(kStamps);           // two a stretch, which marks at least one phase and its end
-        h->stamp_buf.resize(kStamps);
-    } catch (const std::bad_alloc&) {
-        delete h;
-        return SPH_E_CAPACITY;
-    }
+// Streams, arrays and page-locked memory of a new handle (after a failure the caller
+// destroys what there is).
+int init_arrays(sph_handle* h, const sph_config* cfg, int n_capacity) {
     CK(cudaGetDevice(&h->device));
     h->mixed = cfg->precision == SPH_PREC_MIXED;
     h->cap_host = n_capacity;
@@ -1923,8 +1910,7 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     if (cfg->mls_order) m.add(&h->d_mls, cap);
     if (h->mixed) add_sorted(m, h->D32, cap, h->P.max_nbr, h->ncells);
     else add_sorted(m, h->D64, cap, h->P.max_nbr, h->ncells);
-    rc = [&] { CK(m.commit()); return (int)SPH_OK; }();
-    if (rc) { destroy(h); return rc; }
+    CK(m.commit());
     h->cub_tmp = tmp;
     // (every clear in the handle's stream: it does not wait for the default stream, and
     // the caller may have work queued there)
@@ -1935,7 +1921,26 @@ int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
     // (usual copies: a whole state, 60 bytes a particle in seven arrays)
     CK(h->copier.reserve((size_t)60 * n_capacity + 7 * 256, sizeof(HostBox), (void**)&h->box));
     CK(cudaHostGetDevicePointer((void**)&h->d_box, h->box, 0));
-    rc = h->mixed ? clear_sorted(h->D32, cap, h->stream) : clear_sorted(h->D64, cap, h->stream);
+    return h->mixed ? clear_sorted(h->D32, cap, h->stream) : clear_sorted(h->D64, cap, h->stream);
+}
+
+int init_impl(const sph_config* cfg, int n_capacity, sph_handle** out) {
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) return SPH_E_NODEVICE;
+    sph_handle* h = new (std::nothrow) sph_handle();
+    if (!h) return SPH_E_CAPACITY;
+    h->cfg = *cfg;
+    int rc = derive_params(*cfg, h->P);
+    if (rc) { delete h; return rc; }
+    try {
+        h->stamp_of.reserve(kStamps);
+        h->ev_pool.reserve(kStamps);           // two a stretch, which marks at least one phase and its end
+        h->stamp_buf.resize(kStamps);
+    } catch (const std::bad_alloc&) {
+        delete h;
+        return SPH_E_CAPACITY;
+    }
+    rc = init_arrays(h, cfg, n_capacity);
     if (rc) { destroy(h); return rc; }
     *out = h;
     return SPH_OK;
